@@ -135,6 +135,10 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	g.n_vol = n_vol; g.n_s = n_s; g.n_c = n_c; g.n_fl = n_fl; g.n_fc = n_fc; g.K = d * n_c + n_fl * n_fc;
 	g.affine = affine_all;
 	const int K = g.K;
+	// boundary faces or viscous terms: the general chain (the periodic Euler / advection kernels have neither)
+	int general = (sim->pde_index == DPG_PDE_NAVIER_STOKES);
+	for (int f = 0; f < n_face; ++f) general |= (sim->face_vol[2 * f + 1] < 0);
+	if (!general && (rc = dpg::tp_prepare(c, sim))) return fail(rc);
 
 	// operators: Cv, Cf, L = [tw1 | -tw0] (times m_inv_ref when every volume is affine)
 	std::vector<double> L((size_t)n_s * K), Lm((size_t)n_s * K);
@@ -174,17 +178,19 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	} else {
 		// per node metrics [v][k][c] (the host layout is already c fastest within k)
 		if ((rc = dupload(c, (double**)&g.met, sim->metrics_vc, (size_t)n_vol * n_c * d * d))) return fail(rc);
-		std::vector<double> minv((size_t)n_vol * n_s * n_s);
-		for (int v = 0; v < n_vol; ++v) {
-			double* dst = &minv[(size_t)v * n_s * n_s];
-			if (sim->vol_minv_off[v + 1] > sim->vol_minv_off[v]) {
-				memcpy(dst, &sim->m_inv[sim->vol_minv_off[v]], sizeof(double) * n_s * n_s);
-			} else {
-				const double jd = sim->jacobian_det_vc[sim->vol_geo_off[v]];
-				for (int k = 0; k < n_s * n_s; ++k) dst[k] = ops.m_inv_ref[k] / jd;
+		if (!c->tp && !general) {   // the dense kernels' element mass-matrix inverses
+			std::vector<double> minv((size_t)n_vol * n_s * n_s);
+			for (int v = 0; v < n_vol; ++v) {
+				double* dst = &minv[(size_t)v * n_s * n_s];
+				if (sim->vol_minv_off[v + 1] > sim->vol_minv_off[v]) {
+					memcpy(dst, &sim->m_inv[sim->vol_minv_off[v]], sizeof(double) * n_s * n_s);
+				} else {
+					const double jd = sim->jacobian_det_vc[sim->vol_geo_off[v]];
+					for (int k = 0; k < n_s * n_s; ++k) dst[k] = ops.m_inv_ref[k] / jd;
+				}
 			}
+			if ((rc = dupload(c, (double**)&g.minv, minv.data(), minv.size()))) return fail(rc);
 		}
-		if ((rc = dupload(c, (double**)&g.minv, minv.data(), minv.size()))) return fail(rc);
 		g.jinv = nullptr;
 	}
 	std::vector<int> vf((size_t)n_vol * n_fl);
@@ -272,13 +278,7 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 		c->adv_speed = std::sqrt(sim->b_adv[0] * sim->b_adv[0] + sim->b_adv[1] * sim->b_adv[1] + sim->b_adv[2] * sim->b_adv[2]);
 	}
 	if ((rc = dpg::fp64_configure(c))) return fail(rc);
-	// boundary faces or viscous terms: the general chain (the periodic Euler / advection kernels have neither)
-	{
-		int has_bc = 0;
-		for (int f = 0; f < n_face; ++f) has_bc |= (sim->face_vol[2 * f + 1] < 0);
-		if (has_bc || sim->pde_index == DPG_PDE_NAVIER_STOKES)
-			if ((rc = dpg::gen_prepare(c, sim))) return fail(rc);
-	}
+	if (general && (rc = dpg::gen_prepare(c, sim))) return fail(rc);
 	if (cudaDeviceSynchronize() != cudaSuccess) return fail(DPG_ERR_CUDA);
 	*ctx_out = c;
 	return DPG_OK;
@@ -289,6 +289,7 @@ extern "C" void dpg_gpu_destroy(dpg_gpu_ctx* c)
 	if (!c) return;
 	if (c->stream) cudaStreamSynchronize(c->stream);
 	dpg::split_free(c);
+	dpg::tp_free(c);
 	dpg::gen_free(c);
 	dpg::hp_free(c);
 	dpg::implicit_free(c);

@@ -98,6 +98,7 @@ struct dpg_gpu_ctx {
 	int* pos_err = nullptr;      // bit 0: an average density / pressure below EPS_PHYS; bit 1: relaxation underflow
 	double* du_buf = nullptr;    // [n_dof] device copy of a host Newton update (dpg_gpu_positivity_update)
 
+	void* tp = nullptr;         // QUAD / HEX of one order: 1D operators of the FP64 form (kernels_tp.cu)
 	void* general = nullptr;    // boundary faces / Navier-Stokes: the general FP64 chain (kernels_ns.cu)
 	void* hp = nullptr;         // mixed orders: volumes grouped by order (kernels_hp.cu)
 	void* implicit = nullptr;   // Newton-GMRES work space (implicit.cu)
@@ -112,6 +113,15 @@ int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long*
 // of the traces and face fluxes.
 int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t);
 int ensure_tangent_buffers(dpg_gpu_ctx* c);
+
+// tensor-product elements (kernels_tp.cu): traces and weak divergence, then lift, stage and norm; the tangents of the
+// linearisation.  tp_prepare leaves c->tp null where the dense kernels run.
+int  tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);
+int  tp_volume(dpg_gpu_ctx* c);
+int  tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
+int  tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t);
+int  tp_lift_tan(dpg_gpu_ctx* c, const double* nnf_t, double* out);
+void tp_free(dpg_gpu_ctx* c);
 
 // general FP64 chain (kernels_ns.cu): boundary faces and the BR2 Navier-Stokes terms, residual and exact
 // Jacobian-vector products (forward-mode tangents through the same templated kernels)

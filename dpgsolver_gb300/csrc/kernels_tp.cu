@@ -1,0 +1,499 @@
+// FP64 form of the residual on tensor-product meshes of one order (QUAD, HEX, p = 1..4, periodic): the operators are
+// applied one direction at a time in the collocated Gauss basis (tp_ops.cuh).
+//
+//   k_tp_volume : sol_coef -> values at the Gauss points (B passes) -> face traces of every local face, reference volume
+//                 flux and its weak derivative (Dw passes), kept in the collocated basis
+//   k_face      : numerical flux per face node (kernels_fp64.cu)
+//   k_tp_lift   : + the face fluxes over the weights, / detJ, B^-1 passes -> rhs, ||rhs||_inf and the SSP-RK3 stage
+//
+// The FP64 pipe bounds all three (1.6-1.7 lanes per clock and SM on this GPU, 0.53 T operations/s), so the count of FP64
+// instructions decides: HEX p = 3 Euler needs 210 per node in k_tp_volume and 110 in k_tp_lift where the dense
+// operators need 28,672 / 64 x 5 = 2,240.  One thread per (element, node): the operands come from shared memory,
+// whose traffic hides behind the FP64 issue rate.  A block holds as many elements as fill 256 threads, fewer on
+// small meshes so that every SM has work.  32x32x8 HEX p = 3 Euler: k_tp_volume 193 us, k_tp_lift 114 us (0.57 T FP64
+// operations/s, the pipe's measured rate) for 967 + 3,694 us of the dense kernels; the whole residual 0.43 against 4.78 ms.
+//
+// The linearisation (k_tp_volume with TAN, k_face_tan, k_tp_lift) carries (value, tangent) through the same passes.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+#include <vector>
+
+#include "dpg_gpu_internal.cuh"
+#include "dpg_host.h"
+#include "tp_ops.cuh"
+
+namespace dpg {
+
+using namespace tp;
+
+struct TpState {
+	int n1 = 0, E = 1;
+	double* G = nullptr;        // [n_vol][n_var][n1^d] weak divergence in the collocated basis
+	double* jn = nullptr;       // non-affine: [n_vol][n1^d] 1 / detJ at the Gauss points
+	double B[25], Bi[25], Dw[25], lm[5], lp[5], wm[5], wp[5];
+	std::vector<void*> allocs;
+};
+
+struct TpGeo {
+	int n_vol, affine;
+	const double* met;          // affine: [n_vol][d d]; else [n_vol][d d][n1^d]
+	const double* jinv;         // affine: [n_vol]; else [n_vol][n1^d]
+	const int* vol_face;        // [n_vol][2 d]  (face << 1) | side
+	const int* nc_inv;          // [n_face][n_fc]
+};
+
+template <int N1>
+static Ops<N1> ops_of(const TpState* st)
+{
+	Ops<N1> o;
+	for (int k = 0; k < N1 * N1; ++k) { o.B[k] = st->B[k]; o.Bi[k] = st->Bi[k]; o.Dw[k] = st->Dw[k]; }
+	for (int k = 0; k < N1; ++k) { o.lm[k] = st->lm[k]; o.lp[k] = st->lp[k]; o.wm[k] = st->wm[k]; o.wp[k] = st->wp[k]; }
+	return o;
+}
+
+// Shared memory (doubles): the operators, then two buffers of E NW N values and D - 1 of E NV N (the fluxes of direction
+// 0 reuse the buffer the last B pass read from).
+template <int D, int NV, int N1, bool TAN>
+static size_t smem_volume(int E)
+{
+	const size_t N = ipow(N1, D), NW = TAN ? 2 * NV : NV;
+	return sizeof(Ops<N1>) + sizeof(double) * E * N * (2 * NW + (D - 1) * NV);
+}
+
+template <int D, int NV, int N1, bool TAN>
+__global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g,
+                                                   const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
+                                                   double* __restrict__ trace_t, double* __restrict__ G, int E, double bx,
+                                                   double by, double bz)
+{
+	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1), NW = TAN ? 2 * NV : NV;
+	extern __shared__ double sm[];
+	Ops<N1>* so = reinterpret_cast<Ops<N1>*>(sm);
+	double* b0 = sm + sizeof(Ops<N1>) / sizeof(double);
+	double* b1 = b0 + (size_t)E * NW * N;
+	double* fl = b1 + (size_t)E * NW * N;   // [D - 1][E][NV][N]
+	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
+	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
+	const bool live = e < ne;
+	load_ops(so, ops);
+	{
+		const size_t g0 = (size_t)e0 * NV * N;
+		for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) {
+			if constexpr (TAN) {
+				const int ee = k / (NV * N), r = k - ee * NV * N;
+				b0[ee * NW * N + r] = u[g0 + k];
+				b0[ee * NW * N + NV * N + r] = v[g0 + k];
+			} else {
+				b0[k] = u[g0 + k];
+			}
+		}
+	}
+	double m[D][D];   // of this node's element (affine) or node
+	if (live) {
+#pragma unroll
+		for (int x = 0; x < D; ++x)
+#pragma unroll
+			for (int r = 0; r < D; ++r)
+				m[x][r] = g.affine ? g.met[(size_t)(e0 + e) * D * D + x + D * r]
+				                   : g.met[((size_t)(e0 + e) * D * D + x + D * r) * N + i];
+	}
+	__syncthreads();
+	// values at the Gauss points: pass 0 b0 -> b1, pass 1 b1 -> b0, (pass 2 b0 -> b1)
+	double s[NW];
+	auto pass = [&](auto tag, const double* src, double* dst) {
+		constexpr int A = decltype(tag)::value;
+		if (live) {
+			const double* row = so->B + node_along<A, N1>(i) * N1;
+			const int base = pencil_base<A, N1>(i);
+			double op[N1];
+#pragma unroll
+			for (int j = 0; j < N1; ++j) op[j] = row[j];
+#pragma unroll
+			for (int w = 0; w < NW; ++w) {
+				s[w] = pencil_dot<A, N1>(op, src + (e * NW + w) * N, base);
+				dst[(e * NW + w) * N + i] = s[w];
+			}
+		}
+		__syncthreads();
+	};
+	pass(std::integral_constant<int, 0>{}, b0, b1);
+	pass(std::integral_constant<int, 1>{}, b1, b0);
+	if constexpr (D == 3) pass(std::integral_constant<int, 2>{}, b0, b1);
+	const double* sc = D == 3 ? b1 : b0;     // the collocated values
+	double* f0 = D == 3 ? b0 : b1;           // free: the fluxes of direction 0
+	// reference fluxes of this node (TAN: their tangents)
+	if (live) {
+		const double b[3] = {bx, by, bz};
+		auto met = [&](int x, int r) { return m[x][r]; };
+		auto put = [&](int r, int w, double y) { (r == 0 ? f0 : fl + (size_t)(r - 1) * E * NV * N)[(e * NV + w) * N + i] = y; };
+		if constexpr (TAN) {
+			dual sd[NV];
+#pragma unroll
+			for (int w = 0; w < NV; ++w) sd[w] = dual(s[w], s[NV + w]);
+			ref_flux<D, NV>(sd, met, b, [&](int r, const dual (&fr)[NV]) {
+#pragma unroll
+				for (int w = 0; w < NV; ++w) put(r, w, fr[w].d);
+			});
+		} else {
+			ref_flux<D, NV>(s, met, b, [&](int r, const double (&fr)[NV]) {
+#pragma unroll
+				for (int w = 0; w < NV; ++w) put(r, w, fr[w]);
+			});
+		}
+	}
+	// traces of the local faces, in the element's own node order
+	for (int o = threadIdx.x; o < ne * 2 * D * NF; o += blockDim.x) {
+		const int ee = o / (2 * D * NF), r = o - ee * 2 * D * NF, lf = r / NF, q = r - lf * NF, a = lf >> 1;
+		const double* l = (lf & 1) ? so->lp : so->lm;
+		const int S = stride_of<N1>(a), base = face_base<N1>(a, q);
+		const size_t vf = (size_t)g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
+#pragma unroll
+		for (int w = 0; w < NW; ++w) {
+			const double* x = sc + (ee * NW + w) * N + base;
+			double acc = l[0] * x[0];
+#pragma unroll
+			for (int j = 1; j < N1; ++j) acc = fma(l[j], x[j * S], acc);
+			(w < NV ? trace : trace_t)[(vf * NV + (w < NV ? w : w - NV)) * NF + q] = acc;
+		}
+	}
+	__syncthreads();
+	// weak divergence
+	if (live) {
+		double acc[NV];
+		auto add = [&](auto tag, const double* src) {
+			constexpr int A = decltype(tag)::value;
+			const double* row = so->Dw + node_along<A, N1>(i) * N1;
+			const int base = pencil_base<A, N1>(i);
+			double op[N1];
+#pragma unroll
+			for (int j = 0; j < N1; ++j) op[j] = row[j];
+#pragma unroll
+			for (int w = 0; w < NV; ++w) {
+				const double* x = src + (e * NV + w) * N + base;
+#pragma unroll
+				for (int j = 0; j < N1; ++j)
+					acc[w] = (A == 0 && j == 0) ? op[0] * x[0] : fma(op[j], x[j * ipow(N1, A)], acc[w]);
+			}
+		};
+		add(std::integral_constant<int, 0>{}, f0);
+		add(std::integral_constant<int, 1>{}, fl);
+		if constexpr (D == 3) add(std::integral_constant<int, 2>{}, fl + (size_t)E * NV * N);
+#pragma unroll
+		for (int w = 0; w < NV; ++w) G[((size_t)(e0 + e) * NV + w) * N + i] = acc[w];
+	}
+}
+
+template <int D, int NV, int N1>
+static size_t smem_lift(int E)
+{
+	const size_t N = ipow(N1, D), NF = ipow(N1, D - 1);
+	return sizeof(Ops<N1>) + sizeof(double) * E * NV * (2 * N + 2 * D * NF) + 8;
+}
+
+// stage < 0: residual only.  stage 0..2: SSP-RK3 stage update of sol (solp holds the step's initial state).  max_slot may
+// be null (the linearisation).
+template <int D, int NV, int N1>
+__global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, const double* __restrict__ nnf, TpGeo g,
+                                                 const __grid_constant__ Ops<N1> ops, double* __restrict__ sol,
+                                                 double* __restrict__ solp, double* __restrict__ rhs,
+                                                 const double* __restrict__ dt_ptr, unsigned long long* max_slot, int stage,
+                                                 int write_rhs, int E)
+{
+	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1);
+	extern __shared__ double sm[];
+	Ops<N1>* so = reinterpret_cast<Ops<N1>*>(sm);
+	double* b0 = sm + sizeof(Ops<N1>) / sizeof(double);
+	double* b1 = b0 + (size_t)E * NV * N;
+	double* sF = b1 + (size_t)E * NV * N;   // [E][2 D][NV][NF] face fluxes in the element's node order, + outward
+	unsigned long long* s_max = reinterpret_cast<unsigned long long*>(sF + (size_t)E * NV * 2 * D * NF);
+	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
+	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
+	const bool live = e < ne;
+	load_ops(so, ops);
+	const size_t gi0 = (size_t)e0 * NV * N;
+	const size_t gi = gi0 + (size_t)e * NV * N + i;
+	double r[NV], u0[NV], up[NV], ji = 0.0;
+	if (live) {   // every global operand of the node issued before the first barrier
+#pragma unroll
+		for (int w = 0; w < NV; ++w) {
+			r[w] = G[gi + w * N];
+			u0[w] = stage >= 0 ? sol[gi + w * N] : 0.0;
+			up[w] = stage >= 1 ? solp[gi + w * N] : 0.0;
+		}
+		ji = g.affine ? g.jinv[e0 + e] : g.jinv[(size_t)(e0 + e) * N + i];
+	}
+	for (int o = threadIdx.x; o < ne * 2 * D * NF; o += blockDim.x) {
+		const int ee = o / (2 * D * NF), k = o - ee * 2 * D * NF, lf = k / NF, q = k - lf * NF;
+		const int vf = g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
+		const int f = vf >> 1, side = vf & 1;
+		const int qs = side ? g.nc_inv[(size_t)f * NF + q] : q;
+		const long long flip = side ? 0ll : (long long)0x8000000000000000ull;   // - outward flux of this element
+#pragma unroll
+		for (int w = 0; w < NV; ++w)
+			sF[((size_t)(ee * 2 * D + lf) * NV + w) * NF + q] =
+			    __longlong_as_double(__double_as_longlong(nnf[((size_t)f * NV + w) * NF + qs]) ^ flip);
+	}
+	__syncthreads();
+	if (live) {
+		auto face = [&](auto tag) {
+			constexpr int A = decltype(tag)::value;
+			const int ia = node_along<A, N1>(i), q = face_node<A, N1>(i);
+			const double wm = so->wm[ia], wp = so->wp[ia];
+			const double* F = sF + (size_t)(e * 2 * D + 2 * A) * NV * NF + q;
+#pragma unroll
+			for (int w = 0; w < NV; ++w) r[w] = fma(wp, F[(NV + w) * NF], fma(wm, F[w * NF], r[w]));
+		};
+		face(std::integral_constant<int, 0>{});
+		face(std::integral_constant<int, 1>{});
+		if constexpr (D == 3) face(std::integral_constant<int, 2>{});
+#pragma unroll
+		for (int w = 0; w < NV; ++w) b0[(e * NV + w) * N + i] = r[w] * ji;
+	}
+	__syncthreads();
+	// back to the solution nodes: B^-1 in each direction
+	auto pass = [&](auto tag, const double* src, double* dst) {
+		constexpr int A = decltype(tag)::value;
+		if (live) {
+			const double* row = so->Bi + node_along<A, N1>(i) * N1;
+			const int base = pencil_base<A, N1>(i);
+			double op[N1];
+#pragma unroll
+			for (int j = 0; j < N1; ++j) op[j] = row[j];
+#pragma unroll
+			for (int w = 0; w < NV; ++w) {
+				r[w] = pencil_dot<A, N1>(op, src + (e * NV + w) * N, base);
+				if (A < D - 1) dst[(e * NV + w) * N + i] = r[w];
+			}
+		}
+		if (A < D - 1) __syncthreads();
+	};
+	pass(std::integral_constant<int, 0>{}, b0, b1);
+	pass(std::integral_constant<int, 1>{}, b1, b0);
+	if constexpr (D == 3) pass(std::integral_constant<int, 2>{}, b0, b1);
+	unsigned long long lmax = 0;
+	if (live) {
+		const double dt = (stage >= 0 ? *dt_ptr : 0.0);
+#pragma unroll
+		for (int w = 0; w < NV; ++w) {
+			const size_t k = gi + w * N;
+			const unsigned long long ab = abs_bits_of(r[w]);
+			lmax = ab > lmax ? ab : lmax;
+			if (write_rhs) rhs[k] = r[w];
+			if (stage == 0) { solp[k] = u0[w]; sol[k] = u0[w] + dt * r[w]; }
+			else if (stage == 1) sol[k] = (1.0 / 4.0) * (3.0 * up[w] + u0[w] + dt * r[w]);
+			else if (stage == 2) sol[k] = (1.0 / 3.0) * (up[w] + 2.0 * u0[w] + 2.0 * dt * r[w]);
+		}
+	}
+	if (max_slot) block_max_to(lmax, s_max, max_slot);
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// host
+// ------------------------------------------------------------------------------------------------------------
+static bool near(double a, double b, double scale) { return std::fabs(a - b) <= 1e-11 * scale; }
+
+// The 1D operators of order n1 - 1, and whether the element's dense operators are their products.
+static bool build_ops(TpState* st, const dpg_element_ops& o)
+{
+	const int n1 = o.p + 1, d = o.d;
+	double gll[16], wgll[16], gl[16], w[16], val[16], der[16];
+	dpg_nodes_gll(n1, gll, wgll);
+	dpg_nodes_gl(n1, gl, w);
+	for (int q = 0; q < n1; ++q) {
+		dpg_lagrange_1d(n1, gll, gl[q], val, der);
+		for (int i = 0; i < n1; ++i) st->B[q * n1 + i] = val[i];
+		dpg_lagrange_1d(n1, gl, gll[q], val, der);   // the inverse map: the collocated basis at the solution nodes
+		for (int i = 0; i < n1; ++i) st->Bi[q * n1 + i] = val[i];
+		dpg_lagrange_1d(n1, gl, gl[q], val, der);
+		for (int i = 0; i < n1; ++i) st->Dw[i * n1 + q] = w[q] / w[i] * der[i];
+	}
+	dpg_lagrange_1d(n1, gl, -1.0, st->lm, der);
+	dpg_lagrange_1d(n1, gl, 1.0, st->lp, der);
+	for (int i = 0; i < n1; ++i) { st->wm[i] = st->lm[i] / w[i]; st->wp[i] = st->lp[i] / w[i]; }
+	const int n_s = o.n_s, n_c = o.n_c, n_fc = o.n_fc;
+	auto digit = [&](int k, int a) { for (; a > 0; --a) k /= n1; return k % n1; };
+	// interpolation, weak derivative and mass matrix inverse entry by entry
+	for (int c = 0; c < n_c; ++c)
+		for (int s = 0; s < n_s; ++s) {
+			double b = 1.0;
+			for (int a = 0; a < d; ++a) b *= st->B[digit(c, a) * n1 + digit(s, a)];
+			if (!near(o.cv0_vs_vc[(size_t)c * n_s + s], b, 1.0)) return false;
+			for (int r = 0; r < d; ++r) {   // d phi_s / dr at node c = sum over the collocated basis along r
+				double t = 0.0, wc = 1.0;
+				for (int j = 0; j < n1; ++j) {
+					double y = st->Dw[j * n1 + digit(c, r)] * w[j] / w[digit(c, r)];   // l_j'(x_c)
+					for (int a = 0; a < d; ++a) y *= st->B[(a == r ? j : digit(c, a)) * n1 + digit(s, a)];
+					t += y;
+				}
+				for (int a = 0; a < d; ++a) wc *= w[digit(c, a)];
+				if (!near(o.tw1_vt_vc[((size_t)r * n_s + s) * n_c + c], wc * t, 10.0)) return false;
+			}
+		}
+	for (int i = 0; i < n_s; ++i)
+		for (int j = 0; j < n_s; ++j) {
+			double t = 0.0;
+			for (int c = 0; c < n_c; ++c) {
+				double y = 1.0;
+				for (int a = 0; a < d; ++a)
+					y *= st->Bi[digit(i, a) * n1 + digit(c, a)] * st->Bi[digit(j, a) * n1 + digit(c, a)] / w[digit(c, a)];
+				t += y;
+			}
+			if (!near(o.m_inv_ref[(size_t)i * n_s + j], t, 1e3)) return false;
+		}
+	// faces: the collocated basis at the face nodes, the face weights
+	for (int lf = 0; lf < 2 * d; ++lf) {
+		const int a0 = lf >> 1;
+		const double* l = (lf & 1) ? st->lp : st->lm;
+		for (int q = 0; q < n_fc; ++q) {
+			int k[3] = {0, 0, 0}, t = q;
+			double wf = 1.0;
+			for (int a = 0; a < d; ++a)
+				if (a != a0) { k[a] = t % n1; t /= n1; wf *= w[k[a]]; }
+			for (int s = 0; s < n_s; ++s) {
+				double e = 0.0, y = 1.0;
+				for (int j = 0; j < n1; ++j) e += l[j] * st->B[j * n1 + digit(s, a0)];
+				for (int a = 0; a < d; ++a)
+					if (a != a0) y *= st->B[k[a] * n1 + digit(s, a)];
+				if (!near(o.cv0_vs_fc[((size_t)lf * n_fc + q) * n_s + s], e * y, 1.0) ||
+				    !near(o.tw0_vt_fc[((size_t)lf * n_s + s) * n_fc + q], e * y * wf, 1.0))
+					return false;
+			}
+		}
+	}
+	return true;
+}
+
+void tp_free(dpg_gpu_ctx* c)
+{
+	TpState* st = (TpState*)c->tp;
+	if (!st) return;
+	for (void* p : st->allocs) cudaFree(p);
+	delete st;
+	c->tp = nullptr;
+}
+
+// Elements per block: as many as fill 256 threads, but no more than leave two blocks per SM, and at least a warp.
+static constexpr int most_elems(int N) { return 256 / N; }
+static int block_elems(int n_vol, int N, int n_sm)
+{
+	const int fill = (n_vol + 2 * n_sm - 1) / (2 * n_sm), warp = (31 + N) / N;
+	return std::min(most_elems(N), std::max(fill, warp));
+}
+
+// Shared-memory opt-in at the largest block: one limit for every context of the process.
+template <int D, int NV, int N1>
+static int configure()
+{
+	constexpr int E = most_elems(ipow(N1, D));
+	if (cudaFuncSetAttribute(k_tp_volume<D, NV, N1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, false>(E)) ||
+	    cudaFuncSetAttribute(k_tp_volume<D, NV, N1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, true>(E)) ||
+	    cudaFuncSetAttribute(k_tp_lift<D, NV, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lift<D, NV, N1>(E)))
+		return DPG_ERR_CUDA;
+	return DPG_OK;
+}
+
+template <int D, int NV, int N1>
+static int launch_volume(dpg_gpu_ctx* c, const double* u, const double* v, double* trace, double* trace_t)
+{
+	const TpState* st = (const TpState*)c->tp;
+	const GroupDev& g = c->g;
+	constexpr int N = ipow(N1, D);
+	const TpGeo geo{g.n_vol, g.affine, g.met, g.affine ? g.jinv : st->jn, g.vol_face, g.nc_inv};
+	const int E = st->E, grid = (g.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	const Ops<N1> ops = ops_of<N1>(st);
+	if (v)
+		k_tp_volume<D, NV, N1, true><<<grid, threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
+		    u, v, geo, ops, trace, trace_t, st->G, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+	else
+		k_tp_volume<D, NV, N1, false><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
+		    u, nullptr, geo, ops, trace, nullptr, st->G, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
+}
+
+template <int D, int NV, int N1>
+static int launch_lift(dpg_gpu_ctx* c, const double* nnf, double* rhs, unsigned long long* max_slot, int stage, bool write_rhs)
+{
+	const TpState* st = (const TpState*)c->tp;
+	const GroupDev& g = c->g;
+	constexpr int N = ipow(N1, D);
+	const TpGeo geo{g.n_vol, g.affine, g.met, g.affine ? g.jinv : st->jn, g.vol_face, g.nc_inv};
+	const int E = st->E, grid = (g.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	k_tp_lift<D, NV, N1><<<grid, threads, smem_lift<D, NV, N1>(E), c->stream>>>(
+	    st->G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E);
+	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
+}
+
+#define DPG_TP_N1(F, D, NV, ...)                        \
+	switch (((const TpState*)c->tp)->n1) {              \
+	case 2: return F<D, NV, 2>(__VA_ARGS__);            \
+	case 3: return F<D, NV, 3>(__VA_ARGS__);            \
+	case 4: return F<D, NV, 4>(__VA_ARGS__);            \
+	case 5: return F<D, NV, 5>(__VA_ARGS__);            \
+	default: return DPG_ERR_UNSUPPORTED;                \
+	}
+#define DPG_TP_DISPATCH(F, ...)                                             \
+	do {                                                                    \
+		if (c->d == 2 && c->n_var == 4) { DPG_TP_N1(F, 2, 4, __VA_ARGS__) } \
+		if (c->d == 3 && c->n_var == 5) { DPG_TP_N1(F, 3, 5, __VA_ARGS__) } \
+		if (c->d == 2 && c->n_var == 1) { DPG_TP_N1(F, 2, 1, __VA_ARGS__) } \
+		if (c->d == 3 && c->n_var == 1) { DPG_TP_N1(F, 3, 1, __VA_ARGS__) } \
+		return DPG_ERR_UNSUPPORTED;                                         \
+	} while (0)
+
+static int configure_any(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(configure); }
+
+int tp_volume(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(launch_volume, c, c->sol, nullptr, c->trace, nullptr); }
+int tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t)
+{
+	DPG_TP_DISPATCH(launch_volume, c, u, v, c->trace, trace_t);
+}
+int tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
+{
+	DPG_TP_DISPATCH(launch_lift, c, c->nnf, c->rhs, max_slot, stage, write_rhs);
+}
+int tp_lift_tan(dpg_gpu_ctx* c, const double* nnf_t, double* out)
+{
+	DPG_TP_DISPATCH(launch_lift, c, nnf_t, out, nullptr, -1, true);
+}
+
+// Set-up.  Leaves c->tp null (the dense kernels of kernels_fp64.cu run) where the element is not one of the orders above
+// or its operators are not the products of the 1D ones.
+int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim)
+{
+	const dpg_element_ops& o = sim->ops[0];
+	if ((o.e_type != DPG_QUAD && o.e_type != DPG_HEX) || o.p < 1 || o.p + 1 > kN1Max) return DPG_OK;
+	const int N = ipow(o.p + 1, o.d);
+	if (o.n_s != N || o.n_c != N || o.n_fc != ipow(o.p + 1, o.d - 1) || o.n_fl != 2 * o.d) return DPG_OK;
+	// a mesh of fewer nodes than this is bound by the launch chain in either form (QUAD p = 1, 64 elements, one residual
+	// with its host round trip: 68.8 us here, 68.4 us dense; QUAD p = 2, 256 elements, 2,304 nodes: 24.2 us a stage
+	// here, 33.4 us dense) and keeps the dense kernels and their summation order
+	constexpr int64_t kMinNodes = 1024;
+	if ((int64_t)sim->n_vol * N < kMinNodes) return DPG_OK;
+	TpState* st = new TpState();
+	st->n1 = o.p + 1;
+	if (!build_ops(st, o)) { delete st; return DPG_OK; }
+	c->tp = st;
+	auto alloc = [&](double** p, size_t n) {
+		void* q = nullptr;
+		if (cudaMalloc(&q, n * sizeof(double)) != cudaSuccess) return (int)DPG_ERR_CUDA;
+		st->allocs.push_back(q);
+		*p = (double*)q;
+		return (int)DPG_OK;
+	};
+	int rc;
+	if ((rc = alloc(&st->G, (size_t)c->n_dof))) return rc;
+	if (!c->g.affine) {
+		std::vector<double> ji((size_t)sim->n_vol * N);
+		for (int v = 0; v < sim->n_vol; ++v)
+			for (int k = 0; k < N; ++k) ji[(size_t)v * N + k] = 1.0 / sim->jacobian_det_vc[sim->vol_geo_off[v] + k];
+		if ((rc = alloc(&st->jn, ji.size()))) return rc;
+		if (cudaMemcpy(st->jn, ji.data(), sizeof(double) * ji.size(), cudaMemcpyHostToDevice) != cudaSuccess) return DPG_ERR_CUDA;
+	}
+	int n_sm = 0;
+	if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, c->dev) != cudaSuccess || n_sm < 1) n_sm = 1;
+	st->E = block_elems(sim->n_vol, N, n_sm);
+	return configure_any(c);
+}
+
+} // namespace dpg

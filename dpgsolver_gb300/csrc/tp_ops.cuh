@@ -1,0 +1,137 @@
+// One-dimensional operators of the tensor-product elements (QUAD, HEX) and the device passes that apply them one
+// direction at a time.
+//
+// The solution nodes are Gauss-Lobatto points, the cubature nodes of volumes and faces Gauss points, n1 = p + 1 of
+// both per direction.  Every dense operator of the residual is a Kronecker product of 1D factors, and the
+// mass matrix with that cubature is diagonal in the Lagrange basis of the Gauss points (the collocated basis):
+//     cv0_vs_vc           = B (x) B (x) B                     B[q][i]  GLL Lagrange polynomial i at Gauss point q
+//     cv0_vs_fc           = l(+-1)^T in the face's direction of the collocated values
+//     m_inv tw1_vt_vc[r]  = B^-1 (x) .. diag(1 / detJ) Dw_r    Dw[i][j] = w_j / w_i l_i'(x_j)
+//     m_inv tw0_vt_fc     = B^-1 (x) .. diag(1 / detJ) l_i(+-1) / w_i
+// (for a non-affine element too: 1 / detJ is then one number per Gauss point).  An n1^d x n1^d product becomes d
+// passes of n1 terms, a face lift one term per node.
+#pragma once
+
+#include <cstdint>
+
+#include "flux.cuh"
+
+namespace dpg {
+namespace tp {
+
+constexpr int kN1Max = 5;   // orders 1..4
+
+// Kernel parameter (constant bank), copied to shared memory by each block.
+template <int N1>
+struct Ops {
+	double B[N1 * N1];     // [q][i]  GLL -> Gauss values
+	double Bi[N1 * N1];    // [i][q]  its inverse
+	double Dw[N1 * N1];    // [i][j]  weak derivative over the weights
+	double lm[N1], lp[N1]; // collocated basis at -1 and +1
+	double wm[N1], wp[N1]; // the same over the weights
+};
+
+template <int N1>
+__device__ __forceinline__ void load_ops(Ops<N1>* s, const Ops<N1>& p)
+{
+	constexpr int n = (int)(sizeof(Ops<N1>) / sizeof(double));
+	const double* src = reinterpret_cast<const double*>(&p);
+	for (int k = threadIdx.x; k < n; k += blockDim.x) reinterpret_cast<double*>(s)[k] = src[k];
+}
+
+__host__ __device__ constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * ipow(b, e - 1); }
+
+// Node i's value of one direction's pass over an array of n1^d nodes: sum_j op[i_a][j] x[.. j ..].
+template <int A, int N1, class T>
+__device__ __forceinline__ T pencil_dot(const double* row, const T* x, int base)
+{
+	constexpr int S = ipow(N1, A);
+	T acc = row[0] * x[base];
+#pragma unroll
+	for (int j = 1; j < N1; ++j) acc += row[j] * x[base + j * S];
+	return acc;
+}
+
+// Position of node i along direction A, and the first node of its pencil.
+template <int A, int N1>
+__device__ __forceinline__ int node_along(int i) { return (i / ipow(N1, A)) % N1; }
+template <int A, int N1>
+__device__ __forceinline__ int pencil_base(int i) { return i - node_along<A, N1>(i) * ipow(N1, A); }
+
+// Face node q of direction a: the first node of its pencil; node i's face node.
+template <int N1>
+__device__ __forceinline__ int face_base(int a, int q)
+{
+	const int S = a == 0 ? 1 : (a == 1 ? N1 : N1 * N1);
+	return (q % S) + (q / S) * (S * N1);
+}
+template <int A, int N1>
+__device__ __forceinline__ int face_node(int i)
+{
+	constexpr int S = ipow(N1, A);
+	return (i % S) + (i / (S * N1)) * S;
+}
+
+template <int N1>
+__device__ __forceinline__ constexpr int stride_of(int a) { return a == 0 ? 1 : (a == 1 ? N1 : N1 * N1); }
+
+// Reference volume flux of one node, handed to emit(r, fr_r) direction by direction: fr_r[eq] = sum_x m_xr f[x][eq]
+// in contravariant form (the velocity along r once per direction instead of d products per equation).
+template <int D, int NV, class T, class Met, class Emit>
+__device__ __forceinline__ void ref_flux(const T* s, const Met& met, const double* b, Emit&& emit)
+{
+	if constexpr (NV == D + 2) {
+		const T rho_inv = 1.0 / s[0], E = s[D + 1];
+		T u[D], V2 = 0.0;
+#pragma unroll
+		for (int a = 0; a < D; ++a) { u[a] = s[1 + a] * rho_inv; V2 += u[a] * u[a]; }
+		const T p = DPG_GM1_D * (E - 0.5 * s[0] * V2), Ep = E + p;
+#pragma unroll
+		for (int r = 0; r < D; ++r) {
+			double m[D];
+#pragma unroll
+			for (int x = 0; x < D; ++x) m[x] = met(x, r);
+			T W = m[0] * u[0], f0 = m[0] * s[1];
+#pragma unroll
+			for (int x = 1; x < D; ++x) { W += m[x] * u[x]; f0 += m[x] * s[1 + x]; }
+			T fr[NV];
+			fr[0] = f0;
+#pragma unroll
+			for (int a = 0; a < D; ++a) fr[1 + a] = s[1 + a] * W + m[a] * p;
+			fr[D + 1] = Ep * W;
+			emit(r, fr);
+		}
+	} else {
+#pragma unroll
+		for (int r = 0; r < D; ++r) {
+			T fr[NV];
+			double mb = 0.0;
+#pragma unroll
+			for (int x = 0; x < D; ++x) mb += met(x, r) * b[x];
+			fr[0] = mb * s[0];
+			emit(r, fr);
+		}
+	}
+}
+
+__device__ __forceinline__ unsigned long long abs_bits_of(double v)
+{
+	return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+}
+
+// max |v| of the block (IEEE bits: NaN orders above +inf) into *slot; every thread calls.
+__device__ __forceinline__ void block_max_to(unsigned long long m, unsigned long long* s_max, unsigned long long* slot)
+{
+	if (threadIdx.x == 0) *s_max = 0ull;
+	__syncthreads();
+	for (int o = 16; o > 0; o >>= 1) {
+		const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
+		m = t > m ? t : m;
+	}
+	if ((threadIdx.x & 31) == 0) atomicMax(s_max, m);
+	__syncthreads();
+	if (threadIdx.x == 0) atomicMax(slot, *s_max);
+}
+
+} // namespace tp
+} // namespace dpg

@@ -135,10 +135,10 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	g.n_vol = n_vol; g.n_s = n_s; g.n_c = n_c; g.n_fl = n_fl; g.n_fc = n_fc; g.K = d * n_c + n_fl * n_fc;
 	g.affine = affine_all;
 	const int K = g.K;
-	// boundary faces or viscous terms: the general chain (the periodic Euler / advection kernels have neither)
 	int general = (sim->pde_index == DPG_PDE_NAVIER_STOKES);
 	for (int f = 0; f < n_face; ++f) general |= (sim->face_vol[2 * f + 1] < 0);
-	if (!general && (rc = dpg::tp_prepare(c, sim))) return fail(rc);
+	c->walls_or_visc = general;
+	if ((rc = dpg::tp_prepare(c, sim, general))) return fail(rc);
 
 	// operators: Cv, Cf, L = [tw1 | -tw0] (times m_inv_ref when every volume is affine)
 	std::vector<double> L((size_t)n_s * K), Lm((size_t)n_s * K);
@@ -178,7 +178,7 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	} else {
 		// per node metrics [v][k][c] (the host layout is already c fastest within k)
 		if ((rc = dupload(c, (double**)&g.met, sim->metrics_vc, (size_t)n_vol * n_c * d * d))) return fail(rc);
-		if (!c->tp && !general) {   // the dense kernels' element mass-matrix inverses
+		if (!c->tp) {   // the dense kernels' element mass-matrix inverses
 			std::vector<double> minv((size_t)n_vol * n_s * n_s);
 			for (int v = 0; v < n_vol; ++v) {
 				double* dst = &minv[(size_t)v * n_s * n_s];
@@ -238,6 +238,7 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 		c->positivity = 1;
 	} else if ((sim->pde_index == DPG_PDE_EULER || sim->pde_index == DPG_PDE_NAVIER_STOKES) && nv == d + 2) {
 		const int n1 = ops.p + 1;
+		if (n1 * n1 > 25) return fail(DPG_ERR_UNSUPPORTED);   // the limiter's 1D operators: orders 1..4
 		c->pos_n1 = n1;
 		c->pos_amp = (float)(4.0 * (d * (n1 + 2) + 2) * std::ldexp(1.0, -24));
 		for (int i = 0; i < n1 * n1; ++i) { c->bez1_host[i] = ops.bez1[i]; c->bez1_host[25 + i] = ops.bez1_inv[i]; }
@@ -278,7 +279,16 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 		c->adv_speed = std::sqrt(sim->b_adv[0] * sim->b_adv[0] + sim->b_adv[1] * sim->b_adv[1] + sim->b_adv[2] * sim->b_adv[2]);
 	}
 	if ((rc = dpg::fp64_configure(c))) return fail(rc);
-	if (general && (rc = dpg::gen_prepare(c, sim))) return fail(rc);
+	if (general && c->tp) {
+		if ((rc = dpg::tp_general_prepare(c, sim))) return fail(rc);
+	} else if (general) {   // advection: a boundary state is the interior trace
+		if (nv != 1) return fail(DPG_ERR_UNSUPPORTED);
+		std::vector<int> bf;
+		for (int f = 0; f < n_face; ++f)
+			if (sim->face_vol[2 * f + 1] < 0) bf.push_back(f);
+		c->n_bface = (int)bf.size();
+		if ((rc = dupload(c, (int**)&c->bface, bf.data(), bf.size()))) return fail(rc);
+	}
 	if (cudaDeviceSynchronize() != cudaSuccess) return fail(DPG_ERR_CUDA);
 	*ctx_out = c;
 	return DPG_OK;
@@ -290,7 +300,6 @@ extern "C" void dpg_gpu_destroy(dpg_gpu_ctx* c)
 	if (c->stream) cudaStreamSynchronize(c->stream);
 	dpg::split_free(c);
 	dpg::tp_free(c);
-	dpg::gen_free(c);
 	dpg::hp_free(c);
 	dpg::implicit_free(c);
 	dpg::mlp_free(c);
@@ -316,7 +325,7 @@ extern "C" int dpg_gpu_set_precision(dpg_gpu_ctx* c, int mode, int n_slices)
 	if (mode == DPG_PREC_BF16_SLICED && (n_slices < 2 || n_slices > 7)) return DPG_ERR_INVALID;
 	// the split kernels cover periodic meshes of one order without viscous terms (affine elements: checked when
 	// the operators are prepared)
-	if (mode != DPG_PREC_FP64 && (c->general || c->hp)) return DPG_ERR_UNSUPPORTED;
+	if (mode != DPG_PREC_FP64 && (c->walls_or_visc || c->hp)) return DPG_ERR_UNSUPPORTED;
 	c->prec_mode = mode;
 	c->n_slices = n_slices;
 	invalidate_graph(c);
@@ -399,7 +408,7 @@ extern "C" int dpg_gpu_download_rhs(dpg_gpu_ctx* c, double* h)
 static int enqueue_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
 {
 	int rc;
-	if (c->general) return dpg::gen_residual(c, stage, write_rhs, max_slot);
+	if (c->walls_or_visc && c->tp) return dpg::tp_general_residual(c, stage, write_rhs, max_slot);
 	if (c->hp) return dpg::hp_residual(c, stage, write_rhs, max_slot);
 	if (c->prec_mode == DPG_PREC_FP64) {
 		if ((rc = dpg::launch_trace(c))) return rc;
@@ -555,7 +564,7 @@ extern "C" int dpg_gpu_time_rk_steps(dpg_gpu_ctx* c, double dt, int n_steps, dou
 extern "C" int dpg_gpu_launches_per_rhs(dpg_gpu_ctx* c)
 {
 	if (!c) return 0;
-	return c->general ? dpg::gen_launches_per_rhs(c) : 3;
+	return !c->walls_or_visc ? 3 : c->tp ? dpg::tp_general_launches(c) : 4;
 }
 
 extern "C" int dpg_gpu_kernel_times(dpg_gpu_ctx* c, int n_rep, double* ms_out, const char** names_out, int n_max)
@@ -564,11 +573,11 @@ extern "C" int dpg_gpu_kernel_times(dpg_gpu_ctx* c, int n_rep, double* ms_out, c
 	static const char* names[3] = {"trace", "face", "volume"};
 	cudaEvent_t ev[4];
 	for (int i = 0; i < 4; ++i) CK(cudaEventCreate(&ev[i]));
-	if (c->general) {   // the general chain is timed as one residual
+	if (c->walls_or_visc) {   // timed as one residual
 		double acc1 = 0.0;
 		for (int r = 0; r < n_rep; ++r) {
 			CK(cudaEventRecord(ev[0], c->stream));
-			int rc = dpg::gen_residual(c, -1, true, c->dmax + dpg::kMaxStages);
+			int rc = enqueue_residual(c, -1, true, c->dmax + dpg::kMaxStages);
 			if (rc) return rc;
 			CK(cudaEventRecord(ev[1], c->stream));
 			CK(cudaEventSynchronize(ev[1]));

@@ -99,7 +99,10 @@ struct dpg_gpu_ctx {
 	double* du_buf = nullptr;    // [n_dof] device copy of a host Newton update (dpg_gpu_positivity_update)
 
 	void* tp = nullptr;         // QUAD / HEX of one order: 1D operators of the FP64 form (kernels_tp.cu)
-	void* general = nullptr;    // boundary faces / Navier-Stokes: the general FP64 chain (kernels_ns.cu)
+	int walls_or_visc = 0;      // boundary faces or viscous terms: FP64 only, kernels_tp_general.cu (advection above p = 4:
+	                            // the dense kernels, boundary traces copied)
+	const int* bface = nullptr; // [n_bface] the boundary faces of that case
+	int n_bface = 0;
 	void* hp = nullptr;         // mixed orders: volumes grouped by order (kernels_hp.cu)
 	void* implicit = nullptr;   // Newton-GMRES work space (implicit.cu)
 	void* mlp = nullptr;        // learned preconditioner (mlp.cu)
@@ -108,6 +111,7 @@ struct dpg_gpu_ctx {
 namespace dpg {
 int launch_trace (dpg_gpu_ctx* c);
 int launch_face  (dpg_gpu_ctx* c);
+int launch_face_tan(dpg_gpu_ctx* c, const double* trace_t, double* nnf_t);   // tangents of the face fluxes
 int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
 // J v = d(m_inv rhs)/du . v at u (FP64 formulas, forward-mode tangents); trace_t, nnf_t: work buffers of the sizes
 // of the traces and face fluxes.
@@ -116,20 +120,16 @@ int ensure_tangent_buffers(dpg_gpu_ctx* c);
 
 // tensor-product elements (kernels_tp.cu): traces and weak divergence, then lift, stage and norm; the tangents of the
 // linearisation.  tp_prepare leaves c->tp null where the dense kernels run.
-int  tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);
+int  tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general);
 int  tp_volume(dpg_gpu_ctx* c);
 int  tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
 int  tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t);
 int  tp_lift_tan(dpg_gpu_ctx* c, const double* nnf_t, double* out);
 void tp_free(dpg_gpu_ctx* c);
-
-// general FP64 chain (kernels_ns.cu): boundary faces and the BR2 Navier-Stokes terms, residual and exact
-// Jacobian-vector products (forward-mode tangents through the same templated kernels)
-int  gen_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);
-int  gen_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
-int  gen_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out);
-int  gen_launches_per_rhs(dpg_gpu_ctx* c);
-void gen_free(dpg_gpu_ctx* c);
+int  tp_general_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);   // boundary faces, BR2 (after tp_prepare)
+int  tp_general_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
+int  tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t);
+int  tp_general_launches(dpg_gpu_ctx* c);
 
 // mixed orders (kernels_hp.cu): FP64 residual over volume groups of each order; which = 0 traces, 1 face fluxes,
 // 2 volume terms (with the RK stage)

@@ -128,9 +128,9 @@ __device__ __forceinline__ T numflux_upwind(const double* b, T wl, T wr, const d
 // 1000-1040): constant viscosity mu, Prandtl number Pr, g[x][var] the gradient of the conservative variables.
 //   du_i/dx = (d rho u_i/dx - u_i d rho/dx) / rho;  tau_ij = mu (du_j/dx_i + du_i/dx_j) - (2/3) mu div(V) delta_ij;
 //   dTs/dx = (dE/dx rho - E drho/dx) / rho^2 - V . dV/dx  (Ts = p / (rho (gamma - 1)));
-//   f[x] = -(0, tau[0][x], .., tau[d-1][x], gamma/Pr mu dTs/dx + sum_j u_j tau[x][j]).
+//   f[x] = -(0, tau[0][x], .., tau[d-1][x], kappa dTs/dx + sum_j u_j tau[x][j]), kappa = gamma mu / Pr.
 template <int D, class T>
-__device__ __forceinline__ void flux_viscous(double mu, double Pr, const T* s, const T (*g)[D + 2], T f[D][D + 2])
+__device__ __forceinline__ void flux_viscous(double mu, double kappa, const T* s, const T (*g)[D + 2], T f[D][D + 2])
 {
 	const T rho_inv = 1.0 / s[0], E = s[D + 1];
 	T u[D], du[D][D];
@@ -148,17 +148,17 @@ __device__ __forceinline__ void flux_viscous(double mu, double Pr, const T* s, c
 	for (int i = 0; i < D; ++i)
 #pragma unroll
 		for (int j = 0; j < D; ++j)
-			tau[i][j] = (i == j) ? mu * 2.0 * (du[i][i] - divV / 3.0) : mu * (du[j][i] + du[i][j]);
+			tau[i][j] = (i == j) ? mu * 2.0 * (du[i][i] - (1.0 / 3.0) * divV) : mu * (du[j][i] + du[i][j]);
 #pragma unroll
 	for (int x = 0; x < D; ++x) {
 		T dV2 = 0.0, w = 0.0;
 #pragma unroll
 		for (int a = 0; a < D; ++a) { dV2 += u[a] * du[a][x]; w += u[a] * tau[x][a]; }
-		const T dTs = rho_inv * rho_inv * (g[x][D + 1] * s[0] - E * g[x][0]) - 0.5 * (2.0 * dV2);
+		const T dTs = rho_inv * rho_inv * (g[x][D + 1] * s[0] - E * g[x][0]) - dV2;
 		f[x][0] = T(0.0);
 #pragma unroll
 		for (int i = 0; i < D; ++i) f[x][1 + i] = -tau[i][x];
-		f[x][D + 1] = -(DPG_GAMMA_D / Pr * mu * dTs + w);
+		f[x][D + 1] = -(kappa * dTs + w);
 	}
 }
 
@@ -230,8 +230,7 @@ __device__ __forceinline__ void boundary_state(int bc, const T* sl, const double
 		for (int a = 0; a < D; ++a) { sb[1 + a] = w[0] * w[1 + a]; V2 += w[1 + a] * w[1 + a]; }
 		sb[D + 1] = w[D + 1] / DPG_GM1_D + 0.5 * w[0] * V2;
 	} else if (bc == DPG_BC_NOSLIP_ALL_ROTATING) {
-		const double r = ::sqrt(x[0] * x[0] + x[1] * x[1]), th = ::atan2(x[1], x[0]), vt = bp.omega * r;
-		const double uw[3] = {-::sin(th) * vt, ::cos(th) * vt, 0.0};
+		const double uw[3] = {-bp.omega * x[1], bp.omega * x[0], 0.0};   // omega x r
 		sb[0] = -sl[0] + 2.0 * bp.rho_b;
 #pragma unroll
 		for (int a = 0; a < D; ++a) sb[1 + a] = -sl[1 + a] + 2.0 * bp.rho_b * uw[a];

@@ -52,6 +52,21 @@ __global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, G
 	}
 }
 
+// Advection with boundary faces: the boundary state is the interior trace (NV = 1).
+__global__ void __launch_bounds__(128) k_copy_boundary_trace(const int* __restrict__ bface, int n, int n_fc, double* __restrict__ trace)
+{
+	const int t = blockIdx.x * blockDim.x + threadIdx.x;
+	if (t >= n * n_fc) return;
+	const size_t f = (size_t)bface[t / n_fc];
+	trace[(2 * f + 1) * n_fc + t % n_fc] = trace[2 * f * n_fc + t % n_fc];
+}
+
+static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace)
+{
+	const int n = c->n_bface * c->fc.n_fc;
+	if (n) k_copy_boundary_trace<<<(n + 127) / 128, 128, 0, c->stream>>>(c->bface, c->n_bface, c->fc.n_fc, trace);
+}
+
 template <int D, int NV>
 __global__ void __launch_bounds__(256) k_face(const double* __restrict__ trace, FaceDev fd, double* __restrict__ nnf,
                                               int num_flux, double bx, double by, double bz)
@@ -209,6 +224,7 @@ static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs,
 		const size_t smem = (size_t)E_b * NV * g.n_s * sizeof(double);
 		const int grid = (g.n_vol + E_b - 1) / E_b;
 		k_trace<NV><<<grid, 256, smem, c->stream>>>(c->sol, g, c->trace, E_b);
+		copy_boundary_trace(c, c->trace);
 	} else if (which == 1) {
 		const int n = c->fc.n_face * c->fc.n_fc;
 		k_face<D, NV><<<(n + 127) / 128, 128, 0, c->stream>>>(c->trace, c->fc, c->nnf, c->num_flux,
@@ -386,6 +402,24 @@ __global__ void __launch_bounds__(256) k_volume_tan(const double* __restrict__ u
 }
 
 template <int D, int NV>
+static int face_tan_impl(dpg_gpu_ctx* c, const double* trace_t, double* nnf_t)
+{
+	const int n = c->fc.n_face * c->fc.n_fc;
+	k_face_tan<D, NV><<<(n + 127) / 128, 128, 0, c->stream>>>(c->trace, trace_t, c->fc, nnf_t, c->num_flux, c->b_adv[0],
+	                                                         c->b_adv[1], c->b_adv[2]);
+	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
+}
+
+int launch_face_tan(dpg_gpu_ctx* c, const double* trace_t, double* nnf_t)
+{
+	if (c->d == 2 && c->n_var == 4) return face_tan_impl<2, 4>(c, trace_t, nnf_t);
+	if (c->d == 3 && c->n_var == 5) return face_tan_impl<3, 5>(c, trace_t, nnf_t);
+	if (c->d == 2 && c->n_var == 1) return face_tan_impl<2, 1>(c, trace_t, nnf_t);
+	if (c->d == 3 && c->n_var == 1) return face_tan_impl<3, 1>(c, trace_t, nnf_t);
+	return DPG_ERR_UNSUPPORTED;
+}
+
+template <int D, int NV>
 static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t)
 {
 	const GroupDev& g = c->g;
@@ -398,10 +432,10 @@ static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* ou
 		const int grid_t = (g.n_vol + E_t - 1) / E_t;
 		k_trace<NV><<<grid_t, 256, smem_t, c->stream>>>(u, g, c->trace, E_t);
 		k_trace<NV><<<grid_t, 256, smem_t, c->stream>>>(v, g, trace_t, E_t);
+		copy_boundary_trace(c, c->trace);
+		copy_boundary_trace(c, trace_t);
 	}
-	const int n = c->fc.n_face * c->fc.n_fc;
-	k_face_tan<D, NV><<<(n + 127) / 128, 128, 0, c->stream>>>(c->trace, trace_t, c->fc, nnf_t, c->num_flux, c->b_adv[0],
-	                                                         c->b_adv[1], c->b_adv[2]);
+	if ((rc = launch_face_tan(c, trace_t, nnf_t))) return rc;
 	if (c->tp) return tp_lift_tan(c, nnf_t, out);
 	const int E_b = c->tan_block_elems;
 	const size_t smem = (size_t)E_b * NV * (2 * g.n_s + (g.n_c > g.n_s ? g.n_c : g.n_s) + g.n_c + g.K) * sizeof(double);
@@ -412,7 +446,7 @@ static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* ou
 
 int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t)
 {
-	if (c->general) return gen_jvp(c, u, v, out);
+	if (c->walls_or_visc && c->tp) return tp_general_jvp(c, u, v, out, trace_t, nnf_t);
 	if (c->d == 2 && c->n_var == 4) return jvp_impl<2, 4>(c, u, v, out, trace_t, nnf_t);
 	if (c->d == 3 && c->n_var == 5) return jvp_impl<3, 5>(c, u, v, out, trace_t, nnf_t);
 	if (c->d == 2 && c->n_var == 1) return jvp_impl<2, 1>(c, u, v, out, trace_t, nnf_t);

@@ -21,168 +21,11 @@
 
 #include "dpg_gpu_internal.cuh"
 #include "dpg_host.h"
-#include "tp_ops.cuh"
+#include "tp_volume.cuh"
 
 namespace dpg {
 
 using namespace tp;
-
-struct TpState {
-	int n1 = 0, E = 1;
-	double* G = nullptr;        // [n_vol][n_var][n1^d] weak divergence in the collocated basis
-	double* jn = nullptr;       // non-affine: [n_vol][n1^d] 1 / detJ at the Gauss points
-	double B[25], Bi[25], Dw[25], lm[5], lp[5], wm[5], wp[5];
-	std::vector<void*> allocs;
-};
-
-struct TpGeo {
-	int n_vol, affine;
-	const double* met;          // affine: [n_vol][d d]; else [n_vol][d d][n1^d]
-	const double* jinv;         // affine: [n_vol]; else [n_vol][n1^d]
-	const int* vol_face;        // [n_vol][2 d]  (face << 1) | side
-	const int* nc_inv;          // [n_face][n_fc]
-};
-
-template <int N1>
-static Ops<N1> ops_of(const TpState* st)
-{
-	Ops<N1> o;
-	for (int k = 0; k < N1 * N1; ++k) { o.B[k] = st->B[k]; o.Bi[k] = st->Bi[k]; o.Dw[k] = st->Dw[k]; }
-	for (int k = 0; k < N1; ++k) { o.lm[k] = st->lm[k]; o.lp[k] = st->lp[k]; o.wm[k] = st->wm[k]; o.wp[k] = st->wp[k]; }
-	return o;
-}
-
-// Shared memory (doubles): the operators, then two buffers of E NW N values and D - 1 of E NV N (the fluxes of direction
-// 0 reuse the buffer the last B pass read from).
-template <int D, int NV, int N1, bool TAN>
-static size_t smem_volume(int E)
-{
-	const size_t N = ipow(N1, D), NW = TAN ? 2 * NV : NV;
-	return sizeof(Ops<N1>) + sizeof(double) * E * N * (2 * NW + (D - 1) * NV);
-}
-
-template <int D, int NV, int N1, bool TAN>
-__global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g,
-                                                   const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
-                                                   double* __restrict__ trace_t, double* __restrict__ G, int E, double bx,
-                                                   double by, double bz)
-{
-	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1), NW = TAN ? 2 * NV : NV;
-	extern __shared__ double sm[];
-	Ops<N1>* so = reinterpret_cast<Ops<N1>*>(sm);
-	double* b0 = sm + sizeof(Ops<N1>) / sizeof(double);
-	double* b1 = b0 + (size_t)E * NW * N;
-	double* fl = b1 + (size_t)E * NW * N;   // [D - 1][E][NV][N]
-	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
-	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
-	const bool live = e < ne;
-	load_ops(so, ops);
-	{
-		const size_t g0 = (size_t)e0 * NV * N;
-		for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) {
-			if constexpr (TAN) {
-				const int ee = k / (NV * N), r = k - ee * NV * N;
-				b0[ee * NW * N + r] = u[g0 + k];
-				b0[ee * NW * N + NV * N + r] = v[g0 + k];
-			} else {
-				b0[k] = u[g0 + k];
-			}
-		}
-	}
-	double m[D][D];   // of this node's element (affine) or node
-	if (live) {
-#pragma unroll
-		for (int x = 0; x < D; ++x)
-#pragma unroll
-			for (int r = 0; r < D; ++r)
-				m[x][r] = g.affine ? g.met[(size_t)(e0 + e) * D * D + x + D * r]
-				                   : g.met[((size_t)(e0 + e) * D * D + x + D * r) * N + i];
-	}
-	__syncthreads();
-	// values at the Gauss points: pass 0 b0 -> b1, pass 1 b1 -> b0, (pass 2 b0 -> b1)
-	double s[NW];
-	auto pass = [&](auto tag, const double* src, double* dst) {
-		constexpr int A = decltype(tag)::value;
-		if (live) {
-			const double* row = so->B + node_along<A, N1>(i) * N1;
-			const int base = pencil_base<A, N1>(i);
-			double op[N1];
-#pragma unroll
-			for (int j = 0; j < N1; ++j) op[j] = row[j];
-#pragma unroll
-			for (int w = 0; w < NW; ++w) {
-				s[w] = pencil_dot<A, N1>(op, src + (e * NW + w) * N, base);
-				dst[(e * NW + w) * N + i] = s[w];
-			}
-		}
-		__syncthreads();
-	};
-	pass(std::integral_constant<int, 0>{}, b0, b1);
-	pass(std::integral_constant<int, 1>{}, b1, b0);
-	if constexpr (D == 3) pass(std::integral_constant<int, 2>{}, b0, b1);
-	const double* sc = D == 3 ? b1 : b0;     // the collocated values
-	double* f0 = D == 3 ? b0 : b1;           // free: the fluxes of direction 0
-	// reference fluxes of this node (TAN: their tangents)
-	if (live) {
-		const double b[3] = {bx, by, bz};
-		auto met = [&](int x, int r) { return m[x][r]; };
-		auto put = [&](int r, int w, double y) { (r == 0 ? f0 : fl + (size_t)(r - 1) * E * NV * N)[(e * NV + w) * N + i] = y; };
-		if constexpr (TAN) {
-			dual sd[NV];
-#pragma unroll
-			for (int w = 0; w < NV; ++w) sd[w] = dual(s[w], s[NV + w]);
-			ref_flux<D, NV>(sd, met, b, [&](int r, const dual (&fr)[NV]) {
-#pragma unroll
-				for (int w = 0; w < NV; ++w) put(r, w, fr[w].d);
-			});
-		} else {
-			ref_flux<D, NV>(s, met, b, [&](int r, const double (&fr)[NV]) {
-#pragma unroll
-				for (int w = 0; w < NV; ++w) put(r, w, fr[w]);
-			});
-		}
-	}
-	// traces of the local faces, in the element's own node order
-	for (int o = threadIdx.x; o < ne * 2 * D * NF; o += blockDim.x) {
-		const int ee = o / (2 * D * NF), r = o - ee * 2 * D * NF, lf = r / NF, q = r - lf * NF, a = lf >> 1;
-		const double* l = (lf & 1) ? so->lp : so->lm;
-		const int S = stride_of<N1>(a), base = face_base<N1>(a, q);
-		const size_t vf = (size_t)g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
-#pragma unroll
-		for (int w = 0; w < NW; ++w) {
-			const double* x = sc + (ee * NW + w) * N + base;
-			double acc = l[0] * x[0];
-#pragma unroll
-			for (int j = 1; j < N1; ++j) acc = fma(l[j], x[j * S], acc);
-			(w < NV ? trace : trace_t)[(vf * NV + (w < NV ? w : w - NV)) * NF + q] = acc;
-		}
-	}
-	__syncthreads();
-	// weak divergence
-	if (live) {
-		double acc[NV];
-		auto add = [&](auto tag, const double* src) {
-			constexpr int A = decltype(tag)::value;
-			const double* row = so->Dw + node_along<A, N1>(i) * N1;
-			const int base = pencil_base<A, N1>(i);
-			double op[N1];
-#pragma unroll
-			for (int j = 0; j < N1; ++j) op[j] = row[j];
-#pragma unroll
-			for (int w = 0; w < NV; ++w) {
-				const double* x = src + (e * NV + w) * N + base;
-#pragma unroll
-				for (int j = 0; j < N1; ++j)
-					acc[w] = (A == 0 && j == 0) ? op[0] * x[0] : fma(op[j], x[j * ipow(N1, A)], acc[w]);
-			}
-		};
-		add(std::integral_constant<int, 0>{}, f0);
-		add(std::integral_constant<int, 1>{}, fl);
-		if constexpr (D == 3) add(std::integral_constant<int, 2>{}, fl + (size_t)E * NV * N);
-#pragma unroll
-		for (int w = 0; w < NV; ++w) G[((size_t)(e0 + e) * NV + w) * N + i] = acc[w];
-	}
-}
 
 template <int D, int NV, int N1>
 static size_t smem_lift(int E)
@@ -306,7 +149,7 @@ static bool build_ops(TpState* st, const dpg_element_ops& o)
 		dpg_lagrange_1d(n1, gl, gll[q], val, der);   // the inverse map: the collocated basis at the solution nodes
 		for (int i = 0; i < n1; ++i) st->Bi[q * n1 + i] = val[i];
 		dpg_lagrange_1d(n1, gl, gl[q], val, der);
-		for (int i = 0; i < n1; ++i) st->Dw[i * n1 + q] = w[q] / w[i] * der[i];
+		for (int i = 0; i < n1; ++i) { st->Dw[i * n1 + q] = w[q] / w[i] * der[i]; st->Ds[q * n1 + i] = der[i]; }
 	}
 	dpg_lagrange_1d(n1, gl, -1.0, st->lm, der);
 	dpg_lagrange_1d(n1, gl, 1.0, st->lp, der);
@@ -374,7 +217,6 @@ void tp_free(dpg_gpu_ctx* c)
 }
 
 // Elements per block: as many as fill 256 threads, but no more than leave two blocks per SM, and at least a warp.
-static constexpr int most_elems(int N) { return 256 / N; }
 static int block_elems(int n_vol, int N, int n_sm)
 {
 	const int fill = (n_vol + 2 * n_sm - 1) / (2 * n_sm), warp = (31 + N) / N;
@@ -386,8 +228,8 @@ template <int D, int NV, int N1>
 static int configure()
 {
 	constexpr int E = most_elems(ipow(N1, D));
-	if (cudaFuncSetAttribute(k_tp_volume<D, NV, N1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, false>(E)) ||
-	    cudaFuncSetAttribute(k_tp_volume<D, NV, N1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, true>(E)) ||
+	if (cudaFuncSetAttribute(k_tp_volume<D, NV, N1, false, kPeriodic>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, false>(E)) ||
+	    cudaFuncSetAttribute(k_tp_volume<D, NV, N1, true, kPeriodic>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, true>(E)) ||
 	    cudaFuncSetAttribute(k_tp_lift<D, NV, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lift<D, NV, N1>(E)))
 		return DPG_ERR_CUDA;
 	return DPG_OK;
@@ -397,17 +239,16 @@ template <int D, int NV, int N1>
 static int launch_volume(dpg_gpu_ctx* c, const double* u, const double* v, double* trace, double* trace_t)
 {
 	const TpState* st = (const TpState*)c->tp;
-	const GroupDev& g = c->g;
 	constexpr int N = ipow(N1, D);
-	const TpGeo geo{g.n_vol, g.affine, g.met, g.affine ? g.jinv : st->jn, g.vol_face, g.nc_inv};
-	const int E = st->E, grid = (g.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	const TpGeo geo = geo_of(c);
+	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
 	const Ops<N1> ops = ops_of<N1>(st);
 	if (v)
-		k_tp_volume<D, NV, N1, true><<<grid, threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
-		    u, v, geo, ops, trace, trace_t, st->G, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+		k_tp_volume<D, NV, N1, true, kPeriodic><<<grid, threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
+		    u, v, geo, TpBc{}, ops, trace, trace_t, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	else
-		k_tp_volume<D, NV, N1, false><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
-		    u, nullptr, geo, ops, trace, nullptr, st->G, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+		k_tp_volume<D, NV, N1, false, kPeriodic><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
+		    u, nullptr, geo, TpBc{}, ops, trace, nullptr, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
@@ -415,31 +256,13 @@ template <int D, int NV, int N1>
 static int launch_lift(dpg_gpu_ctx* c, const double* nnf, double* rhs, unsigned long long* max_slot, int stage, bool write_rhs)
 {
 	const TpState* st = (const TpState*)c->tp;
-	const GroupDev& g = c->g;
 	constexpr int N = ipow(N1, D);
-	const TpGeo geo{g.n_vol, g.affine, g.met, g.affine ? g.jinv : st->jn, g.vol_face, g.nc_inv};
-	const int E = st->E, grid = (g.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	const TpGeo geo = geo_of(c);
+	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
 	k_tp_lift<D, NV, N1><<<grid, threads, smem_lift<D, NV, N1>(E), c->stream>>>(
 	    st->G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
-
-#define DPG_TP_N1(F, D, NV, ...)                        \
-	switch (((const TpState*)c->tp)->n1) {              \
-	case 2: return F<D, NV, 2>(__VA_ARGS__);            \
-	case 3: return F<D, NV, 3>(__VA_ARGS__);            \
-	case 4: return F<D, NV, 4>(__VA_ARGS__);            \
-	case 5: return F<D, NV, 5>(__VA_ARGS__);            \
-	default: return DPG_ERR_UNSUPPORTED;                \
-	}
-#define DPG_TP_DISPATCH(F, ...)                                             \
-	do {                                                                    \
-		if (c->d == 2 && c->n_var == 4) { DPG_TP_N1(F, 2, 4, __VA_ARGS__) } \
-		if (c->d == 3 && c->n_var == 5) { DPG_TP_N1(F, 3, 5, __VA_ARGS__) } \
-		if (c->d == 2 && c->n_var == 1) { DPG_TP_N1(F, 2, 1, __VA_ARGS__) } \
-		if (c->d == 3 && c->n_var == 1) { DPG_TP_N1(F, 3, 1, __VA_ARGS__) } \
-		return DPG_ERR_UNSUPPORTED;                                         \
-	} while (0)
 
 static int configure_any(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(configure); }
 
@@ -459,7 +282,7 @@ int tp_lift_tan(dpg_gpu_ctx* c, const double* nnf_t, double* out)
 
 // Set-up.  Leaves c->tp null (the dense kernels of kernels_fp64.cu run) where the element is not one of the orders above
 // or its operators are not the products of the 1D ones.
-int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim)
+int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 {
 	const dpg_element_ops& o = sim->ops[0];
 	if ((o.e_type != DPG_QUAD && o.e_type != DPG_HEX) || o.p < 1 || o.p + 1 > kN1Max) return DPG_OK;
@@ -469,7 +292,7 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim)
 	// with its host round trip: 68.8 us here, 68.4 us dense; QUAD p = 2, 256 elements, 2,304 nodes: 24.2 us a stage
 	// here, 33.4 us dense) and keeps the dense kernels and their summation order
 	constexpr int64_t kMinNodes = 1024;
-	if ((int64_t)sim->n_vol * N < kMinNodes) return DPG_OK;
+	if (!general && (int64_t)sim->n_vol * N < kMinNodes) return DPG_OK;
 	TpState* st = new TpState();
 	st->n1 = o.p + 1;
 	if (!build_ops(st, o)) { delete st; return DPG_OK; }

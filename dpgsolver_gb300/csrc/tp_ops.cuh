@@ -13,7 +13,10 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
+#include <vector>
 
+#include "dpg_gpu_internal.cuh"
 #include "flux.cuh"
 
 namespace dpg {
@@ -27,9 +30,80 @@ struct Ops {
 	double B[N1 * N1];     // [q][i]  GLL -> Gauss values
 	double Bi[N1 * N1];    // [i][q]  its inverse
 	double Dw[N1 * N1];    // [i][j]  weak derivative over the weights
+	double Ds[N1 * N1];    // [i][j]  l_j'(x_i)
 	double lm[N1], lp[N1]; // collocated basis at -1 and +1
 	double wm[N1], wp[N1]; // the same over the weights
 };
+
+// Host state of a tensor-product context (dpg_gpu_ctx::tp).
+struct TpState {
+	int n1 = 0, E = 1;          // order + 1, elements per block
+	double* G = nullptr;        // [n_vol][n_var][n1^d] weak divergence in the collocated basis
+	double* jn = nullptr;       // non-affine: [n_vol][n1^d] 1 / detJ at the Gauss points
+	double B[25], Bi[25], Dw[25], Ds[25], lm[5], lp[5], wm[5], wp[5];
+	// boundary faces and viscous terms (kernels_tp_general.cu)
+	int viscous = 0;
+	double mu = 0.0, kappa = 0.0, scale = 0.0;   // viscosity, gamma mu / Pr, BR2 penalty 1.01 NFMAX
+	BcParams bp{};
+	const int* bc = nullptr;    // [n_face] 0 or the boundary code; null without boundary faces
+	const double* xyz = nullptr;// [n_face][n_fc][d]
+	double* Uc = nullptr;       // viscous: [n_dof] collocated values, their tangents (allocated on first use)
+	double* Uc_t = nullptr;
+	double* fvn = nullptr;      // viscous: [n_face][2][n_var][n_fc] normal second-order flux of each side, or its tangent
+	std::vector<void*> allocs;
+};
+
+struct TpGeo {
+	int n_vol, affine;
+	const double* met;          // affine: [n_vol][d d]; else [n_vol][d d][n1^d]
+	const double* jinv;         // affine: [n_vol]; else [n_vol][n1^d]
+	const int* vol_face;        // [n_vol][2 d]  (face << 1) | side
+	const int* nc_inv;          // [n_face][n_fc]
+};
+
+// What boundary faces add: their codes and the positions and normals of the face nodes.
+struct TpBc {
+	const int* bc;
+	const double* xyz;
+	const double* nrm;
+	BcParams bp;
+};
+
+template <int N1>
+inline Ops<N1> ops_of(const TpState* st)
+{
+	Ops<N1> o;
+	for (int k = 0; k < N1 * N1; ++k) { o.B[k] = st->B[k]; o.Bi[k] = st->Bi[k]; o.Dw[k] = st->Dw[k]; o.Ds[k] = st->Ds[k]; }
+	for (int k = 0; k < N1; ++k) { o.lm[k] = st->lm[k]; o.lp[k] = st->lp[k]; o.wm[k] = st->wm[k]; o.wp[k] = st->wp[k]; }
+	return o;
+}
+
+inline TpGeo geo_of(const dpg_gpu_ctx* c)
+{
+	const TpState* st = (const TpState*)c->tp;
+	const GroupDev& g = c->g;
+	return TpGeo{g.n_vol, g.affine, g.met, g.affine ? g.jinv : st->jn, g.vol_face, g.nc_inv};
+}
+
+constexpr int most_elems(int N) { return 256 / N; }   // elements per block: at most 256 threads of one node each
+
+// A launch of a kernel of <D, NV, N1> by the context's sizes.
+#define DPG_TP_N1(F, D, NV, ...)                        \
+	switch (((const TpState*)c->tp)->n1) {              \
+	case 2: return F<D, NV, 2>(__VA_ARGS__);            \
+	case 3: return F<D, NV, 3>(__VA_ARGS__);            \
+	case 4: return F<D, NV, 4>(__VA_ARGS__);            \
+	case 5: return F<D, NV, 5>(__VA_ARGS__);            \
+	default: return DPG_ERR_UNSUPPORTED;                \
+	}
+#define DPG_TP_DISPATCH(F, ...)                                             \
+	do {                                                                    \
+		if (c->d == 2 && c->n_var == 4) { DPG_TP_N1(F, 2, 4, __VA_ARGS__) } \
+		if (c->d == 3 && c->n_var == 5) { DPG_TP_N1(F, 3, 5, __VA_ARGS__) } \
+		if (c->d == 2 && c->n_var == 1) { DPG_TP_N1(F, 2, 1, __VA_ARGS__) } \
+		if (c->d == 3 && c->n_var == 1) { DPG_TP_N1(F, 3, 1, __VA_ARGS__) } \
+		return DPG_ERR_UNSUPPORTED;                                         \
+	} while (0)
 
 template <int N1>
 __device__ __forceinline__ void load_ops(Ops<N1>* s, const Ops<N1>& p)

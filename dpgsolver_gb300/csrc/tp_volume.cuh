@@ -1,0 +1,177 @@
+// First kernel of the tensor-product residual (kernels_tp.cu, kernels_tp_general.cu): one thread per (element, node).
+#pragma once
+
+#include "tp_ops.cuh"
+
+namespace dpg {
+namespace tp {
+
+// Shared memory (doubles): the operators, then two buffers of E NW N values and D - 1 of E NV N (the fluxes of direction
+// 0 reuse the buffer the last B pass read from).
+template <int D, int NV, int N1, bool TAN>
+inline size_t smem_volume(int E)
+{
+	const size_t N = ipow(N1, D), NW = TAN ? 2 * NV : NV;
+	return sizeof(Ops<N1>) + sizeof(double) * E * N * (2 * NW + (D - 1) * NV);
+}
+
+// kPeriodic: every face has two elements.  kWalls: the boundary states of boundary faces go to their side-1 trace slots.
+// kViscous: kWalls, and the collocated values (G, G_t) instead of the weak divergence, which needs the gradients.
+enum { kPeriodic = 0, kWalls = 1, kViscous = 2 };
+
+template <int D, int NV, int N1, bool TAN, int KIND>
+__global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g, TpBc B,
+                                                   const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
+                                                   double* __restrict__ trace_t, double* __restrict__ G,
+                                                   double* __restrict__ G_t, int E, double bx, double by, double bz)
+{
+	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1), NW = TAN ? 2 * NV : NV;
+	extern __shared__ double sm[];
+	Ops<N1>* so = reinterpret_cast<Ops<N1>*>(sm);
+	double* b0 = sm + sizeof(Ops<N1>) / sizeof(double);
+	double* b1 = b0 + (size_t)E * NW * N;
+	double* fl = b1 + (size_t)E * NW * N;   // [D - 1][E][NV][N]
+	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
+	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
+	const bool live = e < ne;
+	load_ops(so, ops);
+	{
+		const size_t g0 = (size_t)e0 * NV * N;
+		for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) {
+			if constexpr (TAN) {
+				const int ee = k / (NV * N), r = k - ee * NV * N;
+				b0[ee * NW * N + r] = u[g0 + k];
+				b0[ee * NW * N + NV * N + r] = v[g0 + k];
+			} else {
+				b0[k] = u[g0 + k];
+			}
+		}
+	}
+	double m[D][D];   // of this node's element (affine) or node
+	if (KIND != kViscous && live) {
+#pragma unroll
+		for (int x = 0; x < D; ++x)
+#pragma unroll
+			for (int r = 0; r < D; ++r)
+				m[x][r] = g.affine ? g.met[(size_t)(e0 + e) * D * D + x + D * r]
+				                   : g.met[((size_t)(e0 + e) * D * D + x + D * r) * N + i];
+	}
+	__syncthreads();
+	// values at the Gauss points: pass 0 b0 -> b1, pass 1 b1 -> b0, (pass 2 b0 -> b1)
+	double s[NW];
+	auto pass = [&](auto tag, const double* src, double* dst) {
+		constexpr int A = decltype(tag)::value;
+		if (live) {
+			const double* row = so->B + node_along<A, N1>(i) * N1;
+			const int base = pencil_base<A, N1>(i);
+			double op[N1];
+#pragma unroll
+			for (int j = 0; j < N1; ++j) op[j] = row[j];
+#pragma unroll
+			for (int w = 0; w < NW; ++w) {
+				s[w] = pencil_dot<A, N1>(op, src + (e * NW + w) * N, base);
+				dst[(e * NW + w) * N + i] = s[w];
+			}
+		}
+		__syncthreads();
+	};
+	pass(std::integral_constant<int, 0>{}, b0, b1);
+	pass(std::integral_constant<int, 1>{}, b1, b0);
+	if constexpr (D == 3) pass(std::integral_constant<int, 2>{}, b0, b1);
+	const double* sc = D == 3 ? b1 : b0;     // the collocated values
+	double* f0 = D == 3 ? b0 : b1;           // free: the fluxes of direction 0
+	if (KIND == kViscous && live) {
+#pragma unroll
+		for (int w = 0; w < NW; ++w)
+			(w < NV ? G : G_t)[((size_t)(e0 + e) * NV + (w < NV ? w : w - NV)) * N + i] = s[w];
+	}
+	// reference fluxes of this node (TAN: their tangents)
+	if (KIND != kViscous && live) {
+		const double b[3] = {bx, by, bz};
+		auto met = [&](int x, int r) { return m[x][r]; };
+		auto put = [&](int r, int w, double y) { (r == 0 ? f0 : fl + (size_t)(r - 1) * E * NV * N)[(e * NV + w) * N + i] = y; };
+		if constexpr (TAN) {
+			dual sd[NV];
+#pragma unroll
+			for (int w = 0; w < NV; ++w) sd[w] = dual(s[w], s[NV + w]);
+			ref_flux<D, NV>(sd, met, b, [&](int r, const dual (&fr)[NV]) {
+#pragma unroll
+				for (int w = 0; w < NV; ++w) put(r, w, fr[w].d);
+			});
+		} else {
+			ref_flux<D, NV>(s, met, b, [&](int r, const double (&fr)[NV]) {
+#pragma unroll
+				for (int w = 0; w < NV; ++w) put(r, w, fr[w]);
+			});
+		}
+	}
+	// traces of the local faces, in the element's own node order
+	for (int o = threadIdx.x; o < ne * 2 * D * NF; o += blockDim.x) {
+		const int ee = o / (2 * D * NF), r = o - ee * 2 * D * NF, lf = r / NF, q = r - lf * NF, a = lf >> 1;
+		const double* l = (lf & 1) ? so->lp : so->lm;
+		const int S = stride_of<N1>(a), base = face_base<N1>(a, q);
+		const size_t vf = (size_t)g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
+		double tr[NW];
+#pragma unroll
+		for (int w = 0; w < NW; ++w) {
+			const double* x = sc + (ee * NW + w) * N + base;
+			tr[w] = l[0] * x[0];
+#pragma unroll
+			for (int j = 1; j < N1; ++j) tr[w] = fma(l[j], x[j * S], tr[w]);
+			(w < NV ? trace : trace_t)[(vf * NV + (w < NV ? w : w - NV)) * NF + q] = tr[w];
+		}
+		if constexpr (KIND != kPeriodic) {
+			const size_t f = vf >> 1;
+			const int code = B.bc ? B.bc[f] : 0;
+			if (code) {   // the only side of a boundary face: its nodes are in this order
+				double n[D], x[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+				for (int k = 0; k < D; ++k) { n[k] = B.nrm[(f * NF + q) * D + k]; x[k] = B.xyz[(f * NF + q) * D + k]; }
+				using T = typename std::conditional<TAN, dual, double>::type;
+				T sl[NV], sb[NV];
+#pragma unroll
+				for (int w = 0; w < NV; ++w) {
+					if constexpr (TAN) sl[w] = dual(tr[w], tr[NV + w]);
+					else sl[w] = tr[w];
+				}
+				if constexpr (NV == D + 2) boundary_state<D>(code, sl, n, x, B.bp, sb);
+				else sb[0] = sl[0];
+#pragma unroll
+				for (int w = 0; w < NV; ++w) {
+					const size_t k = ((vf + 1) * NV + w) * NF + q;
+					if constexpr (TAN) { trace[k] = sb[w].v; trace_t[k] = sb[w].d; }
+					else trace[k] = sb[w];
+				}
+			}
+		}
+	}
+	if constexpr (KIND == kViscous) return;
+	__syncthreads();
+	// weak divergence
+	if (live) {
+		double acc[NV];
+		auto add = [&](auto tag, const double* src) {
+			constexpr int A = decltype(tag)::value;
+			const double* row = so->Dw + node_along<A, N1>(i) * N1;
+			const int base = pencil_base<A, N1>(i);
+			double op[N1];
+#pragma unroll
+			for (int j = 0; j < N1; ++j) op[j] = row[j];
+#pragma unroll
+			for (int w = 0; w < NV; ++w) {
+				const double* x = src + (e * NV + w) * N + base;
+#pragma unroll
+				for (int j = 0; j < N1; ++j)
+					acc[w] = (A == 0 && j == 0) ? op[0] * x[0] : fma(op[j], x[j * ipow(N1, A)], acc[w]);
+			}
+		};
+		add(std::integral_constant<int, 0>{}, f0);
+		add(std::integral_constant<int, 1>{}, fl);
+		if constexpr (D == 3) add(std::integral_constant<int, 2>{}, fl + (size_t)E * NV * N);
+#pragma unroll
+		for (int w = 0; w < NV; ++w) G[((size_t)(e0 + e) * NV + w) * N + i] = acc[w];
+	}
+}
+
+} // namespace tp
+} // namespace dpg

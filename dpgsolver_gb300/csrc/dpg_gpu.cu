@@ -127,6 +127,7 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	for (int a = 0; a < 3; ++a) c->b_adv[a] = sim->b_adv[a];
 	const int n_vol = sim->n_vol, n_face = sim->n_face;
 	c->n_dof = sim->vol_dof_off[n_vol];
+	if (cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, c->dev) != cudaSuccess || c->n_sm < 1) c->n_sm = 1;
 
 	int affine_all = 1;
 	for (int v = 0; v < n_vol; ++v) affine_all &= sim->vol_affine[v];
@@ -303,6 +304,7 @@ extern "C" void dpg_gpu_destroy(dpg_gpu_ctx* c)
 	dpg::hp_free(c);
 	dpg::implicit_free(c);
 	dpg::mlp_free(c);
+	dpg::free_tangent_work(&c->tan);
 	if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
 	for (int i = 0; i < c->n_allocs; ++i) cudaFree(c->allocs[i]);
 	if (c->stream) cudaStreamDestroy(c->stream);
@@ -655,14 +657,42 @@ extern "C" void dpg_newton_params_default(struct dpg_newton_params* p)
 }
 
 namespace dpg {
-// work buffers of the linearisation (tangents of the traces and face fluxes), allocated on first use
-int ensure_tangent_buffers(dpg_gpu_ctx* c)
+TanStride tan_stride(const dpg_gpu_ctx* c)
 {
-	if (c->trace_t && c->nnf_t) return DPG_OK;
-	int rc;
-	if ((rc = dalloc(c, &c->trace_t, (size_t)c->fc.n_face * 2 * c->n_var * c->fc.n_fc))) return rc;
-	return dalloc(c, &c->nnf_t, (size_t)c->fc.n_face * c->n_var * c->fc.n_fc);
+	const size_t nf = (size_t)c->fc.n_face * c->n_var * c->fc.n_fc;
+	return TanStride{(size_t)c->n_dof, 2 * nf, nf};
 }
+
+size_t tangent_bytes(const dpg_gpu_ctx* c)
+{
+	const TanStride s = tan_stride(c);
+	const bool visc = c->tp && tp_viscous(c);
+	return sizeof(double) * (s.tr + s.nf + (c->tp ? s.dof : 0) + (visc ? s.dof + s.tr : 0));
+}
+
+// work buffers of the linearisation for nb directions
+int alloc_tangent_work(dpg_gpu_ctx* c, int nb, TanWork* w)
+{
+	const TanStride s = tan_stride(c);
+	const bool visc = c->tp && tp_viscous(c);
+	auto al = [&](double** p, size_t n) { return cudaMalloc((void**)p, (size_t)nb * n * sizeof(double)) == cudaSuccess; };
+	if (!al(&w->trace_t, s.tr) || !al(&w->nnf_t, s.nf) || (c->tp && !al(&w->G, s.dof)) ||
+	    (visc && (!al(&w->Uc_t, s.dof) || !al(&w->fvn, s.tr)))) {
+		free_tangent_work(w);
+		return DPG_ERR_CUDA;
+	}
+	w->nb = nb;
+	return DPG_OK;
+}
+
+void free_tangent_work(TanWork* w)
+{
+	for (double* p : {w->trace_t, w->nnf_t, w->G, w->Uc_t, w->fvn})
+		if (p) cudaFree(p);
+	*w = TanWork{};
+}
+
+int ensure_tangent_buffers(dpg_gpu_ctx* c) { return c->tan.nb ? DPG_OK : alloc_tangent_work(c, 1, &c->tan); }
 } // namespace dpg
 
 extern "C" int dpg_gpu_jacobian_apply(dpg_gpu_ctx* c, const double* v, double* jv)
@@ -677,7 +707,7 @@ extern "C" int dpg_gpu_jacobian_apply(dpg_gpu_ctx* c, const double* v, double* j
 	if (cudaMalloc(&dj, bytes) != cudaSuccess) { cudaFree(dv); return DPG_ERR_CUDA; }
 	rc = DPG_OK;
 	if (cudaMemcpyAsync(dv, v, bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess) rc = DPG_ERR_CUDA;
-	if (!rc) rc = dpg::jvp_fp64(c, c->sol, dv, dj, c->trace_t, c->nnf_t);
+	if (!rc) rc = dpg::jvp_fp64(c, c->sol, dv, dj, c->tan);
 	if (!rc && cudaMemcpyAsync(jv, dj, bytes, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) rc = DPG_ERR_CUDA;
 	if (cudaStreamSynchronize(c->stream) != cudaSuccess && !rc) rc = DPG_ERR_CUDA;
 	cudaFree(dv);

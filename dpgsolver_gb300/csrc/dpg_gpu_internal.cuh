@@ -33,6 +33,21 @@ struct FaceDev {
 	const int* nc;         // [n_face][n_fc]
 };
 
+// Work space of the linearisation for nb directions at once (their arrays one after another).
+struct TanWork {
+	int nb = 0;
+	double* trace_t = nullptr;  // [nb][n_face][2][n_var][n_fc] tangents of the traces
+	double* nnf_t = nullptr;    // [nb][n_face][n_var][n_fc]    tangents of the face fluxes
+	double* G = nullptr;        // tensor-product meshes: [nb][n_dof] weak divergence
+	double* Uc_t = nullptr;     // viscous: [nb][n_dof] collocated tangents
+	double* fvn = nullptr;      // viscous: [nb][n_face][2][n_var][n_fc]
+};
+
+// Strides between the directions of a launch (blockIdx.y): state-sized arrays, traces, face fluxes.
+struct TanStride {
+	size_t dof = 0, tr = 0, nf = 0;
+};
+
 } // namespace dpg
 
 struct dpg_gpu_ctx {
@@ -68,11 +83,11 @@ struct dpg_gpu_ctx {
 	cudaGraphExec_t step_graph = nullptr;
 	int step_graph_mode = -1;
 
+	int n_sm = 1;
 	int vol_block_elems = 1;
 	int trace_block_elems = 1;
 	int tan_block_elems = 1;     // elements per block of the linearisation's volume kernel
-	double* trace_t = nullptr;   // tangent of the traces (allocated on the first Jacobian-vector product)
-	double* nnf_t = nullptr;     // tangent of the face fluxes
+	dpg::TanWork tan;            // one direction (allocated on the first Jacobian-vector product)
 
 	// positivity of density and pressure (Euler): limiter after every RK stage and Newton update (positivity.cu)
 	int positivity = 0;          // on by default for Euler, as the reference's test_case_requires_positivity
@@ -111,24 +126,29 @@ struct dpg_gpu_ctx {
 namespace dpg {
 int launch_trace (dpg_gpu_ctx* c);
 int launch_face  (dpg_gpu_ctx* c);
-int launch_face_tan(dpg_gpu_ctx* c, const double* trace_t, double* nnf_t);   // tangents of the face fluxes
+int launch_face_tan(dpg_gpu_ctx* c, const TanWork& w);   // tangents of the face fluxes
+TanStride tan_stride(const dpg_gpu_ctx* c);
 int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
-// J v = d(m_inv rhs)/du . v at u (FP64 formulas, forward-mode tangents); trace_t, nnf_t: work buffers of the sizes
-// of the traces and face fluxes.
-int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t);
-int ensure_tangent_buffers(dpg_gpu_ctx* c);
+// J v = d(m_inv rhs)/du . v at u (FP64 formulas, forward-mode tangents) for w.nb directions v[nb][n_dof] -> out[nb][n_dof]
+// in one set of launches.
+int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w);
+int ensure_tangent_buffers(dpg_gpu_ctx* c);             // c->tan
+size_t tangent_bytes(const dpg_gpu_ctx* c);             // of a TanWork, per direction
+int alloc_tangent_work(dpg_gpu_ctx* c, int nb, TanWork* w);
+void free_tangent_work(TanWork* w);
 
 // tensor-product elements (kernels_tp.cu): traces and weak divergence, then lift, stage and norm; the tangents of the
 // linearisation.  tp_prepare leaves c->tp null where the dense kernels run.
 int  tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general);
 int  tp_volume(dpg_gpu_ctx* c);
 int  tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
-int  tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t);
-int  tp_lift_tan(dpg_gpu_ctx* c, const double* nnf_t, double* out);
+int  tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork& w);
+int  tp_lift_tan(dpg_gpu_ctx* c, const TanWork& w, double* out);
+bool tp_viscous(const dpg_gpu_ctx* c);
 void tp_free(dpg_gpu_ctx* c);
 int  tp_general_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);   // boundary faces, BR2 (after tp_prepare)
 int  tp_general_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
-int  tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t);
+int  tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w);
 int  tp_general_launches(dpg_gpu_ctx* c);
 
 // mixed orders (kernels_hp.cu): FP64 residual over volume groups of each order; which = 0 traces, 1 face fluxes,

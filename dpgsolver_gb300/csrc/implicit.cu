@@ -193,6 +193,41 @@ __global__ void k_extract_column(int n_vol, int nb, const double* __restrict__ F
 	}
 }
 
+// Probe directions p0 .. p0 + gridDim.y - 1 of the tangent probing, V[b][n]: probe p = colour * nb + j is e_j on every
+// element of the colour.
+__global__ void k_probe_directions(int n_vol, int nb, const int* __restrict__ colour, int p0, double* __restrict__ V)
+{
+	const int64_t n = (int64_t)n_vol * nb;
+	const int col = (p0 + (int)blockIdx.y) / nb, j = (p0 + (int)blockIdx.y) % nb;
+	double* dst = V + blockIdx.y * n;
+	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+		const int e = (int)(i / nb), k = (int)(i - (int64_t)e * nb);
+		dst[i] = (k == j && colour[e] == col) ? 1.0 : 0.0;
+	}
+}
+
+// The block columns of those probes from their products JV[b][n] (nbr null: diagonal blocks only)
+__global__ void k_extract_probes(int n_vol, int nb, int n_fl, const double* __restrict__ JV, const int* __restrict__ colour,
+                                 const int* __restrict__ nbr, int p0, const double* __restrict__ shift,
+                                 double* __restrict__ diag, double* __restrict__ offd)
+{
+	const int64_t n = (int64_t)n_vol * nb;
+	const int col = (p0 + (int)blockIdx.y) / nb, j = (p0 + (int)blockIdx.y) % nb;
+	const double* src = JV + blockIdx.y * n;
+	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+		const int e = (int)(i / nb), k = (int)(i - (int64_t)e * nb);
+		if (colour[e] == col) {
+			diag[((int64_t)e * nb + k) * nb + j] = (k == j ? shift[e] : 0.0) - src[i];
+			continue;
+		}
+		if (!nbr) continue;
+		for (int s = 0; s < n_fl; ++s) {
+			const int o = nbr[e * n_fl + s];
+			if (o >= 0 && colour[o] == col) offd[(((int64_t)e * n_fl + s) * nb + k) * nb + j] = -src[i];
+		}
+	}
+}
+
 // every element's 1/dtau_e: one value for all
 __global__ void k_fill(int n, double v, double* __restrict__ out)
 {
@@ -743,7 +778,8 @@ struct Implicit {
 	double* forcing = nullptr;    // subtracted from F (nullptr: none)
 	double rho = 0.0;             // mean inf-norm of the element blocks of dF/du (last assembly)
 	double* forcing_buf = nullptr;
-	double* zero = nullptr;       // [n] zeros (tangent probing)
+	TanWork probe;                // tangent probing: work space of a batch of directions,
+	double *pV = nullptr, *pJV = nullptr;   // [probe.nb][n] the directions and their products
 	double* inv_dtau = nullptr;   // [n_vol] 1/dtau_e of the current Newton step
 	bool blocks_valid = false;
 	bool tangent = true;          // Jacobian products by the analytic linearisation (false: finite differences)
@@ -787,9 +823,7 @@ static Implicit* implicit_state(dpg_gpu_ctx* c, int m)
 	al((void**)&im->blocks, (size_t)c->g.n_vol * im->nb * im->nb * 8);
 	al((void**)&im->piv, (size_t)c->g.n_vol * im->nb * 4); al((void**)&im->info, 4);
 	al((void**)&im->colour, (size_t)c->g.n_vol * 4);
-	al((void**)&im->zero, n * 8);
 	al((void**)&im->inv_dtau, (size_t)c->g.n_vol * 8);
-	if (ok && cudaMemset(im->zero, 0, n * 8) != cudaSuccess) ok = false;
 	c->implicit = im;
 	if (!ok) { implicit_free(c); return nullptr; }
 	// greedy element colouring: face neighbours get different colours
@@ -819,10 +853,11 @@ void implicit_free(dpg_gpu_ctx* c)
 	Implicit* im = (Implicit*)c->implicit;
 	if (!im) return;
 	void* ptrs[] = {im->u, im->F0, im->F1, im->up, im->du, im->w, im->V, im->Z, im->h, im->h2, im->partial,
-	                im->blocks, im->piv, im->info, im->colour, im->forcing_buf, im->zero, im->colour2, im->nbr,
+	                im->blocks, im->piv, im->info, im->colour, im->forcing_buf, im->pV, im->pJV, im->colour2, im->nbr,
 	                im->rank, im->level_elems, im->offd, im->wbuf, im->inv_dtau, im->ilu_in, im->ilu_out};
 	if (im->ilu_graph) cudaGraphExecDestroy(im->ilu_graph);
 	for (void* p : ptrs) if (p) cudaFree(p);
+	free_tangent_work(&im->probe);
 	if (im->hcol_host) cudaFreeHost(im->hcol_host);
 	delete im;
 	c->implicit = nullptr;
@@ -863,6 +898,34 @@ static int multidot(dpg_gpu_ctx* c, Implicit* im, int nv, const double* V, const
 	return DPG_OK;
 }
 
+// Block columns by tangent probing: the directions of all (colour, column) pairs are independent, so they go through the
+// linearisation's launches in batches (an 8x8 QUAD p = 2 mesh has 396 probes of ~60 us each one after another, bound by
+// the launch chain on 4 blocks; all of them at once take ~1 ms).  nbr null: diagonal blocks only.
+constexpr size_t kProbeBytes = (size_t)512 << 20;   // work space of a batch, kept with the implicit state
+
+static int probe_blocks(dpg_gpu_ctx* c, Implicit* im, const int* colour, int n_colours, const int* nbr, double* diag, double* offd)
+{
+	const int nb = im->nb, n_vol = c->g.n_vol, n_probes = n_colours * nb;
+	int rc;
+	if (!im->probe.nb) {
+		const size_t per = tangent_bytes(c) + 2 * sizeof(double) * im->n;
+		const int most = (int)std::max<size_t>(1, std::min<size_t>(kProbeBytes / per, (size_t)n_probes));
+		if ((rc = alloc_tangent_work(c, most, &im->probe))) return rc;
+		if (cudaMalloc((void**)&im->pV, (size_t)most * im->n * 8) != cudaSuccess ||
+		    cudaMalloc((void**)&im->pJV, (size_t)most * im->n * 8) != cudaSuccess)
+			return DPG_ERR_CUDA;
+	}
+	for (int p0 = 0; p0 < n_probes; p0 += im->probe.nb) {
+		TanWork w = im->probe;
+		w.nb = std::min(im->probe.nb, n_probes - p0);
+		const dim3 grid((unsigned)std::min<int64_t>((im->n + 255) / 256, 1216), w.nb);
+		k_probe_directions<<<grid, 256, 0, c->stream>>>(n_vol, nb, colour, p0, im->pV);
+		if ((rc = jvp_fp64(c, im->u, im->pV, im->pJV, w))) return rc;
+		k_extract_probes<<<grid, 256, 0, c->stream>>>(n_vol, nb, c->g.n_fl, im->pJV, colour, nbr, p0, im->inv_dtau, diag, offd);
+	}
+	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
+}
+
 static int assemble_block_jacobi(dpg_gpu_ctx* c, Implicit* im, const double* F0)
 {
 	const int nb = im->nb, n_vol = c->g.n_vol;
@@ -870,19 +933,13 @@ static int assemble_block_jacobi(dpg_gpu_ctx* c, Implicit* im, const double* F0)
 	int rc;
 	// block column j of every element of one colour at once (no two face neighbours share a colour): the tangent
 	// along e_j on those elements (exact), or a forward difference of the residual
-	for (int col = 0; col < im->n_colours; ++col)
+	if (im->tangent && (rc = probe_blocks(c, im, im->colour, im->n_colours, nullptr, im->blocks, nullptr))) return rc;
+	for (int col = 0; col < im->n_colours && !im->tangent; ++col)
 		for (int j = 0; j < nb; ++j) {
-			if (im->tangent) {
-				k_perturb<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->zero, im->up, im->colour, col, j, 1.0);
-				if ((rc = jvp_fp64(c, im->u, im->up, im->F1, c->trace_t, c->nnf_t))) return rc;
-				k_extract_column<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->F1, im->zero, im->colour, col, j,
-				                                                          1.0, im->inv_dtau, im->blocks);
-			} else {
-				k_perturb<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->u, im->up, im->colour, col, j, eps);
-				if ((rc = residual(c, im->up, im->F1))) return rc;
-				k_extract_column<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->F1, F0, im->colour, col, j,
-				                                                          1.0 / eps, im->inv_dtau, im->blocks);
-			}
+			k_perturb<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->u, im->up, im->colour, col, j, eps);
+			if ((rc = residual(c, im->up, im->F1))) return rc;
+			k_extract_column<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->F1, F0, im->colour, col, j,
+			                                                          1.0 / eps, im->inv_dtau, im->blocks);
 		}
 	{
 		k_block_norm_partial<<<kRedBlocks, kRedThreads, 0, c->stream>>>(n_vol, nb, im->blocks, im->inv_dtau, im->partial);
@@ -1077,21 +1134,14 @@ static int assemble_block_ilu(dpg_gpu_ctx* c, Implicit* im, const double* F0)
 	const double eps = 1e-7;
 	int rc;
 	im->ilu_valid = false;
-	for (int col = 0; col < im->n_colours2; ++col)
+	if (im->tangent && (rc = probe_blocks(c, im, im->colour2, im->n_colours2, im->nbr, im->blocks, im->offd))) return rc;
+	for (int col = 0; col < im->n_colours2 && !im->tangent; ++col)
 		for (int j = 0; j < nb; ++j) {
-			if (im->tangent) {
-				k_perturb<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->zero, im->up, im->colour2, col, j, 1.0);
-				if ((rc = jvp_fp64(c, im->u, im->up, im->F1, c->trace_t, c->nnf_t))) return rc;
-				k_extract_ilu<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, n_fl, im->F1, im->zero, im->colour2,
-				                                                       im->nbr, col, j, 1.0, im->inv_dtau, im->blocks,
-				                                                       im->offd);
-			} else {
-				k_perturb<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->u, im->up, im->colour2, col, j, eps);
-				if ((rc = residual(c, im->up, im->F1))) return rc;
-				k_extract_ilu<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, n_fl, im->F1, F0, im->colour2,
-				                                                       im->nbr, col, j, 1.0 / eps, im->inv_dtau,
-				                                                       im->blocks, im->offd);
-			}
+			k_perturb<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, im->u, im->up, im->colour2, col, j, eps);
+			if ((rc = residual(c, im->up, im->F1))) return rc;
+			k_extract_ilu<<<grid_for(im->n), 256, 0, c->stream>>>(n_vol, nb, n_fl, im->F1, F0, im->colour2,
+			                                                       im->nbr, col, j, 1.0 / eps, im->inv_dtau,
+			                                                       im->blocks, im->offd);
 		}
 	if (cudaMemsetAsync(im->info, 0, 4, c->stream) != cudaSuccess) return DPG_ERR_CUDA;
 	const size_t smem = 2 * (size_t)nb * nb * 8 + (size_t)nb * 4;
@@ -1139,7 +1189,7 @@ static int apply_precond(dpg_gpu_ctx* c, Implicit* im, int precond, const double
 static int apply_A(dpg_gpu_ctx* c, Implicit* im, const double* z, double* out, double u_norm, double z_norm)
 {
 	if (im->tangent) {
-		int rc = jvp_fp64(c, im->u, z, im->F1, c->trace_t, c->nnf_t);
+		int rc = jvp_fp64(c, im->u, z, im->F1, c->tan);
 		if (rc) return rc;
 		k_shift_minus<<<grid_for(im->n), 256, 0, c->stream>>>(im->n, im->nb, im->inv_dtau, z, im->F1, out);
 		return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;

@@ -12,6 +12,7 @@
 //               stage update of the element (time_step_ssp_rk_33, solve_explicit.c:252-301).
 // Each element's residual is assembled by exactly one thread block in a fixed order: the face-to-element sums are
 // deterministic and use no atomics.  The only atomic is the order-independent max of ||rhs||_inf.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -28,9 +29,12 @@ __device__ __forceinline__ void atomic_max_abs(unsigned long long* slot, double 
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, GroupDev g, double* __restrict__ trace, int E_b)
+__global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, GroupDev g, double* __restrict__ trace, int E_b,
+                                               TanStride st)
 {
 	extern __shared__ double sm[];
+	sol += blockIdx.y * st.dof;
+	trace += blockIdx.y * st.tr;
 	const int n_s = g.n_s, n_fl = g.n_fl, n_fc = g.n_fc;
 	const int e0 = blockIdx.x * E_b;
 	const int ne = min(E_b, g.n_vol - e0);
@@ -53,18 +57,20 @@ __global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, G
 }
 
 // Advection with boundary faces: the boundary state is the interior trace (NV = 1).
-__global__ void __launch_bounds__(128) k_copy_boundary_trace(const int* __restrict__ bface, int n, int n_fc, double* __restrict__ trace)
+__global__ void __launch_bounds__(128) k_copy_boundary_trace(const int* __restrict__ bface, int n, int n_fc, double* __restrict__ trace,
+                                                             size_t stride)
 {
+	trace += blockIdx.y * stride;
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= n * n_fc) return;
 	const size_t f = (size_t)bface[t / n_fc];
 	trace[(2 * f + 1) * n_fc + t % n_fc] = trace[2 * f * n_fc + t % n_fc];
 }
 
-static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace)
+static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace, int nb = 1, size_t stride = 0)
 {
 	const int n = c->n_bface * c->fc.n_fc;
-	if (n) k_copy_boundary_trace<<<(n + 127) / 128, 128, 0, c->stream>>>(c->bface, c->n_bface, c->fc.n_fc, trace);
+	if (n) k_copy_boundary_trace<<<dim3((n + 127) / 128, nb), 128, 0, c->stream>>>(c->bface, c->n_bface, c->fc.n_fc, trace, stride);
 }
 
 template <int D, int NV>
@@ -215,22 +221,29 @@ __global__ void __launch_bounds__(256) k_volume(double* __restrict__ sol, double
 	if ((threadIdx.x & 31) == 0) atomic_max_abs(max_slot, lmax);
 }
 
+// Elements per block of a launch over nb copies of the mesh: the most that the shared memory takes, but no more than
+// leave every SM a block (one direction of a 64-element QUAD p = 2 mesh: k_volume_tan 21 us on 4 blocks of 16).
+static int elems_of(const dpg_gpu_ctx* c, int most, int nb)
+{
+	return std::max(1, (int)std::min<int64_t>(most, ((int64_t)c->g.n_vol * nb + c->n_sm - 1) / c->n_sm));
+}
+
 template <int D, int NV>
 static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsigned long long* max_slot)
 {
 	const GroupDev& g = c->g;
 	if (which == 0) {
-		const int E_b = c->trace_block_elems;
+		const int E_b = elems_of(c, c->trace_block_elems, 1);
 		const size_t smem = (size_t)E_b * NV * g.n_s * sizeof(double);
 		const int grid = (g.n_vol + E_b - 1) / E_b;
-		k_trace<NV><<<grid, 256, smem, c->stream>>>(c->sol, g, c->trace, E_b);
+		k_trace<NV><<<grid, 256, smem, c->stream>>>(c->sol, g, c->trace, E_b, TanStride{});
 		copy_boundary_trace(c, c->trace);
 	} else if (which == 1) {
 		const int n = c->fc.n_face * c->fc.n_fc;
 		k_face<D, NV><<<(n + 127) / 128, 128, 0, c->stream>>>(c->trace, c->fc, c->nnf, c->num_flux,
 		                                                     c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	} else {
-		const int E_b = c->vol_block_elems;
+		const int E_b = elems_of(c, c->vol_block_elems, 1);
 		const size_t smem = (size_t)E_b * NV * (g.n_s + (g.n_c > g.n_s ? g.n_c : g.n_s) + g.K) * sizeof(double);
 		const int grid = (g.n_vol + E_b - 1) / E_b;
 		k_volume<D, NV><<<grid, 256, smem, c->stream>>>(c->sol, c->solp, c->rhs, c->nnf, g, c->ddt, max_slot, stage,
@@ -267,8 +280,10 @@ int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long*
 template <int D, int NV>
 __global__ void __launch_bounds__(256) k_face_tan(const double* __restrict__ trace, const double* __restrict__ trace_t,
                                                   FaceDev fd, double* __restrict__ nnf_t, int num_flux, double bx,
-                                                  double by, double bz)
+                                                  double by, double bz, TanStride st)
 {
+	trace_t += blockIdx.y * st.tr;
+	nnf_t += blockIdx.y * st.nf;
 	const int n_fc = fd.n_fc;
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= fd.n_face * n_fc) return;
@@ -299,9 +314,12 @@ __global__ void __launch_bounds__(256) k_face_tan(const double* __restrict__ tra
 template <int D, int NV>
 __global__ void __launch_bounds__(256) k_volume_tan(const double* __restrict__ u, const double* __restrict__ v,
                                                     const double* __restrict__ nnf_t, GroupDev g, double* __restrict__ out,
-                                                    int E_b, double bx, double by, double bz)
+                                                    int E_b, double bx, double by, double bz, TanStride st)
 {
 	extern __shared__ double sm[];
+	v += blockIdx.y * st.dof;
+	out += blockIdx.y * st.dof;
+	nnf_t += blockIdx.y * st.nf;
 	const int n_s = g.n_s, n_c = g.n_c, n_fl = g.n_fl, n_fc = g.n_fc, K = g.K;
 	const int e0 = blockIdx.x * E_b;
 	const int ne = min(E_b, g.n_vol - e0);
@@ -402,59 +420,61 @@ __global__ void __launch_bounds__(256) k_volume_tan(const double* __restrict__ u
 }
 
 template <int D, int NV>
-static int face_tan_impl(dpg_gpu_ctx* c, const double* trace_t, double* nnf_t)
+static int face_tan_impl(dpg_gpu_ctx* c, const TanWork& w)
 {
 	const int n = c->fc.n_face * c->fc.n_fc;
-	k_face_tan<D, NV><<<(n + 127) / 128, 128, 0, c->stream>>>(c->trace, trace_t, c->fc, nnf_t, c->num_flux, c->b_adv[0],
-	                                                         c->b_adv[1], c->b_adv[2]);
+	k_face_tan<D, NV><<<dim3((n + 127) / 128, w.nb), 128, 0, c->stream>>>(c->trace, w.trace_t, c->fc, w.nnf_t, c->num_flux,
+	                                                                      c->b_adv[0], c->b_adv[1], c->b_adv[2], tan_stride(c));
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
-int launch_face_tan(dpg_gpu_ctx* c, const double* trace_t, double* nnf_t)
+int launch_face_tan(dpg_gpu_ctx* c, const TanWork& w)
 {
-	if (c->d == 2 && c->n_var == 4) return face_tan_impl<2, 4>(c, trace_t, nnf_t);
-	if (c->d == 3 && c->n_var == 5) return face_tan_impl<3, 5>(c, trace_t, nnf_t);
-	if (c->d == 2 && c->n_var == 1) return face_tan_impl<2, 1>(c, trace_t, nnf_t);
-	if (c->d == 3 && c->n_var == 1) return face_tan_impl<3, 1>(c, trace_t, nnf_t);
+	if (c->d == 2 && c->n_var == 4) return face_tan_impl<2, 4>(c, w);
+	if (c->d == 3 && c->n_var == 5) return face_tan_impl<3, 5>(c, w);
+	if (c->d == 2 && c->n_var == 1) return face_tan_impl<2, 1>(c, w);
+	if (c->d == 3 && c->n_var == 1) return face_tan_impl<3, 1>(c, w);
 	return DPG_ERR_UNSUPPORTED;
 }
 
 template <int D, int NV>
-static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t)
+static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w)
 {
 	const GroupDev& g = c->g;
+	const TanStride ts = tan_stride(c);
 	int rc;
 	if (c->tp) {
-		if ((rc = tp_volume_tan(c, u, v, trace_t))) return rc;
+		if ((rc = tp_volume_tan(c, u, v, w))) return rc;
 	} else {
-		const int E_t = c->trace_block_elems;
-		const size_t smem_t = (size_t)E_t * NV * g.n_s * sizeof(double);
-		const int grid_t = (g.n_vol + E_t - 1) / E_t;
-		k_trace<NV><<<grid_t, 256, smem_t, c->stream>>>(u, g, c->trace, E_t);
-		k_trace<NV><<<grid_t, 256, smem_t, c->stream>>>(v, g, trace_t, E_t);
+		const int E1 = elems_of(c, c->trace_block_elems, 1), Et = elems_of(c, c->trace_block_elems, w.nb);
+		const size_t per_t = (size_t)NV * g.n_s * sizeof(double);
+		k_trace<NV><<<(g.n_vol + E1 - 1) / E1, 256, E1 * per_t, c->stream>>>(u, g, c->trace, E1, TanStride{});
+		k_trace<NV><<<dim3((g.n_vol + Et - 1) / Et, w.nb), 256, Et * per_t, c->stream>>>(v, g, w.trace_t, Et, ts);
 		copy_boundary_trace(c, c->trace);
-		copy_boundary_trace(c, trace_t);
+		copy_boundary_trace(c, w.trace_t, w.nb, ts.tr);
 	}
-	if ((rc = launch_face_tan(c, trace_t, nnf_t))) return rc;
-	if (c->tp) return tp_lift_tan(c, nnf_t, out);
-	const int E_b = c->tan_block_elems;
+	if ((rc = launch_face_tan(c, w))) return rc;
+	if (c->tp) return tp_lift_tan(c, w, out);
+	const int E_b = elems_of(c, c->tan_block_elems, w.nb);
 	const size_t smem = (size_t)E_b * NV * (2 * g.n_s + (g.n_c > g.n_s ? g.n_c : g.n_s) + g.n_c + g.K) * sizeof(double);
-	k_volume_tan<D, NV><<<(g.n_vol + E_b - 1) / E_b, 256, smem, c->stream>>>(u, v, nnf_t, g, out, E_b, c->b_adv[0],
-	                                                                       c->b_adv[1], c->b_adv[2]);
+	k_volume_tan<D, NV><<<dim3((g.n_vol + E_b - 1) / E_b, w.nb), 256, smem, c->stream>>>(
+	    u, v, w.nnf_t, g, out, E_b, c->b_adv[0], c->b_adv[1], c->b_adv[2], ts);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
-int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t)
+int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w)
 {
-	if (c->walls_or_visc && c->tp) return tp_general_jvp(c, u, v, out, trace_t, nnf_t);
-	if (c->d == 2 && c->n_var == 4) return jvp_impl<2, 4>(c, u, v, out, trace_t, nnf_t);
-	if (c->d == 3 && c->n_var == 5) return jvp_impl<3, 5>(c, u, v, out, trace_t, nnf_t);
-	if (c->d == 2 && c->n_var == 1) return jvp_impl<2, 1>(c, u, v, out, trace_t, nnf_t);
-	if (c->d == 3 && c->n_var == 1) return jvp_impl<3, 1>(c, u, v, out, trace_t, nnf_t);
+	if (c->walls_or_visc && c->tp) return tp_general_jvp(c, u, v, out, w);
+	if (c->d == 2 && c->n_var == 4) return jvp_impl<2, 4>(c, u, v, out, w);
+	if (c->d == 3 && c->n_var == 5) return jvp_impl<3, 5>(c, u, v, out, w);
+	if (c->d == 2 && c->n_var == 1) return jvp_impl<2, 1>(c, u, v, out, w);
+	if (c->d == 3 && c->n_var == 1) return jvp_impl<3, 1>(c, u, v, out, w);
 	return DPG_ERR_UNSUPPORTED;
 }
 
-// Shared-memory opt-in for the dynamic sizes used above.
+// Shared-memory opt-in of the element kernels: the device's largest block for every context, so that a later context with
+// smaller blocks does not lower the limit of an earlier one.
+constexpr int kSmemOptIn = 227 * 1024;
 int fp64_configure(dpg_gpu_ctx* c)
 {
 	const GroupDev& g = c->g;
@@ -474,12 +494,12 @@ int fp64_configure(dpg_gpu_ctx* c)
 	if (E_j < 1) E_j = 1;
 	if (E_j > 16) E_j = 16;
 	c->tan_block_elems = E_j;
-	const int smem_v = (int)(E_b * per_v), smem_t = (int)(E_t * per_t), smem_j = (int)(E_j * per_j);
+	if (E_b * per_v > kSmemOptIn || E_t * per_t > kSmemOptIn) return DPG_ERR_CUDA;
 	cudaError_t e = cudaSuccess;
-#define SETATTR(KV, KT, KJ)                                                                                      \
-	e = cudaFuncSetAttribute(KV, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_v); if (e) return DPG_ERR_CUDA; \
-	e = cudaFuncSetAttribute(KT, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t); if (e) return DPG_ERR_CUDA; \
-	e = cudaFuncSetAttribute(KJ, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_j); if (e) return DPG_ERR_CUDA;
+#define SETATTR(KV, KT, KJ)                                                                                          \
+	e = cudaFuncSetAttribute(KV, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn); if (e) return DPG_ERR_CUDA; \
+	e = cudaFuncSetAttribute(KT, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn); if (e) return DPG_ERR_CUDA; \
+	e = cudaFuncSetAttribute(KJ, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn); if (e) return DPG_ERR_CUDA;
 	if (c->d == 2 && NV == 4) { SETATTR((k_volume<2, 4>), (k_trace<4>), (k_volume_tan<2, 4>)) }
 	else if (c->d == 3 && NV == 5) { SETATTR((k_volume<3, 5>), (k_trace<5>), (k_volume_tan<3, 5>)) }
 	else if (c->d == 2 && NV == 1) { SETATTR((k_volume<2, 1>), (k_trace<1>), (k_volume_tan<2, 1>)) }
@@ -547,11 +567,11 @@ static int noalloc_launch(const dpg_noalloc_mesh& m, const double* sol, double* 
 	const size_t per_t = (size_t)NV * g.n_s * sizeof(double);
 	int E_t = (int)((32 * 1024) / per_t);
 	E_t = E_t < 1 ? 1 : (E_t > 16 ? 16 : E_t);
-	if (cudaFuncSetAttribute(k_volume<D, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(E_b * per_v)) ||
-	    cudaFuncSetAttribute(k_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(E_t * per_t)))
+	if (cudaFuncSetAttribute(k_volume<D, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) ||
+	    cudaFuncSetAttribute(k_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn))
 		return DPG_ERR_CUDA;
 	if (cudaMemsetAsync(slot, 0, sizeof(unsigned long long), st) != cudaSuccess) return DPG_ERR_CUDA;
-	k_trace<NV><<<(g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st>>>(sol, g, trace, E_t);
+	k_trace<NV><<<(g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st>>>(sol, g, trace, E_t, TanStride{});
 	const int nq = fd.n_face * fd.n_fc;
 	k_face<D, NV><<<(nq + 127) / 128, 128, 0, st>>>(trace, fd, nnf, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
 	k_volume<D, NV><<<(g.n_vol + E_b - 1) / E_b, 256, E_b * per_v, st>>>(

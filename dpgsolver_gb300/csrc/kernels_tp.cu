@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, c
                                                  const __grid_constant__ Ops<N1> ops, double* __restrict__ sol,
                                                  double* __restrict__ solp, double* __restrict__ rhs,
                                                  const double* __restrict__ dt_ptr, unsigned long long* max_slot, int stage,
-                                                 int write_rhs, int E)
+                                                 int write_rhs, int E, TanStride ts)
 {
 	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1);
 	extern __shared__ double sm[];
@@ -50,6 +50,9 @@ __global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, c
 	double* b1 = b0 + (size_t)E * NV * N;
 	double* sF = b1 + (size_t)E * NV * N;   // [E][2 D][NV][NF] face fluxes in the element's node order, + outward
 	unsigned long long* s_max = reinterpret_cast<unsigned long long*>(sF + (size_t)E * NV * 2 * D * NF);
+	G += blockIdx.y * ts.dof;
+	nnf += blockIdx.y * ts.nf;
+	rhs += blockIdx.y * ts.dof;
 	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
 	const bool live = e < ne;
@@ -236,7 +239,7 @@ static int configure()
 }
 
 template <int D, int NV, int N1>
-static int launch_volume(dpg_gpu_ctx* c, const double* u, const double* v, double* trace, double* trace_t)
+static int launch_volume(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w)
 {
 	const TpState* st = (const TpState*)c->tp;
 	constexpr int N = ipow(N1, D);
@@ -244,41 +247,43 @@ static int launch_volume(dpg_gpu_ctx* c, const double* u, const double* v, doubl
 	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
 	const Ops<N1> ops = ops_of<N1>(st);
 	if (v)
-		k_tp_volume<D, NV, N1, true, kPeriodic><<<grid, threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
-		    u, v, geo, TpBc{}, ops, trace, trace_t, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+		k_tp_volume<D, NV, N1, true, kPeriodic><<<dim3(grid, w->nb), threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
+		    u, v, geo, TpBc{}, ops, c->trace, w->trace_t, w->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2], tan_stride(c));
 	else
 		k_tp_volume<D, NV, N1, false, kPeriodic><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
-		    u, nullptr, geo, TpBc{}, ops, trace, nullptr, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+		    u, nullptr, geo, TpBc{}, ops, c->trace, nullptr, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2], TanStride{});
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
 template <int D, int NV, int N1>
-static int launch_lift(dpg_gpu_ctx* c, const double* nnf, double* rhs, unsigned long long* max_slot, int stage, bool write_rhs)
+static int launch_lift(dpg_gpu_ctx* c, const double* G, const double* nnf, double* rhs, unsigned long long* max_slot, int stage,
+                       bool write_rhs, int nb)
 {
 	const TpState* st = (const TpState*)c->tp;
 	constexpr int N = ipow(N1, D);
 	const TpGeo geo = geo_of(c);
 	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
-	k_tp_lift<D, NV, N1><<<grid, threads, smem_lift<D, NV, N1>(E), c->stream>>>(
-	    st->G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E);
+	k_tp_lift<D, NV, N1><<<dim3(grid, nb), threads, smem_lift<D, NV, N1>(E), c->stream>>>(
+	    G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E, tan_stride(c));
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
 static int configure_any(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(configure); }
 
-int tp_volume(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(launch_volume, c, c->sol, nullptr, c->trace, nullptr); }
-int tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t)
+int tp_volume(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(launch_volume, c, c->sol, nullptr, nullptr); }
+int tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork& w)
 {
-	DPG_TP_DISPATCH(launch_volume, c, u, v, c->trace, trace_t);
+	DPG_TP_DISPATCH(launch_volume, c, u, v, &w);
 }
 int tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
 {
-	DPG_TP_DISPATCH(launch_lift, c, c->nnf, c->rhs, max_slot, stage, write_rhs);
+	DPG_TP_DISPATCH(launch_lift, c, ((const TpState*)c->tp)->G, c->nnf, c->rhs, max_slot, stage, write_rhs, 1);
 }
-int tp_lift_tan(dpg_gpu_ctx* c, const double* nnf_t, double* out)
+int tp_lift_tan(dpg_gpu_ctx* c, const TanWork& w, double* out)
 {
-	DPG_TP_DISPATCH(launch_lift, c, nnf_t, out, nullptr, -1, true);
+	DPG_TP_DISPATCH(launch_lift, c, w.G, w.nnf_t, out, nullptr, -1, true, w.nb);
 }
+bool tp_viscous(const dpg_gpu_ctx* c) { return ((const TpState*)c->tp)->viscous != 0; }
 
 // Set-up.  Leaves c->tp null (the dense kernels of kernels_fp64.cu run) where the element is not one of the orders above
 // or its operators are not the products of the 1D ones.
@@ -313,9 +318,7 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 		if ((rc = alloc(&st->jn, ji.size()))) return rc;
 		if (cudaMemcpy(st->jn, ji.data(), sizeof(double) * ji.size(), cudaMemcpyHostToDevice) != cudaSuccess) return DPG_ERR_CUDA;
 	}
-	int n_sm = 0;
-	if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, c->dev) != cudaSuccess || n_sm < 1) n_sm = 1;
-	st->E = block_elems(sim->n_vol, N, n_sm);
+	st->E = block_elems(sim->n_vol, N, c->n_sm);
 	return configure_any(c);
 }
 

@@ -61,7 +61,7 @@ template <class T, int D, int NV, int N1>
 __global__ void __launch_bounds__(256) k_tp_grad(const double* __restrict__ Uc, const double* __restrict__ Uc_t,
                                                  const double* __restrict__ trace, const double* __restrict__ trace_t, TpGeo g,
                                                  TpVisc V, const __grid_constant__ Ops<N1> ops, double* __restrict__ fvn,
-                                                 double* __restrict__ G, int E)
+                                                 double* __restrict__ G, int E, TanStride ts)
 {
 	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1);
 	extern __shared__ double sm[];
@@ -71,6 +71,12 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* __restrict__ Uc, 
 	T* sJ = sG + (size_t)E * D * NV * N;           // [E][2 D][NV][NF] J_f (u_num - u)
 	double* sN = reinterpret_cast<double*>(sJ + (size_t)E * 2 * D * NV * NF);   // [E][2 D][D][NF] normals
 	double* sD = sN + (size_t)E * 2 * D * D * NF;  // [E][N] 1 / detJ
+	if constexpr (Ld<T>::tan) {
+		Uc_t += blockIdx.y * ts.dof;
+		trace_t += blockIdx.y * ts.tr;
+		fvn += blockIdx.y * ts.tr;
+		G += blockIdx.y * ts.dof;
+	}
 	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
 	const bool live = e < ne;
@@ -246,8 +252,13 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* __restrict__ Uc, 
 template <class T, int D, int NV>
 __global__ void __launch_bounds__(128) k_tp_face_br2(const double* __restrict__ trace, const double* __restrict__ trace_t,
                                                      const double* __restrict__ fvn, TpVisc V, int n_face, int n_fc,
-                                                     int num_flux, double* __restrict__ nnf)
+                                                     int num_flux, double* __restrict__ nnf, TanStride ts)
 {
+	if constexpr (Ld<T>::tan) {
+		trace_t += blockIdx.y * ts.tr;
+		fvn += blockIdx.y * ts.tr;
+		nnf += blockIdx.y * ts.nf;
+	}
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= n_face * n_fc) return;
 	const int f = t / n_fc, q = t - f * n_fc, qr = V.nc[t];
@@ -294,71 +305,65 @@ static int configure_general(dpg_gpu_ctx* c)
 	return DPG_OK;
 }
 
-// Everything before the lift: traces, boundary states, (gradients,) face fluxes into nnf, weak divergence into G.
+// Everything before the lift: traces, boundary states, (gradients,) face fluxes, weak divergence -- of the state u (w null)
+// or their tangents along v[nb][n_dof].
 template <int D, int NV, int N1>
-static int front(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t, double* nnf)
+static int front(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w)
 {
 	const TpState* st = (const TpState*)c->tp;
 	constexpr int N = ipow(N1, D);
 	const TpGeo geo = geo_of(c);
 	const TpBc B{st->bc, st->xyz, c->fc.nrm, st->bp};
-	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	const int E = st->E, n_blk = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	const dim3 grid(n_blk, w ? w->nb : 1);
 	const Ops<N1> ops = ops_of<N1>(st);
 	const double bx = c->b_adv[0], by = c->b_adv[1], bz = c->b_adv[2];
+	const size_t sm_v = smem_volume<D, NV, N1, false>(E), sm_t = smem_volume<D, NV, N1, true>(E);
+	const TanStride ts = tan_stride(c);
 	if (!st->viscous) {
-		if (v) k_tp_volume<D, NV, N1, true, kWalls><<<grid, threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
-			u, v, geo, B, ops, c->trace, trace_t, st->G, nullptr, E, bx, by, bz);
-		else k_tp_volume<D, NV, N1, false, kWalls><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
-			u, nullptr, geo, B, ops, c->trace, nullptr, st->G, nullptr, E, bx, by, bz);
+		if (w) k_tp_volume<D, NV, N1, true, kWalls><<<grid, threads, sm_t, c->stream>>>(
+			u, v, geo, B, ops, c->trace, w->trace_t, w->G, nullptr, E, bx, by, bz, ts);
+		else k_tp_volume<D, NV, N1, false, kWalls><<<grid, threads, sm_v, c->stream>>>(
+			u, nullptr, geo, B, ops, c->trace, nullptr, st->G, nullptr, E, bx, by, bz, ts);
 		if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
-		return v ? launch_face_tan(c, trace_t, nnf) : launch_face(c);
+		return w ? launch_face_tan(c, *w) : launch_face(c);
 	}
 	if constexpr (NV == D + 2) {
 		const TpVisc V{st->mu, st->kappa, st->scale, st->bc, c->fc.nc, c->fc.nrm, c->fc.jf};
-		const int nq = c->fc.n_face * c->fc.n_fc;
-		if (v) {
-			k_tp_volume<D, NV, N1, true, kViscous><<<grid, threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
-				u, v, geo, B, ops, c->trace, trace_t, st->Uc, st->Uc_t, E, bx, by, bz);
+		const int n_fb = (c->fc.n_face * c->fc.n_fc + 127) / 128;
+		if (w) {
+			k_tp_volume<D, NV, N1, true, kViscous><<<grid, threads, sm_t, c->stream>>>(
+				u, v, geo, B, ops, c->trace, w->trace_t, st->Uc, w->Uc_t, E, bx, by, bz, ts);
 			k_tp_grad<dual, D, NV, N1><<<grid, threads, smem_grad<dual, D, NV, N1>(E), c->stream>>>(
-				st->Uc, st->Uc_t, c->trace, trace_t, geo, V, ops, st->fvn, st->G, E);
-			k_tp_face_br2<dual, D, NV><<<(nq + 127) / 128, 128, 0, c->stream>>>(c->trace, trace_t, st->fvn, V, c->fc.n_face,
-			                                                                   c->fc.n_fc, c->num_flux, nnf);
+				st->Uc, w->Uc_t, c->trace, w->trace_t, geo, V, ops, w->fvn, w->G, E, ts);
+			k_tp_face_br2<dual, D, NV><<<dim3(n_fb, w->nb), 128, 0, c->stream>>>(
+				c->trace, w->trace_t, w->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, w->nnf_t, ts);
 		} else {
-			k_tp_volume<D, NV, N1, false, kViscous><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
-				u, nullptr, geo, B, ops, c->trace, nullptr, st->Uc, nullptr, E, bx, by, bz);
+			k_tp_volume<D, NV, N1, false, kViscous><<<grid, threads, sm_v, c->stream>>>(
+				u, nullptr, geo, B, ops, c->trace, nullptr, st->Uc, nullptr, E, bx, by, bz, ts);
 			k_tp_grad<double, D, NV, N1><<<grid, threads, smem_grad<double, D, NV, N1>(E), c->stream>>>(
-				st->Uc, nullptr, c->trace, nullptr, geo, V, ops, st->fvn, st->G, E);
-			k_tp_face_br2<double, D, NV><<<(nq + 127) / 128, 128, 0, c->stream>>>(c->trace, nullptr, st->fvn, V, c->fc.n_face,
-			                                                                     c->fc.n_fc, c->num_flux, nnf);
+				st->Uc, nullptr, c->trace, nullptr, geo, V, ops, st->fvn, st->G, E, ts);
+			k_tp_face_br2<double, D, NV><<<n_fb, 128, 0, c->stream>>>(
+				c->trace, nullptr, st->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, c->nnf, ts);
 		}
 		return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 	}
 	return DPG_ERR_UNSUPPORTED;
 }
 
-static int front_any(dpg_gpu_ctx* c, const double* u, const double* v, double* trace_t, double* nnf)
-{
-	DPG_TP_DISPATCH(front, c, u, v, trace_t, nnf);
-}
+static int front_any(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w) { DPG_TP_DISPATCH(front, c, u, v, w); }
 static int configure_general_any(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(configure_general, c); }
 
 int tp_general_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
 {
-	const int rc = front_any(c, c->sol, nullptr, nullptr, c->nnf);
+	const int rc = front_any(c, c->sol, nullptr, nullptr);
 	return rc ? rc : tp_lift(c, stage, write_rhs, max_slot);
 }
 
-int tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, double* trace_t, double* nnf_t)
+int tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w)
 {
-	TpState* st = (TpState*)c->tp;
-	if (st->viscous && !st->Uc_t) {
-		void* p = nullptr;
-		if (cudaMalloc(&p, sizeof(double) * c->n_dof) != cudaSuccess) return DPG_ERR_CUDA;
-		st->allocs.push_back(p);
-		st->Uc_t = (double*)p;
-	}
-	const int rc = front_any(c, u, v, trace_t, nnf_t);
-	return rc ? rc : tp_lift_tan(c, nnf_t, out);
+	const int rc = front_any(c, u, v, &w);
+	return rc ? rc : tp_lift_tan(c, w, out);
 }
 
 int tp_general_launches(dpg_gpu_ctx* c) { return 3 + (((const TpState*)c->tp)->viscous ? 1 : 0); }

@@ -47,9 +47,8 @@ struct TpState {
 	BcParams bp{};
 	const int* bc = nullptr;    // [n_face] 0 or the boundary code; null without boundary faces
 	const double* xyz = nullptr;// [n_face][n_fc][d]
-	double* Uc = nullptr;       // viscous: [n_dof] collocated values, their tangents (allocated on first use)
-	double* Uc_t = nullptr;
-	double* fvn = nullptr;      // viscous: [n_face][2][n_var][n_fc] normal second-order flux of each side, or its tangent
+	double* Uc = nullptr;       // viscous: [n_dof] collocated values
+	double* fvn = nullptr;      // viscous: [n_face][2][n_var][n_fc] normal second-order flux of each side
 	std::vector<void*> allocs;
 };
 

@@ -23,7 +23,7 @@ template <int D, int NV, int N1, bool TAN, int KIND>
 __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g, TpBc B,
                                                    const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
                                                    double* __restrict__ trace_t, double* __restrict__ G,
-                                                   double* __restrict__ G_t, int E, double bx, double by, double bz)
+                                                   double* __restrict__ G_t, int E, double bx, double by, double bz, TanStride ts)
 {
 	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1), NW = TAN ? 2 * NV : NV;
 	extern __shared__ double sm[];
@@ -34,6 +34,12 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
 	const bool live = e < ne;
+	const bool first = blockIdx.y == 0;   // TAN: the direction that writes the values all directions share
+	if constexpr (TAN) {
+		v += blockIdx.y * ts.dof;
+		trace_t += blockIdx.y * ts.tr;
+		(KIND == kViscous ? G_t : G) += blockIdx.y * ts.dof;
+	}
 	load_ops(so, ops);
 	{
 		const size_t g0 = (size_t)e0 * NV * N;
@@ -83,7 +89,7 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 	if (KIND == kViscous && live) {
 #pragma unroll
 		for (int w = 0; w < NW; ++w)
-			(w < NV ? G : G_t)[((size_t)(e0 + e) * NV + (w < NV ? w : w - NV)) * N + i] = s[w];
+			if (w >= NV || !TAN || first) (w < NV ? G : G_t)[((size_t)(e0 + e) * NV + (w < NV ? w : w - NV)) * N + i] = s[w];
 	}
 	// reference fluxes of this node (TAN: their tangents)
 	if (KIND != kViscous && live) {
@@ -118,7 +124,7 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 			tr[w] = l[0] * x[0];
 #pragma unroll
 			for (int j = 1; j < N1; ++j) tr[w] = fma(l[j], x[j * S], tr[w]);
-			(w < NV ? trace : trace_t)[(vf * NV + (w < NV ? w : w - NV)) * NF + q] = tr[w];
+			if (w >= NV || !TAN || first) (w < NV ? trace : trace_t)[(vf * NV + (w < NV ? w : w - NV)) * NF + q] = tr[w];
 		}
 		if constexpr (KIND != kPeriodic) {
 			const size_t f = vf >> 1;
@@ -139,7 +145,7 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 #pragma unroll
 				for (int w = 0; w < NV; ++w) {
 					const size_t k = ((vf + 1) * NV + w) * NF + q;
-					if constexpr (TAN) { trace[k] = sb[w].v; trace_t[k] = sb[w].d; }
+					if constexpr (TAN) { if (first) trace[k] = sb[w].v; trace_t[k] = sb[w].d; }
 					else trace[k] = sb[w];
 				}
 			}

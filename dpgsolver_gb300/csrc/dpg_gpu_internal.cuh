@@ -41,6 +41,7 @@ struct TanWork {
 	double* G = nullptr;        // tensor-product meshes: [nb][n_dof] weak divergence
 	double* Uc_t = nullptr;     // viscous: [nb][n_dof] collocated tangents
 	double* fvn = nullptr;      // viscous: [nb][n_face][2][n_var][n_fc]
+	bool u_traced = false;      // dense kernels: the traces of u are in place (ctx.trace)
 };
 
 // Strides between the directions of a launch (blockIdx.y): state-sized arrays, traces, face fluxes.
@@ -111,6 +112,7 @@ struct dpg_gpu_ctx {
 	double bez1_host[50] = {};   // host copies: bez1 at [0, n1^2), bez1_inv at [25, 25 + n1^2) (kernel parameters)
 	float pos_amp = 0.f;         // FP32 screen: bound of the coefficient error per unit of |A^-1| |u|
 	int* pos_err = nullptr;      // bit 0: an average density / pressure below EPS_PHYS; bit 1: relaxation underflow
+	double* jv_buf = nullptr;    // [2][n_dof] direction and product of dpg_gpu_jacobian_apply
 	double* du_buf = nullptr;    // [n_dof] device copy of a host Newton update (dpg_gpu_positivity_update)
 
 	void* tp = nullptr;         // QUAD / HEX of one order: 1D operators of the FP64 form (kernels_tp.cu)

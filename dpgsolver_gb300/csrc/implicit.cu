@@ -47,47 +47,119 @@ __global__ void k_lincomb3(int64_t n, double a, const double* __restrict__ x, do
 		z[i] = a * x[i] + b * y[i];
 }
 
-// partial[k][block] = sum_i V_k[i] * w[i] for k < nv; V_k = V + k * ld.  Vectors in chunks of 8 with their partial
-// sums in registers (w[i] is re-read once per chunk, from L1/L2); per chunk one warp-shuffle and shared-memory
-// reduction per vector.
-constexpr int kDotChunk = 8;
+constexpr int kDotChunk = 8;   // vectors per block of a multi-vector dot product
+// Sums over the lanes of eight values; lane l returns the value 4 (l >> 4) + 2 ((l >> 3) & 1) + ((l >> 2) & 1).  9 FP64
+// additions instead of 40; each value's tree is the one of eight separate butterflies.
+__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane)
+{
+	double a[4], b[2];
+	const bool h = lane & 16, q = lane & 8, e = lane & 4;
+#pragma unroll
+	for (int k = 0; k < 4; ++k) a[k] = (h ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, h ? v[k] : v[k + 4], 16);
+#pragma unroll
+	for (int k = 0; k < 2; ++k) b[k] = (q ? a[k + 2] : a[k]) + __shfl_xor_sync(0xffffffffu, q ? a[k] : a[k + 2], 8);
+	double s = (e ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, e ? b[0] : b[1], 4);
+	s += __shfl_xor_sync(0xffffffffu, s, 2);
+	s += __shfl_xor_sync(0xffffffffu, s, 1);
+	return s;
+}
+
+// partial[k * gridDim.x + block] = this block's part of V_k . w, eight vectors k per block (blockIdx.y).  With jz: w =
+// shift z - jz first (the product with the pseudo-transient matrix), written by the blocks of the first eight vectors.
 __global__ void __launch_bounds__(kRedThreads) k_multidot_partial(int64_t n, int nv, const double* __restrict__ V, int64_t ld,
-                                                                  const double* __restrict__ w, double* __restrict__ partial)
+                                                                  double* w, double* __restrict__ partial, int nb = 1,
+                                                                  const double* __restrict__ shift = nullptr,
+                                                                  const double* __restrict__ z = nullptr,
+                                                                  const double* __restrict__ jz = nullptr)
 {
 	__shared__ double red[kRedThreads / 32][kDotChunk];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	for (int k0 = 0; k0 < nv; k0 += kDotChunk) {
-		double acc[kDotChunk];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k0 = blockIdx.y * kDotChunk;
+	double acc[kDotChunk];
 #pragma unroll
-		for (int k = 0; k < kDotChunk; ++k) acc[k] = 0.0;
-		if (k0 + kDotChunk <= nv) {
-			for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-				const double wi = w[i];
-#pragma unroll
-				for (int k = 0; k < kDotChunk; ++k) acc[k] += V[(k0 + k) * ld + i] * wi;
-			}
+	for (int k = 0; k < kDotChunk; ++k) acc[k] = 0.0;
+	for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+		double wi;
+		if (jz) {
+			wi = shift[i / nb] * z[i] - jz[i];
+			if (blockIdx.y == 0) w[i] = wi;
 		} else {
-			for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-				const double wi = w[i];
-#pragma unroll
-				for (int k = 0; k < kDotChunk; ++k)
-					if (k0 + k < nv) acc[k] += V[(k0 + k) * ld + i] * wi;
-			}
+			wi = w[i];
 		}
 #pragma unroll
-		for (int k = 0; k < kDotChunk; ++k) {
-			double v = acc[k];
-			for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-			if (lane == 0) red[warp][k] = v;
-		}
-		__syncthreads();
-		if (threadIdx.x < kDotChunk && k0 + (int)threadIdx.x < nv) {
-			double s = 0.0;
-			for (int wv = 0; wv < kRedThreads / 32; ++wv) s += red[wv][threadIdx.x];
-			partial[(int64_t)(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
-		}
-		__syncthreads();
+		for (int k = 0; k < kDotChunk; ++k)
+			if (k0 + k < nv) acc[k] += V[(k0 + k) * ld + i] * wi;
 	}
+	const double v = warp_sum8(acc, lane);
+	if ((lane & 3) == 0) red[warp][4 * (lane >> 4) + 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1)] = v;
+	__syncthreads();
+	if (threadIdx.x < kDotChunk && k0 + (int)threadIdx.x < nv) {
+		double s = 0.0;
+		for (int wv = 0; wv < kRedThreads / 32; ++wv) s += red[wv][threadIdx.x];
+		partial[(int64_t)(k0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+	}
+}
+
+// Orthogonalisation of small systems (at most 32 blocks of one element per thread): each block sums the partial dot
+// products itself, so a Gram-Schmidt pass is two launches instead of three and the norm comes with the second pass
+// (10 -> 5 small launches per Krylov iteration; their chain, not their work, bounds such a system).  The sums are those of
+// k_reduce_partials: lane p holds block p's part.
+//   h_k = sum of the parts of V_k . w;  w -= sum_k V_k h_k;  norm_partial (may be null): this block's part of w . w
+constexpr int kSmallBlocks = 32;
+__global__ void __launch_bounds__(kRedThreads) k_gs_pass(int64_t n, int nv, const double* __restrict__ V, int64_t ld,
+                                                         const double* __restrict__ partial, double* __restrict__ h,
+                                                         double* __restrict__ w, double* __restrict__ norm_partial)
+{
+	extern __shared__ double sh[];   // [nv] h
+	__shared__ double red[kRedThreads / 32];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, np = gridDim.x;
+	for (int k0 = 8 * warp; k0 < nv; k0 += 8 * (kRedThreads / 32)) {
+		double p[8];
+#pragma unroll
+		for (int k = 0; k < 8; ++k) p[k] = (lane < np && k0 + k < nv) ? partial[(int64_t)(k0 + k) * np + lane] : 0.0;
+		const double s = warp_sum8(p, lane);
+		const int k = k0 + 4 * (lane >> 4) + 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1);
+		if ((lane & 3) == 0 && k < nv) {
+			sh[k] = s;
+			if (blockIdx.x == 0) h[k] = s;
+		}
+	}
+	__syncthreads();
+	const int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
+	double wi = 0.0;
+	if (i < n) {
+		double s = 0.0;
+#pragma unroll 8
+		for (int k = 0; k < nv; ++k) s += V[k * ld + i] * sh[k];
+		wi = w[i] - s;
+		w[i] = wi;
+	}
+	if (!norm_partial) return;
+	double v = wi * wi;
+	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+	if (lane == 0) red[warp] = v;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		double s = 0.0;
+		for (int wv = 0; wv < kRedThreads / 32; ++wv) s += red[wv];
+		norm_partial[blockIdx.x] = s;
+	}
+}
+
+// h[i] += h2[i] (the two passes), h[j + 1] = ||w|| from its blocks' parts, w /= ||w|| when positive
+__global__ void __launch_bounds__(kRedThreads) k_gs_finish(int64_t n, int j, const double* __restrict__ norm_partial,
+                                                           double* __restrict__ h, const double* __restrict__ h2,
+                                                           double* __restrict__ w)
+{
+	const int lane = threadIdx.x & 31;
+	double v = lane < (int)gridDim.x ? norm_partial[lane] : 0.0;
+	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+	const double norm = sqrt(fmax(v, 0.0));
+	if (blockIdx.x == 0) {
+		for (int i = threadIdx.x; i <= j; i += blockDim.x) h[i] += h2[i];
+		if (threadIdx.x == 0) h[j + 1] = norm;
+	}
+	const int64_t i = blockIdx.x * (int64_t)kRedThreads + threadIdx.x;
+	if (i < n && norm > 0.0) w[i] *= 1.0 / norm;
 }
 
 __global__ void k_reduce_partials(int nv, int nparts, const double* __restrict__ partial, double* __restrict__ out)
@@ -435,49 +507,123 @@ __global__ void k_extract_ilu(int n_vol, int nb, int n_fl, const double* __restr
 	}
 }
 
-// in-place inverse of the nb x nb row-major matrix a in shared memory (Gauss-Jordan, partial pivoting; the row
-// exchanges are undone as column exchanges at the end); returns false for a zero pivot
-__device__ bool gj_invert_shared(int nb, double* a, int* perm)
+// Per element of the level lists, what its row of the factorisation and of the sweeps touches: {element, number of lower
+// neighbours, number of upper ones, then (slot, neighbour) of the lower and of the upper ones in slot order}.
+constexpr int kIluDesc = 16;   // 3 + 2 * 6 local faces
+
+// D_i = A_ii - sum_{k lower} A_ik D_k^-1 A_ki, kIluSlab columns per block (gridDim.y of them): the columns are independent,
+// and one SM's FP64 pipe would take 14 us for each of a 36 x 36 element's four products (8x8 QUAD p = 2, one level:
+// factor 204 us with a block per element, 40 us for update and inverse here).  diag holds A_ii on entry (elements of
+// earlier levels already hold D_k^-1).
+constexpr int kIluSlab = 4;
+__global__ void __launch_bounds__(256) k_ilu_update_level(const int* __restrict__ desc, int nb, int n_fl,
+                                                          const int* __restrict__ nbr, double* __restrict__ diag,
+                                                          const double* __restrict__ offd)
 {
-	__shared__ int s_p;
-	__shared__ double s_best;
-	for (int k = 0; k < nb; ++k) {
-		if (threadIdx.x < 32) {
-			int p = k;
-			double best = -1.0;
-			for (int i = k + threadIdx.x; i < nb; i += 32) {
-				const double v = fabs(a[i * nb + k]);
-				if (v > best) { best = v; p = i; }
-			}
-			for (int o = 16; o > 0; o >>= 1) {
-				const double bv = __shfl_xor_sync(0xffffffffu, best, o);
-				const int bp = __shfl_xor_sync(0xffffffffu, p, o);
-				if (bv > best || (bv == best && bp < p)) { best = bv; p = bp; }
-			}
-			if (threadIdx.x == 0) { s_p = p; s_best = best; perm[k] = p; }
+	extern __shared__ double sh[];
+	double* M = sh;                       // D_k^-1, then A_ik
+	double* B = M + nb * nb;              // [nb][kIluSlab] A_ki
+	double* T = B + nb * kIluSlab;        // [nb][kIluSlab] D_k^-1 A_ki
+	double* D = T + nb * kIluSlab;        // [nb][kIluSlab]
+	const int* d = desc + (size_t)blockIdx.x * kIluDesc;
+	const int i = d[0], n_low = d[1];
+	if (n_low == 0) return;
+	const int c0 = blockIdx.y * kIluSlab, nc = min(kIluSlab, nb - c0);
+	double* Di = diag + (int64_t)i * nb * nb;
+	for (int t = threadIdx.x; t < nb * kIluSlab; t += blockDim.x) {
+		const int r = t / kIluSlab, c = t - r * kIluSlab;
+		D[t] = c < nc ? Di[r * nb + c0 + c] : 0.0;
+	}
+	for (int q = 0; q < n_low; ++q) {
+		const int s = d[3 + 2 * q], k = d[4 + 2 * q];
+		int sk = -1;
+		for (int t = 0; t < n_fl; ++t)
+			if (nbr[k * n_fl + t] == i) { sk = t; break; }
+		if (sk < 0) continue;
+		const double* Dk = diag + (int64_t)k * nb * nb;                           // D_k^-1
+		const double* Aki = offd + ((int64_t)k * n_fl + sk) * nb * nb;
+		const double* Aik = offd + ((int64_t)i * n_fl + s) * nb * nb;
+		for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) M[t] = Dk[t];
+		for (int t = threadIdx.x; t < nb * kIluSlab; t += blockDim.x) {
+			const int r = t / kIluSlab, c = t - r * kIluSlab;
+			B[t] = c < nc ? Aki[r * nb + c0 + c] : 0.0;
 		}
 		__syncthreads();
-		if (!(s_best > 0.0)) return false;
-		const int p = s_p;
-		if (p != k)
-			for (int c = threadIdx.x; c < nb; c += blockDim.x) {
-				const double t = a[k * nb + c]; a[k * nb + c] = a[p * nb + c]; a[p * nb + c] = t;
-			}
+		for (int t = threadIdx.x; t < nb * kIluSlab; t += blockDim.x) {             // T = D_k^-1 A_ki
+			const int r = t / kIluSlab, c = t - r * kIluSlab;
+			double acc = 0.0;
+			for (int p = 0; p < nb; ++p) acc += M[r * nb + p] * B[p * kIluSlab + c];
+			T[t] = acc;
+		}
 		__syncthreads();
-		const double inv = 1.0 / a[k * nb + k];
+		for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) M[t] = Aik[t];
 		__syncthreads();
-		for (int c = threadIdx.x; c < nb; c += blockDim.x) a[k * nb + c] = (c == k ? inv : a[k * nb + c] * inv);
+		for (int t = threadIdx.x; t < nb * kIluSlab; t += blockDim.x) {             // D -= A_ik T
+			const int r = t / kIluSlab, c = t - r * kIluSlab;
+			double acc = 0.0;
+			for (int p = 0; p < nb; ++p) acc += M[r * nb + p] * T[p * kIluSlab + c];
+			D[t] -= acc;
+		}
+		__syncthreads();
+	}
+	for (int t = threadIdx.x; t < nb * kIluSlab; t += blockDim.x) {
+		const int r = t / kIluSlab, c = t - r * kIluSlab;
+		if (c < nc) Di[r * nb + c0 + c] = D[t];
+	}
+}
+
+// D_i^-1 of the elements of one level, one block each, in shared memory (Gauss-Jordan with partial pivoting; the row
+// exchanges are undone as column exchanges at the end).  Two barriers per pivot: every warp finds the pivot by itself
+// and the exchanged row goes through buffers, since the chain of pivots, not the FP64 work, bounds it.
+__global__ void __launch_bounds__(1024) k_ilu_invert_level(const int* __restrict__ desc, int nb, double* __restrict__ diag,
+                                                           int* __restrict__ info)
+{
+	extern __shared__ double a[];         // [nb][nb]
+	double* row = a + nb * nb;            // the pivot row over the pivot
+	double* old = row + nb;               // the row that the pivot row changes places with
+	double* col = old + nb;               // the factors of the rows after the exchange
+	int* perm = (int*)(col + nb);
+	const int i0 = desc[(size_t)blockIdx.x * kIluDesc];
+	double* Di = diag + (int64_t)i0 * nb * nb;
+	const int lane = threadIdx.x & 31;
+	for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) a[t] = Di[t];
+	__syncthreads();
+	for (int k = 0; k < nb; ++k) {
+		// largest |a_ik|, i >= k (lowest i of equal ones): magnitudes compared as integers, NaN never chosen
+		long long best = -1;
+		int p = k;
+		for (int i = k + lane; i < nb; i += 32) {
+			const long long v = __double_as_longlong(a[i * nb + k]) & 0x7FFFFFFFFFFFFFFFll;
+			if (v <= 0x7FF0000000000000ll && v > best) { best = v; p = i; }
+		}
+		for (int o = 16; o > 0; o >>= 1) {
+			const long long bv = __shfl_xor_sync(0xffffffffu, best, o);
+			const int bp = __shfl_xor_sync(0xffffffffu, p, o);
+			if (bv > best || (bv == best && bp < p)) { best = bv; p = bp; }
+		}
+		if (best <= 0) {   // the same in every warp: the block leaves together
+			if (threadIdx.x == 0) atomicExch(info, i0 + 1);
+			return;
+		}
+		for (int c = threadIdx.x; c < nb; c += blockDim.x) {
+			const double inv = 1.0 / a[p * nb + k];
+			row[c] = c == k ? inv : a[p * nb + c] * inv;
+			old[c] = a[k * nb + c];
+			col[c] = a[(c == p ? k : c) * nb + k];
+			if (c == k) perm[k] = p;
+		}
 		__syncthreads();
 		for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
 			const int i = t / nb, c = t - i * nb;
-			if (i == k) continue;
-			const double f = a[i * nb + k];
-			if (c == k) continue;
-			a[i * nb + c] -= f * a[k * nb + c];
+			double v;
+			if (i == k) v = row[c];
+			else if (c == k) v = -col[i] * row[k];
+			else {
+				v = i == p ? old[c] : a[t];
+				v -= col[i] * row[c];
+			}
+			a[t] = v;
 		}
-		__syncthreads();
-		for (int i = threadIdx.x; i < nb; i += blockDim.x)
-			if (i != k) a[i * nb + k] = -a[i * nb + k] * inv;
 		__syncthreads();
 	}
 	for (int k = nb - 1; k >= 0; --k) {
@@ -488,279 +634,105 @@ __device__ bool gj_invert_shared(int nb, double* a, int* perm)
 			}
 		__syncthreads();
 	}
-	return true;
+	for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) Di[t] = a[t];
 }
 
-// slot of neighbour `want` in the list of element e, -1 if absent
-__device__ __forceinline__ int nbr_slot(const int* __restrict__ nbr, int n_fl, int e, int want)
-{
-	for (int s = 0; s < n_fl; ++s) if (nbr[e * n_fl + s] == want) return s;
-	return -1;
-}
-
-// D_i = A_ii - sum_{k lower} A_ik D_k^-1 A_ki and its inverse, for the elements of one level; diag holds A_ii on
-// entry and D_i^-1 on exit (elements of earlier levels already hold D_k^-1)
-__global__ void k_ilu_factor_level(const int* __restrict__ elems, int nb, int n_fl, const int* __restrict__ nbr,
-                                   const int* __restrict__ rank, double* __restrict__ diag,
-                                   const double* __restrict__ offd, int* __restrict__ info)
-{
-	extern __shared__ double sh[];
-	double* D = sh;
-	double* T = sh + nb * nb;
-	int* perm = (int*)(T + nb * nb);
-	const int i = elems[blockIdx.x];
-	double* Di = diag + (int64_t)i * nb * nb;
-	for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) D[t] = Di[t];
-	__syncthreads();
-	for (int s = 0; s < n_fl; ++s) {
-		const int k = nbr[i * n_fl + s];
-		if (k < 0 || rank[k] >= rank[i]) continue;
-		const int sk = nbr_slot(nbr, n_fl, k, i);
-		if (sk < 0) continue;
-		const double* Dk = diag + (int64_t)k * nb * nb;                           // D_k^-1
-		const double* Aki = offd + ((int64_t)k * n_fl + sk) * nb * nb;
-		const double* Aik = offd + ((int64_t)i * n_fl + s) * nb * nb;
-		for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {                   // T = D_k^-1 A_ki
-			const int r = t / nb, c = t - r * nb;
-			double acc = 0.0;
-			for (int q = 0; q < nb; ++q) acc += Dk[r * nb + q] * Aki[q * nb + c];
-			T[t] = acc;
-		}
-		__syncthreads();
-		for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {                   // D -= A_ik T
-			const int r = t / nb, c = t - r * nb;
-			double acc = 0.0;
-			for (int q = 0; q < nb; ++q) acc += Aik[r * nb + q] * T[q * nb + c];
-			D[t] -= acc;
-		}
-		__syncthreads();
-	}
-	const bool ok = gj_invert_shared(nb, D, perm);
-	if (!ok) {
-		if (threadIdx.x == 0) atomicExch(info, i + 1);
-		return;
-	}
-	for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) Di[t] = D[t];
-}
-
-// Triangular sweeps, one level, one thread block (kIluSweepThreads = 8 warps) per element.  Warp w owns the rows
-// w, w + 8, ... (at most kIluRows of them) and lane l the columns l, l + 32, ... (at most kIluCols); the vector's
-// entries a lane needs are loaded once into registers, and the block rows of all its rows are loaded before any
-// sum is reduced, so a warp has all its loads in flight at once instead of one row after another.
-constexpr int kIluSweepThreads = 256;
-constexpr int kIluRows = 14;   // ceil(112 / 8)
-constexpr int kIluCols = 4;    // ceil(112 / 32)
-
-__device__ __forceinline__ double warp_sum(double v)
-{
-	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-	return v;
-}
-
-// acc[t] += sum_c M[(warp + 8 t) * nb + c] x[c] over this lane's columns; NB > 0 fixes nb at compile time (no
-// predicated padding rows or columns), NB = 0 takes it at run time (nb <= 112)
-template <int NB>
-__device__ __forceinline__ void ilu_rows_times(const double* __restrict__ M, const double* __restrict__ x, int nb_rt,
-                                               int warp, int lane, double (&acc)[kIluRows])
-{
-	const int nb = NB > 0 ? NB : nb_rt;
-	constexpr int R = NB > 0 ? (NB + 7) / 8 : kIluRows;
-	constexpr int CC = NB > 0 ? (NB + 31) / 32 : kIluCols;
-	double xv[CC];
-#pragma unroll
-	for (int j = 0; j < CC; ++j) {
-		const int c = lane + 32 * j;
-		xv[j] = (c < nb) ? x[c] : 0.0;
-	}
-#pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + 8 * t;
-		if (row < nb) {
-#pragma unroll
-			for (int j = 0; j < CC; ++j) {
-				const int c = lane + 32 * j;
-				if (c < nb) acc[t] += M[(int64_t)row * nb + c] * xv[j];
-			}
-		}
-	}
-}
-
-// forward sweep: w_i = D_i^-1 (r_i - sum_{k lower} A_ik w_k)
-template <int NB>
-__global__ void __launch_bounds__(kIluSweepThreads) k_ilu_forward_level(const int* __restrict__ elems, int nb_rt, int n_fl,
-                                                                        const int* __restrict__ nbr, const int* __restrict__ rank,
-                                                                        const double* __restrict__ dinv, const double* __restrict__ offd,
-                                                                        const double* __restrict__ r, double* __restrict__ w)
-{
-	extern __shared__ double y[];
-	const int nb = NB > 0 ? NB : nb_rt;
-	constexpr int R = NB > 0 ? (NB + 7) / 8 : kIluRows;
-	const int i = elems[blockIdx.x];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	double acc[kIluRows];
-#pragma unroll
-	for (int t = 0; t < kIluRows; ++t) acc[t] = 0.0;
-	for (int s = 0; s < n_fl; ++s) {
-		const int k = nbr[i * n_fl + s];
-		if (k < 0 || rank[k] >= rank[i]) continue;
-		ilu_rows_times<NB>(offd + ((int64_t)i * n_fl + s) * nb * nb, w + (int64_t)k * nb, nb, warp, lane, acc);
-	}
-#pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + 8 * t;
-		const double v = warp_sum(acc[t]);
-		if (lane == 0 && row < nb) y[row] = r[(int64_t)i * nb + row] - v;
-	}
-	__syncthreads();
-#pragma unroll
-	for (int t = 0; t < kIluRows; ++t) acc[t] = 0.0;
-	ilu_rows_times<NB>(dinv + (int64_t)i * nb * nb, y, nb, warp, lane, acc);
-#pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + 8 * t;
-		const double v = warp_sum(acc[t]);
-		if (lane == 0 && row < nb) w[(int64_t)i * nb + row] = v;
-	}
-}
-
-// backward sweep (levels in reverse): z_i = w_i - D_i^-1 sum_{j upper} A_ij z_j
-template <int NB>
-__global__ void __launch_bounds__(kIluSweepThreads) k_ilu_backward_level(const int* __restrict__ elems, int nb_rt, int n_fl,
-                                                                         const int* __restrict__ nbr, const int* __restrict__ rank,
-                                                                         const double* __restrict__ dinv, const double* __restrict__ offd,
-                                                                         const double* __restrict__ w, double* __restrict__ z)
-{
-	extern __shared__ double y[];
-	const int nb = NB > 0 ? NB : nb_rt;
-	constexpr int R = NB > 0 ? (NB + 7) / 8 : kIluRows;
-	const int i = elems[blockIdx.x];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	double acc[kIluRows];
-#pragma unroll
-	for (int t = 0; t < kIluRows; ++t) acc[t] = 0.0;
-	for (int s = 0; s < n_fl; ++s) {
-		const int j = nbr[i * n_fl + s];
-		if (j < 0 || rank[j] <= rank[i]) continue;
-		ilu_rows_times<NB>(offd + ((int64_t)i * n_fl + s) * nb * nb, z + (int64_t)j * nb, nb, warp, lane, acc);
-	}
-#pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + 8 * t;
-		const double v = warp_sum(acc[t]);
-		if (lane == 0 && row < nb) y[row] = v;
-	}
-	__syncthreads();
-#pragma unroll
-	for (int t = 0; t < kIluRows; ++t) acc[t] = 0.0;
-	ilu_rows_times<NB>(dinv + (int64_t)i * nb * nb, y, nb, warp, lane, acc);
-#pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + 8 * t;
-		const double v = warp_sum(acc[t]);
-		if (lane == 0 && row < nb) z[(int64_t)i * nb + row] = w[(int64_t)i * nb + row] - v;
-	}
-}
-
-// One level of either sweep for blocks of a size fixed at compile time, with its operands staged in shared memory:
-// every thread first issues asynchronous 16-byte copies (cp.async, completed by cp.async.wait_all, a wait on the
-// thread's own copies) of D_i^-1 and of the blocks A_is of the neighbours the sweep uses, and plain loads of those
-// neighbours' vector entries and of b_i, so a level costs one memory round trip instead of one per neighbour and a
-// dependent one for D_i^-1.  The sums run in the order of the register kernels above (neighbours, then columns
-// lane, lane + 32, ..., per row), so the results are the same bits.
+// One level of either triangular sweep, one thread block per element, four rows per warp (lane l the columns l, l + 32,
+// ...).
 //   FWD: x_i = D_i^-1 (b_i - sum_{k lower} A_ik x_k)    (b = r, x = w)
 //   BWD: x_i = b_i - D_i^-1 sum_{j upper} A_ij x_j      (b = w, x = z)
-constexpr int kIluStagedThreads = 512;
-constexpr int kIluStagedMaxFl = 5;
+// The levels are a chain of dependent launches, each with few elements, so its latency counts: the next level's
+// blocks start early (programmatic dependent launch) and fetch their descriptor and matrices, which no level writes,
+// before they wait for this one; the lane sums of a warp's four rows are folded together (6 FP64 additions instead of
+// 20: the FP64 pipe takes ~20 cycles of the SM for each warp instruction).  A row's sum keeps one order: neighbours, then
+// columns, then lanes l + (l ^ 16), ^ 8, ..  8x8 QUAD p = 2 (36 x 36 blocks): 25 us per level with one row after
+// the other and a plain launch; 64x128 annulus QUAD p = 3 (64 x 64 blocks): 17 us.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-__device__ __forceinline__ void ilu_stage_block(double* dst, const double* __restrict__ src, int n_chunks)
+// Sums over the lanes of four rows' values; lane l returns the row 2 (l >> 4) + ((l >> 3) & 1).
+__device__ __forceinline__ double warp_sum4(const double (&v)[4], int lane)
 {
-	for (int q = threadIdx.x; q < n_chunks; q += blockDim.x)
-		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + 2 * q)),
-		             "l"(src + 2 * q)
-		             : "memory");
+	const bool h = lane & 16, q = lane & 8;
+	const double a = (h ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h ? v[0] : v[2], 16);
+	const double b = (h ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h ? v[1] : v[3], 16);
+	double s = (q ? b : a) + __shfl_xor_sync(0xffffffffu, q ? a : b, 8);
+	for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	return s;
 }
 
-template <int NB, bool FWD>
-__global__ void __launch_bounds__(kIluStagedThreads) k_ilu_level_staged(const int* __restrict__ elems, int n_fl,
-                                                                        const int* __restrict__ nbr, const int* __restrict__ rank,
-                                                                        const double* __restrict__ dinv, const double* __restrict__ offd,
-                                                                        const double* __restrict__ b, double* __restrict__ x)
+template <int CC, bool FWD>
+__global__ void __launch_bounds__(CC <= 2 ? 512 : 896) k_ilu_sweep_level(const int* __restrict__ desc, int nb, int n_fl,
+                                                                         const double* __restrict__ dinv,
+                                                                         const double* __restrict__ offd, const double* b, double* x)
 {
-	extern __shared__ __align__(16) double sm[];   // [1 + used][NB][NB]: D_i^-1, then the used A_is in slot order
-	__shared__ double xs[kIluStagedMaxFl][NB];
-	__shared__ double y[NB];
-	__shared__ int used[kIluStagedMaxFl], n_used;
-	constexpr int NW = kIluStagedThreads / 32, R = (NB + NW - 1) / NW, CC = (NB + 31) / 32;
-	constexpr int kChunks = NB * NB / 2;   // 16-byte copies per block
-	static_assert(NB % 2 == 0, "blocks are copied in 16-byte pieces");
-	const int i = elems[blockIdx.x];
+	constexpr int PRE = CC <= 2 ? 2 : 0;   // neighbour blocks fetched before the wait (register budget)
+	__shared__ double y[128];
+	grid_dependency_launch();
+	int d[kIluDesc];
+#pragma unroll
+	for (int k = 0; k < kIluDesc / 4; ++k) {
+		const int4 t = reinterpret_cast<const int4*>(desc + (size_t)blockIdx.x * kIluDesc)[k];
+		d[4 * k] = t.x; d[4 * k + 1] = t.y; d[4 * k + 2] = t.z; d[4 * k + 3] = t.w;
+	}
+	const int i = d[0], n_low = d[1], n_use = FWD ? n_low : d[2];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	ilu_stage_block(sm, dinv + (int64_t)i * NB * NB, kChunks);
-	if (threadIdx.x == 0) {
-		const int ri = rank[i];
-		int q = 0;
-		for (int s = 0; s < n_fl; ++s) {
-			const int k = nbr[i * n_fl + s];
-			if (k >= 0 && (FWD ? rank[k] < ri : rank[k] > ri)) used[q++] = s;
-		}
-		n_used = q;
-	}
-	__syncthreads();
-	const int nu = n_used;
-	for (int q = 0; q < nu; ++q)
-		ilu_stage_block(sm + (size_t)(q + 1) * NB * NB, offd + ((int64_t)i * n_fl + used[q]) * NB * NB, kChunks);
-	asm volatile("cp.async.commit_group;" ::: "memory");
-	for (int t = threadIdx.x; t < nu * NB; t += blockDim.x) {
-		const int q = t / NB, c = t - q * NB;
-		xs[q][c] = x[(int64_t)nbr[i * n_fl + used[q]] * NB + c];
-	}
-	double bv[R];
+	auto entry = [&](int q, int w) {   // (slot, neighbour) q of this sweep's list
+		int v = 0;
 #pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + NW * t;
-		bv[t] = row < NB ? b[(int64_t)i * NB + row] : 0.0;
-	}
-	asm volatile("cp.async.wait_all;" ::: "memory");
-	__syncthreads();
-	double acc[R];
+		for (int k = 0; k < 6; ++k) v = (k == (FWD ? q : n_low + q)) ? d[3 + 2 * k + w] : v;
+		return v;
+	};
+	auto fetch = [&](const double* M, double (&m)[4][CC]) {
 #pragma unroll
-	for (int t = 0; t < R; ++t) acc[t] = 0.0;
-	for (int q = 0; q < nu; ++q) {
-		const double* M = sm + (size_t)(q + 1) * NB * NB;
+		for (int t = 0; t < 4; ++t)
 #pragma unroll
-		for (int t = 0; t < R; ++t) {
-			const int row = warp + NW * t;
-			if (row < NB) {
-#pragma unroll
-				for (int j = 0; j < CC; ++j) {
-					const int c = lane + 32 * j;
-					if (c < NB) acc[t] += M[row * NB + c] * xs[q][c];
-				}
+			for (int j = 0; j < CC; ++j) {
+				const int row = 4 * warp + t, c = lane + 32 * j;
+				m[t][j] = (row < nb && c < nb) ? M[(int64_t)row * nb + c] : 0.0;
 			}
-		}
-	}
+	};
+	double dm[4][CC], am[PRE > 0 ? PRE : 1][4][CC];
+	fetch(dinv + (int64_t)i * nb * nb, dm);
 #pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + NW * t;
-		const double v = warp_sum(acc[t]);
-		if (lane == 0 && row < NB) y[row] = FWD ? bv[t] - v : v;
+	for (int q = 0; q < PRE; ++q)
+		if (q < n_use) fetch(offd + ((int64_t)i * n_fl + entry(q, 0)) * nb * nb, am[q]);
+	grid_dependency_wait();
+	const int row = 4 * warp + 2 * (lane >> 4) + ((lane >> 3) & 1);   // the row whose sum this lane gets
+	const bool owner = (lane & 7) == 0 && row < nb;
+	const double bv = owner ? __ldcg(b + (int64_t)i * nb + row) : 0.0;
+	double acc[4] = {0.0, 0.0, 0.0, 0.0};
+	auto times = [&](const double (&m)[4][CC], const double (&v)[CC]) {
+#pragma unroll
+		for (int j = 0; j < CC; ++j)
+			if (lane + 32 * j < nb) {
+#pragma unroll
+				for (int t = 0; t < 4; ++t) acc[t] += m[t][j] * v[j];
+			}
+	};
+	for (int q = 0; q < n_use; ++q) {
+		double v[CC];
+#pragma unroll
+		for (int j = 0; j < CC; ++j) v[j] = lane + 32 * j < nb ? __ldcg(x + (int64_t)entry(q, 1) * nb + lane + 32 * j) : 0.0;
+		if constexpr (PRE > 0) {
+			if (q == 0) { times(am[0], v); continue; }
+			if (q == 1) { times(am[1], v); continue; }
+		}
+		double m[4][CC];
+		fetch(offd + ((int64_t)i * n_fl + entry(q, 0)) * nb * nb, m);
+		times(m, v);
 	}
+	const double s = warp_sum4(acc, lane);
+	if (owner) y[row] = FWD ? bv - s : s;
 	__syncthreads();
+#pragma unroll
+	for (int t = 0; t < 4; ++t) acc[t] = 0.0;
 	double yv[CC];
 #pragma unroll
-	for (int j = 0; j < CC; ++j) yv[j] = (lane + 32 * j < NB) ? y[lane + 32 * j] : 0.0;
-#pragma unroll
-	for (int t = 0; t < R; ++t) {
-		const int row = warp + NW * t;
-		double a = 0.0;
-		if (row < NB) {
-#pragma unroll
-			for (int j = 0; j < CC; ++j)
-				if (lane + 32 * j < NB) a += sm[row * NB + lane + 32 * j] * yv[j];
-		}
-		const double v = warp_sum(a);
-		if (lane == 0 && row < NB) x[(int64_t)i * NB + row] = FWD ? v : bv[t] - v;
-	}
+	for (int j = 0; j < CC; ++j) yv[j] = lane + 32 * j < nb ? y[lane + 32 * j] : 0.0;
+	times(dm, yv);
+	const double z = warp_sum4(acc, lane);
+	if (owner) x[(int64_t)i * nb + row] = FWD ? z : bv - z;
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -782,6 +754,7 @@ struct Implicit {
 	double *pV = nullptr, *pJV = nullptr;   // [probe.nb][n] the directions and their products
 	double* inv_dtau = nullptr;   // [n_vol] 1/dtau_e of the current Newton step
 	bool blocks_valid = false;
+	bool u_traced = false;        // c->trace holds the traces of u (within one Krylov solve)
 	bool tangent = true;          // Jacobian products by the analytic linearisation (false: finite differences)
 	// block ILU (built on first use)
 	int ilu_order = -1;           // element order of the levels: DPG_ILU_ORDER_* (-1: not built)
@@ -789,8 +762,7 @@ struct Implicit {
 	int n_colours2 = 0;           // distance-2 colouring: no two elements within two face steps share a colour
 	int* colour2 = nullptr;       // [n_vol]
 	int* nbr = nullptr;           // [n_vol][n_fl] distinct face neighbours (-1: none)
-	int* rank = nullptr;          // [n_vol] position in the element order
-	int* level_elems = nullptr;   // [n_vol] elements grouped by level
+	int* desc = nullptr;          // [n_vol][kIluDesc] rows of the elements grouped by level
 	std::vector<int> level_ptr;   // [n_levels + 1]
 	double* offd = nullptr;       // [n_vol][n_fl][nb][nb] A_{i, nbr[i][s]}
 	double* wbuf = nullptr;       // [n] forward-sweep result
@@ -854,7 +826,7 @@ void implicit_free(dpg_gpu_ctx* c)
 	if (!im) return;
 	void* ptrs[] = {im->u, im->F0, im->F1, im->up, im->du, im->w, im->V, im->Z, im->h, im->h2, im->partial,
 	                im->blocks, im->piv, im->info, im->colour, im->forcing_buf, im->pV, im->pJV, im->colour2, im->nbr,
-	                im->rank, im->level_elems, im->offd, im->wbuf, im->inv_dtau, im->ilu_in, im->ilu_out};
+	                im->desc, im->offd, im->wbuf, im->inv_dtau, im->ilu_in, im->ilu_out};
 	if (im->ilu_graph) cudaGraphExecDestroy(im->ilu_graph);
 	for (void* p : ptrs) if (p) cudaFree(p);
 	free_tangent_work(&im->probe);
@@ -879,6 +851,9 @@ static int residual(dpg_gpu_ctx* c, const double* u, double* F)
 	return rc;
 }
 
+// blocks of a reduction over n values: those past the last value would only add zeros
+static int red_blocks(int64_t n) { return (int)std::min<int64_t>(kRedBlocks, (n + kRedThreads - 1) / kRedThreads); }
+
 static int absmax(dpg_gpu_ctx* c, Implicit* im, const double* x, double* out)
 {
 	k_absmax_partial<<<kRedBlocks, kRedThreads, 0, c->stream>>>(im->n, x, im->partial);
@@ -891,8 +866,10 @@ static int absmax(dpg_gpu_ctx* c, Implicit* im, const double* x, double* out)
 // h[0..nv) = V[0..nv)^T w   (device result in im->h, copied to host_h)
 static int multidot(dpg_gpu_ctx* c, Implicit* im, int nv, const double* V, const double* w, double* host_h)
 {
-	k_multidot_partial<<<kRedBlocks, kRedThreads, 0, c->stream>>>(im->n, nv, V, im->n, w, im->partial);
-	k_reduce_partials<<<nv, 256, 0, c->stream>>>(nv, kRedBlocks, im->partial, im->h);
+	const int blocks = red_blocks(im->n);
+	k_multidot_partial<<<dim3(blocks, (nv + kDotChunk - 1) / kDotChunk), kRedThreads, 0, c->stream>>>(
+	    im->n, nv, V, im->n, const_cast<double*>(w), im->partial);
+	k_reduce_partials<<<nv, 256, 0, c->stream>>>(nv, blocks, im->partial, im->h);
 	if (cudaMemcpyAsync(host_h, im->h, 8 * nv, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) return DPG_ERR_CUDA;
 	if (cudaStreamSynchronize(c->stream) != cudaSuccess) return DPG_ERR_CUDA;
 	return DPG_OK;
@@ -964,48 +941,48 @@ static int assemble_block_jacobi(dpg_gpu_ctx* c, Implicit* im, const double* F0)
 }
 
 // ---- block ILU: structure (once per element order), assembly and factorisation (every Newton step), solve ----
-constexpr int kIluMaxNb = 112;   // D and the product T in shared memory: 2 nb^2 doubles <= 200 KB
+constexpr int kIluMaxNb = 112;   // a block of 4 rows per warp, 28 warps
 
-static bool ilu_staged(int nb, int n_fl) { return nb == 64 && n_fl <= kIluStagedMaxFl; }
+static size_t ilu_update_smem(int nb) { return ((size_t)nb * nb + 3 * (size_t)nb * kIluSlab) * 8; }
+static size_t ilu_invert_smem(int nb) { return ((size_t)nb * nb + 3 * (size_t)nb) * 8 + (size_t)nb * 4; }
 
-static size_t ilu_staged_smem(int nb, int n_fl) { return (size_t)(1 + n_fl) * nb * nb * 8; }
+template <int CC, bool FWD>
+static void launch_sweep_level(dpg_gpu_ctx* c, Implicit* im, int l, bool first, const double* b, double* x)
+{
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3(im->level_ptr[l + 1] - im->level_ptr[l]);
+	cfg.blockDim = dim3(32 * ((im->nb + 3) / 4));
+	cfg.stream = c->stream;
+	cudaLaunchAttribute at{};
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = &at;
+	cfg.numAttrs = first ? 0 : 1;   // the first level waits for what wrote its right-hand side
+	cudaLaunchKernelEx(&cfg, k_ilu_sweep_level<CC, FWD>, (const int*)(im->desc + (size_t)im->level_ptr[l] * kIluDesc), im->nb,
+	                   c->g.n_fl, (const double*)im->blocks, (const double*)im->offd, b, x);
+}
+
+template <int CC>
+static void enqueue_sweeps_of(dpg_gpu_ctx* c, Implicit* im, const double* r, double* z)
+{
+	const int n_levels = (int)im->level_ptr.size() - 1;
+	bool first = true;
+	for (int l = 0; l < n_levels; ++l) {
+		if (im->level_ptr[l + 1] <= im->level_ptr[l]) continue;
+		launch_sweep_level<CC, true>(c, im, l, first, r, im->wbuf);
+		first = false;
+	}
+	for (int l = n_levels - 1; l >= 0; --l)
+		if (im->level_ptr[l + 1] > im->level_ptr[l]) launch_sweep_level<CC, false>(c, im, l, false, im->wbuf, z);
+}
 
 static void enqueue_block_ilu_sweeps(dpg_gpu_ctx* c, Implicit* im, const double* r, double* z)
 {
-	const int nb = im->nb, n_fl = c->g.n_fl;
-	const int n_levels = (int)im->level_ptr.size() - 1;
-	const int threads = kIluSweepThreads;
-	const bool staged = ilu_staged(nb, n_fl);
-	const size_t smem_staged = ilu_staged_smem(nb, n_fl);
-	for (int l = 0; l < n_levels; ++l) {
-		const int cnt = im->level_ptr[l + 1] - im->level_ptr[l];
-		if (cnt <= 0) continue;
-		if (staged)
-			k_ilu_level_staged<64, true><<<cnt, kIluStagedThreads, smem_staged, c->stream>>>(
-			    im->level_elems + im->level_ptr[l], n_fl, im->nbr, im->rank, im->blocks, im->offd, r, im->wbuf);
-		else if (nb == 64)
-			k_ilu_forward_level<64><<<cnt, threads, (size_t)nb * 8, c->stream>>>(im->level_elems + im->level_ptr[l], nb, n_fl,
-			                                                                     im->nbr, im->rank, im->blocks, im->offd, r,
-			                                                                     im->wbuf);
-		else
-			k_ilu_forward_level<0><<<cnt, threads, (size_t)nb * 8, c->stream>>>(im->level_elems + im->level_ptr[l], nb, n_fl,
-			                                                                    im->nbr, im->rank, im->blocks, im->offd, r,
-			                                                                    im->wbuf);
-	}
-	for (int l = n_levels - 1; l >= 0; --l) {
-		const int cnt = im->level_ptr[l + 1] - im->level_ptr[l];
-		if (cnt <= 0) continue;
-		if (staged)
-			k_ilu_level_staged<64, false><<<cnt, kIluStagedThreads, smem_staged, c->stream>>>(
-			    im->level_elems + im->level_ptr[l], n_fl, im->nbr, im->rank, im->blocks, im->offd, im->wbuf, z);
-		else if (nb == 64)
-			k_ilu_backward_level<64><<<cnt, threads, (size_t)nb * 8, c->stream>>>(im->level_elems + im->level_ptr[l], nb,
-			                                                                      n_fl, im->nbr, im->rank, im->blocks,
-			                                                                      im->offd, im->wbuf, z);
-		else
-			k_ilu_backward_level<0><<<cnt, threads, (size_t)nb * 8, c->stream>>>(im->level_elems + im->level_ptr[l], nb,
-			                                                                     n_fl, im->nbr, im->rank, im->blocks,
-			                                                                     im->offd, im->wbuf, z);
+	switch ((im->nb + 31) / 32) {   // columns per lane (nb <= kIluMaxNb)
+	case 1: return enqueue_sweeps_of<1>(c, im, r, z);
+	case 2: return enqueue_sweeps_of<2>(c, im, r, z);
+	case 3: return enqueue_sweeps_of<3>(c, im, r, z);
+	default: return enqueue_sweeps_of<4>(c, im, r, z);
 	}
 }
 
@@ -1085,30 +1062,36 @@ static int ilu_build(dpg_gpu_ctx* c, Implicit* im, int order, int parts)
 	for (int l = 0; l < n_levels; ++l) im->level_ptr[l + 1] += im->level_ptr[l];
 	std::vector<int> elems(n_vol), fill(im->level_ptr.begin(), im->level_ptr.end() - 1);
 	for (int r = 0; r < n_vol; ++r) { const int e = by_rank[r]; elems[fill[level[e]]++] = e; }
+	std::vector<int> desc((size_t)n_vol * kIluDesc, 0);
+	for (int t = 0; t < n_vol; ++t) {
+		int* d = &desc[(size_t)t * kIluDesc];
+		const int e = elems[t];
+		d[0] = e;
+		for (int up = 0; up < 2; ++up)
+			for (int a = 0; a < n_fl; ++a) {
+				const int o = nbr[(size_t)e * n_fl + a];
+				if (o < 0 || (rank[o] > rank[e]) != (up == 1)) continue;
+				const int q = d[1] + d[2];
+				d[3 + 2 * q] = a;
+				d[4 + 2 * q] = o;
+				++d[1 + up];
+			}
+	}
 	bool ok = true;
 	auto al = [&](void** p, size_t bytes) { if (!*p && cudaMalloc(p, bytes ? bytes : 1) != cudaSuccess) ok = false; };
 	al((void**)&im->colour2, (size_t)n_vol * 4); al((void**)&im->nbr, (size_t)n_vol * n_fl * 4);
-	al((void**)&im->rank, (size_t)n_vol * 4); al((void**)&im->level_elems, (size_t)n_vol * 4);
+	al((void**)&im->desc, (size_t)n_vol * kIluDesc * 4);
 	al((void**)&im->offd, (size_t)n_vol * n_fl * nb * nb * 8); al((void**)&im->wbuf, (size_t)im->n * 8);
 	al((void**)&im->ilu_in, (size_t)im->n * 8); al((void**)&im->ilu_out, (size_t)im->n * 8);
 	if (!ok) return DPG_ERR_CUDA;
 	if (cudaMemcpy(im->colour2, col2.data(), (size_t)n_vol * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
 	    cudaMemcpy(im->nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-	    cudaMemcpy(im->rank, rank.data(), (size_t)n_vol * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-	    cudaMemcpy(im->level_elems, elems.data(), (size_t)n_vol * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+	    cudaMemcpy(im->desc, desc.data(), desc.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
 	    cudaMemset(im->offd, 0, (size_t)n_vol * n_fl * nb * nb * 8) != cudaSuccess)
 		return DPG_ERR_CUDA;
-	const int smem = (int)(2 * (size_t)nb * nb * 8 + (size_t)nb * 4);
-	if (cudaFuncSetAttribute(k_ilu_factor_level, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+	if (cudaFuncSetAttribute(k_ilu_update_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ilu_update_smem(kIluMaxNb)) ||
+	    cudaFuncSetAttribute(k_ilu_invert_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ilu_invert_smem(kIluMaxNb)))
 		return DPG_ERR_CUDA;
-	if (ilu_staged(nb, n_fl)) {
-		const int ss = (int)ilu_staged_smem(nb, n_fl);
-		if (cudaFuncSetAttribute(k_ilu_level_staged<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) !=
-		        cudaSuccess ||
-		    cudaFuncSetAttribute(k_ilu_level_staged<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) !=
-		        cudaSuccess)
-			return DPG_ERR_CUDA;
-	}
 	im->n_colours2 = nc2;
 	// the sweeps of one application as a graph: 2 launches per level, replayed with the right-hand side copied into
 	// ilu_in and the result taken from ilu_out (the operands' addresses stay fixed from here on)
@@ -1144,13 +1127,14 @@ static int assemble_block_ilu(dpg_gpu_ctx* c, Implicit* im, const double* F0)
 			                                                       im->blocks, im->offd);
 		}
 	if (cudaMemsetAsync(im->info, 0, 4, c->stream) != cudaSuccess) return DPG_ERR_CUDA;
-	const size_t smem = 2 * (size_t)nb * nb * 8 + (size_t)nb * 4;
-	const int n_levels = (int)im->level_ptr.size() - 1;
+	const int n_levels = (int)im->level_ptr.size() - 1, n_slab = (nb + kIluSlab - 1) / kIluSlab;
+	const int threads = std::min(1024, std::max(128, (nb * nb / 4 + 31) / 32 * 32));
 	for (int l = 0; l < n_levels; ++l) {
 		const int cnt = im->level_ptr[l + 1] - im->level_ptr[l];
+		const int* desc = im->desc + (size_t)im->level_ptr[l] * kIluDesc;
 		if (cnt <= 0) continue;
-		k_ilu_factor_level<<<cnt, 256, smem, c->stream>>>(im->level_elems + im->level_ptr[l], nb, n_fl, im->nbr,
-		                                                  im->rank, im->blocks, im->offd, im->info);
+		if (l > 0) k_ilu_update_level<<<dim3(cnt, n_slab), 256, ilu_update_smem(nb), c->stream>>>(desc, nb, n_fl, im->nbr, im->blocks, im->offd);
+		k_ilu_invert_level<<<cnt, threads, ilu_invert_smem(nb), c->stream>>>(desc, nb, im->blocks, im->info);
 	}
 	int info = 0;
 	if (cudaMemcpyAsync(&info, im->info, 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) return DPG_ERR_CUDA;
@@ -1185,11 +1169,22 @@ static int apply_precond(dpg_gpu_ctx* c, Implicit* im, int precond, const double
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
+// F1 = dF/du z by the tangent; the first product of a Krylov solve also leaves the state's own traces in c->trace, which
+// the next ones read
+static int apply_J(dpg_gpu_ctx* c, Implicit* im, const double* z)
+{
+	TanWork w = c->tan;
+	w.u_traced = im->u_traced;
+	const int rc = jvp_fp64(c, im->u, z, im->F1, w);
+	im->u_traced = true;
+	return rc;
+}
+
 // A z = z / dtau_e - dF/du z: the analytic tangent, or (F(u + eps z) - F(u)) / eps
 static int apply_A(dpg_gpu_ctx* c, Implicit* im, const double* z, double* out, double u_norm, double z_norm)
 {
 	if (im->tangent) {
-		int rc = jvp_fp64(c, im->u, z, im->F1, c->tan);
+		const int rc = apply_J(c, im, z);
 		if (rc) return rc;
 		k_shift_minus<<<grid_for(im->n), 256, 0, c->stream>>>(im->n, im->nb, im->inv_dtau, z, im->F1, out);
 		return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
@@ -1217,6 +1212,7 @@ static int gmres(dpg_gpu_ctx* c, Implicit* im, int precond, double rtol, int max
 	const int m = im->m;
 	const int64_t n = im->n;
 	int rc;
+	im->u_traced = false;
 	if (cudaMemsetAsync(im->du, 0, n * 8, c->stream) != cudaSuccess) return DPG_ERR_CUDA;
 	const double bnorm = host_norm2(c, im, im->F0, &rc);
 	if (rc) return rc;
@@ -1242,18 +1238,38 @@ static int gmres(dpg_gpu_ctx* c, Implicit* im, int precond, double rtol, int max
 				if (rc) return rc;
 			}
 			double* w = im->V + (int64_t)(j + 1) * n;
-			if ((rc = apply_A(c, im, zj, w, u_norm, znorm))) return rc;
-			// classical Gram-Schmidt, twice, and the norm -- all on the device; one copy of the column per iteration
-			k_multidot_partial<<<kRedBlocks, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial);
-			k_reduce_partials<<<j + 1, 256, 0, c->stream>>>(j + 1, kRedBlocks, im->partial, im->h);
-			k_sub_combination<<<grid_for(n), 256, 0, c->stream>>>(n, j + 1, im->V, n, im->h, w);
-			k_multidot_partial<<<kRedBlocks, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial);
-			k_reduce_partials<<<j + 1, 256, 0, c->stream>>>(j + 1, kRedBlocks, im->partial, im->h2);
-			k_sub_combination<<<grid_for(n), 256, 0, c->stream>>>(n, j + 1, im->V, n, im->h2, w);
-			k_multidot_partial<<<kRedBlocks, kRedThreads, 0, c->stream>>>(n, 1, w, n, w, im->partial);
-			k_reduce_partials<<<1, 256, 0, c->stream>>>(1, kRedBlocks, im->partial, im->h2 + j + 1);
-			k_column_finish<<<1, 256, 0, c->stream>>>(j, im->h, im->h2);
-			k_scale_inv<<<grid_for(n), 256, 0, c->stream>>>(n, w, im->h + j + 1);
+			// the product and classical Gram-Schmidt, twice, and the norm -- all on the device; one copy of the column per
+			// iteration
+			const int blocks = red_blocks(n);
+			const dim3 dots(blocks, (j + kDotChunk) / kDotChunk);
+			if (blocks <= kSmallBlocks) {
+				if (im->tangent) {
+					if ((rc = apply_J(c, im, zj))) return rc;
+					k_multidot_partial<<<dots, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial, im->nb, im->inv_dtau,
+					                                                        zj, im->F1);
+				} else {
+					if ((rc = apply_A(c, im, zj, w, u_norm, znorm))) return rc;
+					k_multidot_partial<<<dots, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial);
+				}
+				double* norm_partial = im->partial + (size_t)(m + 1) * kRedBlocks;
+				const size_t sm_h = (size_t)(j + 1) * 8;
+				k_gs_pass<<<blocks, kRedThreads, sm_h, c->stream>>>(n, j + 1, im->V, n, im->partial, im->h, w, nullptr);
+				k_multidot_partial<<<dots, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial);
+				k_gs_pass<<<blocks, kRedThreads, sm_h, c->stream>>>(n, j + 1, im->V, n, im->partial, im->h2, w, norm_partial);
+				k_gs_finish<<<blocks, kRedThreads, 0, c->stream>>>(n, j, norm_partial, im->h, im->h2, w);
+			} else {
+				if ((rc = apply_A(c, im, zj, w, u_norm, znorm))) return rc;
+				k_multidot_partial<<<dots, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial);
+				k_reduce_partials<<<j + 1, 256, 0, c->stream>>>(j + 1, blocks, im->partial, im->h);
+				k_sub_combination<<<grid_for(n), 256, 0, c->stream>>>(n, j + 1, im->V, n, im->h, w);
+				k_multidot_partial<<<dots, kRedThreads, 0, c->stream>>>(n, j + 1, im->V, n, w, im->partial);
+				k_reduce_partials<<<j + 1, 256, 0, c->stream>>>(j + 1, blocks, im->partial, im->h2);
+				k_sub_combination<<<grid_for(n), 256, 0, c->stream>>>(n, j + 1, im->V, n, im->h2, w);
+				k_multidot_partial<<<blocks, kRedThreads, 0, c->stream>>>(n, 1, w, n, w, im->partial);
+				k_reduce_partials<<<1, 256, 0, c->stream>>>(1, blocks, im->partial, im->h2 + j + 1);
+				k_column_finish<<<1, 256, 0, c->stream>>>(j, im->h, im->h2);
+				k_scale_inv<<<grid_for(n), 256, 0, c->stream>>>(n, w, im->h + j + 1);
+			}
 			if (cudaMemcpyAsync(im->hcol_host, im->h, 8 * (j + 2), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
 			    cudaStreamSynchronize(c->stream) != cudaSuccess)
 				return DPG_ERR_CUDA;

@@ -448,9 +448,11 @@ static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* ou
 	} else {
 		const int E1 = elems_of(c, c->trace_block_elems, 1), Et = elems_of(c, c->trace_block_elems, w.nb);
 		const size_t per_t = (size_t)NV * g.n_s * sizeof(double);
-		k_trace<NV><<<(g.n_vol + E1 - 1) / E1, 256, E1 * per_t, c->stream>>>(u, g, c->trace, E1, TanStride{});
+		if (!w.u_traced) {
+			k_trace<NV><<<(g.n_vol + E1 - 1) / E1, 256, E1 * per_t, c->stream>>>(u, g, c->trace, E1, TanStride{});
+			copy_boundary_trace(c, c->trace);
+		}
 		k_trace<NV><<<dim3((g.n_vol + Et - 1) / Et, w.nb), 256, Et * per_t, c->stream>>>(v, g, w.trace_t, Et, ts);
-		copy_boundary_trace(c, c->trace);
 		copy_boundary_trace(c, w.trace_t, w.nb, ts.tr);
 	}
 	if ((rc = launch_face_tan(c, w))) return rc;

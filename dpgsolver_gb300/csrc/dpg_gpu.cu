@@ -65,6 +65,7 @@ static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	c->e_type = sim->ops[0].e_type;
 	for (int a = 0; a < 3; ++a) c->b_adv[a] = sim->b_adv[a];
 	c->n_dof = sim->vol_dof_off[sim->n_vol];
+	if (cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, c->dev) != cudaSuccess || c->n_sm < 1) c->n_sm = 1;
 	if ((rc = dupload(c, &c->sol, sim->sol_coef, (size_t)c->n_dof))) return fail(rc);
 	if ((rc = dalloc(c, &c->solp, (size_t)c->n_dof))) return fail(rc);
 	if ((rc = dalloc(c, &c->rhs, (size_t)c->n_dof))) return fail(rc);

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, G
 	const int ne = min(E_b, g.n_vol - e0);
 	double* sU = sm;  // [ne][NV][n_s]
 	const double* src = sol + (size_t)e0 * NV * n_s;
+	grid_wait();
 	for (int i = threadIdx.x; i < ne * NV * n_s; i += blockDim.x) sU[i] = src[i];
 	__syncthreads();
 	const int per_e = n_fl * NV * n_fc;
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, G
 __global__ void __launch_bounds__(128) k_copy_boundary_trace(const int* __restrict__ bface, int n, int n_fc, double* __restrict__ trace,
                                                              size_t stride)
 {
+	grid_wait();
 	trace += blockIdx.y * stride;
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= n * n_fc) return;
@@ -70,13 +72,14 @@ __global__ void __launch_bounds__(128) k_copy_boundary_trace(const int* __restri
 static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace, int nb = 1, size_t stride = 0)
 {
 	const int n = c->n_bface * c->fc.n_fc;
-	if (n) k_copy_boundary_trace<<<dim3((n + 127) / 128, nb), 128, 0, c->stream>>>(c->bface, c->n_bface, c->fc.n_fc, trace, stride);
+	if (n) launch_chained(k_copy_boundary_trace, dim3((n + 127) / 128, nb), 128, 0, c->stream, c->bface, c->n_bface, c->fc.n_fc, trace, stride);
 }
 
 template <int D, int NV>
 __global__ void __launch_bounds__(256) k_face(const double* __restrict__ trace, FaceDev fd, double* __restrict__ nnf,
                                               int num_flux, double bx, double by, double bz)
 {
+	grid_wait();
 	const int n_fc = fd.n_fc;
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= fd.n_face * n_fc) return;
@@ -116,6 +119,7 @@ __global__ void __launch_bounds__(256) k_volume(double* __restrict__ sol, double
 	double* sU = sm;                          // [E_b][NV][n_s]
 	double* sS = sU + (size_t)E_b * NV * n_s;  // [E_b][NV][n_c]  (reused for the unscaled residual)
 	double* sX = sS + (size_t)E_b * NV * max(n_c, n_s); // [E_b][NV][K]
+	grid_wait();
 	const double* src = sol + (size_t)e0 * NV * n_s;
 	for (int i = threadIdx.x; i < ne * NV * n_s; i += blockDim.x) sU[i] = src[i];
 	__syncthreads();
@@ -236,17 +240,17 @@ static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs,
 		const int E_b = elems_of(c, c->trace_block_elems, 1);
 		const size_t smem = (size_t)E_b * NV * g.n_s * sizeof(double);
 		const int grid = (g.n_vol + E_b - 1) / E_b;
-		k_trace<NV><<<grid, 256, smem, c->stream>>>(c->sol, g, c->trace, E_b, TanStride{});
+		launch_chained(k_trace<NV>, grid, 256, smem, c->stream, c->sol, g, c->trace, E_b, TanStride{});
 		copy_boundary_trace(c, c->trace);
 	} else if (which == 1) {
-		const int n = c->fc.n_face * c->fc.n_fc;
-		k_face<D, NV><<<(n + 127) / 128, 128, 0, c->stream>>>(c->trace, c->fc, c->nnf, c->num_flux,
+		const int n = c->fc.n_face * c->fc.n_fc, t = spread_threads(n, c->n_sm);
+		launch_chained(k_face<D, NV>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
 		                                                     c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	} else {
 		const int E_b = elems_of(c, c->vol_block_elems, 1);
 		const size_t smem = (size_t)E_b * NV * (g.n_s + (g.n_c > g.n_s ? g.n_c : g.n_s) + g.K) * sizeof(double);
 		const int grid = (g.n_vol + E_b - 1) / E_b;
-		k_volume<D, NV><<<grid, 256, smem, c->stream>>>(c->sol, c->solp, c->rhs, c->nnf, g, c->ddt, max_slot, stage,
+		launch_chained(k_volume<D, NV>, grid, 256, smem, c->stream, c->sol, c->solp, c->rhs, c->nnf, g, c->ddt, max_slot, stage,
 		                                               write_rhs ? 1 : 0, E_b, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	}
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
@@ -282,6 +286,7 @@ __global__ void __launch_bounds__(256) k_face_tan(const double* __restrict__ tra
                                                   FaceDev fd, double* __restrict__ nnf_t, int num_flux, double bx,
                                                   double by, double bz, TanStride st)
 {
+	grid_wait();
 	trace_t += blockIdx.y * st.tr;
 	nnf_t += blockIdx.y * st.nf;
 	const int n_fc = fd.n_fc;
@@ -317,6 +322,7 @@ __global__ void __launch_bounds__(256) k_volume_tan(const double* __restrict__ u
                                                     int E_b, double bx, double by, double bz, TanStride st)
 {
 	extern __shared__ double sm[];
+	grid_wait();
 	v += blockIdx.y * st.dof;
 	out += blockIdx.y * st.dof;
 	nnf_t += blockIdx.y * st.nf;
@@ -422,8 +428,8 @@ __global__ void __launch_bounds__(256) k_volume_tan(const double* __restrict__ u
 template <int D, int NV>
 static int face_tan_impl(dpg_gpu_ctx* c, const TanWork& w)
 {
-	const int n = c->fc.n_face * c->fc.n_fc;
-	k_face_tan<D, NV><<<dim3((n + 127) / 128, w.nb), 128, 0, c->stream>>>(c->trace, w.trace_t, c->fc, w.nnf_t, c->num_flux,
+	const int n = c->fc.n_face * c->fc.n_fc, t = spread_threads((int64_t)n * w.nb, c->n_sm);
+	launch_chained(k_face_tan<D, NV>, dim3((n + t - 1) / t, w.nb), t, 0, c->stream, c->trace, w.trace_t, c->fc, w.nnf_t, c->num_flux,
 	                                                                      c->b_adv[0], c->b_adv[1], c->b_adv[2], tan_stride(c));
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
@@ -449,18 +455,17 @@ static int jvp_impl(dpg_gpu_ctx* c, const double* u, const double* v, double* ou
 		const int E1 = elems_of(c, c->trace_block_elems, 1), Et = elems_of(c, c->trace_block_elems, w.nb);
 		const size_t per_t = (size_t)NV * g.n_s * sizeof(double);
 		if (!w.u_traced) {
-			k_trace<NV><<<(g.n_vol + E1 - 1) / E1, 256, E1 * per_t, c->stream>>>(u, g, c->trace, E1, TanStride{});
+			launch_chained(k_trace<NV>, (g.n_vol + E1 - 1) / E1, 256, E1 * per_t, c->stream, u, g, c->trace, E1, TanStride{});
 			copy_boundary_trace(c, c->trace);
 		}
-		k_trace<NV><<<dim3((g.n_vol + Et - 1) / Et, w.nb), 256, Et * per_t, c->stream>>>(v, g, w.trace_t, Et, ts);
+		launch_chained(k_trace<NV>, dim3((g.n_vol + Et - 1) / Et, w.nb), 256, Et * per_t, c->stream, v, g, w.trace_t, Et, ts);
 		copy_boundary_trace(c, w.trace_t, w.nb, ts.tr);
 	}
 	if ((rc = launch_face_tan(c, w))) return rc;
 	if (c->tp) return tp_lift_tan(c, w, out);
 	const int E_b = elems_of(c, c->tan_block_elems, w.nb);
 	const size_t smem = (size_t)E_b * NV * (2 * g.n_s + (g.n_c > g.n_s ? g.n_c : g.n_s) + g.n_c + g.K) * sizeof(double);
-	k_volume_tan<D, NV><<<dim3((g.n_vol + E_b - 1) / E_b, w.nb), 256, smem, c->stream>>>(
-	    u, v, w.nnf_t, g, out, E_b, c->b_adv[0], c->b_adv[1], c->b_adv[2], ts);
+	launch_chained(k_volume_tan<D, NV>, dim3((g.n_vol + E_b - 1) / E_b, w.nb), 256, smem, c->stream, u, v, w.nnf_t, g, out, E_b, c->b_adv[0], c->b_adv[1], c->b_adv[2], ts);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
@@ -573,11 +578,10 @@ static int noalloc_launch(const dpg_noalloc_mesh& m, const double* sol, double* 
 	    cudaFuncSetAttribute(k_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn))
 		return DPG_ERR_CUDA;
 	if (cudaMemsetAsync(slot, 0, sizeof(unsigned long long), st) != cudaSuccess) return DPG_ERR_CUDA;
-	k_trace<NV><<<(g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st>>>(sol, g, trace, E_t, TanStride{});
+	launch_chained(k_trace<NV>, (g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st, sol, g, trace, E_t, TanStride{});
 	const int nq = fd.n_face * fd.n_fc;
-	k_face<D, NV><<<(nq + 127) / 128, 128, 0, st>>>(trace, fd, nnf, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
-	k_volume<D, NV><<<(g.n_vol + E_b - 1) / E_b, 256, E_b * per_v, st>>>(
-	    const_cast<double*>(sol), nullptr, rhs, nnf, g, nullptr, slot, -1, 1, E_b, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
+	launch_chained(k_face<D, NV>, (nq + 127) / 128, 128, 0, st, trace, fd, nnf, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
+	launch_chained(k_volume<D, NV>, (g.n_vol + E_b - 1) / E_b, 256, E_b * per_v, st, const_cast<double*>(sol), nullptr, rhs, nnf, g, nullptr, slot, -1, 1, E_b, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 

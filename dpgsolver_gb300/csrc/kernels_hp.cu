@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(256) k_hp_trace(const double* __restrict__ sol
 	const int e0 = (blockIdx.x - G.blk0) * G.E_b;
 	const int ne = min(G.E_b, G.n_vol - e0);
 	double* sU = sm;   // [ne][NV][n_s]
+	grid_wait();
 	for (int i = threadIdx.x; i < ne * NV * n_s; i += blockDim.x) {
 		const int e = i / (NV * n_s), r = i - e * NV * n_s;
 		sU[i] = sol[h.dof_off[G.vols[e0 + e]] + r];
@@ -112,6 +113,7 @@ template <int D, int NV>
 __global__ void __launch_bounds__(128) k_hp_face(const double* __restrict__ trace, HpDev h, double* __restrict__ nnf,
                                                  int num_flux, double bx, double by, double bz)
 {
+	grid_wait();
 	const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= h.n_fnode) return;
 	const int f = h.node_face[t];
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(256) k_hp_volume(double* __restrict__ sol, dou
 	double* sU = sm;                                    // [E_b][NV][n_s]
 	double* sS = sU + (size_t)E_b * NV * n_s;           // [E_b][NV][max(n_c, n_s)]
 	double* sX = sS + (size_t)E_b * NV * max(n_c, n_s); // [E_b][NV][Kmax]
+	grid_wait();
 	for (int i = threadIdx.x; i < ne * NV * n_s; i += blockDim.x) {
 		const int e = i / (NV * n_s), r = i - e * NV * n_s;
 		sU[i] = sol[h.dof_off[G.vols[e0 + e]] + r];
@@ -448,13 +451,14 @@ static int hp_launch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsig
 	HpState* s = (HpState*)c->hp;
 	const HpDev& h = s->dev;
 	if (which == 0) {
-		k_hp_trace<NV><<<s->blocks, 256, s->smem_trace, c->stream>>>(c->sol, h, s->trace);
+		launch_chained(k_hp_trace<NV>, s->blocks, 256, s->smem_trace, c->stream, c->sol, h, s->trace);
 	} else if (which == 1) {
 		const int64_t n = h.n_fnode;
-		k_hp_face<D, NV><<<(unsigned)((n + 127) / 128), 128, 0, c->stream>>>(s->trace, h, s->nnf, c->num_flux,
+		const int ft = spread_threads(n, c->n_sm);
+		launch_chained(k_hp_face<D, NV>, (unsigned)((n + ft - 1) / ft), ft, 0, c->stream, s->trace, h, s->nnf, c->num_flux,
 		                                                                 c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	} else {
-		k_hp_volume<D, NV><<<s->blocks, 256, s->smem_volume, c->stream>>>(c->sol, c->solp, c->rhs, s->nnf, h, c->ddt,
+		launch_chained(k_hp_volume<D, NV>, s->blocks, 256, s->smem_volume, c->stream, c->sol, c->solp, c->rhs, s->nnf, h, c->ddt,
 		                                                                  max_slot, stage, write_rhs ? 1 : 0,
 		                                                                  c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	}

@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, c
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
 	const bool live = e < ne;
 	load_ops(so, ops);
+	grid_wait();
 	const size_t gi0 = (size_t)e0 * NV * N;
 	const size_t gi = gi0 + (size_t)e * NV * N + i;
 	double r[NV], u0[NV], up[NV], ji = 0.0;
@@ -157,56 +158,60 @@ static bool build_ops(TpState* st, const dpg_element_ops& o)
 	dpg_lagrange_1d(n1, gl, -1.0, st->lm, der);
 	dpg_lagrange_1d(n1, gl, 1.0, st->lp, der);
 	for (int i = 0; i < n1; ++i) { st->wm[i] = st->lm[i] / w[i]; st->wp[i] = st->lp[i] / w[i]; }
+	// the dense operators entry by entry against products of n1 x n1 factors: interpolation, weak derivative, inverse mass
+	// matrix, face traces and lifts
 	const int n_s = o.n_s, n_c = o.n_c, n_fc = o.n_fc;
-	auto digit = [&](int k, int a) { for (; a > 0; --a) k /= n1; return k % n1; };
-	// interpolation, weak derivative and mass matrix inverse entry by entry
+	double D1[25], M1[25], e1[2][5];   // l_s'(Gauss point), 1D inverse mass matrix, solution basis at -1 / +1
+	for (int i = 0; i < n1; ++i)
+		for (int j = 0; j < n1; ++j) {
+			double t = 0.0, m = 0.0;
+			for (int k = 0; k < n1; ++k) {
+				t += st->Ds[i * n1 + k] * st->B[k * n1 + j];
+				m += st->Bi[i * n1 + k] * st->Bi[j * n1 + k] / w[k];
+			}
+			D1[i * n1 + j] = t;
+			M1[i * n1 + j] = m;
+		}
+	for (int s = 0; s < n1; ++s) {
+		e1[0][s] = e1[1][s] = 0.0;
+		for (int j = 0; j < n1; ++j) { e1[0][s] += st->lm[j] * st->B[j * n1 + s]; e1[1][s] += st->lp[j] * st->B[j * n1 + s]; }
+	}
+	std::vector<int> dig((size_t)n_s * 3);   // position along each direction of node k (solution and Gauss nodes alike)
+	for (int k = 0; k < n_s; ++k)
+		for (int a = 0, t = k; a < 3; ++a, t /= n1) dig[3 * k + a] = t % n1;
 	for (int c = 0; c < n_c; ++c)
 		for (int s = 0; s < n_s; ++s) {
-			double b = 1.0;
-			for (int a = 0; a < d; ++a) b *= st->B[digit(c, a) * n1 + digit(s, a)];
-			if (!near(o.cv0_vs_vc[(size_t)c * n_s + s], b, 1.0)) return false;
-			for (int r = 0; r < d; ++r) {   // d phi_s / dr at node c = sum over the collocated basis along r
-				double t = 0.0, wc = 1.0;
-				for (int j = 0; j < n1; ++j) {
-					double y = st->Dw[j * n1 + digit(c, r)] * w[j] / w[digit(c, r)];   // l_j'(x_c)
-					for (int a = 0; a < d; ++a) y *= st->B[(a == r ? j : digit(c, a)) * n1 + digit(s, a)];
-					t += y;
-				}
-				for (int a = 0; a < d; ++a) wc *= w[digit(c, a)];
-				if (!near(o.tw1_vt_vc[((size_t)r * n_s + s) * n_c + c], wc * t, 10.0)) return false;
+			const int *ci = &dig[3 * c], *si = &dig[3 * s];
+			double f[3], g[3], b = 1.0, wc = 1.0, m = 1.0;
+			for (int a = 0; a < d; ++a) {
+				f[a] = st->B[ci[a] * n1 + si[a]];
+				g[a] = D1[ci[a] * n1 + si[a]];
+				b *= f[a];
+				wc *= w[ci[a]];
+				m *= M1[ci[a] * n1 + si[a]];
+			}
+			if (!near(o.cv0_vs_vc[(size_t)c * n_s + s], b, 1.0) || !near(o.m_inv_ref[(size_t)c * n_s + s], m, 1e3)) return false;
+			for (int r = 0; r < d; ++r) {
+				double t = wc;
+				for (int a = 0; a < d; ++a) t *= a == r ? g[a] : f[a];
+				if (!near(o.tw1_vt_vc[((size_t)r * n_s + s) * n_c + c], t, 10.0)) return false;
 			}
 		}
-	for (int i = 0; i < n_s; ++i)
-		for (int j = 0; j < n_s; ++j) {
-			double t = 0.0;
-			for (int c = 0; c < n_c; ++c) {
-				double y = 1.0;
-				for (int a = 0; a < d; ++a)
-					y *= st->Bi[digit(i, a) * n1 + digit(c, a)] * st->Bi[digit(j, a) * n1 + digit(c, a)] / w[digit(c, a)];
-				t += y;
-			}
-			if (!near(o.m_inv_ref[(size_t)i * n_s + j], t, 1e3)) return false;
-		}
-	// faces: the collocated basis at the face nodes, the face weights
-	for (int lf = 0; lf < 2 * d; ++lf) {
-		const int a0 = lf >> 1;
-		const double* l = (lf & 1) ? st->lp : st->lm;
+	for (int lf = 0; lf < 2 * d; ++lf)
 		for (int q = 0; q < n_fc; ++q) {
 			int k[3] = {0, 0, 0}, t = q;
 			double wf = 1.0;
 			for (int a = 0; a < d; ++a)
-				if (a != a0) { k[a] = t % n1; t /= n1; wf *= w[k[a]]; }
+				if (a != (lf >> 1)) { k[a] = t % n1; t /= n1; wf *= w[k[a]]; }
 			for (int s = 0; s < n_s; ++s) {
-				double e = 0.0, y = 1.0;
-				for (int j = 0; j < n1; ++j) e += l[j] * st->B[j * n1 + digit(s, a0)];
+				double y = e1[lf & 1][dig[3 * s + (lf >> 1)]];
 				for (int a = 0; a < d; ++a)
-					if (a != a0) y *= st->B[k[a] * n1 + digit(s, a)];
-				if (!near(o.cv0_vs_fc[((size_t)lf * n_fc + q) * n_s + s], e * y, 1.0) ||
-				    !near(o.tw0_vt_fc[((size_t)lf * n_s + s) * n_fc + q], e * y * wf, 1.0))
+					if (a != (lf >> 1)) y *= st->B[k[a] * n1 + dig[3 * s + a]];
+				if (!near(o.cv0_vs_fc[((size_t)lf * n_fc + q) * n_s + s], y, 1.0) ||
+				    !near(o.tw0_vt_fc[((size_t)lf * n_s + s) * n_fc + q], y * wf, 1.0))
 					return false;
 			}
 		}
-	}
 	return true;
 }
 
@@ -219,11 +224,17 @@ void tp_free(dpg_gpu_ctx* c)
 	c->tp = nullptr;
 }
 
-// Elements per block: as many as fill 256 threads, but no more than leave two blocks per SM, and at least a warp.
+// Elements per block, at most 256 threads: the fewest warps on the fullest SM (a warp's FP64 instruction holds its SM's
+// pipe for ~20 cycles however many of its lanes are in use), the larger block of equal ones.
 static int block_elems(int n_vol, int N, int n_sm)
 {
-	const int fill = (n_vol + 2 * n_sm - 1) / (2 * n_sm), warp = (31 + N) / N;
-	return std::min(most_elems(N), std::max(fill, warp));
+	int best = 1;
+	int64_t cost = INT64_MAX;
+	for (int E = 1; E <= most_elems(N); ++E) {
+		const int64_t blocks = (n_vol + E - 1) / E, c = (blocks + n_sm - 1) / n_sm * ((E * N + 31) / 32);
+		if (c <= cost) { cost = c; best = E; }
+	}
+	return best;
 }
 
 // Shared-memory opt-in at the largest block: one limit for every context of the process.
@@ -247,11 +258,9 @@ static int launch_volume(dpg_gpu_ctx* c, const double* u, const double* v, const
 	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
 	const Ops<N1> ops = ops_of<N1>(st);
 	if (v)
-		k_tp_volume<D, NV, N1, true, kPeriodic><<<dim3(grid, w->nb), threads, smem_volume<D, NV, N1, true>(E), c->stream>>>(
-		    u, v, geo, TpBc{}, ops, c->trace, w->trace_t, w->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2], tan_stride(c));
+		launch_chained(k_tp_volume<D, NV, N1, true, kPeriodic>, dim3(grid, w->nb), threads, smem_volume<D, NV, N1, true>(E), c->stream, u, v, geo, TpBc{}, ops, c->trace, w->trace_t, w->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2], tan_stride(c));
 	else
-		k_tp_volume<D, NV, N1, false, kPeriodic><<<grid, threads, smem_volume<D, NV, N1, false>(E), c->stream>>>(
-		    u, nullptr, geo, TpBc{}, ops, c->trace, nullptr, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2], TanStride{});
+		launch_chained(k_tp_volume<D, NV, N1, false, kPeriodic>, grid, threads, smem_volume<D, NV, N1, false>(E), c->stream, u, nullptr, geo, TpBc{}, ops, c->trace, nullptr, st->G, nullptr, E, c->b_adv[0], c->b_adv[1], c->b_adv[2], TanStride{});
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
@@ -263,8 +272,7 @@ static int launch_lift(dpg_gpu_ctx* c, const double* G, const double* nnf, doubl
 	constexpr int N = ipow(N1, D);
 	const TpGeo geo = geo_of(c);
 	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
-	k_tp_lift<D, NV, N1><<<dim3(grid, nb), threads, smem_lift<D, NV, N1>(E), c->stream>>>(
-	    G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E, tan_stride(c));
+	launch_chained(k_tp_lift<D, NV, N1>, dim3(grid, nb), threads, smem_lift<D, NV, N1>(E), c->stream, G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E, tan_stride(c));
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 

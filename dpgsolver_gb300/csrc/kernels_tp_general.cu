@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* __restrict__ Uc, 
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
 	const bool live = e < ne;
 	load_ops(so, ops);
+	grid_wait();
 	for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) sU[k] = Ld<T>::at(Uc, Uc_t, (size_t)e0 * NV * N + k);
 	double m[D][D], ji = 0.0;
 	if (live) {
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(128) k_tp_face_br2(const double* __restrict__ 
 		fvn += blockIdx.y * ts.tr;
 		nnf += blockIdx.y * ts.nf;
 	}
+	grid_wait();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= n_face * n_fc) return;
 	const int f = t / n_fc, q = t - f * n_fc, qr = V.nc[t];
@@ -321,30 +323,23 @@ static int front(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork
 	const size_t sm_v = smem_volume<D, NV, N1, false>(E), sm_t = smem_volume<D, NV, N1, true>(E);
 	const TanStride ts = tan_stride(c);
 	if (!st->viscous) {
-		if (w) k_tp_volume<D, NV, N1, true, kWalls><<<grid, threads, sm_t, c->stream>>>(
-			u, v, geo, B, ops, c->trace, w->trace_t, w->G, nullptr, E, bx, by, bz, ts);
-		else k_tp_volume<D, NV, N1, false, kWalls><<<grid, threads, sm_v, c->stream>>>(
-			u, nullptr, geo, B, ops, c->trace, nullptr, st->G, nullptr, E, bx, by, bz, ts);
+		if (w) launch_chained(k_tp_volume<D, NV, N1, true, kWalls>, grid, threads, sm_t, c->stream, u, v, geo, B, ops, c->trace, w->trace_t, w->G, nullptr, E, bx, by, bz, ts);
+		else launch_chained(k_tp_volume<D, NV, N1, false, kWalls>, grid, threads, sm_v, c->stream, u, nullptr, geo, B, ops, c->trace, nullptr, st->G, nullptr, E, bx, by, bz, ts);
 		if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
 		return w ? launch_face_tan(c, *w) : launch_face(c);
 	}
 	if constexpr (NV == D + 2) {
 		const TpVisc V{st->mu, st->kappa, st->scale, st->bc, c->fc.nc, c->fc.nrm, c->fc.jf};
-		const int n_fb = (c->fc.n_face * c->fc.n_fc + 127) / 128;
+		const int64_t nq = (int64_t)c->fc.n_face * c->fc.n_fc;
+		const int ft = spread_threads(nq * (w ? w->nb : 1), c->n_sm), n_fb = (int)((nq + ft - 1) / ft);
 		if (w) {
-			k_tp_volume<D, NV, N1, true, kViscous><<<grid, threads, sm_t, c->stream>>>(
-				u, v, geo, B, ops, c->trace, w->trace_t, st->Uc, w->Uc_t, E, bx, by, bz, ts);
-			k_tp_grad<dual, D, NV, N1><<<grid, threads, smem_grad<dual, D, NV, N1>(E), c->stream>>>(
-				st->Uc, w->Uc_t, c->trace, w->trace_t, geo, V, ops, w->fvn, w->G, E, ts);
-			k_tp_face_br2<dual, D, NV><<<dim3(n_fb, w->nb), 128, 0, c->stream>>>(
-				c->trace, w->trace_t, w->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, w->nnf_t, ts);
+			launch_chained(k_tp_volume<D, NV, N1, true, kViscous>, grid, threads, sm_t, c->stream, u, v, geo, B, ops, c->trace, w->trace_t, st->Uc, w->Uc_t, E, bx, by, bz, ts);
+			launch_chained(k_tp_grad<dual, D, NV, N1>, grid, threads, smem_grad<dual, D, NV, N1>(E), c->stream, st->Uc, w->Uc_t, c->trace, w->trace_t, geo, V, ops, w->fvn, w->G, E, ts);
+			launch_chained(k_tp_face_br2<dual, D, NV>, dim3(n_fb, w->nb), ft, 0, c->stream, c->trace, w->trace_t, w->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, w->nnf_t, ts);
 		} else {
-			k_tp_volume<D, NV, N1, false, kViscous><<<grid, threads, sm_v, c->stream>>>(
-				u, nullptr, geo, B, ops, c->trace, nullptr, st->Uc, nullptr, E, bx, by, bz, ts);
-			k_tp_grad<double, D, NV, N1><<<grid, threads, smem_grad<double, D, NV, N1>(E), c->stream>>>(
-				st->Uc, nullptr, c->trace, nullptr, geo, V, ops, st->fvn, st->G, E, ts);
-			k_tp_face_br2<double, D, NV><<<n_fb, 128, 0, c->stream>>>(
-				c->trace, nullptr, st->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, c->nnf, ts);
+			launch_chained(k_tp_volume<D, NV, N1, false, kViscous>, grid, threads, sm_v, c->stream, u, nullptr, geo, B, ops, c->trace, nullptr, st->Uc, nullptr, E, bx, by, bz, ts);
+			launch_chained(k_tp_grad<double, D, NV, N1>, grid, threads, smem_grad<double, D, NV, N1>(E), c->stream, st->Uc, nullptr, c->trace, nullptr, geo, V, ops, st->fvn, st->G, E, ts);
+			launch_chained(k_tp_face_br2<double, D, NV>, n_fb, ft, 0, c->stream, c->trace, nullptr, st->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, c->nnf, ts);
 		}
 		return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 	}

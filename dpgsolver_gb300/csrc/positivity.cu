@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(PencilShape<D, N1>::THREADS, PencilShape<D, N1
 	const bool live = e < n_vol;
 	if (tid < EPB) sflag[tid] = 0;
 
+	grid_wait();
 	// 1. FP32 screen.  b = A^-1 u in FP32 differs from the exact coefficient by at most eps = amp * c, c = |A^-1| |u|
 	//    (amp = 4 (D (n1 + 2) + 2) 2^-24: the truncation of u, the rounding of the operator and the n1-term sums of
 	//    the D passes, with a factor 4 of margin; set by the host), so rho >= b_rho - eps_rho and
@@ -490,6 +491,7 @@ __global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* _
 		sBS[i] = bs64[i];
 		sA32[i] = sb32[i];
 	}
+	grid_wait();
 	__syncthreads();
 	for (int e = blockIdx.x * kDenseWarps + warp; e < n_vol; e += gridDim.x * kDenseWarps) {
 		const int ev = vols ? vols[e] : e;   // mixed orders: the group's volume list and the volumes' offsets
@@ -592,10 +594,10 @@ void launch_limit_dense(dpg_gpu_ctx* c, double* sol, int n_vol, int ns, const fl
 		else cudaFuncSetAttribute(k_positivity_dense<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	}
 	if (c->d == 2)
-		k_positivity_dense<2><<<blocks, kDenseWarps * 32, smem, c->stream>>>(sol, n_vol, ns, sb32, sb64, bs64, amp,
+		launch_chained(k_positivity_dense<2>, blocks, kDenseWarps * 32, smem, c->stream, sol, n_vol, ns, sb32, sb64, bs64, amp,
 		                                                                    c->pos_err, vols, dof_off);
 	else
-		k_positivity_dense<3><<<blocks, kDenseWarps * 32, smem, c->stream>>>(sol, n_vol, ns, sb32, sb64, bs64, amp,
+		launch_chained(k_positivity_dense<3>, blocks, kDenseWarps * 32, smem, c->stream, sol, n_vol, ns, sb32, sb64, bs64, amp,
 		                                                                    c->pos_err, vols, dof_off);
 }
 
@@ -617,7 +619,7 @@ void launch_limit(dpg_gpu_ctx* c, double* sol)
 	}
 	ops.rs = (float)(rs * (1.0 + 1e-6));
 	const int blocks = (c->g.n_vol + S::EPB - 1) / S::EPB;
-	k_positivity<D, N1><<<blocks, S::NT, 0, c->stream>>>(sol, c->g.n_vol, ops, c->pos_amp, c->pos_err);
+	launch_chained(k_positivity<D, N1>, blocks, S::NT, 0, c->stream, sol, c->g.n_vol, ops, c->pos_amp, c->pos_err);
 }
 
 template <int D, int N1>

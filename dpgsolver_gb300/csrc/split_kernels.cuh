@@ -579,6 +579,7 @@ ks_interp(const double* __restrict__ sol, GroupDev g, const float2* __restrict__
 		//    m = tid & 127, K groups kg = (tid >> 7) + kGroups j; column exponent bounds by shared-memory max
 		//    (staged in shared memory so that the digit loop below stays rolled: its unrolled code would be fetched
 		//    once per block, which costs more than the loop)
+		grid_wait();
 		constexpr int NJ = G / kGroups;
 		constexpr int ld_u = 32 * KS + 2;     // +2 doubles: the 16-byte reads of consecutive rows hit distinct banks
 		const int m_r = tid & (kRows - 1), kg0 = tid >> 7;
@@ -947,6 +948,7 @@ ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict_
 		tc::mma_commit_elect(fin);
 		__syncwarp();
 	} else {
+		grid_wait();
 		// column scales from the exponent bounds of the rows: the largest of the row's face parts and volume part
 		if (tid < kRows) {
 			int m = -4000;
@@ -1074,16 +1076,14 @@ __host__ inline SplitArgs args_of(const SplitOp& op) { return SplitArgs{op.tiles
 template <int D, int NV, int KS, int KF, int KC, int FMT, int NP, bool SLICED>
 void launch_interp(dpg_gpu_ctx* c, const SplitState* st)
 {
-	ks_interp<D, NV, KS, KF, KC, FMT, NP, SLICED><<<st->n_blocks, kBlockThreads, st->pi.smem_bytes, c->stream>>>(
-	    c->sol, c->g, st->met2, (float2*)c->trace, st->xl, st->colE, args_of(st->cv), args_of(st->cf), st->pi,
+	launch_chained(ks_interp<D, NV, KS, KF, KC, FMT, NP, SLICED>, st->n_blocks, kBlockThreads, st->pi.smem_bytes, c->stream, c->sol, c->g, st->met2, (float2*)c->trace, st->xl, st->colE, args_of(st->cv), args_of(st->cf), st->pi,
 	    st->EB, st->fp64_eighths, st->b2[0], st->b2[1], st->b2[2], c->b_adv[0], c->b_adv[1], c->b_adv[2], st->err);
 }
 
 template <int D, int NV, int KS, int KF, int KC, int FMT, int NP, bool SLICED>
 void launch_lift(dpg_gpu_ctx* c, const SplitState* st, int stage, int write_rhs, unsigned long long* max_slot)
 {
-	ks_lift<D, NV, KF, KC, FMT, NP, SLICED><<<st->n_blocks, kBlockThreads, st->pl.smem_bytes, c->stream>>>(
-	    c->sol, c->solp, c->rhs, st->xl, st->colE, c->g, args_of(st->lift), st->pl, st->EB,
+	launch_chained(ks_lift<D, NV, KF, KC, FMT, NP, SLICED>, st->n_blocks, kBlockThreads, st->pl.smem_bytes, c->stream, c->sol, c->solp, c->rhs, st->xl, st->colE, c->g, args_of(st->lift), st->pl, st->EB,
 	    c->ddt, max_slot, stage, write_rhs, st->err);
 }
 

@@ -39,10 +39,14 @@ __global__ void __launch_bounds__(256, 4) ks_face(const float2* __restrict__ tra
 #pragma unroll
 	for (int v = 0; v < NV; ++v) { nf[v] = df::mk(0.f); nfd[v] = 0.0; }
 	int elf[2] = {0, 0};
+	int qr = 0;
+	if (active) {   // the side table does not change: before the wait
+		qr = fd.nc[f * n_fc + q];
+		elf[0] = fel[2 * f]; elf[1] = fel[2 * f + 1];
+	}
+	grid_wait();
 	if (active) {
 		const int t = f * n_fc + q;
-		const int qr = fd.nc[t];
-		elf[0] = fel[2 * f]; elf[1] = fel[2 * f + 1];
 		// traces in element order [element][variable][local face * n_fc + node]; the right side at its node qr
 		const int nfq = n_fl * n_fc;
 		const int eL0 = elf[0] / n_fl, eR0 = elf[1] / n_fl;
@@ -354,8 +358,7 @@ template <int D, int NV>
 static void launch_face_k(dpg_gpu_ctx* c, const SplitState* st)
 {
 	const int warps_per_block = st->face_block_warps, threads = 32 * warps_per_block;
-	ks_face<D, NV><<<(st->n_face_warps + warps_per_block - 1) / warps_per_block, threads, 0, c->stream>>>(
-	    (const float2*)c->trace, c->fc, st->nrm2, st->jf2, st->fel, c->g.n_fl, st->xl, 32 * st->KL, st->colE,
+	launch_chained(ks_face<D, NV>, (st->n_face_warps + warps_per_block - 1) / warps_per_block, threads, 0, c->stream, (const float2*)c->trace, c->fc, st->nrm2, st->jf2, st->fel, c->g.n_fl, st->xl, 32 * st->KL, st->colE,
 	    c->num_flux, st->b2[0], st->b2[1], st->b2[2]);
 }
 

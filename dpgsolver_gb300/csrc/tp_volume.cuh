@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 		(KIND == kViscous ? G_t : G) += blockIdx.y * ts.dof;
 	}
 	load_ops(so, ops);
+	grid_wait();
 	{
 		const size_t g0 = (size_t)e0 * NV * N;
 		for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) {

@@ -465,7 +465,11 @@ static int build_step_graph(dpg_gpu_ctx* c)
 	CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
 	int rc = DPG_OK;
 	if (cudaMemsetAsync(c->dmax, 0, sizeof(unsigned long long) * dpg::kMaxStages, c->stream) != cudaSuccess) rc = DPG_ERR_CUDA;
-	for (int stage = 0; stage < 3 && rc == DPG_OK; ++stage) rc = enqueue_stage(c, stage, c->dmax + stage);
+	if (c->tp && c->prec_mode == DPG_PREC_FP64) {
+		if (rc == DPG_OK) rc = dpg::tp_step(c, c->dmax);
+	} else {
+		for (int stage = 0; stage < 3 && rc == DPG_OK; ++stage) rc = enqueue_stage(c, stage, c->dmax + stage);
+	}
 	cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
 	if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
 	if (e != cudaSuccess) return DPG_ERR_CUDA;

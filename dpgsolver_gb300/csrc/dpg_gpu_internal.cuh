@@ -193,6 +193,10 @@ int  tp_general_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);   // boundar
 int  tp_general_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
 int  tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w);
 int  tp_general_launches(dpg_gpu_ctx* c);
+int  tp_general_front(dpg_gpu_ctx* c);     // its first kernel, and those up to the face fluxes (the fused stages of tp_step)
+int  tp_general_fluxes(dpg_gpu_ctx* c);
+int  tp_configure_stage(dpg_gpu_ctx* c);
+int  tp_step(dpg_gpu_ctx* c, unsigned long long* max_slots);   // one SSP-RK3 step with the limiter (kernels_tp_stage.cu)
 
 // mixed orders (kernels_hp.cu): FP64 residual over volume groups of each order; which = 0 traces, 1 face fluxes,
 // 2 volume terms (with the RK stage)

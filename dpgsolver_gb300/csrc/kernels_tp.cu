@@ -21,18 +21,12 @@
 
 #include "dpg_gpu_internal.cuh"
 #include "dpg_host.h"
+#include "tp_lift.cuh"
 #include "tp_volume.cuh"
 
 namespace dpg {
 
 using namespace tp;
-
-template <int D, int NV, int N1>
-static size_t smem_lift(int E)
-{
-	const size_t N = ipow(N1, D), NF = ipow(N1, D - 1);
-	return sizeof(Ops<N1>) + sizeof(double) * E * NV * (2 * N + 2 * D * NF) + 8;
-}
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update of sol (solp holds the step's initial state).  max_slot may
 // be null (the linearisation).
@@ -70,54 +64,7 @@ __global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, c
 		}
 		ji = g.affine ? g.jinv[e0 + e] : g.jinv[(size_t)(e0 + e) * N + i];
 	}
-	for (int o = threadIdx.x; o < ne * 2 * D * NF; o += blockDim.x) {
-		const int ee = o / (2 * D * NF), k = o - ee * 2 * D * NF, lf = k / NF, q = k - lf * NF;
-		const int vf = g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
-		const int f = vf >> 1, side = vf & 1;
-		const int qs = side ? g.nc_inv[(size_t)f * NF + q] : q;
-		const long long flip = side ? 0ll : (long long)0x8000000000000000ull;   // - outward flux of this element
-#pragma unroll
-		for (int w = 0; w < NV; ++w)
-			sF[((size_t)(ee * 2 * D + lf) * NV + w) * NF + q] =
-			    __longlong_as_double(__double_as_longlong(nnf[((size_t)f * NV + w) * NF + qs]) ^ flip);
-	}
-	__syncthreads();
-	if (live) {
-		auto face = [&](auto tag) {
-			constexpr int A = decltype(tag)::value;
-			const int ia = node_along<A, N1>(i), q = face_node<A, N1>(i);
-			const double wm = so->wm[ia], wp = so->wp[ia];
-			const double* F = sF + (size_t)(e * 2 * D + 2 * A) * NV * NF + q;
-#pragma unroll
-			for (int w = 0; w < NV; ++w) r[w] = fma(wp, F[(NV + w) * NF], fma(wm, F[w * NF], r[w]));
-		};
-		face(std::integral_constant<int, 0>{});
-		face(std::integral_constant<int, 1>{});
-		if constexpr (D == 3) face(std::integral_constant<int, 2>{});
-#pragma unroll
-		for (int w = 0; w < NV; ++w) b0[(e * NV + w) * N + i] = r[w] * ji;
-	}
-	__syncthreads();
-	// back to the solution nodes: B^-1 in each direction
-	auto pass = [&](auto tag, const double* src, double* dst) {
-		constexpr int A = decltype(tag)::value;
-		if (live) {
-			const double* row = so->Bi + node_along<A, N1>(i) * N1;
-			const int base = pencil_base<A, N1>(i);
-			double op[N1];
-#pragma unroll
-			for (int j = 0; j < N1; ++j) op[j] = row[j];
-#pragma unroll
-			for (int w = 0; w < NV; ++w) {
-				r[w] = pencil_dot<A, N1>(op, src + (e * NV + w) * N, base);
-				if (A < D - 1) dst[(e * NV + w) * N + i] = r[w];
-			}
-		}
-		if (A < D - 1) __syncthreads();
-	};
-	pass(std::integral_constant<int, 0>{}, b0, b1);
-	pass(std::integral_constant<int, 1>{}, b1, b0);
-	if constexpr (D == 3) pass(std::integral_constant<int, 2>{}, b0, b1);
+	lift_body<D, NV, N1>(so, b0, b1, sF, e0, ne, g, nnf, ji, r);
 	unsigned long long lmax = 0;
 	if (live) {
 		const double dt = (stage >= 0 ? *dt_ptr : 0.0);
@@ -127,9 +74,8 @@ __global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, c
 			const unsigned long long ab = abs_bits_of(r[w]);
 			lmax = ab > lmax ? ab : lmax;
 			if (write_rhs) rhs[k] = r[w];
-			if (stage == 0) { solp[k] = u0[w]; sol[k] = u0[w] + dt * r[w]; }
-			else if (stage == 1) sol[k] = (1.0 / 4.0) * (3.0 * up[w] + u0[w] + dt * r[w]);
-			else if (stage == 2) sol[k] = (1.0 / 3.0) * (up[w] + 2.0 * u0[w] + 2.0 * dt * r[w]);
+			if (stage == 0) solp[k] = u0[w];
+			if (stage >= 0) sol[k] = stage_value(stage, u0[w], up[w], r[w], dt);
 		}
 	}
 	if (max_slot) block_max_to(lmax, s_max, max_slot);
@@ -327,7 +273,8 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 		if (cudaMemcpy(st->jn, ji.data(), sizeof(double) * ji.size(), cudaMemcpyHostToDevice) != cudaSuccess) return DPG_ERR_CUDA;
 	}
 	st->E = block_elems(sim->n_vol, N, c->n_sm);
-	return configure_any(c);
+	const int rc2 = configure_any(c);
+	return rc2 ? rc2 : tp_configure_stage(c);
 }
 
 } // namespace dpg

@@ -307,57 +307,75 @@ static int configure_general(dpg_gpu_ctx* c)
 	return DPG_OK;
 }
 
-// Everything before the lift: traces, boundary states, (gradients,) face fluxes, weak divergence -- of the state u (w null)
-// or their tangents along v[nb][n_dof].
+// What comes before the lift, of the state u (w null) or its tangents along v[nb][n_dof]: the traces and boundary states with
+// the weak divergence or the collocated values (kFront), then (the gradients and) the face fluxes (kFluxes).
+enum { kFront = 1, kFluxes = 2 };
+
 template <int D, int NV, int N1>
-static int front(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w)
+static int before_lift(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w, int parts)
 {
 	const TpState* st = (const TpState*)c->tp;
 	constexpr int N = ipow(N1, D);
 	const TpGeo geo = geo_of(c);
-	const TpBc B{st->bc, st->xyz, c->fc.nrm, st->bp};
 	const int E = st->E, n_blk = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
 	const dim3 grid(n_blk, w ? w->nb : 1);
 	const Ops<N1> ops = ops_of<N1>(st);
-	const double bx = c->b_adv[0], by = c->b_adv[1], bz = c->b_adv[2];
-	const size_t sm_v = smem_volume<D, NV, N1, false>(E), sm_t = smem_volume<D, NV, N1, true>(E);
 	const TanStride ts = tan_stride(c);
-	if (!st->viscous) {
-		if (w) launch_chained(k_tp_volume<D, NV, N1, true, kWalls>, grid, threads, sm_t, c->stream, u, v, geo, B, ops, c->trace, w->trace_t, w->G, nullptr, E, bx, by, bz, ts);
-		else launch_chained(k_tp_volume<D, NV, N1, false, kWalls>, grid, threads, sm_v, c->stream, u, nullptr, geo, B, ops, c->trace, nullptr, st->G, nullptr, E, bx, by, bz, ts);
-		if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
-		return w ? launch_face_tan(c, *w) : launch_face(c);
+	if (parts & kFront) {
+		const TpBc B{st->bc, st->xyz, c->fc.nrm, st->bp};
+		auto go = [&](auto kernel, size_t smem, double* G, double* G_t) {
+			launch_chained(kernel, grid, threads, smem, c->stream, u, v, geo, B, ops, c->trace, w ? w->trace_t : nullptr, G, G_t, E,
+			               c->b_adv[0], c->b_adv[1], c->b_adv[2], ts);
+		};
+		const size_t sm_v = smem_volume<D, NV, N1, false>(E), sm_t = smem_volume<D, NV, N1, true>(E);
+		if constexpr (NV == D + 2) {
+			if (st->viscous && w) go(k_tp_volume<D, NV, N1, true, kViscous>, sm_t, st->Uc, w->Uc_t);
+			else if (st->viscous) go(k_tp_volume<D, NV, N1, false, kViscous>, sm_v, st->Uc, nullptr);
+		}
+		if (!st->viscous && w) go(k_tp_volume<D, NV, N1, true, kWalls>, sm_t, w->G, nullptr);
+		else if (!st->viscous) go(k_tp_volume<D, NV, N1, false, kWalls>, sm_v, st->G, nullptr);
 	}
+	if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
+	if (!(parts & kFluxes)) return DPG_OK;
+	if (!st->viscous) return w ? launch_face_tan(c, *w) : launch_face(c);
 	if constexpr (NV == D + 2) {
 		const TpVisc V{st->mu, st->kappa, st->scale, st->bc, c->fc.nc, c->fc.nrm, c->fc.jf};
 		const int64_t nq = (int64_t)c->fc.n_face * c->fc.n_fc;
 		const int ft = spread_threads(nq * (w ? w->nb : 1), c->n_sm), n_fb = (int)((nq + ft - 1) / ft);
 		if (w) {
-			launch_chained(k_tp_volume<D, NV, N1, true, kViscous>, grid, threads, sm_t, c->stream, u, v, geo, B, ops, c->trace, w->trace_t, st->Uc, w->Uc_t, E, bx, by, bz, ts);
-			launch_chained(k_tp_grad<dual, D, NV, N1>, grid, threads, smem_grad<dual, D, NV, N1>(E), c->stream, st->Uc, w->Uc_t, c->trace, w->trace_t, geo, V, ops, w->fvn, w->G, E, ts);
-			launch_chained(k_tp_face_br2<dual, D, NV>, dim3(n_fb, w->nb), ft, 0, c->stream, c->trace, w->trace_t, w->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, w->nnf_t, ts);
+			launch_chained(k_tp_grad<dual, D, NV, N1>, grid, threads, smem_grad<dual, D, NV, N1>(E), c->stream, st->Uc, w->Uc_t,
+			               c->trace, w->trace_t, geo, V, ops, w->fvn, w->G, E, ts);
+			launch_chained(k_tp_face_br2<dual, D, NV>, dim3(n_fb, w->nb), ft, 0, c->stream, c->trace, w->trace_t, w->fvn, V,
+			               c->fc.n_face, c->fc.n_fc, c->num_flux, w->nnf_t, ts);
 		} else {
-			launch_chained(k_tp_volume<D, NV, N1, false, kViscous>, grid, threads, sm_v, c->stream, u, nullptr, geo, B, ops, c->trace, nullptr, st->Uc, nullptr, E, bx, by, bz, ts);
-			launch_chained(k_tp_grad<double, D, NV, N1>, grid, threads, smem_grad<double, D, NV, N1>(E), c->stream, st->Uc, nullptr, c->trace, nullptr, geo, V, ops, st->fvn, st->G, E, ts);
-			launch_chained(k_tp_face_br2<double, D, NV>, n_fb, ft, 0, c->stream, c->trace, nullptr, st->fvn, V, c->fc.n_face, c->fc.n_fc, c->num_flux, c->nnf, ts);
+			launch_chained(k_tp_grad<double, D, NV, N1>, grid, threads, smem_grad<double, D, NV, N1>(E), c->stream, st->Uc, nullptr,
+			               c->trace, nullptr, geo, V, ops, st->fvn, st->G, E, ts);
+			launch_chained(k_tp_face_br2<double, D, NV>, n_fb, ft, 0, c->stream, c->trace, nullptr, st->fvn, V, c->fc.n_face,
+			               c->fc.n_fc, c->num_flux, c->nnf, ts);
 		}
 		return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 	}
 	return DPG_ERR_UNSUPPORTED;
 }
 
-static int front_any(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w) { DPG_TP_DISPATCH(front, c, u, v, w); }
+static int before_lift_any(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork* w, int parts)
+{
+	DPG_TP_DISPATCH(before_lift, c, u, v, w, parts);
+}
 static int configure_general_any(dpg_gpu_ctx* c) { DPG_TP_DISPATCH(configure_general, c); }
+
+int tp_general_front(dpg_gpu_ctx* c) { return before_lift_any(c, c->sol, nullptr, nullptr, kFront); }
+int tp_general_fluxes(dpg_gpu_ctx* c) { return before_lift_any(c, c->sol, nullptr, nullptr, kFluxes); }
 
 int tp_general_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
 {
-	const int rc = front_any(c, c->sol, nullptr, nullptr);
+	const int rc = before_lift_any(c, c->sol, nullptr, nullptr, kFront | kFluxes);
 	return rc ? rc : tp_lift(c, stage, write_rhs, max_slot);
 }
 
 int tp_general_jvp(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w)
 {
-	const int rc = front_any(c, u, v, &w);
+	const int rc = before_lift_any(c, u, v, &w, kFront | kFluxes);
 	return rc ? rc : tp_lift_tan(c, w, out);
 }
 

@@ -19,41 +19,17 @@ inline size_t smem_volume(int E)
 // kViscous: kWalls, and the collocated values (G, G_t) instead of the weak divergence, which needs the gradients.
 enum { kPeriodic = 0, kWalls = 1, kViscous = 2 };
 
+// What follows the state in b0 (all threads synchronised): values at the Gauss points, traces, (boundary states,) and the weak
+// divergence or the collocated values.
 template <int D, int NV, int N1, bool TAN, int KIND>
-__global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g, TpBc B,
-                                                   const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
-                                                   double* __restrict__ trace_t, double* __restrict__ G,
-                                                   double* __restrict__ G_t, int E, double bx, double by, double bz, TanStride ts)
+__device__ __forceinline__ void volume_body(const Ops<N1>* so, double* b0, double* b1, double* fl, int e0, int ne, int E, bool first,
+                                            const TpGeo& g, const TpBc& B, double* __restrict__ trace,
+                                            double* __restrict__ trace_t, double* __restrict__ G, double* __restrict__ G_t,
+                                            double bx, double by, double bz)
 {
 	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1), NW = TAN ? 2 * NV : NV;
-	extern __shared__ double sm[];
-	Ops<N1>* so = reinterpret_cast<Ops<N1>*>(sm);
-	double* b0 = sm + sizeof(Ops<N1>) / sizeof(double);
-	double* b1 = b0 + (size_t)E * NW * N;
-	double* fl = b1 + (size_t)E * NW * N;   // [D - 1][E][NV][N]
-	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
 	const bool live = e < ne;
-	const bool first = blockIdx.y == 0;   // TAN: the direction that writes the values all directions share
-	if constexpr (TAN) {
-		v += blockIdx.y * ts.dof;
-		trace_t += blockIdx.y * ts.tr;
-		(KIND == kViscous ? G_t : G) += blockIdx.y * ts.dof;
-	}
-	load_ops(so, ops);
-	grid_wait();
-	{
-		const size_t g0 = (size_t)e0 * NV * N;
-		for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) {
-			if constexpr (TAN) {
-				const int ee = k / (NV * N), r = k - ee * NV * N;
-				b0[ee * NW * N + r] = u[g0 + k];
-				b0[ee * NW * N + NV * N + r] = v[g0 + k];
-			} else {
-				b0[k] = u[g0 + k];
-			}
-		}
-	}
 	double m[D][D];   // of this node's element (affine) or node
 	if (KIND != kViscous && live) {
 #pragma unroll
@@ -63,7 +39,6 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 				m[x][r] = g.affine ? g.met[(size_t)(e0 + e) * D * D + x + D * r]
 				                   : g.met[((size_t)(e0 + e) * D * D + x + D * r) * N + i];
 	}
-	__syncthreads();
 	// values at the Gauss points: pass 0 b0 -> b1, pass 1 b1 -> b0, (pass 2 b0 -> b1)
 	double s[NW];
 	auto pass = [&](auto tag, const double* src, double* dst) {
@@ -178,6 +153,41 @@ __global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u,
 #pragma unroll
 		for (int w = 0; w < NV; ++w) G[((size_t)(e0 + e) * NV + w) * N + i] = acc[w];
 	}
+}
+
+template <int D, int NV, int N1, bool TAN, int KIND>
+__global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g, TpBc B,
+                                                   const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
+                                                   double* __restrict__ trace_t, double* __restrict__ G,
+                                                   double* __restrict__ G_t, int E, double bx, double by, double bz, TanStride ts)
+{
+	constexpr int N = ipow(N1, D), NW = TAN ? 2 * NV : NV;
+	extern __shared__ double sm[];
+	Ops<N1>* so = reinterpret_cast<Ops<N1>*>(sm);
+	double* b0 = sm + sizeof(Ops<N1>) / sizeof(double);
+	double* b1 = b0 + (size_t)E * NW * N;
+	double* fl = b1 + (size_t)E * NW * N;   // [D - 1][E][NV][N]
+	const int e0 = blockIdx.x * E, ne = min(E, g.n_vol - e0);
+	const bool first = blockIdx.y == 0;   // TAN: the direction that writes the values all directions share
+	if constexpr (TAN) {
+		v += blockIdx.y * ts.dof;
+		trace_t += blockIdx.y * ts.tr;
+		(KIND == kViscous ? G_t : G) += blockIdx.y * ts.dof;
+	}
+	load_ops(so, ops);
+	grid_wait();
+	const size_t g0 = (size_t)e0 * NV * N;
+	for (int k = threadIdx.x; k < ne * NV * N; k += blockDim.x) {
+		if constexpr (TAN) {
+			const int ee = k / (NV * N), r = k - ee * NV * N;
+			b0[ee * NW * N + r] = u[g0 + k];
+			b0[ee * NW * N + NV * N + r] = v[g0 + k];
+		} else {
+			b0[k] = u[g0 + k];
+		}
+	}
+	__syncthreads();
+	volume_body<D, NV, N1, TAN, KIND>(so, b0, b1, fl, e0, ne, E, first, g, B, trace, trace_t, G, G_t, bx, by, bz);
 }
 
 } // namespace tp

@@ -29,7 +29,7 @@ __device__ __forceinline__ void atomic_max_abs(unsigned long long* slot, double 
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) k_trace(const double* __restrict__ sol, GroupDev g, double* __restrict__ trace, int E_b,
+__global__ void __launch_bounds__(256) k_trace(const double* sol, GroupDev g, double* __restrict__ trace, int E_b,
                                                TanStride st)
 {
 	extern __shared__ double sm[];
@@ -76,7 +76,7 @@ static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace, int nb = 1, size_
 }
 
 template <int D, int NV>
-__global__ void __launch_bounds__(256) k_face(const double* __restrict__ trace, FaceDev fd, double* __restrict__ nnf,
+__global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, double* __restrict__ nnf,
                                               int num_flux, double bx, double by, double bz)
 {
 	grid_wait();
@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(256) k_face(const double* __restrict__ trace, 
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update of sol (solp holds the step's initial state).
 template <int D, int NV>
-__global__ void __launch_bounds__(256) k_volume(double* __restrict__ sol, double* __restrict__ solp, double* __restrict__ rhs,
-                                                const double* __restrict__ nnf, GroupDev g, const double* __restrict__ dt_ptr,
+__global__ void __launch_bounds__(256) k_volume(double* sol, double* solp, double* __restrict__ rhs,
+                                                const double* nnf, GroupDev g, const double* __restrict__ dt_ptr,
                                                 unsigned long long* max_slot, int stage, int write_rhs, int E_b,
                                                 double bx, double by, double bz)
 {
@@ -282,7 +282,7 @@ int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long*
 // (no difference quotient): the element blocks and the Krylov products of the implicit solver use them.
 // ------------------------------------------------------------------------------------------------------------
 template <int D, int NV>
-__global__ void __launch_bounds__(256) k_face_tan(const double* __restrict__ trace, const double* __restrict__ trace_t,
+__global__ void __launch_bounds__(256) k_face_tan(const double* trace, const double* trace_t,
                                                   FaceDev fd, double* __restrict__ nnf_t, int num_flux, double bx,
                                                   double by, double bz, TanStride st)
 {
@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(256) k_face_tan(const double* __restrict__ tra
 }
 
 template <int D, int NV>
-__global__ void __launch_bounds__(256) k_volume_tan(const double* __restrict__ u, const double* __restrict__ v,
-                                                    const double* __restrict__ nnf_t, GroupDev g, double* __restrict__ out,
+__global__ void __launch_bounds__(256) k_volume_tan(const double* u, const double* v,
+                                                    const double* nnf_t, GroupDev g, double* __restrict__ out,
                                                     int E_b, double bx, double by, double bz, TanStride st)
 {
 	extern __shared__ double sm[];

@@ -78,7 +78,7 @@ __device__ __forceinline__ void hp_atomic_max_abs(unsigned long long* slot, doub
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) k_hp_trace(const double* __restrict__ sol, HpDev h, double* __restrict__ trace)
+__global__ void __launch_bounds__(256) k_hp_trace(const double* sol, HpDev h, double* __restrict__ trace)
 {
 	extern __shared__ double sm[];
 	const HpGroup& G = h.grp[hp_group_of(h, blockIdx.x)];
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) k_hp_trace(const double* __restrict__ sol
 }
 
 template <int D, int NV>
-__global__ void __launch_bounds__(128) k_hp_face(const double* __restrict__ trace, HpDev h, double* __restrict__ nnf,
+__global__ void __launch_bounds__(128) k_hp_face(const double* trace, HpDev h, double* __restrict__ nnf,
                                                  int num_flux, double bx, double by, double bz)
 {
 	grid_wait();
@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(128) k_hp_face(const double* __restrict__ trac
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update (solp holds the step's initial state).
 template <int D, int NV>
-__global__ void __launch_bounds__(256) k_hp_volume(double* __restrict__ sol, double* __restrict__ solp,
-                                                   double* __restrict__ rhs, const double* __restrict__ nnf, HpDev h,
+__global__ void __launch_bounds__(256) k_hp_volume(double* sol, double* solp,
+                                                   double* __restrict__ rhs, const double* nnf, HpDev h,
                                                    const double* __restrict__ dt_ptr, unsigned long long* max_slot,
                                                    int stage, int write_rhs, double bx, double by, double bz)
 {

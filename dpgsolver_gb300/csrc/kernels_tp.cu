@@ -31,9 +31,9 @@ using namespace tp;
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update of sol (solp holds the step's initial state).  max_slot may
 // be null (the linearisation).
 template <int D, int NV, int N1>
-__global__ void __launch_bounds__(256) k_tp_lift(const double* __restrict__ G, const double* __restrict__ nnf, TpGeo g,
-                                                 const __grid_constant__ Ops<N1> ops, double* __restrict__ sol,
-                                                 double* __restrict__ solp, double* __restrict__ rhs,
+__global__ void __launch_bounds__(256) k_tp_lift(const double* G, const double* nnf, TpGeo g,
+                                                 const __grid_constant__ Ops<N1> ops, double* sol,
+                                                 double* solp, double* __restrict__ rhs,
                                                  const double* __restrict__ dt_ptr, unsigned long long* max_slot, int stage,
                                                  int write_rhs, int E, TanStride ts)
 {

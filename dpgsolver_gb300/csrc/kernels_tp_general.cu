@@ -58,8 +58,8 @@ static size_t smem_grad(int E)
 }
 
 template <class T, int D, int NV, int N1>
-__global__ void __launch_bounds__(256) k_tp_grad(const double* __restrict__ Uc, const double* __restrict__ Uc_t,
-                                                 const double* __restrict__ trace, const double* __restrict__ trace_t, TpGeo g,
+__global__ void __launch_bounds__(256) k_tp_grad(const double* Uc, const double* Uc_t,
+                                                 const double* trace, const double* trace_t, TpGeo g,
                                                  TpVisc V, const __grid_constant__ Ops<N1> ops, double* __restrict__ fvn,
                                                  double* __restrict__ G, int E, TanStride ts)
 {
@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* __restrict__ Uc, 
 }
 
 template <class T, int D, int NV>
-__global__ void __launch_bounds__(128) k_tp_face_br2(const double* __restrict__ trace, const double* __restrict__ trace_t,
-                                                     const double* __restrict__ fvn, TpVisc V, int n_face, int n_fc,
+__global__ void __launch_bounds__(128) k_tp_face_br2(const double* trace, const double* trace_t,
+                                                     const double* fvn, TpVisc V, int n_face, int n_fc,
                                                      int num_flux, double* __restrict__ nnf, TanStride ts)
 {
 	if constexpr (Ld<T>::tan) {

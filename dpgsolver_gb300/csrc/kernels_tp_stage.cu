@@ -17,7 +17,7 @@ using namespace pos;
 // same size as work space, flag [E].  All threads call; the pencil of thread t < E P is t % P of element t / P.
 template <int D, int N1>
 __device__ __forceinline__ void limit_block(const PosOps& ops, float amp, double* b0, double* b1, int* flag, int E, int ne,
-                                            double* __restrict__ sol, int* __restrict__ err)
+                                            double* sol, int* __restrict__ err)
 {
 	constexpr int NS = ipow(N1, D), NV = D + 2, P = NS / N1;
 	const int tid = threadIdx.x, el = tid / P, q = tid - el * P;
@@ -157,10 +157,10 @@ static size_t smem_stage(int E)
 }
 
 template <int D, int NV, int N1, int KIND>
-__global__ void __launch_bounds__(256) k_tp_stage(double* G, const double* __restrict__ nnf, TpGeo g, TpBc B,
+__global__ void __launch_bounds__(256) k_tp_stage(double* G, const double* nnf, TpGeo g, TpBc B,
                                                   const __grid_constant__ Ops<N1> ops, const __grid_constant__ PosOps pops,
-                                                  float amp, int* __restrict__ pos_err, double* __restrict__ sol,
-                                                  double* __restrict__ solp, const double* __restrict__ dt_ptr,
+                                                  float amp, int* __restrict__ pos_err, double* sol,
+                                                  double* solp, const double* __restrict__ dt_ptr,
                                                   unsigned long long* max_slot, int stage, int limit, int next,
                                                   double* __restrict__ trace, double* Gn, int E, double bx, double by, double bz)
 {

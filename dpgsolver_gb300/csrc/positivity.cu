@@ -108,7 +108,7 @@ __device__ __forceinline__ void tp_pencils64(const PosOps& ops, double* s, int e
 }
 
 template <int D, int N1>
-__global__ void __launch_bounds__(PencilShape<D, N1>::THREADS, PencilShape<D, N1>::MINB) k_positivity(double* __restrict__ sol, int n_vol,
+__global__ void __launch_bounds__(PencilShape<D, N1>::THREADS, PencilShape<D, N1>::MINB) k_positivity(double* sol, int n_vol,
                                                                           const __grid_constant__ PosOps ops,
                                                                           float amp, int* __restrict__ err)
 {
@@ -369,7 +369,7 @@ __device__ bool limit_volume_n(double* w, int ns)
 }
 
 template <int D>
-__global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* __restrict__ sol, int n_vol, int ns,
+__global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* sol, int n_vol, int ns,
                                                                      const float* __restrict__ sb32,
                                                                      const double* __restrict__ sb64,
                                                                      const double* __restrict__ bs64, float amp,

@@ -330,6 +330,14 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
 }
 
+// 32 bytes, a whole sector, in one load (32-byte aligned), where a thread's neighbours read other rows: as two 16-byte loads
+// each sector is fetched twice (ks_lift on 196,608 TETs p = 3, two steps: 17.8 -> 17.5 ms; 32x32x8 HEX p = 3: 3,665 -> 3,631 us).
+// Volatile: it stays behind grid_wait.
+__device__ __forceinline__ void load_sector(const double* p, double* x)
+{
+	asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p));
+}
+
 __device__ __forceinline__ void fail(int* err, int code) { atomicExch(err, code); }
 
 // Barrier of the compute warps only (the issuing warp runs its own loop meanwhile).
@@ -508,7 +516,7 @@ struct InterpChunk {
 
 template <int D, int NV, int KS, int KF, int KC, int FMT, int NP, bool SLICED>
 __global__ void __launch_bounds__(kBlockThreads, 1)
-ks_interp(const double* __restrict__ sol, GroupDev g, const float2* __restrict__ met2, float2* __restrict__ trace,
+ks_interp(const double* sol, GroupDev g, const float2* __restrict__ met2, float2* __restrict__ trace,
           double* __restrict__ xl, int* __restrict__ colE, SplitArgs Acv, SplitArgs Acf, Plan P, int EB,
           int fp64_eighths, float2 bx, float2 by, float2 bz, double bxd, double byd, double bzd, int* err)
 {
@@ -876,8 +884,8 @@ __device__ __forceinline__ void store_digits8_tmem(uint32_t ta, const double (&x
 
 template <int D, int NV, int KF, int KC, int FMT, int NP, bool SLICED>
 __global__ void __launch_bounds__(kBlockThreads, 1)
-ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict__ rhs, const double* __restrict__ xl,
-        const int* __restrict__ colE, GroupDev g,
+ks_lift(double* sol, double* solp, double* __restrict__ rhs, const double* xl,
+        const int* colE, GroupDev g,
         SplitArgs Al, Plan P, int EB, const double* __restrict__ dt_ptr, unsigned long long* max_slot, int stage,
         int write_rhs, int* err)
 {
@@ -949,7 +957,24 @@ ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict_
 		__syncwarp();
 	} else {
 		grid_wait();
-		// column scales from the exponent bounds of the rows: the largest of the row's face parts and volume part
+		// thread items: data row m_r, K group kg0 = tid >> 7 of each chunk, i.e. half h_r = kg0 >> 1 (threads
+		// 256 h_r ..) at K offset 8 (kg0 & 1) within it; the raw values of a chunk are loaded two chunks ahead of
+		// its digits (registers), so the global latency is covered
+		const int m_r = tid & (kRows - 1), kg0 = tid >> 7, h_r = kg0 >> 1;
+		const double* xrow = xl + ((size_t)e0 * NV + m_r) * LDX;   // the block's rows are contiguous
+		const uint32_t ta0 = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kDigCol + (uint32_t)((kg0 & 1) * (pc / 2));
+		auto load_chunk = [&](int c, double (&xv)[8]) {
+			if (m_r >= rows) {
+#pragma unroll
+				for (int jj = 0; jj < 8; ++jj) xv[jj] = 0.0;
+			} else {
+				load_sector(xrow + 32 * c + 8 * kg0, xv);
+				load_sector(xrow + 32 * c + 8 * kg0 + 4, xv + 4);
+			}
+		};
+		// column scales from the exponent bounds of the rows: the largest of the row's face parts and volume part.  The
+		// first chunks are loaded behind the barrier: in front of it they take the L2's time from other blocks' digits
+		// (196,608 TETs p = 3, two steps: 17.5 -> 17.8 ms).
 		if (tid < kRows) {
 			int m = -4000;
 			if (tid < rows) {   // the row's 8 slots in two 16-byte loads
@@ -960,24 +985,12 @@ ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict_
 			colF[tid] = tid < rows ? col_exp_of(m, NP) : 0;
 		}
 		compute_sync();
-
-		// thread items: data row m_r, K group kg0 = tid >> 7 of each chunk, i.e. half h_r = kg0 >> 1 (threads
-		// 256 h_r ..) at K offset 8 (kg0 & 1) within it; the raw values of a chunk are loaded two chunks ahead of
-		// its digits (registers), so the global latency is covered
-		const int m_r = tid & (kRows - 1), kg0 = tid >> 7, h_r = kg0 >> 1;
 		const int F_r = colF[m_r];
-		const double* xrow = xl + ((size_t)e0 * NV + m_r) * LDX;   // the block's rows are contiguous
-		const uint32_t ta0 = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kDigCol + (uint32_t)((kg0 & 1) * (pc / 2));
-		auto load_chunk = [&](int c, double (&xv)[8]) {
-			if (m_r >= rows) {
-#pragma unroll
-				for (int jj = 0; jj < 8; ++jj) xv[jj] = 0.0;
-			} else {
-				const double2* p = (const double2*)(xrow + 32 * c + 8 * kg0);
-#pragma unroll
-				for (int h = 0; h < 4; ++h) { const double2 t2 = p[h]; xv[2 * h] = t2.x; xv[2 * h + 1] = t2.y; }
-			}
-		};
+		double x0[8], x1[8], x2[8];
+		load_chunk(0, x0);
+		if (KL > 1) load_chunk(1, x1);
+		if (KL > 2) load_chunk(2, x2);
+
 		// three register sets in rotation, the loop unrolled by three: chunk c + 3 is loaded into the set of chunk c
 		// right after its digits are written, so every load has two chunks of digit work to land in (a register move
 		// of a set would wait for its pending loads, i.e. shorten that distance to one chunk)
@@ -991,10 +1004,6 @@ ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict_
 			tc::fence_before_sync();
 			mbar_arrive(&hready[s]);
 		};
-		double x0[8], x1[8], x2[8];
-		load_chunk(0, x0);
-		if (KL > 1) load_chunk(1, x1);
-		if (KL > 2) load_chunk(2, x2);
 #pragma unroll 1
 		for (int c = 0; c < KL; c += 3) {
 			digits(c, x0);
@@ -1020,11 +1029,13 @@ ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict_
 		const int Fm = colF[m];
 		const size_t rbase = ((size_t)e0 * NV + m) * n_s;   // the row's first node
 		double u0[8], up[8];
+		int re[8];   // with the state: a load between the stores below would wait for them one by one
 		auto load_state = [&](int c8) {
 #pragma unroll
 			for (int j = 0; j < 8; ++j) {
 				const int node = 8 * c8 + j;
 				const bool in = live && node < n_s;
+				if constexpr (SLICED) re[j] = Al.row_exp[node];
 				u0[j] = (in && stage >= 0) ? sol[rbase + node] : 0.0;
 				up[j] = (in && stage >= 1) ? solp[rbase + node] : 0.0;
 			}
@@ -1043,7 +1054,7 @@ ks_lift(double* __restrict__ sol, double* __restrict__ solp, double* __restrict_
 				const int node = 8 * c8 + j;
 				if (!live || node >= n_s) continue;
 				df::df64 y = v8[j];
-				if constexpr (SLICED) y = df::scale_pow2(y, Al.row_exp[node] + Fm - 48);
+				if constexpr (SLICED) y = df::scale_pow2(y, re[j] + Fm - 48);
 				// the residual in double-float (~2^-47 relative): it enters the state only through dt * r, so the
 				// stage update below (FP64, the only FP64 instructions here) keeps the state's full precision
 				const double r = df::to_double(df::mul(y, jv));

@@ -17,7 +17,7 @@ inline size_t smem_lift(int E)
 // nodes.  b0, b1: [E][NV][N]; sF: [E][2 D][NV][NF].
 template <int D, int NV, int N1>
 __device__ __forceinline__ void lift_body(const Ops<N1>* so, double* b0, double* b1, double* sF, int e0, int ne,
-                                          const TpGeo& g, const double* __restrict__ nnf, double ji, double (&r)[NV])
+                                          const TpGeo& g, const double* nnf, double ji, double (&r)[NV])
 {
 	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1);
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;

@@ -156,7 +156,7 @@ __device__ __forceinline__ void volume_body(const Ops<N1>* so, double* b0, doubl
 }
 
 template <int D, int NV, int N1, bool TAN, int KIND>
-__global__ void __launch_bounds__(256) k_tp_volume(const double* __restrict__ u, const double* __restrict__ v, TpGeo g, TpBc B,
+__global__ void __launch_bounds__(256) k_tp_volume(const double* u, const double* v, TpGeo g, TpBc B,
                                                    const __grid_constant__ Ops<N1> ops, double* __restrict__ trace,
                                                    double* __restrict__ trace_t, double* __restrict__ G,
                                                    double* __restrict__ G_t, int E, double bx, double by, double bz, TanStride ts)

@@ -46,6 +46,12 @@ __device__ __forceinline__ dual sqrt(dual a)
 	const double s = ::sqrt(a.v);
 	return dual(s, s > 0.0 ? a.d / (2.0 * s) : 0.0);
 }
+using ::rsqrt;
+__device__ __forceinline__ dual rsqrt(dual a)
+{
+	const double r = ::rsqrt(a.v);
+	return dual(r, -0.5 * r * r * r * a.d);
+}
 using ::pow;
 __device__ __forceinline__ dual pow(dual a, double e)
 {

@@ -75,7 +75,7 @@ static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace, int nb = 1, size_
 	if (n) launch_chained(k_copy_boundary_trace, dim3((n + 127) / 128, nb), 128, 0, c->stream, c->bface, c->n_bface, c->fc.n_fc, trace, stride);
 }
 
-template <int D, int NV>
+template <int D, int NV, bool RS>
 __global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, double* __restrict__ nnf,
                                               int num_flux, double bx, double by, double bz)
 {
@@ -94,8 +94,14 @@ __global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, d
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = fd.nrm[(size_t)t * D + a];
 	if constexpr (NV == D + 2) {
-		if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike<D>(WL, WR, n, nf);
-		else                                   numflux_lax_friedrichs<D>(WL, WR, n, nf);
+		if constexpr (RS) {
+			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
+			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
+		} else if (num_flux == DPG_NUM_FLUX_ROE_PIKE) {
+			numflux_roe_pike<D>(WL, WR, n, nf);
+		} else {
+			numflux_lax_friedrichs<D>(WL, WR, n, nf);
+		}
 	} else {
 		const double b[3] = {bx, by, bz};
 		nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
@@ -244,7 +250,7 @@ static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs,
 		copy_boundary_trace(c, c->trace);
 	} else if (which == 1) {
 		const int n = c->fc.n_face * c->fc.n_fc, t = spread_threads(n, c->n_sm);
-		launch_chained(k_face<D, NV>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
+		launch_chained(c->tp ? k_face<D, NV, true> : k_face<D, NV, false>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
 		                                                     c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	} else {
 		const int E_b = elems_of(c, c->vol_block_elems, 1);
@@ -281,7 +287,7 @@ int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long*
 // physical flux and lifts the tangents of [fr ; nnf] with the same operators.  The products are exact to rounding
 // (no difference quotient): the element blocks and the Krylov products of the implicit solver use them.
 // ------------------------------------------------------------------------------------------------------------
-template <int D, int NV>
+template <int D, int NV, bool RS>
 __global__ void __launch_bounds__(256) k_face_tan(const double* trace, const double* trace_t,
                                                   FaceDev fd, double* __restrict__ nnf_t, int num_flux, double bx,
                                                   double by, double bz, TanStride st)
@@ -305,8 +311,14 @@ __global__ void __launch_bounds__(256) k_face_tan(const double* trace, const dou
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = fd.nrm[(size_t)t * D + a];
 	if constexpr (NV == D + 2) {
-		if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike<D>(WL, WR, n, nf);
-		else                                   numflux_lax_friedrichs<D>(WL, WR, n, nf);
+		if constexpr (RS) {
+			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
+			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
+		} else if (num_flux == DPG_NUM_FLUX_ROE_PIKE) {
+			numflux_roe_pike<D>(WL, WR, n, nf);
+		} else {
+			numflux_lax_friedrichs<D>(WL, WR, n, nf);
+		}
 	} else {
 		const double b[3] = {bx, by, bz};
 		nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
@@ -429,7 +441,7 @@ template <int D, int NV>
 static int face_tan_impl(dpg_gpu_ctx* c, const TanWork& w)
 {
 	const int n = c->fc.n_face * c->fc.n_fc, t = spread_threads((int64_t)n * w.nb, c->n_sm);
-	launch_chained(k_face_tan<D, NV>, dim3((n + t - 1) / t, w.nb), t, 0, c->stream, c->trace, w.trace_t, c->fc, w.nnf_t, c->num_flux,
+	launch_chained(c->tp ? k_face_tan<D, NV, true> : k_face_tan<D, NV, false>, dim3((n + t - 1) / t, w.nb), t, 0, c->stream, c->trace, w.trace_t, c->fc, w.nnf_t, c->num_flux,
 	                                                                      c->b_adv[0], c->b_adv[1], c->b_adv[2], tan_stride(c));
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
@@ -580,7 +592,7 @@ static int noalloc_launch(const dpg_noalloc_mesh& m, const double* sol, double* 
 	if (cudaMemsetAsync(slot, 0, sizeof(unsigned long long), st) != cudaSuccess) return DPG_ERR_CUDA;
 	launch_chained(k_trace<NV>, (g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st, sol, g, trace, E_t, TanStride{});
 	const int nq = fd.n_face * fd.n_fc;
-	launch_chained(k_face<D, NV>, (nq + 127) / 128, 128, 0, st, trace, fd, nnf, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
+	launch_chained(k_face<D, NV, false>, (nq + 127) / 128, 128, 0, st, trace, fd, nnf, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
 	launch_chained(k_volume<D, NV>, (g.n_vol + E_b - 1) / E_b, 256, E_b * per_v, st, const_cast<double*>(sol), nullptr, rhs, nnf, g, nullptr, slot, -1, 1, E_b, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }

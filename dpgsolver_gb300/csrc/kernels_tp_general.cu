@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(128) k_tp_face_br2(const double* trace, const 
 	}
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = V.nrm[(size_t)t * D + a];
-	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike<D>(WL, WR, n, nf);
-	else                                   numflux_lax_friedrichs<D>(WL, WR, n, nf);
+	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
+	else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
 	const double j = V.jf[t];
 	const bool adiabatic = V.bc && V.bc[f] == DPG_BC_NOSLIP_ADIABATIC;
 #pragma unroll

@@ -73,6 +73,7 @@ static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	if ((rc = dalloc(c, &c->ddt, 1))) return fail(rc);
 	if (cudaMemset(c->rhs, 0, sizeof(double) * c->n_dof) != cudaSuccess) return fail(DPG_ERR_CUDA);
 	if ((rc = dpg::hp_prepare(c, sim))) return fail(rc);
+	if ((rc = dpg::oz_prepare(c, sim, dpg::hp_tables(c, sim)))) return fail(rc);
 	// Euler: the dense positivity limiter per order group (Bezier operators of each order, n_s <= 64)
 	if (sim->pde_index == DPG_PDE_EULER && nv == d + 2) {
 		std::vector<std::vector<int>> members(sim->n_ops);
@@ -281,6 +282,12 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 		c->adv_speed = std::sqrt(sim->b_adv[0] * sim->b_adv[0] + sim->b_adv[1] * sim->b_adv[1] + sim->b_adv[2] * sim->b_adv[2]);
 	}
 	if ((rc = dpg::fp64_configure(c))) return fail(rc);
+	if (affine_all) {
+		dpg::OzTables t;
+		t.met[0] = g.met; t.jinv[0] = g.jinv; t.vol_face = g.vol_face;
+		t.nc = fd.nc; t.nrm = fd.nrm; t.jf = fd.jf;
+		if ((rc = dpg::oz_prepare(c, sim, t))) return fail(rc);
+	}
 	if (general && c->tp) {
 		if ((rc = dpg::tp_general_prepare(c, sim))) return fail(rc);
 	} else if (general) {   // advection: a boundary state is the interior trace
@@ -302,6 +309,7 @@ extern "C" void dpg_gpu_destroy(dpg_gpu_ctx* c)
 	if (c->stream) cudaStreamSynchronize(c->stream);
 	dpg::split_free(c);
 	dpg::tp_free(c);
+	dpg::oz_free(c);
 	dpg::hp_free(c);
 	dpg::implicit_free(c);
 	dpg::mlp_free(c);
@@ -412,6 +420,7 @@ static int enqueue_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned 
 {
 	int rc;
 	if (c->walls_or_visc && c->tp) return dpg::tp_general_residual(c, stage, write_rhs, max_slot);
+	if (c->oz && c->prec_mode == DPG_PREC_FP64) return dpg::oz_residual(c, stage, write_rhs, max_slot);
 	if (c->hp) return dpg::hp_residual(c, stage, write_rhs, max_slot);
 	if (c->prec_mode == DPG_PREC_FP64) {
 		if ((rc = dpg::launch_trace(c))) return rc;
@@ -444,7 +453,7 @@ static int read_max(dpg_gpu_ctx* c, int slot, double* out)
 	double v;
 	memcpy(&v, &bits, sizeof v);
 	if (out) *out = v;
-	if (c->prec_mode != DPG_PREC_FP64 && dpg::split_error(c)) return DPG_ERR_TIMEOUT;
+	if (c->prec_mode != DPG_PREC_FP64 ? dpg::split_error(c) : c->oz && dpg::oz_error(c)) return DPG_ERR_TIMEOUT;
 	if (dpg::positivity_error(c)) return DPG_ERR_NONFINITE;   // the reference stops: average density / pressure ~ 0
 	return std::isfinite(v) ? DPG_OK : DPG_ERR_NONFINITE;
 }
@@ -461,6 +470,10 @@ extern "C" int dpg_gpu_compute_rhs(dpg_gpu_ctx* c, double* max_rhs)
 static int build_step_graph(dpg_gpu_ctx* c)
 {
 	invalidate_graph(c);
+	if (c->oz && c->prec_mode == DPG_PREC_FP64) {   // allocations are not possible during the capture
+		const int r = dpg::oz_ready(c);
+		if (r) return r;
+	}
 	cudaGraph_t graph = nullptr;
 	CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
 	int rc = DPG_OK;
@@ -601,15 +614,16 @@ extern "C" int dpg_gpu_kernel_times(dpg_gpu_ctx* c, int n_rep, double* ms_out, c
 	unsigned long long* slot = c->dmax + dpg::kMaxStages;
 	for (int r = 0; r < n_rep; ++r) {
 		CK(cudaEventRecord(ev[0], c->stream));
-		int rc = (c->hp ? dpg::hp_launch_part(c, 0, -1, true, slot)
+		const bool oz = c->oz && c->prec_mode == DPG_PREC_FP64;
+		int rc = (oz ? dpg::oz_launch_part(c, 0, -1, true, slot) : c->hp ? dpg::hp_launch_part(c, 0, -1, true, slot)
 		          : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_trace(c) : dpg::split_launch_trace(c));
 		if (rc) return rc;
 		CK(cudaEventRecord(ev[1], c->stream));
-		rc = (c->hp ? dpg::hp_launch_part(c, 1, -1, true, slot)
+		rc = (oz ? dpg::oz_launch_part(c, 1, -1, true, slot) : c->hp ? dpg::hp_launch_part(c, 1, -1, true, slot)
 		      : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_face(c) : dpg::split_launch_face(c));
 		if (rc) return rc;
 		CK(cudaEventRecord(ev[2], c->stream));
-		rc = (c->hp ? dpg::hp_launch_part(c, 2, -1, true, slot)
+		rc = (oz ? dpg::oz_launch_part(c, 2, -1, true, slot) : c->hp ? dpg::hp_launch_part(c, 2, -1, true, slot)
 		      : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_volume(c, -1, true, slot)
 		                                      : dpg::split_launch_volume(c, -1, true, slot));
 		if (rc) return rc;

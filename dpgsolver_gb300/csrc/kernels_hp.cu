@@ -445,6 +445,20 @@ int hp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim)
 	return DPG_ERR_UNSUPPORTED;
 }
 
+OzTables hp_tables(const dpg_gpu_ctx* c, const struct dpg_sim* sim)
+{
+	const HpState* s = (const HpState*)c->hp;
+	const HpDev& h = s->dev;
+	OzTables t;
+	t.n_groups = h.n_groups;
+	for (const HpGroup& g : s->host_groups)
+		for (int k = 0; k < sim->n_ops; ++k)
+			if (sim->ops[k].p == g.p) { t.vols[k] = g.vols; t.met[k] = g.met; t.jinv[k] = g.jinv; }
+	t.dof_off = h.dof_off; t.vol_face = h.vol_face; t.face_p = h.face_p; t.fnode_off = h.fnode_off; t.node_face = h.node_face;
+	t.nc = h.nc; t.nrm = h.nrm; t.jf = h.jf;
+	return t;
+}
+
 template <int D, int NV>
 static int hp_launch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsigned long long* max_slot)
 {

@@ -118,9 +118,9 @@ __device__ __forceinline__ void numflux_lax_friedrichs(const T* WL, const T* WR,
 // does 1.6 per clock and SM, ~90 cycles apart when they depend on one another): the densities enter as 1 / sqrt(rho),
 // whose square is 1 / rho and whose multiple by rho is the Roe weight sqrt(rho); c comes from 1 / sqrt(c^2).
 // Roe-Pike: one division and three reciprocal square roots instead of four and two, three in a row instead of five;
-// Lax-Friedrichs: two divisions and four roots instead of 2 D + 4 and four.  For the tensor-product kernels (k_face,
-// 32x32x8 HEX p = 3, FP64
-// step: 1,517 -> 1,480 us); results differ from the functions above by rounding.
+// Lax-Friedrichs: two divisions and four roots instead of 2 D + 4 and four.  Results differ from the functions above by
+// rounding.  For the tensor-product kernels (32x32x8 HEX p = 3, FP64 step: 1,517 -> 1,483 us) and k_oz_flux.
+
 // y with its sign flipped where x is negative; sign(a) != sign(b).
 __device__ __forceinline__ double signed_as(double y, double x)
 {

@@ -72,7 +72,7 @@ static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	if ((rc = dalloc(c, &c->dmax, dpg::kMaxStages + 1))) return fail(rc);
 	if ((rc = dalloc(c, &c->ddt, 1))) return fail(rc);
 	if (cudaMemset(c->rhs, 0, sizeof(double) * c->n_dof) != cudaSuccess) return fail(DPG_ERR_CUDA);
-	if ((rc = dpg::hp_prepare(c, sim))) return fail(rc);
+	if ((rc = dpg::hp_prepare(c, sim, nullptr))) return fail(rc);
 	if ((rc = dpg::oz_prepare(c, sim, dpg::hp_tables(c, sim)))) return fail(rc);
 	// Euler: the dense positivity limiter per order group (Bezier operators of each order, n_s <= 64)
 	if (sim->pde_index == DPG_PDE_EULER && nv == d + 2) {
@@ -285,8 +285,11 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	if (affine_all) {
 		dpg::OzTables t;
 		t.met[0] = g.met; t.jinv[0] = g.jinv; t.vol_face = g.vol_face;
-		t.nc = fd.nc; t.nrm = fd.nrm; t.jf = fd.jf;
+		t.nc = fd.nc; t.nc_inv = g.nc_inv; t.nrm = fd.nrm; t.jf = fd.jf;
 		if ((rc = dpg::oz_prepare(c, sim, t))) return fail(rc);
+		// advection on simplices, all sizes: 1.15 to 3.5 times as fast as the dense kernels (figures in kernels_hp.cu), which
+		// keep meshes with boundary faces, whose traces they copy
+		if (nv == 1 && (c->e_type == DPG_TRI || c->e_type == DPG_TET) && !general && (rc = dpg::hp_prepare(c, sim, &t))) return fail(rc);
 	}
 	if (general && c->tp) {
 		if ((rc = dpg::tp_general_prepare(c, sim))) return fail(rc);
@@ -421,7 +424,7 @@ static int enqueue_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned 
 	int rc;
 	if (c->walls_or_visc && c->tp) return dpg::tp_general_residual(c, stage, write_rhs, max_slot);
 	if (c->oz && c->prec_mode == DPG_PREC_FP64) return dpg::oz_residual(c, stage, write_rhs, max_slot);
-	if (c->hp) return dpg::hp_residual(c, stage, write_rhs, max_slot);
+	if (c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64)) return dpg::hp_residual(c, stage, write_rhs, max_slot);
 	if (c->prec_mode == DPG_PREC_FP64) {
 		if ((rc = dpg::launch_trace(c))) return rc;
 		if ((rc = dpg::launch_face(c))) return rc;
@@ -480,6 +483,8 @@ static int build_step_graph(dpg_gpu_ctx* c)
 	if (cudaMemsetAsync(c->dmax, 0, sizeof(unsigned long long) * dpg::kMaxStages, c->stream) != cudaSuccess) rc = DPG_ERR_CUDA;
 	if (c->tp && c->prec_mode == DPG_PREC_FP64) {
 		if (rc == DPG_OK) rc = dpg::tp_step(c, c->dmax);
+	} else if (dpg::hp_steps(c)) {
+		if (rc == DPG_OK) rc = dpg::hp_step(c, c->dmax);
 	} else {
 		for (int stage = 0; stage < 3 && rc == DPG_OK; ++stage) rc = enqueue_stage(c, stage, c->dmax + stage);
 	}
@@ -584,6 +589,7 @@ extern "C" int dpg_gpu_time_rk_steps(dpg_gpu_ctx* c, double dt, int n_steps, dou
 extern "C" int dpg_gpu_launches_per_rhs(dpg_gpu_ctx* c)
 {
 	if (!c) return 0;
+	if (c->n_var == 1 && (c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64))) return 2;   // no launch of its own for the face fluxes
 	return !c->walls_or_visc ? 3 : c->tp ? dpg::tp_general_launches(c) : 4;
 }
 
@@ -614,16 +620,16 @@ extern "C" int dpg_gpu_kernel_times(dpg_gpu_ctx* c, int n_rep, double* ms_out, c
 	unsigned long long* slot = c->dmax + dpg::kMaxStages;
 	for (int r = 0; r < n_rep; ++r) {
 		CK(cudaEventRecord(ev[0], c->stream));
-		const bool oz = c->oz && c->prec_mode == DPG_PREC_FP64;
-		int rc = (oz ? dpg::oz_launch_part(c, 0, -1, true, slot) : c->hp ? dpg::hp_launch_part(c, 0, -1, true, slot)
+		const bool oz = c->oz && c->prec_mode == DPG_PREC_FP64, hp = c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64);
+		int rc = (oz ? dpg::oz_launch_part(c, 0, -1, true, slot) : hp ? dpg::hp_launch_part(c, 0, -1, true, slot)
 		          : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_trace(c) : dpg::split_launch_trace(c));
 		if (rc) return rc;
 		CK(cudaEventRecord(ev[1], c->stream));
-		rc = (oz ? dpg::oz_launch_part(c, 1, -1, true, slot) : c->hp ? dpg::hp_launch_part(c, 1, -1, true, slot)
+		rc = (oz ? dpg::oz_launch_part(c, 1, -1, true, slot) : hp ? dpg::hp_launch_part(c, 1, -1, true, slot)
 		      : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_face(c) : dpg::split_launch_face(c));
 		if (rc) return rc;
 		CK(cudaEventRecord(ev[2], c->stream));
-		rc = (oz ? dpg::oz_launch_part(c, 2, -1, true, slot) : c->hp ? dpg::hp_launch_part(c, 2, -1, true, slot)
+		rc = (oz ? dpg::oz_launch_part(c, 2, -1, true, slot) : hp ? dpg::hp_launch_part(c, 2, -1, true, slot)
 		      : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_volume(c, -1, true, slot)
 		                                      : dpg::split_launch_volume(c, -1, true, slot));
 		if (rc) return rc;

@@ -122,6 +122,7 @@ struct dpg_gpu_ctx {
 	int n_bface = 0;
 	void* oz = nullptr;         // simplices: FP64 dense products on the tensor cores (kernels_oz.cu)
 	void* hp = nullptr;         // mixed orders: volumes grouped by order (kernels_hp.cu)
+	void* adv = nullptr;        // one order, simplices, advection: the same for the FP64 residual
 	void* implicit = nullptr;   // Newton-GMRES work space (implicit.cu)
 	void* mlp = nullptr;        // learned preconditioner (mlp.cu)
 };
@@ -202,8 +203,9 @@ int  tp_step(dpg_gpu_ctx* c, unsigned long long* max_slots);   // one SSP-RK3 st
 
 // mixed orders (kernels_hp.cu): FP64 residual over volume groups of each order; which = 0 traces, 1 face fluxes,
 // 2 volume terms (with the RK stage)
-int  hp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);
 int  hp_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
+bool hp_steps(const dpg_gpu_ctx* c);                            // advection on affine elements:
+int  hp_step(dpg_gpu_ctx* c, unsigned long long* max_slots);   // one SSP-RK3 step
 int  hp_launch_part(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsigned long long* max_slot);
 void hp_free(dpg_gpu_ctx* c);
 
@@ -218,10 +220,11 @@ struct OzTables {                       // device tables of the context, by orde
 	const int* face_p = nullptr;
 	const int64_t* fnode_off = nullptr;
 	const int* node_face = nullptr;
-	const int* nc = nullptr;
+	const int *nc = nullptr, *nc_inv = nullptr;
 	const double* nrm = nullptr;
 	const double* jf = nullptr;
 };
+int  hp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, const OzTables* share);
 OzTables hp_tables(const dpg_gpu_ctx* c, const struct dpg_sim* sim);
 int  oz_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, const OzTables& tab);
 int  oz_ready(dpg_gpu_ctx* c);

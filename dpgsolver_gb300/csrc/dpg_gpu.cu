@@ -47,6 +47,23 @@ static int dupload(dpg_gpu_ctx* c, T** p, const T* host, size_t n)
 	return DPG_OK;
 }
 
+// A group of the dense positivity limiter; its FP32 screen's bound: 4 (n_s + 5) 2^-24 per unit of |ccSB0| |u| (truncation
+// of u, rounding of the operator, n_s-term sums, a factor 4 of margin).
+static int dense_limiter(dpg_gpu_ctx* c, const dpg_element_ops& o, int n_vol, const int* vols)
+{
+	if (o.n_s > 64 || !o.ccSB0_vs_vs || !o.ccBS0_vs_vs || c->n_pos_grp >= DPG_P_MAX) return DPG_ERR_UNSUPPORTED;
+	std::vector<float> screen;
+	std::vector<double> sbT, bsT;
+	dpg::dense_limiter_tables(o, screen, sbT, bsT);
+	dpg_gpu_ctx::PosGroup& g = c->pos_grp[c->n_pos_grp++];
+	g.n_vol = n_vol; g.ns = o.n_s; g.vols = vols;
+	g.amp = (float)(4.0 * (o.n_s + 5) * std::ldexp(1.0, -24));
+	int rc;
+	if ((rc = dupload(c, (float**)&g.screen, screen.data(), screen.size()))) return rc;
+	if ((rc = dupload(c, (double**)&g.sbT, sbT.data(), sbT.size()))) return rc;
+	return dupload(c, (double**)&g.bsT, bsT.data(), bsT.size());
+}
+
 // Mixed orders: state, the per-order volume groups and the face tables of kernels_hp.cu (periodic meshes, FP64
 // residual and explicit steps).
 static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
@@ -81,19 +98,9 @@ static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 		for (int k = 0; k < sim->n_ops; ++k) {
 			const dpg_element_ops& o = sim->ops[k];
 			if (members[k].empty()) continue;
-			if (o.n_s > 64 || !o.ccSB0_vs_vs || !o.ccBS0_vs_vs || c->n_pos_grp >= DPG_P_MAX) return fail(DPG_ERR_UNSUPPORTED);
-			dpg_gpu_ctx::PosGroup& g = c->pos_grp[c->n_pos_grp++];
-			g.n_vol = (int)members[k].size();
-			g.ns = o.n_s;
-			g.amp = (float)(4.0 * (o.n_s + 5) * std::ldexp(1.0, -24));
-			std::vector<float> sb32((size_t)o.n_s * o.n_s);
-			for (size_t i = 0; i < sb32.size(); ++i) sb32[i] = (float)o.ccSB0_vs_vs[i];
-			int* dv; float* d32; double* d64; double* dbs;
+			int* dv;
 			if ((rc = dupload(c, &dv, members[k].data(), members[k].size()))) return fail(rc);
-			if ((rc = dupload(c, &d32, sb32.data(), sb32.size()))) return fail(rc);
-			if ((rc = dupload(c, &d64, o.ccSB0_vs_vs, sb32.size()))) return fail(rc);
-			if ((rc = dupload(c, &dbs, o.ccBS0_vs_vs, sb32.size()))) return fail(rc);
-			g.vols = dv; g.sb32 = d32; g.sb64 = d64; g.bs64 = dbs;
+			if ((rc = dense_limiter(c, o, (int)members[k].size(), dv))) return fail(rc);
 		}
 		int64_t* doff;
 		if ((rc = dupload(c, &doff, sim->vol_dof_off, (size_t)sim->n_vol + 1))) return fail(rc);
@@ -225,17 +232,8 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	// 4 (D (n1 + 2) + 2) 2^-24 (input truncation, operator rounding and n1-term sums in each of the D passes)
 	const bool simplex_e = (ops.e_type == DPG_TRI || ops.e_type == DPG_TET);
 	if ((sim->pde_index == DPG_PDE_EULER || sim->pde_index == DPG_PDE_NAVIER_STOKES) && nv == d + 2 && simplex_e) {
-		// simplices: dense operators; the FP32 screen's bound (n_s + 5) 2^-24 per unit of |ccSB0| |u| (truncation of u,
-		// rounding of the operator, n_s-term sums), with a factor 4 of margin
-		if (n_s > 64) return fail(DPG_ERR_UNSUPPORTED);
 		c->pos_dense = 1;
-		c->pos_amp = (float)(4.0 * (n_s + 5) * std::ldexp(1.0, -24));
-		std::vector<float> sb32((size_t)n_s * n_s);
-		for (size_t i = 0; i < sb32.size(); ++i) sb32[i] = (float)ops.ccSB0_vs_vs[i];
-		if ((rc = dupload(c, &c->bez_bs, ops.ccBS0_vs_vs, (size_t)n_s * n_s))) return fail(rc);
-		if ((rc = dalloc(c, &c->bez_sb32, (size_t)n_s * n_s))) return fail(rc);
-		if (cudaMemcpy(c->bez_sb32, sb32.data(), sizeof(float) * sb32.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-			return fail(DPG_ERR_CUDA);
+		if ((rc = dense_limiter(c, ops, n_vol, nullptr))) return fail(rc);
 		if ((rc = dalloc(c, &c->pos_err, 1))) return fail(rc);
 		if (cudaMemset(c->pos_err, 0, sizeof(int)) != cudaSuccess) return fail(DPG_ERR_CUDA);
 		c->positivity = 1;

@@ -1,6 +1,7 @@
 // Device context and kernel launch declarations shared by the CUDA translation units.
 #pragma once
 
+#include <vector>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -95,15 +96,12 @@ struct dpg_gpu_ctx {
 	int pos_n1 = 0;              // solution points per direction
 	double* bez1 = nullptr;      // [n1 x n1] Bernstein polynomials at the GLL nodes (Bezier -> solution coefficients)
 	double* bez1_inv = nullptr;  // [n1 x n1] its inverse
-	int pos_dense = 0;           // simplices: dense Bezier operators (no 1D factors), n_s solution nodes
-	double* bez_bs = nullptr;    // [n_s x n_s] Bezier -> solution coefficients (ccBS0_vs_vs), dense limiter
-	float* bez_sb32 = nullptr;   // [n_s x n_s] ccSB0_vs_vs in FP32 (the dense limiter's screen)
-	// mixed orders (Euler): the dense limiter per order group -- its volumes, operators and screen bound
-	struct PosGroup { int n_vol = 0, ns = 0; const int* vols = nullptr; const float* sb32 = nullptr;
-	                  const double* sb64 = nullptr; const double* bs64 = nullptr; float amp = 0.f; };
-	PosGroup pos_grp[DPG_P_MAX];
+	int pos_dense = 0;           // simplices, mixed orders: dense Bezier operators (no 1D factors)
+	// the dense limiter per order group: its volumes (null: all, one order), operators (dense_limiter_tables), screen bound
+	struct PosGroup { int n_vol, ns; const int* vols; const float* screen; const double *sbT, *bsT; float amp; };
+	PosGroup pos_grp[DPG_P_MAX] = {};
 	int n_pos_grp = 0;
-	const int64_t* pos_dof_off = nullptr;   // [n_vol + 1]
+	const int64_t* pos_dof_off = nullptr;   // [n_vol + 1], or null (one order)
 	// local pseudo time steps of the implicit solve (the reference's CFL ramping)
 	double* h_min = nullptr;     // [n_vol] shortest edge of each volume (chord between its end vertices)
 	double* bez_full = nullptr;  // [n_s x n_s] solution -> Bezier coefficients (ccSB0_vs_vs), Euler-like PDEs
@@ -253,6 +251,7 @@ int  enqueue_residual_raw(dpg_gpu_ctx* c, unsigned long long* max_slot);
 
 // positivity (positivity.cu): the limiter on a state (no-op when c->positivity is 0) and the Newton update
 // u += relax du with the per-volume under-relaxation (positivity on only); errors in c->pos_err
+void dense_limiter_tables(const dpg_element_ops& o, std::vector<float>& screen, std::vector<double>& sbT, std::vector<double>& bsT);
 int  launch_positivity(dpg_gpu_ctx* c, double* sol);
 int  launch_relaxed_update(dpg_gpu_ctx* c, double* u, const double* du);
 int  positivity_error(dpg_gpu_ctx* c);   // reads and clears c->pos_err

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <vector>
 
 #include "positivity.cuh"
 
@@ -335,14 +336,21 @@ __global__ void __launch_bounds__(kPosThreads) k_relax_update(double* __restrict
 	}
 }
 
-// The limiter on simplices (TRI, TET): dense Bezier operators (the Bernstein polynomials of a simplex have no 1D
-// factors).  One warp per volume, grid-stride over the volumes; a lane per Bezier coefficient (n_s <= 64, two per
-// lane).  The FP32 screen as above with b = ccSB0 u and c = |ccSB0| |u| summed directly (amp = 4 (n_s + 5) 2^-24,
-// set by the host); a volume that does not clear it runs the reference's algorithm in FP64: ccSB0 u, primitive
-// variables, limit_volume's serial steps on lane 0, conservative variables, u = ccBS0 b.  The operators sit in
-// shared memory (FP32 ccSB0 for the screen, FP64 ccSB0 and ccBS0), with a [NV][n_s] FP32 and two FP64 buffers per
-// warp.
-constexpr int kDenseWarps = 4;
+// The limiter on simplices (TRI, TET) and mixed orders: dense Bezier operators (the Bernstein polynomials of a simplex
+// have no 1D factors), one launch over the groups of volumes of an order.
+//
+// Screen in FP32: a block per 32 volumes, a lane per volume and a warp per kRowsT rows of b = ccSB0 u; the rounding bound amp |ccSB0| |u| as
+// amp (row sum of |ccSB0|) max |u|, amp = 4 (n_s + 5) 2^-24 (truncation of u, rounding of the operator, n_s-term sums, a
+// factor 4).  A lane reads its volume's column of the staged coefficients (volume fastest, odd stride: no bank
+// conflicts either way) and the warp the same operator entries, so 25 multiply-adds (TET) take 7 shared-memory
+// reads; a lane per row of one volume with the whole of |ccSB0| |u| took 6 reads, 4-way conflicts among them, for ten.
+// 196,608 TETs of order 3 (157 MB of state, 23 us at the copy rate): 297 -> 71 us (107 with the
+// staging loads one after the other); 24,576 TETs of orders 1..4 in one launch instead of four: 56 -> 16 us.
+// A volume that does not clear it runs the reference's algorithm in FP64 on a warp: ccSB0 u, primitive variables,
+// limit_volume's serial steps on lane 0, conservative variables, u = ccBS0 b (operators K-major, from L1).
+constexpr int kDenseWarps = 8, kDenseThreads = 32 * kDenseWarps;
+constexpr int kRowsT = 5, kRowsPad = 8;
+constexpr int kDenseVols = 32, kDenseLd = kDenseVols + 1, kBatch = 5;
 
 template <int D>
 __device__ bool limit_volume_n(double* w, int ns)
@@ -368,65 +376,103 @@ __device__ bool limit_volume_n(double* w, int ns)
 	return true;
 }
 
+struct DenseLimit {
+	int n_groups;
+	struct { dpg_gpu_ctx::PosGroup t; int blk0; } g[DPG_P_MAX];
+	const int64_t* dof_off;
+};
+
+__host__ __device__ constexpr int dense_row_groups(int ns) { return (ns + kRowsT - 1) / kRowsT; }
+
 template <int D>
-__global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* sol, int n_vol, int ns,
-                                                                     const float* __restrict__ sb32,
-                                                                     const double* __restrict__ sb64,
-                                                                     const double* __restrict__ bs64, float amp,
-                                                                     int* __restrict__ err,
-                                                                     const int* __restrict__ vols,
-                                                                     const int64_t* __restrict__ dof_off)
+__global__ void __launch_bounds__(kDenseThreads) k_positivity_dense(double* sol, const __grid_constant__ DenseLimit P, int* __restrict__ err)
 {
 	constexpr int NV = D + 2;
-	extern __shared__ double dsm[];
-	const int nn = ns * ns, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	double* sSB = dsm;                                   // [ns][ns]
-	double* sBS = sSB + nn;                              // [ns][ns]
-	double* sW = sBS + nn + (size_t)warp * 2 * NV * ns;  // this warp's [2][NV][ns]
-	float* sA32 = reinterpret_cast<float*>(sBS + nn + (size_t)kDenseWarps * 2 * NV * ns);   // [ns][ns]
-	float* sX = sA32 + nn + (size_t)warp * NV * ns;       // this warp's [NV][ns]
-	for (int i = threadIdx.x; i < nn; i += blockDim.x) {
-		sSB[i] = sb64[i];
-		sBS[i] = bs64[i];
-		sA32[i] = sb32[i];
+	extern __shared__ __align__(16) double dsm[];
+	int gi = 0;
+	while (gi + 1 < P.n_groups && P.g[gi + 1].blk0 <= (int)blockIdx.x) ++gi;
+	const dpg_gpu_ctx::PosGroup& G = P.g[gi].t;
+	const int ns = G.ns, ng = dense_row_groups(ns);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nu = NV * ns;
+	const int e0 = (blockIdx.x - P.g[gi].blk0) * kDenseVols, ne = min(kDenseVols, G.n_vol - e0);
+	int64_t* sBase = reinterpret_cast<int64_t*>(dsm);             // [kDenseVols] first coefficient
+	float* sA = reinterpret_cast<float*>(dsm + kDenseVols);               // [ng][ns][kRowsPad], then the row sums [ng][kRowsPad]
+	float* sX = sA + ng * (ns + 1) * kRowsPad;                    // [NV ns][kDenseLd]
+	__shared__ unsigned sBad;
+	if (threadIdx.x < kDenseVols) {   // mixed orders: the group's volumes and their offsets
+		const int e = threadIdx.x, ev = e < ne ? (G.vols ? G.vols[e0 + e] : e0 + e) : 0;
+		sBase[e] = P.dof_off ? P.dof_off[ev] : (int64_t)ev * nu;
 	}
+	for (int i = threadIdx.x; i < ng * (ns + 1) * kRowsPad; i += kDenseThreads) sA[i] = G.screen[i];
+	if (threadIdx.x == 0) sBad = 0;
 	grid_wait();
 	__syncthreads();
-	for (int e = blockIdx.x * kDenseWarps + warp; e < n_vol; e += gridDim.x * kDenseWarps) {
-		const int ev = vols ? vols[e] : e;   // mixed orders: the group's volume list and the volumes' offsets
-		double* u = sol + (dof_off ? (size_t)dof_off[ev] : (size_t)ev * NV * ns);
-		for (int i = lane; i < NV * ns; i += 32) sX[i] = trunc_to_float(u[i]);
-		__syncwarp();
-		bool bad = false;
-		for (int i = lane; i < ns; i += 32) {
-			float b[NV], c[NV];
+	{
+		const int de = kDenseThreads / nu, dr = kDenseThreads - de * nu;
+		int e = threadIdx.x / nu, r = threadIdx.x - e * nu;
+		for (int i = threadIdx.x; i < ne * nu; i += kBatch * kDenseThreads) {   // kBatch loads on their way at once
+			double x[kBatch];
+			int at[kBatch];
+#pragma unroll
+			for (int j = 0; j < kBatch; ++j) {
+				at[j] = i + j * kDenseThreads < ne * nu ? r * kDenseLd + e : -1;
+				x[j] = at[j] >= 0 ? sol[sBase[e] + r] : 0.0;
+				e += de; r += dr;
+				if (r >= nu) { r -= nu; ++e; }
+			}
+#pragma unroll
+			for (int j = 0; j < kBatch; ++j)
+				if (at[j] >= 0) sX[at[j]] = trunc_to_float(x[j]);
+		}
+	}
+	__syncthreads();
+	for (int grp = warp; grp < ng; grp += kDenseWarps) {
+		float acc[kRowsT][NV], mx[NV];
+#pragma unroll
+		for (int v = 0; v < NV; ++v) {
+			mx[v] = 0.f;
+#pragma unroll
+			for (int t = 0; t < kRowsT; ++t) acc[t][v] = 0.f;
+		}
+		const float *a = sA + grp * ns * kRowsPad, *x = sX + lane;
+#pragma unroll 2
+		for (int k = 0; k < ns; ++k) {
+			const float4 a4 = *reinterpret_cast<const float4*>(a + k * kRowsPad);
+			const float ar[kRowsT] = {a4.x, a4.y, a4.z, a4.w, a[k * kRowsPad + 4]};
 #pragma unroll
 			for (int v = 0; v < NV; ++v) {
-				float yb = 0.f, yc = 0.f;
-				for (int k = 0; k < ns; ++k) {
-					const float a = sA32[i * ns + k], x = sX[v * ns + k];
-					yb += a * x;
-					yc += fabsf(a) * fabsf(x);
-				}
-				b[v] = yb;
-				c[v] = yc;
+				const float xv = x[(v * ns + k) * kDenseLd];
+				mx[v] = fmaxf(mx[v], fabsf(xv));
+#pragma unroll
+				for (int t = 0; t < kRowsT; ++t) acc[t][v] += ar[t] * xv;
 			}
-			const float rho_lo = b[0] - amp * c[0];
+		}
+		bool bad = false;
+#pragma unroll
+		for (int t = 0; t < kRowsT; ++t) {
+			const float amp = G.amp * sA[ng * ns * kRowsPad + grp * kRowsPad + t];
+			const float rho_lo = acc[t][0] - amp * mx[0];
 			float m2 = 0.f;
 #pragma unroll
-			for (int a = 0; a < D; ++a) {
-				const float m = fabsf(b[1 + a]) + amp * c[1 + a];
+			for (int d = 0; d < D; ++d) {
+				const float m = fabsf(acc[t][1 + d]) + amp * mx[1 + d];
 				m2 += m * m;
 			}
-			const float eE = amp * c[NV - 1];
-			const float q2 = 0.5f * m2 / rho_lo, E_lo = b[NV - 1] - eE;
-			const float p_lo = 0.4f * (E_lo - q2) - 9.5367431640625e-07f * (fabsf(b[NV - 1]) + eE + q2);
-			bad |= !(rho_lo > 2.0f * (float)DPG_EPS_PHYS) || !(p_lo > 2.0f * (float)DPG_EPS_PHYS);
+			const float bE = acc[t][NV - 1], eE = amp * mx[NV - 1];
+			const float q2 = 0.5f * m2 / rho_lo, E_lo = bE - eE;
+			const float p_lo = 0.4f * (E_lo - q2) - 9.5367431640625e-07f * (fabsf(bE) + eE + q2);
+			bad |= grp * kRowsT + t < ns && (!(rho_lo > 2.0f * (float)DPG_EPS_PHYS) || !(p_lo > 2.0f * (float)DPG_EPS_PHYS));
 		}
-		if (!__any_sync(0xffffffffu, bad)) {
-			__syncwarp();
-			continue;
-		}
+		const unsigned m = __ballot_sync(0xffffffffu, bad && lane < ne);   // lanes beyond ne: whatever was there
+		if (lane == 0 && m) atomicOr(&sBad, m);
+	}
+	__syncthreads();
+	if (!sBad) return;
+	double* sW = reinterpret_cast<double*>(sX) + (size_t)warp * 2 * nu;   // this warp's [2][NV][ns] over the staged coefficients
+	int turn = 0;
+	for (int e = 0; e < ne; ++e) {
+		if (!(sBad >> e & 1u) || (turn++ & (kDenseWarps - 1)) != warp) continue;
+		double* u = sol + sBase[e];
 		// the reference's algorithm in FP64
 		double* w0 = sW;              // u, then the primitive Bezier coefficients
 		double* w1 = sW + NV * ns;    // the Bezier coefficients, then the limited conservative ones
@@ -435,7 +481,7 @@ __global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* s
 		for (int o = lane; o < NV * ns; o += 32) {
 			const int v = o / ns, i = o - v * ns;
 			double acc = 0.0;
-			for (int k = 0; k < ns; ++k) acc += sSB[i * ns + k] * w0[v * ns + k];
+			for (int k = 0; k < ns; ++k) acc += G.sbT[k * ns + i] * w0[v * ns + k];
 			w1[o] = acc;
 		}
 		__syncwarp();
@@ -468,7 +514,7 @@ __global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* s
 			for (int o = lane; o < NV * ns; o += 32) {
 				const int v = o / ns, i = o - v * ns;
 				double acc = 0.0;
-				for (int k = 0; k < ns; ++k) acc += sBS[i * ns + k] * w1[v * ns + k];
+				for (int k = 0; k < ns; ++k) acc += G.bsT[k * ns + i] * w1[v * ns + k];
 				u[o] = acc;
 			}
 		}
@@ -478,26 +524,30 @@ __global__ void __launch_bounds__(kDenseWarps * 32) k_positivity_dense(double* s
 
 size_t dense_smem(int d, int ns)
 {
-	const int nv = d + 2;
-	return sizeof(double) * (2 * (size_t)ns * ns + (size_t)kDenseWarps * 2 * nv * ns) +
-	       sizeof(float) * ((size_t)ns * ns + (size_t)kDenseWarps * nv * ns);
+	const size_t nu = (size_t)(d + 2) * ns;
+	const size_t x = std::max(sizeof(float) * nu * kDenseLd, sizeof(double) * kDenseWarps * 2 * nu);
+	return sizeof(int64_t) * kDenseVols + sizeof(float) * dense_row_groups(ns) * (ns + 1) * kRowsPad + x;
 }
 
-void launch_limit_dense(dpg_gpu_ctx* c, double* sol, int n_vol, int ns, const float* sb32, const double* sb64,
-                        const double* bs64, float amp, const int* vols, const int64_t* dof_off)
+template <int D>
+int launch_limit_dense(dpg_gpu_ctx* c, double* sol)
 {
-	const size_t smem = dense_smem(c->d, ns);
-	const int blocks = std::max(1, std::min((n_vol + kDenseWarps - 1) / kDenseWarps, 152 * 8));
-	if (smem > 48 * 1024) {   // n_s above 40 (TRI orders above 7)
-		if (c->d == 2) cudaFuncSetAttribute(k_positivity_dense<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		else cudaFuncSetAttribute(k_positivity_dense<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	DenseLimit P{};
+	size_t smem = 0;
+	int blocks = 0;
+	for (int k = c->n_pos_grp - 1; k >= 0; --k) {   // the highest order (the longest blocks) first
+		const dpg_gpu_ctx::PosGroup& t = c->pos_grp[k];
+		P.g[P.n_groups].t = t;
+		P.g[P.n_groups++].blk0 = blocks;
+		blocks += (t.n_vol + kDenseVols - 1) / kDenseVols;
+		smem = std::max(smem, dense_smem(D, t.ns));
 	}
-	if (c->d == 2)
-		launch_chained(k_positivity_dense<2>, blocks, kDenseWarps * 32, smem, c->stream, sol, n_vol, ns, sb32, sb64, bs64, amp,
-		                                                                    c->pos_err, vols, dof_off);
-	else
-		launch_chained(k_positivity_dense<3>, blocks, kDenseWarps * 32, smem, c->stream, sol, n_vol, ns, sb32, sb64, bs64, amp,
-		                                                                    c->pos_err, vols, dof_off);
+	P.dof_off = c->pos_dof_off;
+	// once per launch: the attribute is a maximum, and other contexts may have set a smaller one
+	if (smem > 48 * 1024 && cudaFuncSetAttribute(k_positivity_dense<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+		return DPG_ERR_CUDA;
+	launch_chained(k_positivity_dense<D>, blocks, kDenseThreads, smem, c->stream, sol, P, c->pos_err);
+	return DPG_OK;
 }
 
 template <int D, int N1>
@@ -519,19 +569,35 @@ void launch_relax(dpg_gpu_ctx* c, double* u, const double* du)
 
 } // namespace
 
+// The dense limiter's operators: ccSB0 in FP32 by groups of rows for the screen, [row group][k][kRowsPad], with the row sums
+// of |ccSB0| [row group][kRowsPad] (rounded up) behind it; ccSB0 and ccBS0 K-major.
+void dense_limiter_tables(const dpg_element_ops& o, std::vector<float>& screen, std::vector<double>& sbT, std::vector<double>& bsT)
+{
+	const int ns = o.n_s, ng = dense_row_groups(ns);
+	screen.assign((size_t)ng * (ns + 1) * kRowsPad, 0.f);
+	sbT.resize((size_t)ns * ns);
+	bsT.resize((size_t)ns * ns);
+	for (int i = 0; i < ns; ++i) {
+		const int g = i / kRowsT, t = i - g * kRowsT;
+		double sum = 0.0;
+		for (int k = 0; k < ns; ++k) {
+			const double a = o.ccSB0_vs_vs[(size_t)i * ns + k];
+			screen[((size_t)g * ns + k) * kRowsPad + t] = (float)a;
+			sum += std::fabs(a);
+			sbT[(size_t)k * ns + i] = a;
+			bsT[(size_t)k * ns + i] = o.ccBS0_vs_vs[(size_t)i * ns + k];
+		}
+		screen[((size_t)ng * ns + g) * kRowsPad + t] = (float)(sum * (1.0 + 1e-6));
+	}
+}
+
 // (d, points per direction) of the Euler element groups: QUAD and HEX, p = 1..4; simplices: the dense form
 int launch_positivity(dpg_gpu_ctx* c, double* sol)
 {
 	if (!c->positivity) return DPG_OK;
 	if (c->pos_dense) {
-		if (c->n_pos_grp == 0)
-			launch_limit_dense(c, sol, c->g.n_vol, c->g.n_s, c->bez_sb32, c->bez_full, c->bez_bs, c->pos_amp, nullptr,
-			                   nullptr);
-		for (int k = 0; k < c->n_pos_grp; ++k) {   // mixed orders: one launch per order group
-			const dpg_gpu_ctx::PosGroup& g = c->pos_grp[k];
-			launch_limit_dense(c, sol, g.n_vol, g.ns, g.sb32, g.sb64, g.bs64, g.amp, g.vols, c->pos_dof_off);
-		}
-		return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
+		const int rc = c->d == 2 ? launch_limit_dense<2>(c, sol) : launch_limit_dense<3>(c, sol);
+		return rc ? rc : cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 	}
 	const int n1 = c->pos_n1;
 	if (c->d == 2 && n1 == 2) launch_limit<2, 2>(c, sol);

@@ -152,22 +152,5 @@ __device__ __forceinline__ int exp_bound(df64 x)
 	return be == 0 ? -4000 : be - 126;
 }
 
-// round(f * 2^sc) for an FP32 value f, |f 2^sc| < 2^62, with integer operations.
-__device__ __forceinline__ long long f32_scaled(float f, int sc)
-{
-	const uint32_t b = __float_as_uint(f);
-	const int be = (int)((b >> 23) & 0xFF);
-	if (be == 0) return 0;
-	const long long mant = (long long)((b & 0x7FFFFFu) | 0x800000u);
-	const int sh = be - 150 + sc;
-	long long m = 0;
-	if (sh >= 0) m = mant << sh;
-	else if (sh > -26) m = (mant + (1ll << (-sh - 1))) >> (-sh);
-	return (b & 0x80000000u) ? -m : m;
-}
-
-// (hi + lo) * 2^sc rounded to an integer (each part rounded: at most one unit off).
-__device__ __forceinline__ long long scaled_mantissa(df64 x, int sc) { return f32_scaled(x.hi, sc) + f32_scaled(x.lo, sc); }
-
 } // namespace df
 } // namespace dpg

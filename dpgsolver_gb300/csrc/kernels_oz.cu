@@ -108,7 +108,7 @@ __device__ __forceinline__ void write_digits(uint8_t* chunk, int m, int kk0, con
 	uint32_t lo[8], hi[8], lead[8];
 #pragma unroll
 	for (int j = 0; j < 8; ++j) {
-		const long long mm = scaled_mantissa(x[j], 8 * S - F) + digit_bias<S>();
+		const long long mm = biased_mantissa<S>(x[j], 8 * S - F);
 		lo[j] = (uint32_t)mm;
 		hi[j] = (uint32_t)((unsigned long long)mm >> 32);
 		lead[j] = (uint32_t)((int)(mm >> (8 * (S - 1))) + 128);

@@ -158,22 +158,6 @@ __device__ __forceinline__ int col_exp_of(int emax, int S)
 	return F < lo ? lo : (F > hi ? hi : F);
 }
 
-// round(x * 2^sc) from the bits of x with integer operations only (the FP64 pipe is kept for the fluxes):
-// x = +-mant * 2^(be - 1075), so the result is +-mant * 2^(be - 1075 + sc) (|result| < 2^(8S-1) by the choice of sc).
-// Branch-free: a left shift by max(sh, 0) and a rounding right shift by min(max(-sh, 0), 63).
-__device__ __forceinline__ long long scaled_mantissa(double x, int sc)
-{
-	const long long bits = __double_as_longlong(x);
-	const int be = (int)((bits >> 52) & 0x7FF);
-	const long long mant = (bits & 0xFFFFFFFFFFFFFll) | (1ll << 52);
-	const int sh = be - 1075 + sc;
-	const int rs = min(max(-sh, 0), 63);
-	const long long half = rs > 0 ? (1ll << (rs - 1)) : 0ll;
-	long long m = ((mant << max(sh, 0)) + half) >> rs;
-	m = be == 0 ? 0ll : m;
-	return bits < 0 ? -m : m;
-}
-
 // 128 in each of the S-1 low digit bytes: m + bias has the biased digits d_s + 128 in [0, 255] as its low bytes and
 // the leading digit d_0 in [-128, 128] above them.
 template <int S>
@@ -182,6 +166,24 @@ __host__ __device__ constexpr long long digit_bias()
 	long long C = 0;
 	for (int s = 0; s < S - 1; ++s) C |= 128ll << (8 * s);
 	return C;
+}
+
+// round(x 2^sc) + digit_bias<S>() from the bits of x, ties away from zero, with integer operations only (the FP64 pipe is kept
+// for the fluxes): x = +-mant 2^(be - 1075).  The choice of sc keeps the result below 2^(8S - 1) (S = 8: 2^62), i.e. twice
+// its magnitude is mant 2^10 >> r with r >= 0; zeros and subnormals have r > 62 and give 0.  With v = mant 2^10 >> r, the
+// rounded half is (v + 1) >> 1, its negative (-v) >> 1: both are ((v ^ sign) + 1) >> 1.  17 instructions (with shifts either way,
+// a rounding term and a negation: ~30; ks_lift's pipe for them was 48 % busy, the others less).
+template <int S>
+__device__ __forceinline__ long long biased_mantissa(double x, int sc)
+{
+	const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+	const int r = min(1084 - sc - (int)((hi >> 20) & 0x7FF), 63);
+	const uint32_t mh = (__funnelshift_l(lo, hi, 10) & 0x3FFFFFFFu) | 0x40000000u;
+	const unsigned long long v = (((unsigned long long)mh << 32) | (lo << 10)) >> r;
+	const uint32_t sign = (uint32_t)((int)hi >> 31);
+	const long long t = (long long)(v ^ (((unsigned long long)sign << 32) | sign));
+	if constexpr (S < 8) return (t + (2 * digit_bias<S>() + 1)) >> 1;
+	else                 return ((t + 1) >> 1) + digit_bias<S>();
 }
 
 __host__ __device__ constexpr float pow2f(int e) { return e >= 0 ? (e == 0 ? 1.0f : 2.0f * pow2f(e - 1)) : 0.5f * pow2f(e + 1); }
@@ -199,26 +201,32 @@ __device__ __forceinline__ uint32_t tf32_bits(float x)
 	return r;
 }
 
-// Digit s >= 1 (byte S-1-s of the biased integer) of 8 values as floats d * 2^(-8s), exactly: one byte permute
-// places the byte u in the low mantissa bits under the exponent field 150 - 8s, i.e. the float
-// 2^(23-8s) + u 2^(-8s), and one add removes 2^(23-8s) + 128 * 2^(-8s).  The leading digit (s = 0, 9 bits with
-// its bias) is placed by an OR into the mantissa of 2^23.
+// Digit s of 8 values as BF16 d 2^(-8s), exactly.  s >= 1: byte u = d + 128 of the biased integer, two values at once: 128 + (u & 127)
+// and 128, or 256 where u < 128, are BF16 numbers with u's bits in place under the exponent of 2^(7 - 8s), and d is their difference
+// (a byte permute, two logical operations and one subtraction for two values; a value at a time as FP32, then packed,
+// takes five).  The leading digit (s = 0, 9 bits with its bias) is placed by an OR into the mantissa of 2^23.
 template <int S, int s>
 __device__ __forceinline__ uint4 digit_row(const uint32_t (&lo)[8], const uint32_t (&hi)[8], const uint32_t (&lead)[8])
 {
-	float f[8];
 	if constexpr (s == 0) {
+		float f[8];
 #pragma unroll
 		for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(0x4B000000u | lead[j]) - 8388736.0f;
+		return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 	} else {
 		constexpr int k = S - 1 - s;
-		constexpr uint32_t K = (uint32_t)(150 - 8 * s) << 23;
-		constexpr uint32_t sel = 0x7650u | (uint32_t)(k & 3);
-		constexpr float sub = -8388736.0f * pow2f(-8 * s);
+		constexpr uint32_t E = (0x4300u - 0x400u * s) * 0x10001u;
+		constexpr uint32_t sel = (uint32_t)(k & 3) | (uint32_t)(4 + (k & 3)) << 8;
+		uint32_t y[4];
 #pragma unroll
-		for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(__byte_perm(k < 4 ? lo[j] : hi[j], K, sel)) + sub;
+		for (int j = 0; j < 4; ++j) {
+			const uint32_t w = __byte_perm(k < 4 ? lo[2 * j] : hi[2 * j], k < 4 ? lo[2 * j + 1] : hi[2 * j + 1], sel);
+			const uint32_t p = (w & 0x007F007Fu) | E, q = (~w & 0x00800080u) | E;
+			const __nv_bfloat162 d = __hsub2(*(const __nv_bfloat162*)&p, *(const __nv_bfloat162*)&q);
+			y[j] = *(const uint32_t*)&d;
+		}
+		return make_uint4(y[0], y[1], y[2], y[3]);
 	}
-	return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
 
 template <int S, int s>
@@ -234,15 +242,8 @@ __device__ __forceinline__ void store_slices(uint8_t* dst, int part_bytes, const
 // Digits / split parts of 8 consecutive K values (kk0 .. kk0+7 of a 32-K chunk) of data row m, written as one
 // 16-byte core-matrix row per part (two for TF32).  Eight consecutive threads taking eight consecutive rows of one
 // K group fill one whole 128-byte core matrix (conflict-free).  F = column scale (sliced mode).
-// Value access for the digit writers: FP64 values (the solution coefficients) or double-floats (the streamed lift
-// operand, which the producing kernels keep as FP32 pairs).
-__device__ __forceinline__ long long mantissa_of(double x, int sc) { return scaled_mantissa(x, sc); }
-__device__ __forceinline__ long long mantissa_of(df::df64 x, int sc) { return df::scaled_mantissa(x, sc); }
-__device__ __forceinline__ float float_of(double x) { return (float)x; }
-__device__ __forceinline__ float float_of(df::df64 x) { return x.hi + x.lo; }
-
-template <int FMT, int NP, bool SLICED, class T>
-__device__ __forceinline__ void store_digits8(uint8_t* chunk, int m, int kk0, const T (&x)[8], int F)
+template <int FMT, int NP, bool SLICED>
+__device__ __forceinline__ void store_digits8(uint8_t* chunk, int m, int kk0, const double (&x)[8], int F)
 {
 	constexpr int es = (FMT == 1 ? 2 : 4);
 	constexpr int part_bytes = kRows * 32 * es;
@@ -251,7 +252,7 @@ __device__ __forceinline__ void store_digits8(uint8_t* chunk, int m, int kk0, co
 		uint32_t lo[8], hi[8], lead[8];
 #pragma unroll
 		for (int j = 0; j < 8; ++j) {
-			const long long mm = mantissa_of(x[j], sc) + digit_bias<NP>();
+			const long long mm = biased_mantissa<NP>(x[j], sc);
 			lo[j] = (uint32_t)mm;
 			hi[j] = (uint32_t)((unsigned long long)mm >> 32);
 			lead[j] = (uint32_t)((int)(mm >> (8 * (NP - 1))) + 128);
@@ -261,7 +262,7 @@ __device__ __forceinline__ void store_digits8(uint8_t* chunk, int m, int kk0, co
 		float hi[8], lo[8];
 #pragma unroll
 		for (int j = 0; j < 8; ++j) {
-			const float xf = float_of(x[j]);
+			const float xf = (float)x[j];
 			hi[j] = __bfloat162float(__float2bfloat16_rn(xf));
 			lo[j] = xf - hi[j];
 		}
@@ -274,7 +275,7 @@ __device__ __forceinline__ void store_digits8(uint8_t* chunk, int m, int kk0, co
 		uint32_t hi[8], lo[8];
 #pragma unroll
 		for (int j = 0; j < 8; ++j) {
-			const float xf = float_of(x[j]);
+			const float xf = (float)x[j];
 			hi[j] = tf32_bits(xf);
 			lo[j] = tf32_bits(xf - __uint_as_float(hi[j]));
 		}
@@ -853,7 +854,7 @@ __device__ __forceinline__ void store_digits8_tmem(uint32_t ta, const double (&x
 		uint32_t lo[8], hi[8], lead[8];
 #pragma unroll
 		for (int j = 0; j < 8; ++j) {
-			const long long mm = scaled_mantissa(x[j], sc) + digit_bias<NP>();
+			const long long mm = biased_mantissa<NP>(x[j], sc);
 			lo[j] = (uint32_t)mm;
 			hi[j] = (uint32_t)((unsigned long long)mm >> 32);
 			lead[j] = (uint32_t)((int)(mm >> (8 * (NP - 1))) + 128);

@@ -3,8 +3,8 @@
 // SM against ~128 for FP32, so pointwise physics in double-float runs several times faster than in FP64 while
 // staying within ~1e-14 of it.  The building blocks are the error-free transformations TwoSum (Knuth), FastTwoSum
 // (Dekker) and the FMA-based TwoProd; addition, multiplication and division follow the "double-word" algorithms
-// analysed by Joldes, Muller and Popescu (ACM TOMS 44, 2017: AccurateDWPlusDW, DWTimesDW, DWDivDW); the square
-// root is one Newton step in double-float from the FP32 root (its correction term by the fast FP32 division).  The
+// analysed by Joldes, Muller and Popescu (ACM TOMS 44, 2017: AccurateDWPlusDW, DWTimesDW, DWDivDW); reciprocal and
+// reciprocal square root are one series step in double-float from the hardware's approximations.  The
 // conversion to FP64 and the digit extraction of the tensor-core path avoid FP64 instructions (integer and FP32
 // operations only).
 #pragma once
@@ -56,13 +56,40 @@ __device__ __forceinline__ df64 add_s(df64 x, df64 y)
 	return fast_two_sum(s.hi, s.lo + (x.lo + y.lo));
 }
 __device__ __forceinline__ df64 sub_s(df64 x, df64 y) { return add_s(x, neg(y)); }
-__device__ __forceinline__ df64 mul(df64 x, df64 y)
+// x y as an unnormalised pair: the leading product and its error with both cross terms (x.lo y.lo is below 2^-48).
+__device__ __forceinline__ df64 prod(df64 x, df64 y)
 {
 	const float p = x.hi * y.hi;
-	float e = fmaf(x.hi, y.hi, -p);
-	const float t = fmaf(x.lo, y.hi, x.hi * y.lo);
-	e += t;
-	return fast_two_sum(p, e);
+	return df64{p, fmaf(x.lo, y.hi, fmaf(x.hi, y.lo, fmaf(x.hi, y.hi, -p)))};
+}
+__device__ __forceinline__ df64 mul(df64 x, df64 y)
+{
+	const df64 p = prod(x, y);
+	return fast_two_sum(p.hi, p.lo);
+}
+// Sums of products and values: the leading parts by TwoSum, everything else in one FP32 number, normalised at the end only.
+// Each term costs 8 instructions (12 with its product); with a normalised product and a normalised sum per term it is 19.
+// The error stays within ~2^-47 of the largest term or partial sum, as with add_s.
+struct Sum {
+	float s, c;
+	__device__ __forceinline__ explicit Sum(df64 x) : s(x.hi), c(x.lo) {}
+	__device__ __forceinline__ Sum& operator+=(df64 x)   // x normalised or not
+	{
+		const df64 t = two_sum(s, x.hi);
+		s = t.hi;
+		c += t.lo + x.lo;
+		return *this;
+	}
+	__device__ __forceinline__ Sum& operator-=(df64 x) { return *this += df64{-x.hi, -x.lo}; }
+	__device__ __forceinline__ df64 value() const { return fast_two_sum(s, c); }
+};
+template <int N>
+__device__ __forceinline__ df64 dot(const df64* x, const df64* y)
+{
+	Sum s(prod(x[0], y[0]));
+#pragma unroll
+	for (int k = 1; k < N; ++k) s += prod(x[k], y[k]);
+	return s.value();
 }
 __device__ __forceinline__ df64 mulf(df64 x, float y)
 {
@@ -81,24 +108,26 @@ __device__ __forceinline__ df64 div(df64 x, df64 y)
 	const float tl = __fdiv_rn(d, y.hi);
 	return fast_two_sum(th, tl);
 }
-// 1 / y: the correctly rounded FP32 reciprocal of hi, then one Newton step r + r (1 - y r) whose residual is formed
-// with FMAs (exact for the hi part); relative error below 2^-45.
+// 1 / y: the hardware's FP32 approximation r (relative error e ~ 2^-23), then r (1 + e + e^2) with e = 1 - y r formed by
+// FMAs; relative error below 2^-45.
 __device__ __forceinline__ df64 rcp(df64 y)
 {
-	const float r = __frcp_rn(y.hi);
-	float e = fmaf(-y.hi, r, 1.f);
-	e = fmaf(-y.lo, r, e);
-	return fast_two_sum(r, r * e);
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y.hi));
+	const float e = fmaf(-y.lo, r, fmaf(-y.hi, r, 1.f));
+	return fast_two_sum(r, r * fmaf(e, e, e));
 }
-__device__ __forceinline__ df64 sqrt(df64 x)
+// 1 / sqrt(x): the hardware's approximation y, then y (1 + e/2 + 3/8 e^2), e = 1 - x y^2; NaN for x <= 0 (x = 0: infinity, NaN).
+__device__ __forceinline__ df64 rsqrt(df64 x)
 {
-	if (!(x.hi > 0.f)) return mk(0.f);
-	const float s = __fsqrt_rn(x.hi);
-	const float p = s * s;
-	const float e = fmaf(s, s, -p);
-	const float r = ((x.hi - p) - e) + x.lo;
-	return fast_two_sum(s, __fdividef(r, 2.f * s));   // the correction term needs ~24 bits: 2-ulp division
+	float y;
+	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x.hi));
+	const float p = y * y, pe = fmaf(y, y, -p);
+	const float e = fmaf(-x.lo, p, fmaf(-x.hi, pe, fmaf(-x.hi, p, 1.f)));
+	return fast_two_sum(y, y * fmaf(0.375f * e, e, 0.5f * e));
 }
+// x > 0: x / sqrt(x); else 0.
+__device__ __forceinline__ df64 sqrt(df64 x) { return x.hi > 0.f ? mul(x, rsqrt(x)) : mk(0.f); }
 __device__ __forceinline__ bool gt0(df64 a) { return a.hi > 0.f || (a.hi == 0.f && a.lo > 0.f); }
 __device__ __forceinline__ df64 absd(df64 a) { return a.hi < 0.f ? neg(a) : a; }
 __device__ __forceinline__ bool abs_less(df64 a, df64 b)   // |a| < |b|

@@ -247,11 +247,12 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 	if ((o.e_type != DPG_QUAD && o.e_type != DPG_HEX) || o.p < 1 || o.p + 1 > kN1Max) return DPG_OK;
 	const int N = ipow(o.p + 1, o.d);
 	if (o.n_s != N || o.n_c != N || o.n_fc != ipow(o.p + 1, o.d - 1) || o.n_fl != 2 * o.d) return DPG_OK;
-	// a mesh of fewer nodes than this is bound by the launch chain in either form (QUAD p = 1, 64 elements, one residual
-	// with its host round trip: 68.8 us here, 68.4 us dense; QUAD p = 2, 256 elements, 2,304 nodes: 24.2 us a stage
-	// here, 33.4 us dense) and keeps the dense kernels and their summation order
-	constexpr int64_t kMinNodes = 1024;
-	if (!general && (int64_t)sim->n_vol * N < kMinNodes) return DPG_OK;
+	// A mesh of fewer nodes than this is bound by the launch chain in either form and keeps the dense kernels and their
+	// summation order.  us here / dense: one residual with its host round trip, HEX p = 1, 1,728 nodes: 83.5 / 76.1, 4,096: 83.4 /
+	// 83.1; QUAD p = 1, 1,600 nodes: 72.4 / 69.7; a step of QUAD p = 1, 1,600 nodes: 48.0 / 49.3, 6,400: 51.6 / 55.5; of
+	// QUAD p = 2, 1,296: 53.6 / 56.0; of HEX p = 2, 1,728: 70.1 / 98.5.
+	const int64_t min_nodes = o.p == 1 ? 4096 : 1024;
+	if (!general && (int64_t)sim->n_vol * N < min_nodes) return DPG_OK;
 	TpState* st = new TpState();
 	st->n1 = o.p + 1;
 	if (!build_ops(st, o)) { delete st; return DPG_OK; }

@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, d
 	for (int a = 0; a < D; ++a) n[a] = fd.nrm[(size_t)t * D + a];
 	if constexpr (NV == D + 2) {
 		if constexpr (RS) {
-			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
-			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
+			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, 0.5 * fd.jf[t], nf);
+			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, 0.5 * fd.jf[t], nf);
 		} else if (num_flux == DPG_NUM_FLUX_ROE_PIKE) {
 			numflux_roe_pike<D>(WL, WR, n, nf);
 		} else {
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, d
 		const double b[3] = {bx, by, bz};
 		nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
 	}
-	const double j = fd.jf[t];
+	const double j = RS && NV == D + 2 ? 1.0 : fd.jf[t];   // the _rs fluxes come scaled
 #pragma unroll
 	for (int v = 0; v < NV; ++v) nnf[((size_t)f * NV + v) * n_fc + q] = nf[v] * j;
 }
@@ -250,7 +250,9 @@ static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs,
 		copy_boundary_trace(c, c->trace);
 	} else if (which == 1) {
 		const int n = c->fc.n_face * c->fc.n_fc, t = spread_threads(n, c->n_sm);
-		launch_chained(c->tp ? k_face<D, NV, true> : k_face<D, NV, false>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
+		// QUAD and HEX without the 1D operators keep the sums of numflux_roe_pike (small meshes of the Newton iteration)
+		const bool rs = c->tp || c->e_type == DPG_TRI || c->e_type == DPG_TET;
+		launch_chained(rs ? k_face<D, NV, true> : k_face<D, NV, false>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
 		                                                     c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	} else {
 		const int E_b = elems_of(c, c->vol_block_elems, 1);
@@ -312,8 +314,8 @@ __global__ void __launch_bounds__(256) k_face_tan(const double* trace, const dou
 	for (int a = 0; a < D; ++a) n[a] = fd.nrm[(size_t)t * D + a];
 	if constexpr (NV == D + 2) {
 		if constexpr (RS) {
-			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
-			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
+			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, 0.5 * fd.jf[t], nf);
+			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, 0.5 * fd.jf[t], nf);
 		} else if (num_flux == DPG_NUM_FLUX_ROE_PIKE) {
 			numflux_roe_pike<D>(WL, WR, n, nf);
 		} else {
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(256) k_face_tan(const double* trace, const dou
 		const double b[3] = {bx, by, bz};
 		nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
 	}
-	const double j = fd.jf[t];
+	const double j = RS && NV == D + 2 ? 1.0 : fd.jf[t];   // the _rs fluxes come scaled
 #pragma unroll
 	for (int v = 0; v < NV; ++v) nnf_t[((size_t)f * NV + v) * n_fc + q] = nf[v].d * j;
 }

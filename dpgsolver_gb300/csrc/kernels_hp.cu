@@ -170,11 +170,11 @@ __global__ void __launch_bounds__(128) k_hp_face(const double* trace, const __gr
 	}
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = h.nrm[t * D + a];
-	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike<D>(WL, WR, n, nf);
-	else                                   numflux_lax_friedrichs<D>(WL, WR, n, nf);
-	const double j = h.jf[t];
+	const double h2 = 0.5 * h.jf[t];
+	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, h2, nf);
+	else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, h2, nf);
 #pragma unroll
-	for (int v = 0; v < NV; ++v) nnf[NV * off + (size_t)v * n_fc + q] = nf[v] * j;
+	for (int v = 0; v < NV; ++v) nnf[NV * off + (size_t)v * n_fc + q] = nf[v];
 }
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update (solp holds the step's initial state).  flux: face fluxes

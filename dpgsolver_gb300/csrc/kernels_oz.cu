@@ -325,18 +325,18 @@ __global__ void __launch_bounds__(128) k_oz_flux(const double* trace, const doub
 #pragma unroll
 		for (int a = 0; a < D; ++a) n[a] = d.nrm[t * D + a];
 		if constexpr (NV == D + 2) {
-			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
-			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
+			const double h = 0.5 * d.jf[t];
+			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, h, nf);
+			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, h, nf);
 		} else {
-			nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
+			nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n) * d.jf[t];
 		}
-		const double j = d.jf[t];
 		double* xL = xl + d.face_xl[2 * f] + q;
 		double* xR = xl + d.face_xl[2 * f + 1] + qr;
 		const int lL = d.face_ld[2 * f], lR = d.face_ld[2 * f + 1];
 #pragma unroll
 		for (int v = 0; v < NV; ++v) {
-			const double y = nf[v] * j;
+			const double y = nf[v];
 			xL[(size_t)v * lL] = y;
 			xR[(size_t)v * lR] = __longlong_as_double(__double_as_longlong(y) ^ (long long)0x8000000000000000ull);
 		}

@@ -274,15 +274,15 @@ __global__ void __launch_bounds__(128) k_tp_face_br2(const double* trace, const 
 	}
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = V.nrm[(size_t)t * D + a];
-	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, nf);
-	else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, nf);
-	const double j = V.jf[t];
+	const double h = 0.5 * V.jf[t];
+	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, h, nf);
+	else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, h, nf);
 	const bool adiabatic = V.bc && V.bc[f] == DPG_BC_NOSLIP_ADIABATIC;
 #pragma unroll
 	for (int v = 0; v < NV; ++v) {
-		double y = Ld<T>::out(nf[v]) + 0.5 * (fvn[iL + (size_t)v * n_fc] + fvn[iR + (size_t)v * n_fc]);
+		double y = Ld<T>::out(nf[v]) + h * (fvn[iL + (size_t)v * n_fc] + fvn[iR + (size_t)v * n_fc]);
 		if (v == D + 1 && adiabatic) y = 0.0;   // prescribed: no energy flux through the wall
-		nnf[((size_t)f * NV + v) * n_fc + q] = y * j;
+		nnf[((size_t)f * NV + v) * n_fc + q] = y;
 	}
 }
 

@@ -155,18 +155,19 @@ __device__ __forceinline__ void ref_flux(const T* s, const Met& met, const doubl
 {
 	if constexpr (NV == D + 2) {
 		const T rho_inv = 1.0 / s[0], E = s[D + 1];
-		T u[D], V2 = 0.0;
+		T q = 0.0;   // (rho V)^2
 #pragma unroll
-		for (int a = 0; a < D; ++a) { u[a] = s[1 + a] * rho_inv; V2 += u[a] * u[a]; }
-		const T p = DPG_GM1_D * (E - 0.5 * s[0] * V2), Ep = E + p;
+		for (int a = 0; a < D; ++a) q += s[1 + a] * s[1 + a];
+		const T p = DPG_GM1_D * (E - 0.5 * (q * rho_inv)), Ep = E + p;
 #pragma unroll
 		for (int r = 0; r < D; ++r) {
 			double m[D];
 #pragma unroll
 			for (int x = 0; x < D; ++x) m[x] = met(x, r);
-			T W = m[0] * u[0], f0 = m[0] * s[1];
+			T f0 = m[0] * s[1];
 #pragma unroll
-			for (int x = 1; x < D; ++x) { W += m[x] * u[x]; f0 += m[x] * s[1 + x]; }
+			for (int x = 1; x < D; ++x) f0 += m[x] * s[1 + x];
+			const T W = f0 * rho_inv;
 			T fr[NV];
 			fr[0] = f0;
 #pragma unroll

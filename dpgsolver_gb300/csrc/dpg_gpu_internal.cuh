@@ -188,6 +188,7 @@ int  tp_volume(dpg_gpu_ctx* c);
 int  tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
 int  tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork& w);
 int  tp_lift_tan(dpg_gpu_ctx* c, const TanWork& w, double* out);
+bool tp_own_faces(const dpg_gpu_ctx* c);   // no k_face: the lift and stage kernels form their elements' face fluxes
 bool tp_viscous(const dpg_gpu_ctx* c);
 void tp_free(dpg_gpu_ctx* c);
 int  tp_general_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);   // boundary faces, BR2 (after tp_prepare)

@@ -276,7 +276,11 @@ static int dispatch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsign
 // Tensor-product meshes take the 1D operators of kernels_tp.cu for the element kernels (32x32x8 HEX p = 3 Euler:
 // 0.31 ms for the two against 4.66 ms here; 47x61 jittered QUAD p = 3: 26 us against 120 us).
 int launch_trace(dpg_gpu_ctx* c) { return c->tp ? tp_volume(c) : dispatch(c, 0, -1, false, nullptr); }
-int launch_face(dpg_gpu_ctx* c) { return dispatch(c, 1, -1, false, nullptr); }
+int launch_face(dpg_gpu_ctx* c)
+{
+	if (c->tp && tp_own_faces(c)) return DPG_OK;   // the lift forms them
+	return dispatch(c, 1, -1, false, nullptr);
+}
 int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
 {
 	return c->tp ? tp_lift(c, stage, write_rhs, max_slot) : dispatch(c, 2, stage, write_rhs, max_slot);

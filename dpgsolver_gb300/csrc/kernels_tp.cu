@@ -30,8 +30,8 @@ using namespace tp;
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update of sol (solp holds the step's initial state).  max_slot may
 // be null (the linearisation).
-template <int D, int NV, int N1>
-__global__ void __launch_bounds__(256) k_tp_lift(const double* G, const double* nnf, TpGeo g,
+template <int D, int NV, int N1, bool OWN>
+__global__ void __launch_bounds__(256) k_tp_lift(const double* G, const double* nnf, TpGeo g, TpFaces fa,
                                                  const __grid_constant__ Ops<N1> ops, double* sol,
                                                  double* solp, double* __restrict__ rhs,
                                                  const double* __restrict__ dt_ptr, unsigned long long* max_slot, int stage,
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) k_tp_lift(const double* G, const double* 
 		}
 		ji = g.affine ? g.jinv[e0 + e] : g.jinv[(size_t)(e0 + e) * N + i];
 	}
-	lift_body<D, NV, N1>(so, b0, b1, sF, e0, ne, g, nnf, ji, r);
+	lift_body<D, NV, N1, OWN>(so, b0, b1, sF, e0, ne, g, nnf, fa, ji, r);
 	unsigned long long lmax = 0;
 	if (live) {
 		const double dt = (stage >= 0 ? *dt_ptr : 0.0);
@@ -190,7 +190,8 @@ static int configure()
 	constexpr int E = most_elems(ipow(N1, D));
 	if (cudaFuncSetAttribute(k_tp_volume<D, NV, N1, false, kPeriodic>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, false>(E)) ||
 	    cudaFuncSetAttribute(k_tp_volume<D, NV, N1, true, kPeriodic>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_volume<D, NV, N1, true>(E)) ||
-	    cudaFuncSetAttribute(k_tp_lift<D, NV, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lift<D, NV, N1>(E)))
+	    cudaFuncSetAttribute(k_tp_lift<D, NV, N1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lift<D, NV, N1>(E)) ||
+	    cudaFuncSetAttribute(k_tp_lift<D, NV, N1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lift<D, NV, N1>(E)))
 		return DPG_ERR_CUDA;
 	return DPG_OK;
 }
@@ -217,8 +218,9 @@ static int launch_lift(dpg_gpu_ctx* c, const double* G, const double* nnf, doubl
 	const TpState* st = (const TpState*)c->tp;
 	constexpr int N = ipow(N1, D);
 	const TpGeo geo = geo_of(c);
-	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
-	launch_chained(k_tp_lift<D, NV, N1>, dim3(grid, nb), threads, smem_lift<D, NV, N1>(E), c->stream, G, nnf, geo, ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E, tan_stride(c));
+	const bool own = st->own && nnf == c->nnf;
+	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = own ? own_threads<D, N1>(E) : (E * N + 31) / 32 * 32;
+	launch_chained(own ? k_tp_lift<D, NV, N1, true> : k_tp_lift<D, NV, N1, false>, dim3(grid, nb), threads, smem_lift<D, NV, N1>(E), c->stream, G, nnf, geo, faces_of(c, c->trace), ops_of<N1>(st), c->sol, c->solp, rhs, c->ddt, max_slot, stage, write_rhs ? 1 : 0, E, tan_stride(c));
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 
@@ -237,6 +239,7 @@ int tp_lift_tan(dpg_gpu_ctx* c, const TanWork& w, double* out)
 {
 	DPG_TP_DISPATCH(launch_lift, c, w.G, w.nnf_t, out, nullptr, -1, true, w.nb);
 }
+bool tp_own_faces(const dpg_gpu_ctx* c) { return ((const TpState*)c->tp)->own; }
 bool tp_viscous(const dpg_gpu_ctx* c) { return ((const TpState*)c->tp)->viscous != 0; }
 
 // Set-up.  Leaves c->tp null (the dense kernels of kernels_fp64.cu run) where the element is not one of the orders above
@@ -274,6 +277,17 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 		if (cudaMemcpy(st->jn, ji.data(), sizeof(double) * ji.size(), cudaMemcpyHostToDevice) != cudaSuccess) return DPG_ERR_CUDA;
 	}
 	st->E = block_elems(sim->n_vol, N, c->n_sm);
+	// Below this many face nodes the lift and stage kernels form their elements' face fluxes (each flux twice, one launch less);
+	// the FP64 pipe has the time.  us per step (with the limiter), so / with k_face: QUAD p = 1, 4,096 face nodes:
+	// 41.3 / 47.6, 16,384: 55.5 / 50.1; QUAD p = 2, 1,536: 47.7 / 51.6, 15,000: 59.8 / 59.5; QUAD p = 3, 8,192: 51.5 / 53.8,
+	// 20,000: 84.6 / 80.4; HEX p = 1, 6,144: 53.5 / 64.4, 12,000: 61.8 / 65.7, 32,928: 98.5 / 80.3; HEX p = 2, 13,824: 74.1 / 71.8;
+	// HEX p = 3, 10,368: 76.0 / 76.1.  One residual gains 3 to 7 us of 31 to 36.
+	constexpr int64_t kOwnFaceNodes = 10000;
+	const int64_t face_nodes = sim->face_geo_off[sim->n_face];
+	if (!general && face_nodes <= kOwnFaceNodes) {
+		if ((rc = alloc(&st->trace2, (size_t)2 * c->n_var * face_nodes))) return rc;
+		st->own = true;
+	}
 	const int rc2 = configure_any(c);
 	return rc2 ? rc2 : tp_configure_stage(c);
 }

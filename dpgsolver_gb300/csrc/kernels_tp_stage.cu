@@ -156,8 +156,8 @@ static size_t smem_stage(int E)
 	return sizeof(Ops<N1>) + sizeof(double) * E * NV * (2 * N + work) + 8 + sizeof(int) * E;
 }
 
-template <int D, int NV, int N1, int KIND>
-__global__ void __launch_bounds__(256) k_tp_stage(double* G, const double* nnf, TpGeo g, TpBc B,
+template <int D, int NV, int N1, int KIND, bool OWN>
+__global__ void __launch_bounds__(256) k_tp_stage(double* G, const double* nnf, TpGeo g, TpFaces fa, TpBc B,
                                                   const __grid_constant__ Ops<N1> ops, const __grid_constant__ PosOps pops,
                                                   float amp, int* __restrict__ pos_err, double* sol,
                                                   double* solp, const double* __restrict__ dt_ptr,
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(256) k_tp_stage(double* G, const double* nnf, 
 		}
 		ji = g.affine ? g.jinv[e0 + e] : g.jinv[(size_t)(e0 + e) * N + i];
 	}
-	lift_body<D, NV, N1>(so, b0, b1, sW, e0, ne, g, nnf, ji, r);
+	lift_body<D, NV, N1, OWN>(so, b0, b1, sW, e0, ne, g, nnf, fa, ji, r);
 	unsigned long long lmax = 0;
 	__syncthreads();   // the last pass has read its buffer
 	if (live) {
@@ -219,10 +219,11 @@ static int configure_stage(dpg_gpu_ctx* c)
 	constexpr int E = most_elems(ipow(N1, D));
 	constexpr cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
 	const int sm = (int)smem_stage<D, NV, N1>(E);
-	if (cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kPeriodic>, A, sm) || cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kWalls>, A, sm))
+	if (cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kPeriodic, false>, A, sm) || cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kPeriodic, true>, A, sm) ||
+	    cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kWalls, false>, A, sm))
 		return DPG_ERR_CUDA;
 	if constexpr (NV == D + 2)
-		if (cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kViscous>, A, sm)) return DPG_ERR_CUDA;
+		if (cudaFuncSetAttribute(k_tp_stage<D, NV, N1, kViscous, false>, A, sm)) return DPG_ERR_CUDA;
 	return DPG_OK;
 }
 
@@ -233,22 +234,27 @@ static int launch_stage(dpg_gpu_ctx* c, int stage, unsigned long long* max_slot,
 	constexpr int N = ipow(N1, D);
 	const TpGeo geo = geo_of(c);
 	const TpBc B{st->bc, st->xyz, c->fc.nrm, st->bp};
-	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = (E * N + 31) / 32 * 32;
+	const int E = st->E, grid = (geo.n_vol + E - 1) / E, threads = st->own ? own_threads<D, N1>(E) : (E * N + 31) / 32 * 32;
+	// own face fluxes: the neighbours still read this stage's traces, so the next stage's go to the other array
+	double* const from = st->own && stage == 1 ? st->trace2 : c->trace;
+	double* const to = st->own && stage == 0 ? st->trace2 : c->trace;
 	const size_t sm = smem_stage<D, NV, N1>(E);
 	const Ops<N1> ops = ops_of<N1>(st);
 	const int limit = NV == D + 2 && c->positivity;
 	const PosOps pops = limit ? pos_ops<N1>(c) : PosOps{};
 	auto go = [&](auto kernel) {
-		return launch_chained(kernel, grid, threads, sm, c->stream, st->G, c->nnf, geo, B, ops, pops, c->pos_amp, c->pos_err, c->sol,
-		                      c->solp, c->ddt, max_slot, stage, limit, next, c->trace, st->Uc, E, c->b_adv[0], c->b_adv[1],
+		return launch_chained(kernel, grid, threads, sm, c->stream, st->G, c->nnf, geo, faces_of(c, from), B, ops, pops, c->pos_amp,
+		                      c->pos_err, c->sol, c->solp, c->ddt, max_slot, stage, limit, next, to, st->Uc, E, c->b_adv[0], c->b_adv[1],
 		                      c->b_adv[2]);
 	};
 	cudaError_t e;
 	if constexpr (NV == D + 2) {
-		e = st->viscous ? go(k_tp_stage<D, NV, N1, kViscous>)
-		                : c->walls_or_visc ? go(k_tp_stage<D, NV, N1, kWalls>) : go(k_tp_stage<D, NV, N1, kPeriodic>);
+		e = st->viscous ? go(k_tp_stage<D, NV, N1, kViscous, false>)
+		    : c->walls_or_visc ? go(k_tp_stage<D, NV, N1, kWalls, false>)
+		    : st->own ? go(k_tp_stage<D, NV, N1, kPeriodic, true>) : go(k_tp_stage<D, NV, N1, kPeriodic, false>);
 	} else {
-		e = c->walls_or_visc ? go(k_tp_stage<D, NV, N1, kWalls>) : go(k_tp_stage<D, NV, N1, kPeriodic>);
+		e = c->walls_or_visc ? go(k_tp_stage<D, NV, N1, kWalls, false>)
+		    : st->own ? go(k_tp_stage<D, NV, N1, kPeriodic, true>) : go(k_tp_stage<D, NV, N1, kPeriodic, false>);
 	}
 	return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }

@@ -15,9 +15,10 @@ inline size_t smem_lift(int E)
 
 // r (in: the weak divergence of this thread's node, collocated) += the lifted face fluxes, times 1 / detJ, at the solution
 // nodes.  b0, b1: [E][NV][N]; sF: [E][2 D][NV][NF].
-template <int D, int NV, int N1>
+// OWN: the face fluxes are formed here from the traces, the same value on both sides, instead of read from nnf.
+template <int D, int NV, int N1, bool OWN>
 __device__ __forceinline__ void lift_body(const Ops<N1>* so, double* b0, double* b1, double* sF, int e0, int ne,
-                                          const TpGeo& g, const double* nnf, double ji, double (&r)[NV])
+                                          const TpGeo& g, const double* nnf, const TpFaces& fa, double ji, double (&r)[NV])
 {
 	constexpr int N = ipow(N1, D), NF = ipow(N1, D - 1);
 	const int e = threadIdx.x / N, i = threadIdx.x - e * N;
@@ -29,10 +30,31 @@ __device__ __forceinline__ void lift_body(const Ops<N1>* so, double* b0, double*
 		const int f = vf >> 1, side = vf & 1;
 		const int qs = side ? g.nc_inv[(size_t)f * NF + q] : q;
 		const long long flip = side ? 0ll : (long long)0x8000000000000000ull;   // - outward flux of this element
+		double y[NV];
+		if constexpr (OWN) {
+			const size_t t = (size_t)f * NF + qs;
+			const int qr = side ? q : fa.nc[t];
+			double WL[NV], WR[NV], n[D];
+#pragma unroll
+			for (int w = 0; w < NV; ++w) {
+				WL[w] = fa.trace[((size_t)2 * f * NV + w) * NF + qs];
+				WR[w] = fa.trace[((size_t)(2 * f + 1) * NV + w) * NF + qr];
+			}
+#pragma unroll
+			for (int x = 0; x < D; ++x) n[x] = fa.nrm[t * D + x];
+			if constexpr (NV == D + 2) {
+				if (fa.num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, 0.5 * fa.jf[t], y);
+				else                                      numflux_lax_friedrichs_rs<D>(WL, WR, n, 0.5 * fa.jf[t], y);
+			} else {
+				y[0] = numflux_upwind<D>(fa.b, WL[0], WR[0], n) * fa.jf[t];
+			}
+		} else {
+#pragma unroll
+			for (int w = 0; w < NV; ++w) y[w] = nnf[((size_t)f * NV + w) * NF + qs];
+		}
 #pragma unroll
 		for (int w = 0; w < NV; ++w)
-			sF[((size_t)(ee * 2 * D + lf) * NV + w) * NF + q] =
-			    __longlong_as_double(__double_as_longlong(nnf[((size_t)f * NV + w) * NF + qs]) ^ flip);
+			sF[((size_t)(ee * 2 * D + lf) * NV + w) * NF + q] = __longlong_as_double(__double_as_longlong(y[w]) ^ flip);
 	}
 	__syncthreads();
 	if (live) {

@@ -12,6 +12,7 @@
 // passes of n1 terms, a face lift one term per node.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 #include <vector>
@@ -38,6 +39,8 @@ struct Ops {
 // Host state of a tensor-product context (dpg_gpu_ctx::tp).
 struct TpState {
 	int n1 = 0, E = 1;          // order + 1, elements per block
+	bool own = false;           // small meshes: k_tp_lift and k_tp_stage form their elements' face fluxes
+	double* trace2 = nullptr;   // own: the traces of every other stage
 	double* G = nullptr;        // [n_vol][n_var][n1^d] weak divergence in the collocated basis
 	double* jn = nullptr;       // non-affine: [n_vol][n1^d] 1 / detJ at the Gauss points
 	double B[25], Bi[25], Dw[25], Ds[25], lm[5], lp[5], wm[5], wp[5];
@@ -58,6 +61,16 @@ struct TpGeo {
 	const double* jinv;         // affine: [n_vol]; else [n_vol][n1^d]
 	const int* vol_face;        // [n_vol][2 d]  (face << 1) | side
 	const int* nc_inv;          // [n_face][n_fc]
+};
+
+// What a kernel needs to form the numerical fluxes of its elements' faces by itself.
+struct TpFaces {
+	const double* trace;        // [n_face][2][n_var][n_fc]
+	const int* nc;              // [n_face][n_fc]
+	const double* nrm;          // [n_face][n_fc][d]
+	const double* jf;           // [n_face][n_fc]
+	int num_flux;
+	double b[3];
 };
 
 // What boundary faces add: their codes and the positions and normals of the face nodes.
@@ -84,6 +97,10 @@ inline TpGeo geo_of(const dpg_gpu_ctx* c)
 	return TpGeo{g.n_vol, g.affine, g.met, g.affine ? g.jinv : st->jn, g.vol_face, g.nc_inv};
 }
 
+inline TpFaces faces_of(const dpg_gpu_ctx* c, const double* trace)
+{
+	return {trace, c->fc.nc, c->fc.nrm, c->fc.jf, c->num_flux, {c->b_adv[0], c->b_adv[1], c->b_adv[2]}};
+}
 constexpr int most_elems(int N) { return 256 / N; }   // elements per block: at most 256 threads of one node each
 
 // A launch of a kernel of <D, NV, N1> by the context's sizes.
@@ -123,6 +140,13 @@ __device__ __forceinline__ T pencil_dot(const double* row, const T* x, int base)
 #pragma unroll
 	for (int j = 1; j < N1; ++j) acc += row[j] * x[base + j * S];
 	return acc;
+}
+// A thread per face node too, as far as a block goes.
+template <int D, int N1>
+inline int own_threads(int E)
+{
+	const int n = ipow(N1, D), nf = 2 * D * ipow(N1, D - 1);
+	return std::min(256, (E * (n > nf ? n : nf) + 31) / 32 * 32);
 }
 
 // Position of node i along direction A, and the first node of its pencil.

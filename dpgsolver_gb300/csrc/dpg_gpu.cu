@@ -588,8 +588,8 @@ extern "C" int dpg_gpu_launches_per_rhs(dpg_gpu_ctx* c)
 {
 	if (!c) return 0;
 	// no launch of its own for the face fluxes
-	if (c->n_var == 1 && (c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64))) return 2;
-	if (!c->walls_or_visc && c->tp && c->prec_mode == DPG_PREC_FP64 && dpg::tp_own_faces(c)) return 2;
+	if (!c->walls_or_visc && c->prec_mode == DPG_PREC_FP64 && !c->oz &&
+	    (c->hp || c->adv ? dpg::hp_launches(c) == 2 : c->tp ? dpg::tp_own_faces(c) : dpg::dense_own_faces(c))) return 2;
 	return !c->walls_or_visc ? 3 : c->tp ? dpg::tp_general_launches(c) : 4;
 }
 

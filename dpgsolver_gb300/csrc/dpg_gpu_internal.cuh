@@ -168,6 +168,9 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
 	return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Up to this many face nodes of a mesh its volume or lift kernels form their elements' face fluxes themselves.
+constexpr int64_t kOwnFaceNodes = 10000;
+
 int launch_trace (dpg_gpu_ctx* c);
 int launch_face  (dpg_gpu_ctx* c);
 int launch_face_tan(dpg_gpu_ctx* c, const TanWork& w);   // tangents of the face fluxes
@@ -188,7 +191,8 @@ int  tp_volume(dpg_gpu_ctx* c);
 int  tp_lift(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
 int  tp_volume_tan(dpg_gpu_ctx* c, const double* u, const double* v, const TanWork& w);
 int  tp_lift_tan(dpg_gpu_ctx* c, const TanWork& w, double* out);
-bool tp_own_faces(const dpg_gpu_ctx* c);   // no k_face: the lift and stage kernels form their elements' face fluxes
+bool dense_own_faces(const dpg_gpu_ctx* c);  // no k_face: the dense volume kernel forms its elements' face fluxes
+bool tp_own_faces(const dpg_gpu_ctx* c);     // the same: the lift and stage kernels form their elements' face fluxes
 bool tp_viscous(const dpg_gpu_ctx* c);
 void tp_free(dpg_gpu_ctx* c);
 int  tp_general_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim);   // boundary faces, BR2 (after tp_prepare)
@@ -203,6 +207,7 @@ int  tp_step(dpg_gpu_ctx* c, unsigned long long* max_slots);   // one SSP-RK3 st
 // mixed orders (kernels_hp.cu): FP64 residual over volume groups of each order; which = 0 traces, 1 face fluxes,
 // 2 volume terms (with the RK stage)
 int  hp_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot);
+int  hp_launches(const dpg_gpu_ctx* c);
 bool hp_steps(const dpg_gpu_ctx* c);                            // advection on affine elements:
 int  hp_step(dpg_gpu_ctx* c, unsigned long long* max_slots);   // one SSP-RK3 step
 int  hp_launch_part(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsigned long long* max_slot);

@@ -75,6 +75,27 @@ static void copy_boundary_trace(dpg_gpu_ctx* c, double* trace, int nb = 1, size_
 	if (n) launch_chained(k_copy_boundary_trace, dim3((n + 127) / 128, nb), 128, 0, c->stream, c->bface, c->n_bface, c->fc.n_fc, trace, stride);
 }
 
+// The numerical flux of a face node times its face Jacobian; RS: the shorter form (flux.cuh).
+template <int D, int NV, bool RS>
+__device__ __forceinline__ void face_flux(const double* WL, const double* WR, const double* n, double j, int num_flux, double bx,
+                                          double by, double bz, double* nf)
+{
+	if constexpr (NV == D + 2 && RS) {
+		if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, 0.5 * j, nf);
+		else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, 0.5 * j, nf);
+	} else {
+		if constexpr (NV == D + 2) {
+			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike<D>(WL, WR, n, nf);
+			else                                   numflux_lax_friedrichs<D>(WL, WR, n, nf);
+		} else {
+			const double b[3] = {bx, by, bz};
+			nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
+		}
+#pragma unroll
+		for (int v = 0; v < NV; ++v) nf[v] = nf[v] * j;
+	}
+}
+
 template <int D, int NV, bool RS>
 __global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, double* __restrict__ nnf,
                                               int num_flux, double bx, double by, double bz)
@@ -93,29 +114,19 @@ __global__ void __launch_bounds__(256) k_face(const double* trace, FaceDev fd, d
 	}
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = fd.nrm[(size_t)t * D + a];
-	if constexpr (NV == D + 2) {
-		if constexpr (RS) {
-			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, 0.5 * fd.jf[t], nf);
-			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, 0.5 * fd.jf[t], nf);
-		} else if (num_flux == DPG_NUM_FLUX_ROE_PIKE) {
-			numflux_roe_pike<D>(WL, WR, n, nf);
-		} else {
-			numflux_lax_friedrichs<D>(WL, WR, n, nf);
-		}
-	} else {
-		const double b[3] = {bx, by, bz};
-		nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n);
-	}
-	const double j = RS && NV == D + 2 ? 1.0 : fd.jf[t];   // the _rs fluxes come scaled
+	face_flux<D, NV, RS>(WL, WR, n, fd.jf[t], num_flux, bx, by, bz, nf);
 #pragma unroll
-	for (int v = 0; v < NV; ++v) nnf[((size_t)f * NV + v) * n_fc + q] = nf[v] * j;
+	for (int v = 0; v < NV; ++v) nnf[((size_t)f * NV + v) * n_fc + q] = nf[v];
 }
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update of sol (solp holds the step's initial state).
-template <int D, int NV>
+enum { kFaceRead = 0, kFaceOwn = 1, kFaceOwnRs = 2 };
+
+// FACES: the face fluxes are read from nnf, or formed here from the traces in its place (with numflux_.. or numflux_.._rs).
+template <int D, int NV, int FACES>
 __global__ void __launch_bounds__(256) k_volume(double* sol, double* solp, double* __restrict__ rhs,
-                                                const double* nnf, GroupDev g, const double* __restrict__ dt_ptr,
-                                                unsigned long long* max_slot, int stage, int write_rhs, int E_b,
+                                                const double* nnf, GroupDev g, FaceDev fd, const double* __restrict__ dt_ptr,
+                                                unsigned long long* max_slot, int stage, int write_rhs, int E_b, int num_flux,
                                                 double bx, double by, double bz)
 {
 	extern __shared__ double sm[];
@@ -147,9 +158,25 @@ __global__ void __launch_bounds__(256) k_volume(double* sol, double* solp, doubl
 		const int f = vf >> 1, side = vf & 1;
 		const int qs = side ? g.nc_inv[(size_t)f * n_fc + q] : q;
 		const double sgn = side ? -1.0 : 1.0;
+		double nf[NV];
+		if constexpr (FACES != kFaceRead) {
+			const size_t t = (size_t)f * n_fc + qs;
+			const int qr = side ? q : fd.nc[t];
+			double WL[NV], WR[NV], n[D];
 #pragma unroll
-		for (int v = 0; v < NV; ++v)
-			sX[((size_t)e * NV + v) * K + D * n_c + r] = sgn * nnf[((size_t)f * NV + v) * n_fc + qs];
+			for (int v = 0; v < NV; ++v) {
+				WL[v] = nnf[((size_t)(2 * f + 0) * NV + v) * n_fc + qs];
+				WR[v] = nnf[((size_t)(2 * f + 1) * NV + v) * n_fc + qr];
+			}
+#pragma unroll
+			for (int a = 0; a < D; ++a) n[a] = fd.nrm[t * D + a];
+			face_flux<D, NV, FACES == kFaceOwnRs>(WL, WR, n, fd.jf[t], num_flux, bx, by, bz, nf);
+		} else {
+#pragma unroll
+			for (int v = 0; v < NV; ++v) nf[v] = nnf[((size_t)f * NV + v) * n_fc + qs];
+		}
+#pragma unroll
+		for (int v = 0; v < NV; ++v) sX[((size_t)e * NV + v) * K + D * n_c + r] = sgn * nf[v];
 	}
 	__syncthreads();
 	// 3. physical flux and reference flux fr[eq][r][c] = sum_x m_{x r} f[x][eq]
@@ -238,6 +265,19 @@ static int elems_of(const dpg_gpu_ctx* c, int most, int nb)
 	return std::max(1, (int)std::min<int64_t>(most, ((int64_t)c->g.n_vol * nb + c->n_sm - 1) / c->n_sm));
 }
 
+// QUAD and HEX without the 1D operators (small meshes) keep the sums of numflux_roe_pike: a Newton iteration that stagnates at
+// rounding amplifies a change of the last bit.
+static bool rs_fluxes(const dpg_gpu_ctx* c) { return c->tp || c->e_type == DPG_TRI || c->e_type == DPG_TET; }
+
+// Small meshes: k_volume forms its elements' face fluxes, each flux twice (the FP64 pipe has the time), one launch less.  us per
+// step, so / with k_face: QUAD p = 1, 64 elements: 46.0 / 49.5; TRI p = 1, 1,152: 47.2 / 51.3; TRI p = 2, 2,048 (9,216 face
+// nodes): 65.9 / 70.0; TET p = 2, 384: 71.9 / 76.2; one residual gains 2 to 5 us of 27 to 35.  Beyond the line (TRI p = 2, 13,824
+// face nodes) the doubled fluxes cost more.
+bool dense_own_faces(const dpg_gpu_ctx* c)
+{
+	return !c->tp && !c->walls_or_visc && (int64_t)c->fc.n_face * c->fc.n_fc <= kOwnFaceNodes;
+}
+
 template <int D, int NV>
 static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsigned long long* max_slot)
 {
@@ -250,16 +290,15 @@ static int launch_all_impl(dpg_gpu_ctx* c, int which, int stage, bool write_rhs,
 		copy_boundary_trace(c, c->trace);
 	} else if (which == 1) {
 		const int n = c->fc.n_face * c->fc.n_fc, t = spread_threads(n, c->n_sm);
-		// QUAD and HEX without the 1D operators keep the sums of numflux_roe_pike (small meshes of the Newton iteration)
-		const bool rs = c->tp || c->e_type == DPG_TRI || c->e_type == DPG_TET;
-		launch_chained(rs ? k_face<D, NV, true> : k_face<D, NV, false>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
+		launch_chained(rs_fluxes(c) ? k_face<D, NV, true> : k_face<D, NV, false>, (n + t - 1) / t, t, 0, c->stream, c->trace, c->fc, c->nnf, c->num_flux,
 		                                                     c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	} else {
 		const int E_b = elems_of(c, c->vol_block_elems, 1);
 		const size_t smem = (size_t)E_b * NV * (g.n_s + (g.n_c > g.n_s ? g.n_c : g.n_s) + g.K) * sizeof(double);
 		const int grid = (g.n_vol + E_b - 1) / E_b;
-		launch_chained(k_volume<D, NV>, grid, 256, smem, c->stream, c->sol, c->solp, c->rhs, c->nnf, g, c->ddt, max_slot, stage,
-		                                               write_rhs ? 1 : 0, E_b, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+		auto kernel = !dense_own_faces(c) ? k_volume<D, NV, kFaceRead> : rs_fluxes(c) ? k_volume<D, NV, kFaceOwnRs> : k_volume<D, NV, kFaceOwn>;
+		launch_chained(kernel, grid, 256, smem, c->stream, c->sol, c->solp, c->rhs, dense_own_faces(c) ? c->trace : c->nnf, g, c->fc, c->ddt,
+		               max_slot, stage, write_rhs ? 1 : 0, E_b, c->num_flux, c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	}
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
@@ -278,7 +317,7 @@ static int dispatch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsign
 int launch_trace(dpg_gpu_ctx* c) { return c->tp ? tp_volume(c) : dispatch(c, 0, -1, false, nullptr); }
 int launch_face(dpg_gpu_ctx* c)
 {
-	if (c->tp && tp_own_faces(c)) return DPG_OK;   // the lift forms them
+	if (c->tp ? tp_own_faces(c) : dense_own_faces(c)) return DPG_OK;   // the lift, or the volume kernel, forms them
 	return dispatch(c, 1, -1, false, nullptr);
 }
 int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
@@ -520,18 +559,16 @@ int fp64_configure(dpg_gpu_ctx* c)
 	if (E_j > 16) E_j = 16;
 	c->tan_block_elems = E_j;
 	if (E_b * per_v > kSmemOptIn || E_t * per_t > kSmemOptIn) return DPG_ERR_CUDA;
-	cudaError_t e = cudaSuccess;
-#define SETATTR(KV, KT, KJ)                                                                                          \
-	e = cudaFuncSetAttribute(KV, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn); if (e) return DPG_ERR_CUDA; \
-	e = cudaFuncSetAttribute(KT, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn); if (e) return DPG_ERR_CUDA; \
-	e = cudaFuncSetAttribute(KJ, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn); if (e) return DPG_ERR_CUDA;
-	if (c->d == 2 && NV == 4) { SETATTR((k_volume<2, 4>), (k_trace<4>), (k_volume_tan<2, 4>)) }
-	else if (c->d == 3 && NV == 5) { SETATTR((k_volume<3, 5>), (k_trace<5>), (k_volume_tan<3, 5>)) }
-	else if (c->d == 2 && NV == 1) { SETATTR((k_volume<2, 1>), (k_trace<1>), (k_volume_tan<2, 1>)) }
-	else if (c->d == 3 && NV == 1) { SETATTR((k_volume<3, 1>), (k_trace<1>), (k_volume_tan<3, 1>)) }
-	else return DPG_ERR_UNSUPPORTED;
-#undef SETATTR
-	return DPG_OK;
+	auto set = [&](auto... kernels) {
+		return ((cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) == cudaSuccess) && ...) ? DPG_OK : DPG_ERR_CUDA;
+	};
+#define DENSE_KERNELS(D, NV) k_volume<D, NV, kFaceRead>, k_volume<D, NV, kFaceOwn>, k_volume<D, NV, kFaceOwnRs>, k_trace<NV>, k_volume_tan<D, NV>
+	if (c->d == 2 && NV == 4) return set(DENSE_KERNELS(2, 4));
+	if (c->d == 3 && NV == 5) return set(DENSE_KERNELS(3, 5));
+	if (c->d == 2 && NV == 1) return set(DENSE_KERNELS(2, 1));
+	if (c->d == 3 && NV == 1) return set(DENSE_KERNELS(3, 1));
+#undef DENSE_KERNELS
+	return DPG_ERR_UNSUPPORTED;
 }
 
 } // namespace dpg
@@ -592,14 +629,14 @@ static int noalloc_launch(const dpg_noalloc_mesh& m, const double* sol, double* 
 	const size_t per_t = (size_t)NV * g.n_s * sizeof(double);
 	int E_t = (int)((32 * 1024) / per_t);
 	E_t = E_t < 1 ? 1 : (E_t > 16 ? 16 : E_t);
-	if (cudaFuncSetAttribute(k_volume<D, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) ||
+	if (cudaFuncSetAttribute(k_volume<D, NV, kFaceRead>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) ||
 	    cudaFuncSetAttribute(k_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn))
 		return DPG_ERR_CUDA;
 	if (cudaMemsetAsync(slot, 0, sizeof(unsigned long long), st) != cudaSuccess) return DPG_ERR_CUDA;
 	launch_chained(k_trace<NV>, (g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st, sol, g, trace, E_t, TanStride{});
 	const int nq = fd.n_face * fd.n_fc;
 	launch_chained(k_face<D, NV, false>, (nq + 127) / 128, 128, 0, st, trace, fd, nnf, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
-	launch_chained(k_volume<D, NV>, (g.n_vol + E_b - 1) / E_b, 256, E_b * per_v, st, const_cast<double*>(sol), nullptr, rhs, nnf, g, nullptr, slot, -1, 1, E_b, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
+	launch_chained(k_volume<D, NV, kFaceRead>, (g.n_vol + E_b - 1) / E_b, 256, E_b * per_v, st, const_cast<double*>(sol), nullptr, rhs, nnf, g, fd, nullptr, slot, -1, 1, E_b, m.num_flux, m.b_adv[0], m.b_adv[1], m.b_adv[2]);
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
 

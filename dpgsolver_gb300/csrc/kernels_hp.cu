@@ -27,7 +27,8 @@
 //     TRI 1..4 (mixed),  8,192: 105 / 58     TET 1..4 (mixed), 34,992: 2,288 / 918
 //     TRI 1,   8,192: 39 / 27                TRI 4, 288: 46 / 24, 8,192: 103 / 80, 32,768: 308 / 263
 //     TET 2,  34,992: 322 / 281              TET 3, 3,072: 165 / 93, 34,992: 906 / 783      TET 4, 3,072: 683 / 193
-//   Euler TRI 1..3 (mixed), us per residual: 1,152 volumes 48 / 45, 8,192: 75 / 70
+//   Euler (mixed), us per step: TRI 1..3, 1,152 volumes: 91 / 88; QUAD 1..4, 64: 337 / 131, 10,000: 792 / 514; HEX 1..3, 64:
+//   1,659 / 449, 1,728: 2,998 / 1,012
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -84,6 +85,7 @@ struct HpState {
 	size_t smem_trace = 0, smem_volume = 0;
 	int blocks = 0;
 	bool folded = false;                   // k_hp_advect in the place of k_hp_volume
+	bool own = false;                      // Euler, small meshes: k_hp_volume forms its elements' face fluxes
 };
 
 __device__ __forceinline__ int hp_group_of(const HpDev& h, int blk)
@@ -151,6 +153,18 @@ __global__ void __launch_bounds__(kHpThreads) k_hp_trace(const double* sol, cons
 	hp_traces<NV>(sU, sSide, G, G.n_stage ? sT : G.ops + G.n_tr0, n_fl, h.nfc_max, ne, trace);
 }
 
+// The numerical flux of a face node times its face Jacobian.
+template <int D, int NV>
+__device__ __forceinline__ void hp_numflux(const double* WL, const double* WR, const double* n, double j, int num_flux, const double* b, double* nf)
+{
+	if constexpr (NV == 1) {
+		nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n) * j;
+	} else {
+		if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, 0.5 * j, nf);
+		else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, 0.5 * j, nf);
+	}
+}
+
 template <int D, int NV>
 __global__ void __launch_bounds__(128) k_hp_face(const double* trace, const __grid_constant__ HpDev h, double* __restrict__ nnf,
                                                  int num_flux)
@@ -170,19 +184,17 @@ __global__ void __launch_bounds__(128) k_hp_face(const double* trace, const __gr
 	}
 #pragma unroll
 	for (int a = 0; a < D; ++a) n[a] = h.nrm[t * D + a];
-	const double h2 = 0.5 * h.jf[t];
-	if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, h2, nf);
-	else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, h2, nf);
+	hp_numflux<D, NV>(WL, WR, n, h.jf[t], num_flux, nullptr, nf);
 #pragma unroll
 	for (int v = 0; v < NV; ++v) nnf[NV * off + (size_t)v * n_fc + q] = nf[v];
 }
 
 // stage < 0: residual only.  stage 0..2: SSP-RK3 stage update (solp holds the step's initial state).  flux: face fluxes
-// (Euler) or traces (advection).
-template <int D, int NV>
+// or, OWN, traces: the block forms its elements' face fluxes itself.
+template <int D, int NV, bool OWN>
 __global__ void __launch_bounds__(kHpThreads) k_hp_volume(double* sol, double* solp, double* __restrict__ rhs, const double* flux,
                                                    const __grid_constant__ HpDev h, const double* __restrict__ dt_ptr,
-                                                   unsigned long long* max_slot, int stage, int write_rhs,
+                                                   unsigned long long* max_slot, int stage, int write_rhs, int num_flux,
                                                    double bx, double by, double bz)
 {
 	extern __shared__ __align__(16) double sm[];
@@ -215,13 +227,19 @@ __global__ void __launch_bounds__(kHpThreads) k_hp_volume(double* sol, double* s
 		const int64_t off = side_offset(t);
 		const double sgn = side ? -1.0 : 1.0;
 		double* x = sX + (size_t)e * NV * Kx + t.x + q;
-		if constexpr (NV == 1) {
-			const int other = side ? h.nc_inv[off + q] : h.nc[off + q], ql = side ? other : q;
-			const double wl = flux[2 * off + ql], wr = flux[2 * off + n_fc + (side ? q : other)];
-			double n[D];
+		if constexpr (OWN) {
+			const int other = side ? h.nc_inv[off + q] : h.nc[off + q], ql = side ? other : q, qr = side ? q : other;
+			double WL[NV], WR[NV], n[D], nf[NV];
+#pragma unroll
+			for (int v = 0; v < NV; ++v) {
+				WL[v] = flux[2 * NV * off + (size_t)v * n_fc + ql];
+				WR[v] = flux[2 * NV * off + (size_t)(NV + v) * n_fc + qr];
+			}
 #pragma unroll
 			for (int a = 0; a < D; ++a) n[a] = h.nrm[(off + ql) * D + a];
-			*x = sgn * (numflux_upwind<D>(b, wl, wr, n) * h.jf[off + ql]);
+			hp_numflux<D, NV>(WL, WR, n, h.jf[off + ql], num_flux, b, nf);
+#pragma unroll
+			for (int v = 0; v < NV; ++v) x[(size_t)v * Kx] = sgn * nf[v];
 		} else {
 			const int qs = side ? h.nc_inv[off + q] : q;
 #pragma unroll
@@ -480,7 +498,8 @@ template <int D, int NV>
 static int hp_set_smem(HpState* s)
 {
 	if (cudaFuncSetAttribute(k_hp_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_trace) ||
-	    cudaFuncSetAttribute(k_hp_volume<D, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume) ||
+	    cudaFuncSetAttribute(k_hp_volume<D, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume) ||
+	    cudaFuncSetAttribute(k_hp_volume<D, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume) ||
 	    cudaFuncSetAttribute(k_hp_advect<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume))
 		return DPG_ERR_CUDA;
 	return DPG_OK;
@@ -582,6 +601,9 @@ int hp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, const OzTables* share)
 		const size_t per_v = sizeof(double) * (2 * n_fl + NV * (o.n_s + ((kv + n_fl * h.nfc_max) | 1) + (folded || !G.affine ? o.n_s : 0)));
 		const size_t per_t = sizeof(double) * (2 * n_fl + NV * o.n_s);
 		G.E_b = std::max(1, std::min({16, kHpThreads / o.n_s, (int)((96 * 1024) / per_v)}));
+		// small meshes leave every SM a block (us per Euler step, 288 TRI 1..3: 109 -> 80; k_hp_advect has less work than
+		// staging per volume: 288 TRI 4 23 -> 31)
+		if (!folded) G.E_b = std::min(G.E_b, (n_vol + c->n_sm - 1) / c->n_sm);
 		smem_t = std::max(smem_t, G.E_b * per_t + (G.n_stage ? G.n_tr : 0) * sizeof(double));
 		smem_v = std::max(smem_v, G.E_b * per_v + G.n_stage * sizeof(double));
 		G.blk0 = blocks;
@@ -644,7 +666,8 @@ int hp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, const OzTables* share)
 	}
 	for (int k = 0; k < (folded ? 2 : 1); ++k)
 		if ((rc = hp_upload(s, &s->trace[k], (const double*)nullptr, (size_t)2 * NV * n_fnode))) return rc;
-	if (NV > 1 && (rc = hp_upload(s, &s->nnf, (const double*)nullptr, (size_t)NV * n_fnode))) return rc;
+	s->own = NV > 1 && n_fnode <= kOwnFaceNodes;
+	if (NV > 1 && !s->own && (rc = hp_upload(s, &s->nnf, (const double*)nullptr, (size_t)NV * n_fnode))) return rc;
 	if (d == 2 && NV == 1) return hp_set_smem<2, 1>(s);
 	if (d == 3 && NV == 1) return hp_set_smem<3, 1>(s);
 	if (d == 2 && NV == 4) return hp_set_smem<2, 4>(s);
@@ -678,6 +701,7 @@ static int hp_launch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsig
 		if constexpr (NV > 1) {
 			const int64_t n = h.n_fnode;
 			const int ft = spread_threads(n, c->n_sm);
+			if (s->own) return DPG_OK;
 			launch_chained(k_hp_face<D, NV>, (unsigned)((n + ft - 1) / ft), ft, 0, c->stream, s->trace[0], h, s->nnf, c->num_flux);
 		}
 	} else if (NV == 1 && s->folded) {
@@ -685,9 +709,10 @@ static int hp_launch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsig
 		               c->ddt, max_slot, stage, write_rhs ? 1 : 0, next ? s->trace[1 - from] : nullptr, c->b_adv[0], c->b_adv[1],
 		               c->b_adv[2]);
 	} else {
-		launch_chained(k_hp_volume<D, NV>, s->blocks, kHpThreads, s->smem_volume, c->stream, c->sol, c->solp, c->rhs,
-		               NV > 1 ? s->nnf : s->trace[0], h, c->ddt, max_slot, stage, write_rhs ? 1 : 0, c->b_adv[0], c->b_adv[1],
-		               c->b_adv[2]);
+		const bool own = NV == 1 || s->own;
+		launch_chained(own ? k_hp_volume<D, NV, true> : k_hp_volume<D, NV, false>, s->blocks, kHpThreads, s->smem_volume, c->stream,
+		               c->sol, c->solp, c->rhs, own ? s->trace[0] : s->nnf, h, c->ddt, max_slot, stage, write_rhs ? 1 : 0, c->num_flux,
+		               c->b_adv[0], c->b_adv[1], c->b_adv[2]);
 	}
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }
@@ -713,6 +738,9 @@ int hp_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* m
 	if ((rc = hp_launch_part(c, 1, stage, write_rhs, max_slot))) return rc;
 	return hp_launch_part(c, 2, stage, write_rhs, max_slot);
 }
+
+// Kernels of one residual.
+int hp_launches(const dpg_gpu_ctx* c) { return c->n_var == 1 || hp_state(c)->own ? 2 : 3; }
 
 // Whether hp_step may take the place of three stages.
 bool hp_steps(const dpg_gpu_ctx* c) { return c->prec_mode == DPG_PREC_FP64 && hp_state(c) && hp_state(c)->folded; }

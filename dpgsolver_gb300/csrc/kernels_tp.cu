@@ -251,11 +251,10 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 	const int N = ipow(o.p + 1, o.d);
 	if (o.n_s != N || o.n_c != N || o.n_fc != ipow(o.p + 1, o.d - 1) || o.n_fl != 2 * o.d) return DPG_OK;
 	// A mesh of fewer nodes than this is bound by the launch chain in either form and keeps the dense kernels and their
-	// summation order.  us here / dense: one residual with its host round trip, HEX p = 1, 1,728 nodes: 83.5 / 76.1, 4,096: 83.4 /
-	// 83.1; QUAD p = 1, 1,600 nodes: 72.4 / 69.7; a step of QUAD p = 1, 1,600 nodes: 48.0 / 49.3, 6,400: 51.6 / 55.5; of
-	// QUAD p = 2, 1,296: 53.6 / 56.0; of HEX p = 2, 1,728: 70.1 / 98.5.
-	const int64_t min_nodes = o.p == 1 ? 4096 : 1024;
-	if (!general && (int64_t)sim->n_vol * N < min_nodes) return DPG_OK;
+	// summation order.  us per step here / dense (both with their own face fluxes): QUAD p = 1, 1,024 nodes: 41.2 / 46.0;
+	// QUAD p = 2, 1,296: 47.7 / 52; HEX p = 1, 1,728: 53.5 / 60.
+	constexpr int64_t kMinNodes = 1024;
+	if (!general && (int64_t)sim->n_vol * N < kMinNodes) return DPG_OK;
 	TpState* st = new TpState();
 	st->n1 = o.p + 1;
 	if (!build_ops(st, o)) { delete st; return DPG_OK; }
@@ -282,7 +281,6 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 	// 41.3 / 47.6, 16,384: 55.5 / 50.1; QUAD p = 2, 1,536: 47.7 / 51.6, 15,000: 59.8 / 59.5; QUAD p = 3, 8,192: 51.5 / 53.8,
 	// 20,000: 84.6 / 80.4; HEX p = 1, 6,144: 53.5 / 64.4, 12,000: 61.8 / 65.7, 32,928: 98.5 / 80.3; HEX p = 2, 13,824: 74.1 / 71.8;
 	// HEX p = 3, 10,368: 76.0 / 76.1.  One residual gains 3 to 7 us of 31 to 36.
-	constexpr int64_t kOwnFaceNodes = 10000;
 	const int64_t face_nodes = sim->face_geo_off[sim->n_face];
 	if (!general && face_nodes <= kOwnFaceNodes) {
 		if ((rc = alloc(&st->trace2, (size_t)2 * c->n_var * face_nodes))) return rc;

@@ -1,5 +1,5 @@
-"""Tensor-product meshes small enough that the lift and stage kernels form their elements' face fluxes themselves, against the
-CPU oracle: every order, both fluxes, affine and jittered elements, advection, residual and steps (with the limiter), sizes that
+"""Meshes small enough that their last kernel forms its elements' face fluxes itself (1D operators, dense operators, mixed
+orders), against the CPU oracle: every order, both fluxes, affine and jittered elements, advection, residual and steps (with the limiter), sizes that
 leave the last block of elements partly filled, and the side of the line where the fluxes have a kernel of their own.
 
 Tolerance 1e-11 of the largest entry, the repository's FP64 bound."""
@@ -28,6 +28,12 @@ CASES = {
     "hex-p2-jitter": (dict(EUL, d=3, p=2, n_elem=(5, 4, 3), jitter=0.1, seed=4), 2),
     "hex-p3-lf": (dict(EUL, d=3, p=3, n_elem=(4, 3, 3), num_flux="Lax-Friedrichs"), 2),
     "hex-p4": (dict(EUL, d=3, p=4, n_elem=(3, 3, 2)), 2),
+    "dense-quad-p2": (dict(EUL, d=2, p=2, n_elem=(7, 5, 1)), 2),
+    "dense-hex-p1-lf": (dict(EUL, d=3, p=1, n_elem=(5, 4, 3), num_flux="Lax-Friedrichs"), 2),
+    "tri-p2": (dict(EUL, d=2, element="tri", p=2, n_elem=(33, 33, 1), jitter=0.1, seed=3), 2),
+    "tri-p2-beyond": (dict(EUL, d=2, element="tri", p=2, n_elem=(34, 33, 1), jitter=0.1, seed=3), 3),
+    "tri-p1to3": (dict(EUL, d=2, element="tri", p=1, p_max=3, p_seed=5, n_elem=(11, 9, 1), jitter=0.1, seed=3), 2),
+    "hex-p1to2": (dict(EUL, d=3, p=1, p_max=2, p_seed=5, n_elem=(4, 3, 3), jitter=0.1, seed=3), 2),
     "quad-p2-advection": (dict(ADV, d=2, p=2, n_elem=(13, 11, 1), jitter=0.1, seed=3), 2),
     "hex-p2-advection": (dict(ADV, d=3, p=2, n_elem=(4, 4, 3)), 2),
 }

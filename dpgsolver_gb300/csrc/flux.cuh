@@ -205,36 +205,69 @@ __device__ __forceinline__ T numflux_upwind(const double* b, T wl, T wr, const d
 //   dTs/dx = (dE/dx rho - E drho/dx) / rho^2 - V . dV/dx  (Ts = p / (rho (gamma - 1)));
 //   f[x] = -(0, tau[0][x], .., tau[d-1][x], kappa dTs/dx + sum_j u_j tau[x][j]), kappa = gamma mu / Pr.
 template <int D, class T>
-__device__ __forceinline__ void flux_viscous(double mu, double kappa, const T* s, const T (*g)[D + 2], T f[D][D + 2])
+__device__ __forceinline__ void viscous_terms(double mu, const T* s, const T (*g)[D + 2], T (&u)[D], T (&tau)[D][D], T (&dTs)[D])
 {
-	const T rho_inv = 1.0 / s[0], E = s[D + 1];
-	T u[D], du[D][D];
+	const T rho_inv = 1.0 / s[0], e = s[D + 1] * rho_inv;
+	T du[D][D];
 #pragma unroll
 	for (int a = 0; a < D; ++a) u[a] = s[1 + a] * rho_inv;
 #pragma unroll
 	for (int i = 0; i < D; ++i)
 #pragma unroll
 		for (int x = 0; x < D; ++x) du[i][x] = rho_inv * (g[x][1 + i] - g[x][0] * u[i]);
-	T divV = 0.0;
+	T divV = du[0][0];
 #pragma unroll
-	for (int a = 0; a < D; ++a) divV += du[a][a];
-	T tau[D][D];
+	for (int a = 1; a < D; ++a) divV += du[a][a];
+	const T third = (-2.0 / 3.0 * mu) * divV;
 #pragma unroll
 	for (int i = 0; i < D; ++i)
 #pragma unroll
-		for (int j = 0; j < D; ++j)
-			tau[i][j] = (i == j) ? mu * 2.0 * (du[i][i] - (1.0 / 3.0) * divV) : mu * (du[j][i] + du[i][j]);
+		for (int j = 0; j < D; ++j) tau[i][j] = (i == j) ? (2.0 * mu) * du[i][i] + third : mu * (du[j][i] + du[i][j]);
 #pragma unroll
 	for (int x = 0; x < D; ++x) {
-		T dV2 = 0.0, w = 0.0;
+		dTs[x] = rho_inv * (g[x][D + 1] - e * g[x][0]);
 #pragma unroll
-		for (int a = 0; a < D; ++a) { dV2 += u[a] * du[a][x]; w += u[a] * tau[x][a]; }
-		const T dTs = rho_inv * rho_inv * (g[x][D + 1] * s[0] - E * g[x][0]) - dV2;
+		for (int a = 0; a < D; ++a) dTs[x] = dTs[x] - u[a] * du[a][x];
+	}
+}
+
+template <int D, class T>
+__device__ __forceinline__ void flux_viscous(double mu, double kappa, const T* s, const T (*g)[D + 2], T f[D][D + 2])
+{
+	T u[D], tau[D][D], dTs[D];
+	viscous_terms<D>(mu, s, g, u, tau, dTs);
+#pragma unroll
+	for (int x = 0; x < D; ++x) {
+		T w = kappa * dTs[x];
+#pragma unroll
+		for (int a = 0; a < D; ++a) w += u[a] * tau[x][a];
 		f[x][0] = T(0.0);
 #pragma unroll
 		for (int i = 0; i < D; ++i) f[x][1 + i] = -tau[i][x];
-		f[x][D + 1] = -(kappa * dTs + w);
+		f[x][D + 1] = -w;
 	}
+}
+
+// The same along a normal: fn = sum_x n_x f[x].
+template <int D, class T>
+__device__ __forceinline__ void flux_viscous_normal(double mu, double kappa, const T* s, const T (*g)[D + 2], const double* n, T* fn)
+{
+	T u[D], tau[D][D], dTs[D];
+	viscous_terms<D>(mu, s, g, u, tau, dTs);
+	T q = n[0] * dTs[0];
+#pragma unroll
+	for (int x = 1; x < D; ++x) q += n[x] * dTs[x];
+	T w = kappa * q;
+	fn[0] = T(0.0);
+#pragma unroll
+	for (int i = 0; i < D; ++i) {
+		T t = n[0] * tau[i][0];
+#pragma unroll
+		for (int x = 1; x < D; ++x) t += n[x] * tau[i][x];
+		w += u[i] * t;
+		fn[1 + i] = -t;
+	}
+	fn[D + 1] = -w;
 }
 
 // Parameters of the boundary states.

@@ -115,6 +115,11 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* Uc, const double*
 	// volume gradient at this node
 	T gx[D][NV];
 	if (live) {
+		double jm[D][D];
+#pragma unroll
+		for (int x = 0; x < D; ++x)
+#pragma unroll
+			for (int r = 0; r < D; ++r) jm[x][r] = ji * m[x][r];
 #pragma unroll
 		for (int w = 0; w < NV; ++w) {
 			T dr[D];
@@ -128,10 +133,10 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* Uc, const double*
 			if constexpr (D == 3) along(std::integral_constant<int, 2>{});
 #pragma unroll
 			for (int x = 0; x < D; ++x) {
-				T acc = m[x][0] * dr[0];
+				T acc = jm[x][0] * dr[0];
 #pragma unroll
-				for (int r = 1; r < D; ++r) acc += m[x][r] * dr[r];
-				gx[x][w] = ji * acc;
+				for (int r = 1; r < D; ++r) acc += jm[x][r] * dr[r];
+				gx[x][w] = acc;
 				sG[((size_t)(x * E + e) * NV + w) * N + i] = gx[x][w];
 			}
 		}
@@ -142,11 +147,11 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* Uc, const double*
 		const int ee = o / (2 * D * NF), k = o - ee * 2 * D * NF, lf = k / NF, q = k - lf * NF, a = lf >> 1;
 		const int vf = g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
 		const double* l = (lf & 1) ? so->lp : so->lm;
-		const double* lw = (lf & 1) ? so->wp : so->wm;
+		const double* lw = (lf & 1) ? so->lwp : so->lwm;
 		const int S = stride_of<N1>(a), base = face_base<N1>(a, q);
 		double cq = 0.0, n[D];
 #pragma unroll
-		for (int j = 0; j < N1; ++j) cq = fma(l[j] * lw[j], sD[ee * N + base + j * S], cq);
+		for (int j = 0; j < N1; ++j) cq = fma(lw[j], sD[ee * N + base + j * S], cq);
 		cq *= V.scale;
 #pragma unroll
 		for (int x = 0; x < D; ++x) n[x] = sN[((size_t)(ee * 2 * D + lf) * D + x) * NF + q];
@@ -165,15 +170,10 @@ __global__ void __launch_bounds__(256) k_tp_grad(const double* Uc, const double*
 			W[w] = Ld<T>::at(trace, trace_t, ((size_t)vf * NV + w) * NF + q);
 		}
 		auto emit = [&](int slot) {
-			T F[D][NV];
-			flux_viscous<D>(V.mu, V.kappa, W, gq, F);
+			T F[NV];
+			flux_viscous_normal<D>(V.mu, V.kappa, W, gq, n, F);
 #pragma unroll
-			for (int w = 0; w < NV; ++w) {
-				T acc = n[0] * F[0][w];
-#pragma unroll
-				for (int x = 1; x < D; ++x) acc += n[x] * F[x][w];
-				fvn[((size_t)slot * NV + w) * NF + q] = Ld<T>::out(acc);
-			}
+			for (int w = 0; w < NV; ++w) fvn[((size_t)slot * NV + w) * NF + q] = Ld<T>::out(F[w]);
 		};
 		emit(vf);
 		if (V.bc && V.bc[vf >> 1]) {   // boundary face: the boundary state with the interior gradient

@@ -34,6 +34,7 @@ struct Ops {
 	double Ds[N1 * N1];    // [i][j]  l_j'(x_i)
 	double lm[N1], lp[N1]; // collocated basis at -1 and +1
 	double wm[N1], wp[N1]; // the same over the weights
+	double lwm[N1], lwp[N1]; // lm wm, lp wp
 };
 
 // Host state of a tensor-product context (dpg_gpu_ctx::tp).
@@ -86,7 +87,10 @@ inline Ops<N1> ops_of(const TpState* st)
 {
 	Ops<N1> o;
 	for (int k = 0; k < N1 * N1; ++k) { o.B[k] = st->B[k]; o.Bi[k] = st->Bi[k]; o.Dw[k] = st->Dw[k]; o.Ds[k] = st->Ds[k]; }
-	for (int k = 0; k < N1; ++k) { o.lm[k] = st->lm[k]; o.lp[k] = st->lp[k]; o.wm[k] = st->wm[k]; o.wp[k] = st->wp[k]; }
+	for (int k = 0; k < N1; ++k) {
+		o.lm[k] = st->lm[k]; o.lp[k] = st->lp[k]; o.wm[k] = st->wm[k]; o.wp[k] = st->wp[k];
+		o.lwm[k] = st->lm[k] * st->wm[k]; o.lwp[k] = st->lp[k] * st->wp[k];
+	}
 	return o;
 }
 

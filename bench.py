@@ -570,7 +570,7 @@ def _advection_tri(dg, np, lib):
     """The advection configuration's element type and mesh: 2D linear advection, velocity (1, 0.5), upwind flux, on a
     periodic unit square of 64 x 64 cells split into 8,192 triangles with vertices jittered by up to 0.1 h (seeded).
     One uniform order per run, p = 1..4, and the configuration itself: each triangle's order drawn uniformly from
-    {1, 2, 3, 4} (seeded), all orders in each of the three launches of a residual.  FP64 residual throughput (CUDA
+    {1, 2, 3, 4} (seeded), all orders in each launch of a residual.  FP64 residual throughput (CUDA
     events on the library stream) and parity with the oracle's own set-up (all host threads); at one order per mesh
     also the split-precision modes' parity and the S = 7 residual time."""
     from oracle import Oracle

@@ -109,16 +109,16 @@ __device__ __forceinline__ df64 div(df64 x, df64 y)
 	return fast_two_sum(th, tl);
 }
 // 1 / y: the hardware's FP32 approximation r (relative error e ~ 2^-23), then r (1 + e + e^2) with e = 1 - y r formed by
-// FMAs; relative error below 2^-45.
+// FMAs; relative error below 2^-45 (|y| beyond 2^126: r is a subnormal number, 2^-22).
 __device__ __forceinline__ df64 rcp(df64 y)
 {
 	float r;
-	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y.hi));
+	asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y.hi));
 	const float e = fmaf(-y.lo, r, fmaf(-y.hi, r, 1.f));
 	return fast_two_sum(r, r * fmaf(e, e, e));
 }
-// 1 / sqrt(x): the hardware's approximation y, then y (1 + e/2 + 3/8 e^2), e = 1 - x y^2; NaN for x <= 0 (x = 0: infinity, NaN).
-__device__ __forceinline__ df64 rsqrt(df64 x)
+// 1 / sqrt(x) of a normal x > 0: the hardware's approximation y, then y (1 + e/2 + 3/8 e^2), e = 1 - x y^2.
+__device__ __forceinline__ df64 rsqrt_normal(df64 x)
 {
 	float y;
 	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x.hi));
@@ -126,8 +126,22 @@ __device__ __forceinline__ df64 rsqrt(df64 x)
 	const float e = fmaf(-x.lo, p, fmaf(-x.hi, pe, fmaf(-x.hi, p, 1.f)));
 	return fast_two_sum(y, y * fmaf(0.375f * e, e, 0.5f * e));
 }
+// The instruction takes a subnormal number for zero, and |V|^2 of a gas nearly at rest is one (|V| < 1.1e-19): such an x goes
+// through 2^64 x, a branch that is hardly ever taken.  Negative x, zero and NaN give NaN.
+constexpr float kMinNormal = 1.17549435e-38f;   // 2^-126
+__device__ __forceinline__ df64 rsqrt(df64 x)
+{
+	if (x.hi > 0.f && x.hi < kMinNormal) return scale(rsqrt_normal(scale(x, 0x1p64f)), 0x1p32f);
+	return rsqrt_normal(x);
+}
 // x > 0: x / sqrt(x); else 0.
-__device__ __forceinline__ df64 sqrt(df64 x) { return x.hi > 0.f ? mul(x, rsqrt(x)) : mk(0.f); }
+__device__ __forceinline__ df64 sqrt(df64 x)
+{
+	if (x.hi >= kMinNormal) return mul(x, rsqrt_normal(x));
+	if (!(x.hi > 0.f)) return mk(0.f);
+	const df64 t = scale(x, 0x1p64f);
+	return scale(mul(t, rsqrt_normal(t)), 0x1p-32f);
+}
 __device__ __forceinline__ bool gt0(df64 a) { return a.hi > 0.f || (a.hi == 0.f && a.lo > 0.f); }
 __device__ __forceinline__ df64 absd(df64 a) { return a.hi < 0.f ? neg(a) : a; }
 __device__ __forceinline__ bool abs_less(df64 a, df64 b)   // |a| < |b|

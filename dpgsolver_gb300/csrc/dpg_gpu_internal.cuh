@@ -168,6 +168,15 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, s
 	return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Shared-memory opt-in of a kernel without static shared memory: the device's largest block, for every context of the process.
+// The attribute belongs to the function: a limit of this context's size would refuse the launches of an earlier one with larger
+// blocks.
+constexpr int kSmemOptIn = 227 * 1024;
+inline bool allow_smem(const void* kernel)
+{
+	return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) == cudaSuccess;
+}
+
 // Up to this many face nodes of a mesh its volume or lift kernels form their elements' face fluxes themselves.
 constexpr int64_t kOwnFaceNodes = 10000;
 

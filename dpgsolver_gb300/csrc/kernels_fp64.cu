@@ -536,9 +536,6 @@ int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, cons
 	return DPG_ERR_UNSUPPORTED;
 }
 
-// Shared-memory opt-in of the element kernels: the device's largest block for every context, so that a later context with
-// smaller blocks does not lower the limit of an earlier one.
-constexpr int kSmemOptIn = 227 * 1024;
 int fp64_configure(dpg_gpu_ctx* c)
 {
 	const GroupDev& g = c->g;
@@ -560,7 +557,7 @@ int fp64_configure(dpg_gpu_ctx* c)
 	c->tan_block_elems = E_j;
 	if (E_b * per_v > kSmemOptIn || E_t * per_t > kSmemOptIn) return DPG_ERR_CUDA;
 	auto set = [&](auto... kernels) {
-		return ((cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) == cudaSuccess) && ...) ? DPG_OK : DPG_ERR_CUDA;
+		return (allow_smem((const void*)kernels) && ...) ? DPG_OK : DPG_ERR_CUDA;
 	};
 #define DENSE_KERNELS(D, NV) k_volume<D, NV, kFaceRead>, k_volume<D, NV, kFaceOwn>, k_volume<D, NV, kFaceOwnRs>, k_trace<NV>, k_volume_tan<D, NV>
 	if (c->d == 2 && NV == 4) return set(DENSE_KERNELS(2, 4));
@@ -629,9 +626,7 @@ static int noalloc_launch(const dpg_noalloc_mesh& m, const double* sol, double* 
 	const size_t per_t = (size_t)NV * g.n_s * sizeof(double);
 	int E_t = (int)((32 * 1024) / per_t);
 	E_t = E_t < 1 ? 1 : (E_t > 16 ? 16 : E_t);
-	if (cudaFuncSetAttribute(k_volume<D, NV, kFaceRead>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn) ||
-	    cudaFuncSetAttribute(k_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOptIn))
-		return DPG_ERR_CUDA;
+	if (!allow_smem((const void*)k_volume<D, NV, kFaceRead>) || !allow_smem((const void*)k_trace<NV>)) return DPG_ERR_CUDA;
 	if (cudaMemsetAsync(slot, 0, sizeof(unsigned long long), st) != cudaSuccess) return DPG_ERR_CUDA;
 	launch_chained(k_trace<NV>, (g.n_vol + E_t - 1) / E_t, 256, E_t * per_t, st, sol, g, trace, E_t, TanStride{});
 	const int nq = fd.n_face * fd.n_fc;

@@ -495,14 +495,11 @@ void hp_free(dpg_gpu_ctx* c)
 }
 
 template <int D, int NV>
-static int hp_set_smem(HpState* s)
+static int hp_set_smem(const HpState* s)
 {
-	if (cudaFuncSetAttribute(k_hp_trace<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_trace) ||
-	    cudaFuncSetAttribute(k_hp_volume<D, NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume) ||
-	    cudaFuncSetAttribute(k_hp_volume<D, NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume) ||
-	    cudaFuncSetAttribute(k_hp_advect<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem_volume))
-		return DPG_ERR_CUDA;
-	return DPG_OK;
+	if (s->smem_trace > kSmemOptIn || s->smem_volume > kSmemOptIn) return DPG_ERR_CUDA;
+	return allow_smem((const void*)k_hp_trace<NV>) && allow_smem((const void*)k_hp_volume<D, NV, false>) &&
+	       allow_smem((const void*)k_hp_volume<D, NV, true>) && allow_smem((const void*)k_hp_advect<D>) ? DPG_OK : DPG_ERR_CUDA;
 }
 
 // share: null with mixed orders (c->hp); else the device tables of a context of one order that takes hp_step and

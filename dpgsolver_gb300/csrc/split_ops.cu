@@ -13,7 +13,6 @@
 namespace dpg {
 namespace split {
 
-constexpr int kSmemMax = 227 * 1024;
 constexpr int kSmemOneBlock = 116 * 1024;   // requests at least this much: one block per SM (512 TMEM columns)
 
 // ------------------------------------------------------------------------------------------------------------
@@ -290,7 +289,7 @@ int split_prepare(dpg_gpu_ctx* c)
 	pl.off_dig = kSlotsL * pl.stage_bytes;
 	pl.off_tab = pl.off_dig;   // digits live in TMEM; the epilogue writes from registers
 	pl.off_colF = pl.off_tab;
-	if (pi.smem_bytes > kSmemMax || pl.off_colF + 4 * kRows + 8 * (2 * kSlotsL + 2 * kMaxHalfSlots + 1) + 16 > kSmemMax) {
+	if (pi.smem_bytes > kSmemOptIn || pl.off_colF + 4 * kRows + 8 * (2 * kSlotsL + 2 * kMaxHalfSlots + 1) + 16 > kSmemOptIn) {
 		split_free(c);
 		return DPG_ERR_UNSUPPORTED;
 	}
@@ -346,8 +345,7 @@ int split_prepare(dpg_gpu_ctx* c)
 		if (cudaMalloc(&st->met2, sizeof(float2) * n_met) ||
 		    cudaMemcpy(st->met2, m2.data(), sizeof(float2) * n_met, cudaMemcpyHostToDevice)) { split_free(c); return DPG_ERR_CUDA; }
 	}
-	if (cudaFuncSetAttribute(st->kt.interp_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pi.smem_bytes) ||
-	    cudaFuncSetAttribute(st->kt.lift_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem_bytes)) {
+	if (!allow_smem(st->kt.interp_fn) || !allow_smem(st->kt.lift_fn)) {
 		split_free(c);
 		return DPG_ERR_CUDA;
 	}

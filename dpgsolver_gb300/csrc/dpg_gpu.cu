@@ -695,19 +695,18 @@ size_t tangent_bytes(const dpg_gpu_ctx* c)
 	return sizeof(double) * (s.tr + s.nf + (c->tp ? s.dof : 0) + (visc ? s.dof + s.tr : 0));
 }
 
-// work buffers of the linearisation for nb directions
-int alloc_tangent_work(dpg_gpu_ctx* c, int nb, TanWork* w)
+int alloc_tangent_work(dpg_gpu_ctx* c, int most, TanWork* w, std::initializer_list<DirBuffer> more)
 {
 	const TanStride s = tan_stride(c);
-	const bool visc = c->tp && tp_viscous(c);
-	auto al = [&](double** p, size_t n) { return cudaMalloc((void**)p, (size_t)nb * n * sizeof(double)) == cudaSuccess; };
-	if (!al(&w->trace_t, s.tr) || !al(&w->nnf_t, s.nf) || (c->tp && !al(&w->G, s.dof)) ||
-	    (visc && (!al(&w->Uc_t, s.dof) || !al(&w->fvn, s.tr)))) {
-		free_tangent_work(w);
-		return DPG_ERR_CUDA;
-	}
-	w->nb = nb;
-	return DPG_OK;
+	const size_t dof = c->tp ? s.dof : 0, visc = c->tp && tp_viscous(c) ? 1 : 0;
+	auto get = [](void** p, size_t bytes) {
+		if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+		cudaGetLastError();   // answered here: the next launch does not see it
+		return false;
+	};
+	w->nb = alloc_directions(most, {{&w->trace_t, s.tr}, {&w->nnf_t, s.nf}, {&w->G, dof}, {&w->Uc_t, visc * s.dof}, {&w->fvn, visc * s.tr}},
+	                         more, get, [](void* p) { cudaFree(p); });
+	return w->nb ? DPG_OK : DPG_ERR_CUDA;
 }
 
 void free_tangent_work(TanWork* w)

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "batch_alloc.h"
 #include "dpg_gb300.h"
 #include "dpg_simulation.h"
 
@@ -190,7 +191,8 @@ int launch_volume(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long*
 int jvp_fp64(dpg_gpu_ctx* c, const double* u, const double* v, double* out, const TanWork& w);
 int ensure_tangent_buffers(dpg_gpu_ctx* c);             // c->tan
 size_t tangent_bytes(const dpg_gpu_ctx* c);             // of a TanWork, per direction
-int alloc_tangent_work(dpg_gpu_ctx* c, int nb, TanWork* w);
+// w for the largest batch up to `most` directions that fits (w->nb), with more buffers of the same batch: all or none
+int alloc_tangent_work(dpg_gpu_ctx* c, int most, TanWork* w, std::initializer_list<DirBuffer> more = {});
 void free_tangent_work(TanWork* w);
 
 // tensor-product elements (kernels_tp.cu): traces and weak divergence, then lift, stage and norm; the tangents of the

@@ -878,7 +878,7 @@ static int multidot(dpg_gpu_ctx* c, Implicit* im, int nv, const double* V, const
 // Block columns by tangent probing: the directions of all (colour, column) pairs are independent, so they go through the
 // linearisation's launches in batches (an 8x8 QUAD p = 2 mesh has 396 probes of ~60 us each one after another, bound by
 // the launch chain on 4 blocks; all of them at once take ~1 ms).  nbr null: diagonal blocks only.
-constexpr size_t kProbeBytes = (size_t)512 << 20;   // work space of a batch, kept with the implicit state
+constexpr size_t kProbeBytes = (size_t)512 << 20;   // work space of a batch, kept with the implicit state; less where it does not fit
 
 static int probe_blocks(dpg_gpu_ctx* c, Implicit* im, const int* colour, int n_colours, const int* nbr, double* diag, double* offd)
 {
@@ -887,18 +887,18 @@ static int probe_blocks(dpg_gpu_ctx* c, Implicit* im, const int* colour, int n_c
 	if (!im->probe.nb) {
 		const size_t per = tangent_bytes(c) + 2 * sizeof(double) * im->n;
 		const int most = (int)std::max<size_t>(1, std::min<size_t>(kProbeBytes / per, (size_t)n_probes));
-		if ((rc = alloc_tangent_work(c, most, &im->probe))) return rc;
-		if (cudaMalloc((void**)&im->pV, (size_t)most * im->n * 8) != cudaSuccess ||
-		    cudaMalloc((void**)&im->pJV, (size_t)most * im->n * 8) != cudaSuccess)
-			return DPG_ERR_CUDA;
+		alloc_tangent_work(c, most, &im->probe, {{&im->pV, (size_t)im->n}, {&im->pJV, (size_t)im->n}});
 	}
-	for (int p0 = 0; p0 < n_probes; p0 += im->probe.nb) {
-		TanWork w = im->probe;
-		w.nb = std::min(im->probe.nb, n_probes - p0);
+	// no room for one direction more: one after another through the buffers of the Krylov products
+	const TanWork all = im->probe.nb ? im->probe : c->tan;
+	double *V = im->probe.nb ? im->pV : im->up, *JV = im->probe.nb ? im->pJV : im->F1;
+	for (int p0 = 0; p0 < n_probes; p0 += all.nb) {
+		TanWork w = all;
+		w.nb = std::min(all.nb, n_probes - p0);
 		const dim3 grid((unsigned)std::min<int64_t>((im->n + 255) / 256, 1216), w.nb);
-		k_probe_directions<<<grid, 256, 0, c->stream>>>(n_vol, nb, colour, p0, im->pV);
-		if ((rc = jvp_fp64(c, im->u, im->pV, im->pJV, w))) return rc;
-		k_extract_probes<<<grid, 256, 0, c->stream>>>(n_vol, nb, c->g.n_fl, im->pJV, colour, nbr, p0, im->inv_dtau, diag, offd);
+		k_probe_directions<<<grid, 256, 0, c->stream>>>(n_vol, nb, colour, p0, V);
+		if ((rc = jvp_fp64(c, im->u, V, JV, w))) return rc;
+		k_extract_probes<<<grid, 256, 0, c->stream>>>(n_vol, nb, c->g.n_fl, JV, colour, nbr, p0, im->inv_dtau, diag, offd);
 	}
 	return cudaGetLastError() == cudaSuccess ? DPG_OK : DPG_ERR_CUDA;
 }

@@ -64,6 +64,14 @@ static int dense_limiter(dpg_gpu_ctx* c, const dpg_element_ops& o, int n_vol, co
 	return dupload(c, (double**)&g.bsT, bsT.data(), bsT.size());
 }
 
+// The sliced FP64 form where it is the faster one; the dense kernels where there is no room for its tables.
+static void prepare_oz(dpg_gpu_ctx* c, const struct dpg_sim* sim, const dpg::OzTables& t)
+{
+	if (dpg::oz_prepare(c, sim, t) == DPG_OK) return;
+	dpg::oz_free(c);
+	cudaGetLastError();
+}
+
 // Mixed orders: state, the per-order volume groups and the face tables of kernels_hp.cu (periodic meshes, FP64
 // residual and explicit steps).
 static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
@@ -90,7 +98,7 @@ static int create_mixed_orders(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 	if ((rc = dalloc(c, &c->ddt, 1))) return fail(rc);
 	if (cudaMemset(c->rhs, 0, sizeof(double) * c->n_dof) != cudaSuccess) return fail(DPG_ERR_CUDA);
 	if ((rc = dpg::hp_prepare(c, sim, nullptr))) return fail(rc);
-	if ((rc = dpg::oz_prepare(c, sim, dpg::hp_tables(c, sim)))) return fail(rc);
+	prepare_oz(c, sim, dpg::hp_tables(c, sim));
 	// Euler: the dense positivity limiter per order group (Bezier operators of each order, n_s <= 64)
 	if (sim->pde_index == DPG_PDE_EULER && nv == d + 2) {
 		std::vector<std::vector<int>> members(sim->n_ops);
@@ -284,7 +292,7 @@ extern "C" int dpg_gpu_create(const struct dpg_sim* sim, dpg_gpu_ctx** ctx_out)
 		dpg::OzTables t;
 		t.met[0] = g.met; t.jinv[0] = g.jinv; t.vol_face = g.vol_face;
 		t.nc = fd.nc; t.nc_inv = g.nc_inv; t.nrm = fd.nrm; t.jf = fd.jf;
-		if ((rc = dpg::oz_prepare(c, sim, t))) return fail(rc);
+		prepare_oz(c, sim, t);
 		// advection on simplices, all sizes: 1.15 to 3.5 times as fast as the dense kernels (figures in kernels_hp.cu), which
 		// keep meshes with boundary faces, whose traces they copy
 		if (nv == 1 && (c->e_type == DPG_TRI || c->e_type == DPG_TET) && !general && (rc = dpg::hp_prepare(c, sim, &t))) return fail(rc);
@@ -416,12 +424,21 @@ extern "C" int dpg_gpu_download_rhs(dpg_gpu_ctx* c, double* h)
 	return DPG_OK;
 }
 
+// Whether the sliced form takes the FP64 residual.  Without room for its work arrays the dense kernels do, from here on.
+static bool oz_takes(dpg_gpu_ctx* c)
+{
+	if (!c->oz || c->prec_mode != DPG_PREC_FP64) return false;
+	if (dpg::oz_ready(c) == DPG_OK) return true;
+	dpg::oz_free(c);
+	return false;
+}
+
 // One residual evaluation (optionally an RK stage) on the context stream; no synchronisation.
 static int enqueue_residual(dpg_gpu_ctx* c, int stage, bool write_rhs, unsigned long long* max_slot)
 {
 	int rc;
 	if (c->walls_or_visc && c->tp) return dpg::tp_general_residual(c, stage, write_rhs, max_slot);
-	if (c->oz && c->prec_mode == DPG_PREC_FP64) return dpg::oz_residual(c, stage, write_rhs, max_slot);
+	if (oz_takes(c)) return dpg::oz_residual(c, stage, write_rhs, max_slot);
 	if (c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64)) return dpg::hp_residual(c, stage, write_rhs, max_slot);
 	if (c->prec_mode == DPG_PREC_FP64) {
 		if ((rc = dpg::launch_trace(c))) return rc;
@@ -471,10 +488,7 @@ extern "C" int dpg_gpu_compute_rhs(dpg_gpu_ctx* c, double* max_rhs)
 static int build_step_graph(dpg_gpu_ctx* c)
 {
 	invalidate_graph(c);
-	if (c->oz && c->prec_mode == DPG_PREC_FP64) {   // allocations are not possible during the capture
-		const int r = dpg::oz_ready(c);
-		if (r) return r;
-	}
+	oz_takes(c);   // allocations are not possible during the capture
 	cudaGraph_t graph = nullptr;
 	CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
 	int rc = DPG_OK;
@@ -620,7 +634,7 @@ extern "C" int dpg_gpu_kernel_times(dpg_gpu_ctx* c, int n_rep, double* ms_out, c
 	unsigned long long* slot = c->dmax + dpg::kMaxStages;
 	for (int r = 0; r < n_rep; ++r) {
 		CK(cudaEventRecord(ev[0], c->stream));
-		const bool oz = c->oz && c->prec_mode == DPG_PREC_FP64, hp = c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64);
+		const bool oz = oz_takes(c), hp = c->hp || (c->adv && c->prec_mode == DPG_PREC_FP64);
 		int rc = (oz ? dpg::oz_launch_part(c, 0, -1, true, slot) : hp ? dpg::hp_launch_part(c, 0, -1, true, slot)
 		          : c->prec_mode == DPG_PREC_FP64 ? dpg::launch_trace(c) : dpg::split_launch_trace(c));
 		if (rc) return rc;

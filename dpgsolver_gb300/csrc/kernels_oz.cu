@@ -730,15 +730,13 @@ int oz_ready(dpg_gpu_ctx* c)
 {
 	State* st = (State*)c->oz;
 	if (!st || st->xl) return DPG_OK;
-	auto al = [&](double** p, size_t n) {
-		void* q = nullptr;
-		if (cudaMalloc(&q, n * sizeof(double)) != cudaSuccess) return false;
-		st->allocs.push_back(q);
-		*p = (double*)q;
-		return true;
-	};
 	double* xl = nullptr;
-	if (!al(&st->svc, st->n_svc) || !al(&st->trace, st->n_trace) || !al(&xl, st->n_xl)) return DPG_ERR_CUDA;
+	auto get = [](void** p, size_t bytes) { return cudaMalloc(p, bytes) == cudaSuccess; };
+	if (!alloc_directions(1, {{&st->svc, st->n_svc}, {&st->trace, st->n_trace}, {&xl, st->n_xl}}, {}, get, [](void* p) { cudaFree(p); })) {
+		cudaGetLastError();   // answered by the caller: the dense kernels take over
+		return DPG_ERR_CUDA;
+	}
+	for (double* p : {st->svc, st->trace, xl}) st->allocs.push_back(p);
 	// the K slots of other face orders and the padding stay zero
 	if (cudaMemsetAsync(xl, 0, st->n_xl * sizeof(double), c->stream) != cudaSuccess) return DPG_ERR_CUDA;
 	st->xl = xl;

@@ -121,6 +121,12 @@ __device__ __forceinline__ void numflux_lax_friedrichs(const T* WL, const T* WR,
 // Lax-Friedrichs: two divisions and four roots instead of 2 D + 4 and four.  Results differ from the functions above by
 // rounding.  For the tensor-product kernels (32x32x8 HEX p = 3, FP64 step: 1,517 -> 1,483 us) and
 // simplices.
+// The rounding error is that of the functions above or below it: differences of the two states are formed before they are
+// multiplied by a wave speed (a wave speed times each state rounds the speed of sound into the mass flux of a gas at
+// rest), small terms are added first, and 1 / rho, the square of a rounded root, gets one Newton step.  rms over random states
+// against extended precision, in 2^-53, mass / momentum / energy, 3D, M ~ 0.5, jumps of 1e-3: Roe-Pike 0.40 / 0.58 / 1.56 (above:
+// 0.43 / 0.60 / 1.64; without these three: 0.52 / 0.66 / 2.22), Lax-Friedrichs 0.30 / 0.53 / 1.17 (above: 0.34 / 0.70 / 1.40;
+// without: 0.76 / 0.59 / 3.88, and at M ~ 1e-6 a mass flux of 0.6 where it is 4e-7).
 
 // y with its sign flipped where x is negative; sign(a) != sign(b).
 __device__ __forceinline__ double signed_as(double y, double x)
@@ -128,19 +134,21 @@ __device__ __forceinline__ double signed_as(double y, double x)
 	return __longlong_as_double(__double_as_longlong(y) ^ (__double_as_longlong(x) & (long long)0x8000000000000000ull));
 }
 __device__ __forceinline__ dual signed_as(dual y, dual x) { return dual(signed_as(y.v, x.v), signed_as(y.d, x.v)); }
+// y near 1 / x, one Newton step (the tangent of y is exact to rounding as it is).
+__device__ __forceinline__ double refined_inverse(double y, double x) { return fma(y, fma(-x, y, 1.0), y); }
+__device__ __forceinline__ dual refined_inverse(dual y, dual x) { return dual(refined_inverse(y.v, x.v), y.d); }
 __device__ __forceinline__ bool signs_differ(double a, double b) { return (__double_as_longlong(a) ^ __double_as_longlong(b)) < 0; }
 
 // The FP64 pipe bounds their kernels, so instructions count: velocities appear only where they are needed (V . n and V^2 through
-// the momenta), the states take the central part and |V . n| times their difference in one coefficient each, and the flux comes
-// scaled, 2 h F . n (h = half the face Jacobian): 113 instructions and the four chains for Roe-Pike in 3D, 141 with the terms
-// written out.  32x32x8 HEX p = 3, FP64 step: 1,483 -> 1,408 us.
+// the momenta), and the flux comes scaled, 2 h F . n (h = half the face Jacobian).  32x32x8 HEX p = 3, FP64 step: 1,483 -> 1,443 us
+// (1,410 with |V . n| folded into the states' coefficients and no Newton step, at the rounding given above).
 template <int D, class T>
 __device__ __forceinline__ void numflux_roe_pike_rs(const T* WL, const T* WR, const double* n, double h, T* nF)
 {
 	const T rhoL = WL[0], rhoR = WR[0], EL = WL[D + 1], ER = WR[D + 1];
 	// sqrt(rhoR / rhoL) exists for two densities of one sign; as there, the weights of others are NaN
 	const T aL_ = abs_i(rhoL), aR_ = abs_i(rhoR), isL = rsqrt(aL_), isR = rsqrt(aR_), sL = aL_ * isL, sR = aR_ * isR;
-	const T rhoL_inv = signed_as(isL * isL, rhoL), rhoR_inv = signed_as(isR * isR, rhoR);
+	const T rhoL_inv = refined_inverse(signed_as(isL * isL, rhoL), rhoL), rhoR_inv = refined_inverse(signed_as(isR * isR, rhoR), rhoR);
 	const T s_sum = signs_differ(value_of(rhoL), value_of(rhoR)) ? T(__longlong_as_double(0x7FF8000000000000ll)) : sL + sR;
 	const T s_inv = 1.0 / s_sum, kL = signed_as(isL * s_inv, rhoL), kR = signed_as(isR * s_inv, rhoR);   // Roe weight / rho
 	T qL = 0.0, qR = 0.0, mnL = 0.0, mnR = 0.0;   // (rho V)^2, rho V . n
@@ -161,11 +169,12 @@ __device__ __forceinline__ void numflux_roe_pike_rs(const T* WL, const T* WR, co
 	const T lc1 = 0.5 * (l5 + l1) - l234, lc2 = 0.5 * (l5 - l1);
 	const T dpc = dp * c_inv, rdV = rho * dVn;
 	const T disInter1 = (lc1 * dpc + lc2 * rdV) * c_inv, disInter2 = lc1 * rdV + lc2 * dpc;
-	const T wL = VnL + l234, wR = VnR - l234, np = (pL + pR) - disInter2;
-	nF[0] = h * (rhoL * wL + rhoR * wR - disInter1);
+	const T np = (pL + pR) - disInter2;
+	nF[0] = h * ((mnL + mnR) - (l234 * (rhoR - rhoL) + disInter1));
 #pragma unroll
-	for (int a = 0; a < D; ++a) nF[1 + a] = h * (WL[1 + a] * wL + WR[1 + a] * wR + n[a] * np - disInter1 * u[a]);
-	nF[D + 1] = h * (EpL * wL + EpR * wR + l234 * dp - disInter1 * H - disInter2 * Vn);
+	for (int a = 0; a < D; ++a)
+		nF[1 + a] = h * (n[a] * np + (WL[1 + a] * VnL + (WR[1 + a] * VnR - (l234 * (WR[1 + a] - WL[1 + a]) + disInter1 * u[a]))));
+	nF[D + 1] = h * (EpL * VnL + (EpR * VnR - (l234 * (ER - EL) + disInter1 * H + disInter2 * Vn)));
 }
 
 template <int D, class T>
@@ -182,11 +191,12 @@ __device__ __forceinline__ void numflux_lax_friedrichs_rs(const T* WL, const T* 
 	const T pL = DPG_GM1_D * (WL[D + 1] - 0.5 * mVL), pR = DPG_GM1_D * (WR[D + 1] - 0.5 * mVR);
 	const T maxlL = sqrt(mVL * rhoL_inv) + sqrt(DPG_GAMMA_D * pL * rhoL_inv);
 	const T maxlR = sqrt(mVR * rhoR_inv) + sqrt(DPG_GAMMA_D * pR * rhoR_inv);
-	const T maxV = (maxlL > maxlR ? maxlL : maxlR), wL = VnL + maxV, wR = VnR - maxV, pLR = pL + pR;
-	nF[0] = h * (WL[0] * wL + WR[0] * wR);
+	const T maxV = (maxlL > maxlR ? maxlL : maxlR), pLR = pL + pR;
+	nF[0] = h * (maxV * (WL[0] - WR[0]) + (mnL + mnR));
 #pragma unroll
-	for (int a = 0; a < D; ++a) nF[1 + a] = h * (WL[1 + a] * wL + WR[1 + a] * wR + n[a] * pLR);
-	nF[D + 1] = h * ((WL[D + 1] + pL) * wL + (WR[D + 1] + pR) * wR + maxV * (pR - pL));
+	for (int a = 0; a < D; ++a)
+		nF[1 + a] = h * (n[a] * pLR + (WL[1 + a] * VnL + (WR[1 + a] * VnR + maxV * (WL[1 + a] - WR[1 + a]))));
+	nF[D + 1] = h * ((WL[D + 1] + pL) * VnL + ((WR[D + 1] + pR) * VnR + maxV * (WL[D + 1] - WR[D + 1])));
 }
 
 template <int D, class T>

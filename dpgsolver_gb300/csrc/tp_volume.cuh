@@ -20,7 +20,8 @@ inline size_t smem_volume(int E)
 enum { kPeriodic = 0, kWalls = 1, kViscous = 2 };
 
 // What follows the state in b0 (all threads synchronised): values at the Gauss points, traces, (boundary states,) and the weak
-// divergence or the collocated values.
+// divergence or the collocated values.  Each buffer is read by the traces between the barriers of the passes that write and
+// overwrite it.
 template <int D, int NV, int N1, bool TAN, int KIND>
 __device__ __forceinline__ void volume_body(const Ops<N1>* so, double* b0, double* b1, double* fl, int e0, int ne, int E, bool first,
                                             const TpGeo& g, const TpBc& B, double* __restrict__ trace,
@@ -57,15 +58,15 @@ __device__ __forceinline__ void volume_body(const Ops<N1>* so, double* b0, doubl
 		}
 		__syncthreads();
 	};
-	// traces of the local faces, in the element's own node order; value(element, local face, face node, variable)
-	auto traces = [&](auto value) {
-		for (int o = threadIdx.x; o < ne * 2 * D * NF; o += blockDim.x) {
-			const int ee = o / (2 * D * NF), r = o - ee * 2 * D * NF, lf = r / NF, q = r - lf * NF;
-			const size_t vf = (size_t)g.vol_face[(size_t)(e0 + ee) * 2 * D + lf];
+	// traces of the two local faces of direction a, in the element's own node order; value(element, side, face node, variable)
+	auto traces = [&](int a, auto value) {
+		for (int o = threadIdx.x; o < ne * 2 * NF; o += blockDim.x) {
+			const int ee = o / (2 * NF), r = o - ee * 2 * NF, side = r / NF, q = r - side * NF;
+			const size_t vf = (size_t)g.vol_face[(size_t)(e0 + ee) * 2 * D + 2 * a + side];
 			double tr[NW];
 #pragma unroll
 			for (int w = 0; w < NW; ++w) {
-				tr[w] = value(ee, lf, q, w);
+				tr[w] = value(ee, side, q, w);
 				if (w >= NV || !TAN || first) (w < NV ? trace : trace_t)[(vf * NV + (w < NV ? w : w - NV)) * NF + q] = tr[w];
 			}
 			if constexpr (KIND != kPeriodic) {
@@ -94,42 +95,48 @@ __device__ __forceinline__ void volume_body(const Ops<N1>* so, double* b0, doubl
 			}
 		}
 	};
+	// The traces come straight from the solution nodes, whose first and last of a direction lie on the faces: only the tangential
+	// directions are interpolated, N1 or no multiply-adds per face node, variable and step (2D: N1 for direction 0, none for
+	// direction 1; 3D: 2 N1, N1, none).  Extrapolated from the Gauss points they would carry the rounding of three passes
+	// with sums of up to 2.1 in magnitude: rms error of the residual of a vortex against extended precision, this way /
+	// extrapolated / dense, HEX p = 1 1.16e-14 / 1.37e-14 / 1.40e-14, p = 2 1.20e-14 / 2.02e-14 / 1.70e-14, p = 3 2.67e-14 / 3.15e-14 / 5.17e-14, QUAD p = 1
+	// 9.35e-14 / 9.73e-14 / 9.45e-14, jittered p = 3 3.12e-13 / 3.17e-13 / 3.36e-13.  Viscous face gradients amplify a jump's error by
+	// ~4 p^2 / h: extrapolated, the energy residual at the 64x128 annulus' steady state stays at 2e-10 (this way and dense: below
+	// 1e-10).
+	auto along = [&](const double* u, int S, int q) {   // sum_j B[q][j] u[j S]
+		double y = so->B[q * N1] * u[0];
+#pragma unroll
+		for (int j = 1; j < N1; ++j) y = fma(so->B[q * N1 + j], u[j * S], y);
+		return y;
+	};
+	if constexpr (D == 2) {
+		traces(0, [&](int ee, int side, int q, int w) { return along(b0 + (ee * NW + w) * N + side * (N1 - 1), N1, q); });
+	} else {   // direction 0: along direction 1 first, into the space of the fluxes, [element][side][variable][k][q]
+		for (int o = threadIdx.x; o < ne * 2 * NF; o += blockDim.x) {
+			const int ee = o / (2 * NF), r = o - ee * 2 * NF, side = r / NF, kq = r - side * NF, k = kq / N1, q = kq - k * N1;
+#pragma unroll
+			for (int w = 0; w < NW; ++w)
+				fl[((ee * 2 + side) * NW + w) * NF + kq] = along(b0 + (ee * NW + w) * N + side * (N1 - 1) + N1 * N1 * k, N1, q);
+		}
+	}
 	pass(std::integral_constant<int, 0>{}, b0, b1);
-	if constexpr (KIND == kViscous) {
-		// From the solution nodes, whose first and last of a direction lie on the faces: only the tangential directions are
-		// interpolated.  The face gradients amplify a rounding error of a jump by ~4 p^2 / h; through the Gauss points
-		// the energy residual at the 64x128 annulus' steady state stays at 2e-10 (this way and dense: below 1e-10).
-		traces([&](int ee, int lf, int q, int w) {
-			const int a = lf >> 1, end = (lf & 1) ? N1 - 1 : 0;
-			const double *u0 = b0 + (ee * NW + w) * N, *u1 = b1 + (ee * NW + w) * N;   // at the solution nodes; interpolated along 0
-			double y = 0.0;
-			if constexpr (D == 2) {
-				if (a == 1) return u1[q + N1 * end];
-#pragma unroll
-				for (int j = 0; j < N1; ++j) y = fma(so->B[q * N1 + j], u0[end + N1 * j], y);
-			} else {
-				const int qa = q % N1, qb = q / N1;
-				if (a == 0) {
-#pragma unroll
-					for (int k = 0; k < N1; ++k) {
-						double z = 0.0;
-#pragma unroll
-						for (int j = 0; j < N1; ++j) z = fma(so->B[qa * N1 + j], u0[end + N1 * (j + N1 * k)], z);
-						y = fma(so->B[qb * N1 + k], z, y);
-					}
-				} else {
-					const int base = a == 1 ? qa + N1 * end : qa + N1 * N1 * end, S = a == 1 ? N1 * N1 : N1;
-#pragma unroll
-					for (int j = 0; j < N1; ++j) y = fma(so->B[qb * N1 + j], u1[base + S * j], y);
-				}
-			}
-			return y;
+	if constexpr (D == 2) {
+		traces(1, [&](int ee, int side, int q, int w) { return b1[(ee * NW + w) * N + q + N1 * side * (N1 - 1)]; });
+	} else {
+		traces(0, [&](int ee, int side, int q, int w) {
+			const int qb = q / N1;
+			return along(fl + ((ee * 2 + side) * NW + w) * NF + q - qb * N1, N1, qb);
 		});
-		__syncthreads();   // the next pass overwrites b0
+		traces(1, [&](int ee, int side, int q, int w) {
+			const int qb = q / N1;
+			return along(b1 + (ee * NW + w) * N + q - qb * N1 + N1 * side * (N1 - 1), N1 * N1, qb);
+		});
 	}
 	pass(std::integral_constant<int, 1>{}, b1, b0);
-	if constexpr (D == 3) pass(std::integral_constant<int, 2>{}, b0, b1);
-	const double* sc = D == 3 ? b1 : b0;     // the collocated values
+	if constexpr (D == 3) {
+		traces(2, [&](int ee, int side, int q, int w) { return b0[(ee * NW + w) * N + q + N1 * N1 * side * (N1 - 1)]; });
+		pass(std::integral_constant<int, 2>{}, b0, b1);
+	}
 	double* f0 = D == 3 ? b0 : b1;           // free: the fluxes of direction 0
 	if (KIND == kViscous && live) {
 #pragma unroll
@@ -157,15 +164,6 @@ __device__ __forceinline__ void volume_body(const Ops<N1>* so, double* b0, doubl
 		}
 	}
 	if constexpr (KIND == kViscous) return;
-	traces([&](int ee, int lf, int q, int w) {
-		const int a = lf >> 1, S = stride_of<N1>(a);
-		const double* l = (lf & 1) ? so->lp : so->lm;
-		const double* x = sc + (ee * NW + w) * N + face_base<N1>(a, q);
-		double y = l[0] * x[0];
-#pragma unroll
-		for (int j = 1; j < N1; ++j) y = fma(l[j], x[j * S], y);
-		return y;
-	});
 	__syncthreads();
 	// weak divergence
 	if (live) {

@@ -170,7 +170,7 @@ __host__ __device__ inline float2 split_double(double v)
 // or just below it when hi is a power of two and lo has the opposite sign: spacing halved there).  lo / spacing is
 // an exact FP32 scaling by a power of two (two factors when it leaves the FP32 range), |k| <= 2^29, and the
 // round-to-nearest-even of the conversion is that of the double (k carries the parity of its last bit).  A
-// subnormal or zero hi (|x| < 2^-126) gives 0.
+// subnormal or zero hi (|x| < 2^-126) gives 0, an infinity or NaN a number in [2^128, 2^129).
 __device__ __forceinline__ double to_double(df64 x)
 {
 	const uint32_t bh = __float_as_uint(x.hi), ah = bh & 0x7FFFFFFFu;

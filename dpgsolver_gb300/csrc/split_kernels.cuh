@@ -186,6 +186,11 @@ __device__ __forceinline__ long long biased_mantissa(double x, int sc)
 	else                 return ((t + 1) >> 1) + digit_bias<S>();
 }
 
+// Exponent bounds beyond the double-float range, which ends at 2^128: of an infinity or NaN of the double-float arithmetic
+// (df::to_double makes a number in [2^128, 2^129) of it) and of a state that large or not finite.  A row of the lift's
+// data with such a bound gives NaN.
+constexpr int kExpBeyond = 129, kExpNan = 1025;
+
 __host__ __device__ constexpr float pow2f(int e) { return e >= 0 ? (e == 0 ? 1.0f : 2.0f * pow2f(e - 1)) : 0.5f * pow2f(e + 1); }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
@@ -765,7 +770,7 @@ ks_interp(const double* sol, GroupDev g, const float2* __restrict__ met2, float2
 			}
 		}
 		compute_sync();   // every volume-flux item done: the exponent bounds are complete
-		if (tid < rows) colE[((size_t)e0 * NV + tid) * kColSlots + g.n_fl] = emx[tid];
+		if (tid < rows) colE[((size_t)e0 * NV + tid) * kColSlots + g.n_fl] = colF[tid] > kExpBeyond ? kExpNan : emx[tid];
 	}
 	tc::fence_before_sync();
 	__syncthreads();
@@ -983,7 +988,7 @@ ks_lift(double* sol, double* solp, double* __restrict__ rhs, const double* xl,
 				const int4 a = ce[0], b = ce[1];
 				m = max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w)));
 			}
-			colF[tid] = tid < rows ? col_exp_of(m, NP) : 0;
+			colF[tid] = tid < rows ? col_exp_of(m >= kExpBeyond ? kExpNan : m, NP) : 0;
 		}
 		compute_sync();
 		const int F_r = colF[m_r];
@@ -1025,9 +1030,11 @@ ks_lift(double* sol, double* solp, double* __restrict__ rhs, const double* xl,
 		const int m = 32 * (warp & 3) + lane;
 		const bool live = m < rows;
 		const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-		const double dt = (stage >= 0 ? *dt_ptr : 0.0);
 		const df::df64 jv = df::from2(df::split_double(live ? g.jinv[e0 + m / NV] : 0.0));
 		const int Fm = colF[m];
+		const bool bad = Fm == col_exp_of(kExpNan, NP);   // NaN in the residual, the new state and the norm
+		const double nan = __longlong_as_double(0x7FF8000000000000ll);
+		const double dt = bad ? nan : (stage >= 0 ? *dt_ptr : 0.0);
 		const size_t rbase = ((size_t)e0 * NV + m) * n_s;   // the row's first node
 		double u0[8], up[8];
 		int re[8];   // with the state: a load between the stores below would wait for them one by one
@@ -1062,13 +1069,14 @@ ks_lift(double* sol, double* solp, double* __restrict__ rhs, const double* xl,
 				const unsigned long long ab = (unsigned long long)__double_as_longlong(r) & 0x7FFFFFFFFFFFFFFFull;
 				lmax = ab > lmax ? ab : lmax;
 				const size_t gi = rbase + node;
-				if (write_rhs) rhs[gi] = r;
+				if (write_rhs) rhs[gi] = bad ? nan : r;
 				if (stage == 0) { solp[gi] = u0[j]; sol[gi] = u0[j] + dt * r; }
 				else if (stage == 1) sol[gi] = (1.0 / 4.0) * (3.0 * up[j] + u0[j] + dt * r);
 				else if (stage == 2) sol[gi] = (1.0 / 3.0) * (up[j] + 2.0 * u0[j] + 2.0 * dt * r);
 			}
 			if (c8 + kColStride < Al.N_pad / 8) load_state(c8 + kColStride);
 		}
+		if ((bad && live) || lmax >= 0x47F0000000000000ull) lmax = 0x7FF8000000000000ull;   // 2^128 and more: not finite either
 		for (int off = 16; off > 0; off >>= 1) {
 			const unsigned long long o = __shfl_xor_sync(0xffffffffu, lmax, off);
 			lmax = o > lmax ? o : lmax;

@@ -5,11 +5,15 @@
 // 4 needs 110,000 of them per residual (Euler), 93 % in dense products.  Here every product runs as the sliced (Ozaki)
 // scheme: operator rows and data columns are scaled by powers of two, cut into S = 8 signed 8-bit digits (62 bits of
 // each operand's largest value) held as BF16, and the digit products of level a + b < 8 are accumulated in FP32,
-// each level in an accumulator of its own (integers below 2^24, exact; 8 x 64 TMEM columns).  The level sums are
-// joined in 64-bit integers and rounded to FP64 once, so an output is a correctly rounded sum up to the digits cut off,
-// 2^-61 K of the largest products.  Residuals against binary128 (TRI, TET, orders 2..4 and mixed; smooth and noisy
-// states): 0.3 to 0.8 of the dense FP64 kernels' largest error, 0.25 to 0.6 of their mean.  Fluxes, mass matrix scaling, RK stages
-// and norms are FP64 instructions.  A row with a value that is not finite gives NaN in all its outputs.
+// each level in an accumulator of its own (8 x 64 TMEM columns).  The level sums are joined in 64-bit integers and rounded
+// to FP64 once, so an output is a correctly rounded sum up to the digits cut off, 2^-61 K of the largest products.
+// An accumulator is exact while its integer sum is below 2^24 (random digits: an rms of 0.02 times that or less).  In the worst
+// case, data digits at their extremes in line with the operator's own, levels 0 to 4 stay below it for every element (0.79
+// times 2^24 at most), and all levels for every element but the TET of order 4 (K = 439), whose levels 5, 6 and 7 can
+// reach 1.01, 1.23 and 1.45 times: an addition above 2^24 rounds by two units, 2^-51 of the largest product or less.
+// Residuals against binary128 (TRI, TET, orders 2..4 and mixed; smooth and noisy states): 0.3 to 0.8 of the dense FP64
+// kernels' largest error, 0.25 to 0.6 of their mean.  Fluxes, mass matrix scaling, RK stages and norms are FP64
+// instructions.  A row with a value that is not finite gives NaN in all its outputs.
 //
 //   k_oz_interp : rows (element, variable) of the state -> values at the volume cubature nodes and face traces (a local
 //                 face's operators for every order its face may have; the one it has is written)

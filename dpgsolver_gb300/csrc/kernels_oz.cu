@@ -309,12 +309,11 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_oz_interp(const double* so
 // Face nodes first, then the volume nodes of the groups.
 template <int D, int NV>
 __global__ void __launch_bounds__(128) k_oz_flux(const double* trace, const double* svc,
-                                                 const __grid_constant__ Dev d, double* __restrict__ xl, int num_flux, double bx,
-                                                 double by, double bz)
+                                                 const __grid_constant__ Dev d, double* __restrict__ xl, int num_flux)
 {
+	static_assert(NV == D + 2, "Euler");
 	grid_wait();
 	const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	const double b[3] = {bx, by, bz};
 	if (t < d.n_fnode) {
 		const int f = d.node_face ? d.node_face[t] : (int)(t / d.n_fc[d.p_min]);
 		const int64_t off = d.fnode_off ? d.fnode_off[f] : (int64_t)f * d.n_fc[d.p_min];
@@ -328,13 +327,9 @@ __global__ void __launch_bounds__(128) k_oz_flux(const double* trace, const doub
 		}
 #pragma unroll
 		for (int a = 0; a < D; ++a) n[a] = d.nrm[t * D + a];
-		if constexpr (NV == D + 2) {
-			const double h = 0.5 * d.jf[t];
-			if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, h, nf);
-			else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, h, nf);
-		} else {
-			nf[0] = numflux_upwind<D>(b, WL[0], WR[0], n) * d.jf[t];
-		}
+		const double h = 0.5 * d.jf[t];
+		if (num_flux == DPG_NUM_FLUX_ROE_PIKE) numflux_roe_pike_rs<D>(WL, WR, n, h, nf);
+		else                                   numflux_lax_friedrichs_rs<D>(WL, WR, n, h, nf);
 		double* xL = xl + d.face_xl[2 * f] + q;
 		double* xR = xl + d.face_xl[2 * f + 1] + qr;
 		const int lL = d.face_ld[2 * f], lR = d.face_ld[2 * f + 1];
@@ -358,7 +353,7 @@ __global__ void __launch_bounds__(128) k_oz_flux(const double* trace, const doub
 	for (int v = 0; v < NV; ++v) s[v] = svc[g.svc0 + ((size_t)e * NV + v) * g.n_c + c];
 	double* x = xl + g.xl0 + (size_t)e * NV * g.ldx + c;
 	const double* m = g.met + (size_t)e * D * D;
-	tp::ref_flux<D, NV>(s, [&](int a, int dir) { return m[a + D * dir]; }, b, [&](int dir, const double (&fr)[NV]) {
+	tp::ref_flux<D, NV>(s, [&](int a, int dir) { return m[a + D * dir]; }, nullptr, [&](int dir, const double (&fr)[NV]) {
 #pragma unroll
 		for (int v = 0; v < NV; ++v) x[(size_t)v * g.ldx + dir * g.n_c] = fr[v];
 	});
@@ -756,8 +751,7 @@ static int launch_part(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, uns
 		launch_chained(k_oz_interp<NV>, d.n_blocks, kBlockThreads, kSmem, c->stream, c->sol, d, st->svc, st->trace, st->err);
 	} else if (which == 1) {
 		const int64_t n = d.n_fnode + d.n_vnode;
-		launch_chained(k_oz_flux<D, NV>, (unsigned)((n + 127) / 128), 128, 0, c->stream, st->trace, st->svc, d, st->xl, c->num_flux,
-		               c->b_adv[0], c->b_adv[1], c->b_adv[2]);
+		launch_chained(k_oz_flux<D, NV>, (unsigned)((n + 127) / 128), 128, 0, c->stream, st->trace, st->svc, d, st->xl, c->num_flux);
 	} else {
 		launch_chained(k_oz_lift<NV>, d.n_blocks, kBlockThreads, kSmem, c->stream, st->xl, d, c->sol, c->solp, c->rhs, c->ddt, max_slot,
 		               stage, write_rhs ? 1 : 0, st->err);

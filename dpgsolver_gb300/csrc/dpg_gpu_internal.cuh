@@ -129,11 +129,14 @@ struct dpg_gpu_ctx {
 namespace dpg {
 // The kernels of a residual are a chain, each a few us long on small meshes: the next kernel's launch is processed while the
 // previous one runs (programmatic dependent launch), and its blocks wait for that kernel's end and memory before they
-// touch anything a kernel writes.  Every kernel launched by launch_chained calls grid_wait first, so the wait covers all
-// kernels before it.  Their inputs that another kernel writes are not `__restrict__`: such loads count as invariant (or
-// as untouched by the wait), may be moved above it and go through the read-only path.  Blocks of small grids (two of which fit the SMs side by side) let the next kernel's blocks start
-// at once (16x16 QUAD p = 2, 36 stages: 870 us with plain launches, 834 without this, 788 with it); for larger grids the
-// early blocks pack onto the first free SMs and share their FP64 pipes (61x47 QUAD p = 3: 473 us without, 553 with it).
+// touch anything a kernel writes.  In every kernel launched by launch_chained each thread that reads or writes what another
+// kernel writes calls grid_wait before it does, and every block has such threads (in ks_* and k_oz_* the compute warps; the
+// loading and issuing warps touch operators and shared memory only).  So a kernel that has ended means that all before it have.
+// Inputs that another kernel writes are not `__restrict__`: such loads count as invariant (or as untouched by the wait),
+// may be moved above it and go through the read-only path.  Blocks of small grids (at most half of the 152 SMs: two grids
+// fit side by side) let the next kernel's blocks start at once (16x16 QUAD p = 2, 36 stages: 870 us with plain launches,
+// 834 without this, 788 with it); for larger grids the early blocks pack onto the first free SMs and share their FP64
+// pipes (61x47 QUAD p = 3: 473 us without, 553 with it).
 __device__ __forceinline__ void grid_wait()
 {
 	if (gridDim.x * gridDim.y <= 76) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

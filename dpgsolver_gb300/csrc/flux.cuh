@@ -4,12 +4,13 @@
 // Follows compute_Flux_T_euler (flux_euler_T.c:71-143, f at :259-298), compute_Numerical_Flux_T_euler_roe_pike
 // (numerical_flux_euler_T.c:470-..., entropy fix from min/max_abs_real_T, math_functions_T.c:222-236),
 // compute_Numerical_Flux_T_euler_lax_friedrichs (numerical_flux_euler_T.c:60-...) and
-// compute_Numerical_Flux_T_advection_upwind (numerical_flux_advection_T.c:39-75).  The operation order of each
-// formula is the reference's (up to taking repeated divisors as one reciprocal), so that FP64 results agree with
-// the CPU oracle to rounding.
+// compute_Numerical_Flux_T_advection_upwind (numerical_flux_advection_T.c:39-75).  The operation order of flux_euler,
+// numflux_roe_pike and numflux_lax_friedrichs is the reference's (up to taking repeated divisors as one reciprocal); the
+// numflux_.._rs forms, which all but small dense QUAD and HEX meshes and the allocation-free residual take, and the viscous fluxes order the same
+// formulas for fewer FP64 instructions.  All agree with the CPU oracle to rounding.
 //
 // The flux functions are templated on the scalar type: double (the residual) or dual (dual.cuh: the tangent of the
-// linearisation); the double instantiations are the FP64 formulas above, operation for operation.
+// linearisation).
 #pragma once
 
 #include "dual.cuh"

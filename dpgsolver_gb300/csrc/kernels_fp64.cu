@@ -313,7 +313,7 @@ static int dispatch(dpg_gpu_ctx* c, int which, int stage, bool write_rhs, unsign
 }
 
 // Tensor-product meshes take the 1D operators of kernels_tp.cu for the element kernels (32x32x8 HEX p = 3 Euler:
-// 0.31 ms for the two against 4.66 ms here; 47x61 jittered QUAD p = 3: 26 us against 120 us).
+// 0.28 ms for the two against 4.66 ms here; 47x61 jittered QUAD p = 3: 28 us against 120 us).
 int launch_trace(dpg_gpu_ctx* c) { return c->tp ? tp_volume(c) : dispatch(c, 0, -1, false, nullptr); }
 int launch_face(dpg_gpu_ctx* c)
 {

@@ -21,8 +21,8 @@
 //                 data (the right side of a face negated, in its own node order)
 //   k_oz_lift   : data rows -> rhs (operators [tw1 | -tw0[p_f]] times m_inv), 1 / detJ, norm, SSP-RK3 stage
 //
-// A block holds 128 data rows (the MMA's M): 25 TETs or 32 TRIs of Euler.  24,576 TETs of orders 1..4: 779 us per residual
-// (interpolation 241, fluxes 263, lift 276), dense kernels 2,116.  The fluxes are bound by the FP64 pipe (~210 slots per
+// A block holds 128 data rows (the MMA's M): 25 TETs or 32 TRIs of Euler.  24,576 TETs of orders 1..4: 739 us per residual
+// (interpolation 239, fluxes 232, lift 268), dense kernels 2,116.  The fluxes are bound by the FP64 pipe (~210 slots per
 // node: Roe-Pike and the volume flux); the other two by the chain digits -> MMAs -> accumulators of the one block that
 // an SM holds (512 TMEM columns, 193 KB of shared memory): the products are 36 digit pairs per K of 32 columns.
 // Moving a chunk's loads to whole sectors of 8 rows (lane = row, 32-byte part) and one barrier arrival per warp instead

@@ -10,8 +10,8 @@
 // instructions decides: HEX p = 3 Euler needs 210 per node in k_tp_volume and 110 in k_tp_lift where the dense
 // operators need 28,672 / 64 x 5 = 2,240.  One thread per (element, node): the operands come from shared memory,
 // whose traffic hides behind the FP64 issue rate.  A block holds as many elements as fill 256 threads, fewer on
-// small meshes so that every SM has work.  32x32x8 HEX p = 3 Euler: k_tp_volume 193 us, k_tp_lift 114 us (0.57 T FP64
-// operations/s, the pipe's measured rate) for 967 + 3,694 us of the dense kernels; the whole residual 0.43 against 4.78 ms.
+// small meshes so that every SM has work.  32x32x8 HEX p = 3 Euler: k_tp_volume 183 us, k_tp_lift 100 us (the FP64
+// pipe's measured rate) for 967 + 3,694 us of the dense kernels; the whole residual 0.39 against 4.78 ms.
 //
 // The linearisation (k_tp_volume with TAN, k_face_tan, k_tp_lift) carries (value, tangent) through the same passes.
 #include <algorithm>
@@ -250,9 +250,12 @@ int tp_prepare(dpg_gpu_ctx* c, const struct dpg_sim* sim, bool general)
 	if ((o.e_type != DPG_QUAD && o.e_type != DPG_HEX) || o.p < 1 || o.p + 1 > kN1Max) return DPG_OK;
 	const int N = ipow(o.p + 1, o.d);
 	if (o.n_s != N || o.n_c != N || o.n_fc != ipow(o.p + 1, o.d - 1) || o.n_fl != 2 * o.d) return DPG_OK;
-	// A mesh of fewer nodes than this is bound by the launch chain in either form and keeps the dense kernels and their
-	// summation order.  us per step here / dense (both with their own face fluxes): QUAD p = 1, 1,024 nodes: 41.2 / 46.0;
-	// QUAD p = 2, 1,296: 47.7 / 52; HEX p = 1, 1,728: 53.5 / 60.
+	// Periodic meshes of fewer nodes keep the dense kernels for their summation order, not for speed: a Newton solve there runs
+	// until its systems are near-singular and its residual is rounding, and ends elsewhere when a sum is
+	// reordered (8x8 QUAD p = 2, uniform stream: by 6e-5 of the state).  The line lies above the small Newton problems of
+	// the tests and the benchmark (900 nodes at most), whose results are kept.  us per step, 1D operators / dense (both with their own face fluxes): QUAD p = 1, 64 nodes 38.9 / 45.1, 900: 41.0 /
+	// 45.1, 1,024: 41.2 / 46.0; QUAD p = 2, 576: 45.1 / 51.2, 1,296: 47.7 / 52; QUAD p = 4, 900: 53.4 / 67.6; HEX p = 1, 1,000: 55.3 / 59.0;
+	// HEX p = 2, 729: 164 / 201; HEX p = 3, 768: 256 / 508.  One residual is equal on both sides up to p = 3 (37 to 47 us).
 	constexpr int64_t kMinNodes = 1024;
 	if (!general && (int64_t)sim->n_vol * N < kMinNodes) return DPG_OK;
 	TpState* st = new TpState();

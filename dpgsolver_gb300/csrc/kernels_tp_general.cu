@@ -19,7 +19,7 @@
 //
 // Four launches per Navier-Stokes residual, three for Euler with walls.  Every sum is formed by one thread in a fixed
 // order.  Bound: the FP64 pipe (about 320 instructions per node in k_tp_grad, which runs at its rate).  64x128 annulus, QUAD
-// p = 3, one residual: k_tp_volume 22, k_tp_grad 85, k_tp_face_br2 19, k_tp_lift 18 us, 144 us in all; the dense form with
+// p = 3, one residual: k_tp_volume 22, k_tp_grad 86, k_tp_face_br2 21, k_tp_lift 18 us, 146 us in all; the dense form with
 // stored gradients (two passes of element mass-matrix inverses per face, six launches) took 957 us.
 // T = double: the residual; T = dual: its tangent (fvn, the face fluxes and G then hold tangents only).
 #include <vector>

@@ -124,7 +124,8 @@ __device__ __forceinline__ void numflux_lax_friedrichs(const T* WL, const T* WR,
 // simplices.
 // The rounding error is that of the functions above or below it: differences of the two states are formed before they are
 // multiplied by a wave speed (a wave speed times each state rounds the speed of sound into the mass flux of a gas at
-// rest), small terms are added first, and 1 / rho, the square of a rounded root, gets one Newton step.  rms over random states
+// rest; only Roe-Pike's momenta take Vn +- |Vn| in one coefficient), small terms are added first, and 1 / rho, the square
+// of a rounded root, gets one Newton step.  rms over random states
 // against extended precision, in 2^-53, mass / momentum / energy, 3D, M ~ 0.5, jumps of 1e-3: Roe-Pike 0.40 / 0.58 / 1.56 (above:
 // 0.43 / 0.60 / 1.64; without these three: 0.52 / 0.66 / 2.22), Lax-Friedrichs 0.30 / 0.53 / 1.17 (above: 0.34 / 0.70 / 1.40;
 // without: 0.76 / 0.59 / 3.88, and at M ~ 1e-6 a mass flux of 0.6 where it is 4e-7).
@@ -141,8 +142,8 @@ __device__ __forceinline__ dual refined_inverse(dual y, dual x) { return dual(re
 __device__ __forceinline__ bool signs_differ(double a, double b) { return (__double_as_longlong(a) ^ __double_as_longlong(b)) < 0; }
 
 // The FP64 pipe bounds their kernels, so instructions count: velocities appear only where they are needed (V . n and V^2 through
-// the momenta), and the flux comes scaled, 2 h F . n (h = half the face Jacobian).  32x32x8 HEX p = 3, FP64 step: 1,483 -> 1,443 us
-// (1,410 with |V . n| folded into the states' coefficients and no Newton step, at the rounding given above).
+// the momenta), and the flux comes scaled, 2 h F . n (h = half the face Jacobian).  32x32x8 HEX p = 3, FP64 step: 1,483 -> 1,432 us
+// (1,410 with |V . n| in the coefficients of all states and no Newton step, at the rounding given above).
 template <int D, class T>
 __device__ __forceinline__ void numflux_roe_pike_rs(const T* WL, const T* WR, const double* n, double h, T* nF)
 {
@@ -170,11 +171,10 @@ __device__ __forceinline__ void numflux_roe_pike_rs(const T* WL, const T* WR, co
 	const T lc1 = 0.5 * (l5 + l1) - l234, lc2 = 0.5 * (l5 - l1);
 	const T dpc = dp * c_inv, rdV = rho * dVn;
 	const T disInter1 = (lc1 * dpc + lc2 * rdV) * c_inv, disInter2 = lc1 * rdV + lc2 * dpc;
-	const T np = (pL + pR) - disInter2;
+	const T wL = VnL + l234, wR = VnR - l234, np = (pL + pR) - disInter2;
 	nF[0] = h * ((mnL + mnR) - (l234 * (rhoR - rhoL) + disInter1));
 #pragma unroll
-	for (int a = 0; a < D; ++a)
-		nF[1 + a] = h * (n[a] * np + (WL[1 + a] * VnL + (WR[1 + a] * VnR - (l234 * (WR[1 + a] - WL[1 + a]) + disInter1 * u[a]))));
+	for (int a = 0; a < D; ++a) nF[1 + a] = h * (n[a] * np + (WL[1 + a] * wL + (WR[1 + a] * wR - disInter1 * u[a])));
 	nF[D + 1] = h * (EpL * VnL + (EpR * VnR - (l234 * (ER - EL) + disInter1 * H + disInter2 * Vn)));
 }
 
